@@ -80,6 +80,28 @@ def test_ties_at_the_top_k_cut_keep_the_earliest_indices(dev):
   assert tokens.download().tolist() == expected(logits, queries)
 
 
+@pytest.mark.parametrize("vocab", [64, 1003, 4096, 16388])
+def test_small_and_odd_vocabularies(dev, vocab):
+  """Fewer logits than the cluster has threads, a length that no vector load fits, and parts of uneven size."""
+  rng = np.random.default_rng(vocab)
+  logits = (2.0 * rng.standard_normal((6, vocab))).astype(np.float32)
+  logits[1, [vocab - 1, vocab - 2]] = 12.0  # a tie in the last part
+  queries, count = make_queries([(0.0, 1.0, 0, 1), (0.0, 1.0, 0, 1), (0.7, 0.9, 40, 1), (1.2, 1.0, 64, 1), (0.9, 0.8, 1, 1), (0.5, 0.0, 3, 1)])
+  tokens = dev.empty(count, np.int32)
+  dev.sample(dev.array(logits), vocab, dev.queries(queries), len(queries), count, 0, tokens)
+  assert tokens.download().tolist() == expected(logits, queries)
+
+
+def test_more_ties_than_the_collection_holds(dev):
+  """3000 logits share the largest value but one: the row takes the radix select, and the earliest of them are kept."""
+  logits = np.full((2, VOCAB), -5.0, np.float32)
+  logits[:, 5000:8000], logits[:, 100000] = 2.0, 3.0
+  queries, count = make_queries([(0.7, 1.0, 40, 1), (1.0, 0.95, 64, 1)])
+  tokens = dev.empty(count, np.int32)
+  dev.sample(dev.array(logits), VOCAB, dev.queries(queries), len(queries), count, 0, tokens)
+  assert tokens.download().tolist() == expected(logits, queries)
+
+
 # ---- draft verification on the device against the host loop of the reference ----
 def host_acceptance(samples, speculative, sampled, proposals, draft_width, stops):
   """runtime/engine.cpp:205-216 for one query: returns (accepted, emitted, stopped)."""
