@@ -2,10 +2,10 @@
 //
 // Replaces dequant_tile for q5_k / q8_0 / iq4_xs (quant_linear.metal:50-67, 87-115), linear_decode_q5_k and
 // linear_decode_q8_0 (:329-434, 514-570), the q5_k / iq4_xs variants of mlp_gate_up (fused_kernels.metal:80-200) and the
-// embedding gather for tables of these types. The synthetic benchmark models are all Q4_K / Q6_K, so these kernels
-// are written for correctness and moderate speed, not for the roofline: one warp per weight row, the row's blocks
-// dequantised in registers (bit-exact with the CPU oracle's values), fp32 multiply-adds against up to 8 activation rows
-// at a time, a shuffle reduction, and the residual add or SiLU * up epilogue.
+// embedding gather for tables of these types. Matrices in whole 16-row tiles with 16-byte aligned rows take the tensor-core
+// GEMV of gemv.cu (a layer of mixed types with 7 rows: 595 -> 89 us); the plain kernel here serves every other shape: one
+// warp per weight row, the row's blocks dequantised in registers (bit-exact with the CPU oracle's values), fp32
+// multiply-adds against up to 8 activation rows at a time, a shuffle reduction, and the residual add or SiLU * up epilogue.
 #include "common.cuh"
 #include "ops.h"
 

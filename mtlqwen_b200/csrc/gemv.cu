@@ -1,8 +1,9 @@
-// Dequant-fused fp16 tensor-core GEMV for decode (M <= 8 activation rows) over GGUF Q4_K / Q6_K weights. It serves
-// every Q6_K matrix (lm_head) and, when the integer kernel of q4k_decode.cu is switched off, the Q4_K ones.
+// Dequant-fused fp16 tensor-core GEMV for decode (M <= 8 activation rows) over GGUF Q4_K / Q5_K / Q6_K / Q8_0 / IQ4_XS
+// weights. It serves every Q6_K matrix (lm_head), the Q5_K, Q8_0 and IQ4_XS ones whose shape it takes (formats.cu has the
+// rest) and, when the integer kernel of q4k_decode.cu is switched off, the Q4_K ones.
 //
-// Replaces linear_decode_q4_k[_add] (quant_linear.metal:245-327), linear_decode_q6_k[_add] (:436-512) and
-// mlp_gate_up_q4_k_decode (fused_kernels.metal:11-78). The reference re-reads the weights once per
+// Replaces linear_decode_q4_k[_add] (quant_linear.metal:245-327), linear_decode_q5_k / q6_k / q8_0[_add] (:329-570) and
+// mlp_gate_up of Q4_K, Q5_K and IQ4_XS (fused_kernels.metal:11-200). The reference re-reads the weights once per
 // activation row (grid.y = rows); here up to 8 rows share one pass over the weights.
 //
 // Design (one persistent CTA per SM, 8 consumer warps + 1 producer warp):
@@ -22,6 +23,7 @@
 //    accuracy; XSPLIT = 1 drops lo (relative error ~3e-4, still inside the 1e-3 contract).
 //  * Every mbarrier wait is bounded; on a timeout the kernel raises an abort flag, records a status code
 //    and all roles leave their loops.
+#include <type_traits>
 #include "common.cuh"
 #include "kernels.h"
 
@@ -35,19 +37,33 @@ constexpr int kStageBlocks = kGemvStageBlocks;  // super-blocks per ring stage (
 constexpr int kMaxStages = 8;
 constexpr int kTileRows = kGemvTileRows;
 
+// How a block type lies in a ring stage: kBoxes tiled copies of 16 rows x kStageBlocks / kBoxes super-blocks (a box is at
+// most 256 elements of 8 bytes wide, which eight super-blocks of Q8_0 exceed), each row kPad bytes wider than its
+// super-blocks where the pitch would otherwise put the eight rows of a warp-wide load into the same banks.
 struct Q4K {
-  static constexpr int kBlockBytes = 144;
-  static constexpr int kRowStride = kStageBlocks * kBlockBytes;  // rows of a TMA box are dense in shared memory
-  static constexpr bool kMinTerm = true;
-  static constexpr int kStageBytes = kTileRows * kRowStride;
+  static constexpr int kBlockBytes = 144, kBoxes = 1, kPad = 0;
+  static constexpr bool kMinTerm = true, kRotated = true;
 };
-
+struct Q5K {
+  static constexpr int kBlockBytes = 176, kBoxes = 1, kPad = 16;  // pitch 1424 = 16 mod 128
+  static constexpr bool kMinTerm = true, kRotated = false;
+};
 struct Q6K {
-  static constexpr int kBlockBytes = 210;
-  static constexpr int kRowStride = kStageBlocks * kBlockBytes;  // 1680 == 16 mod 128
-  static constexpr bool kMinTerm = false;
-  static constexpr int kStageBytes = kTileRows * kRowStride;
+  static constexpr int kBlockBytes = 210, kBoxes = 1, kPad = 0;  // pitch 1680 = 16 mod 128
+  static constexpr bool kMinTerm = false, kRotated = false;
 };
+struct Q8 {
+  static constexpr int kBlockBytes = 272, kBoxes = 2, kPad = 16;  // eight Q8_0 blocks; pitch 1104 = 80 mod 128
+  static constexpr bool kMinTerm = false, kRotated = false;
+};
+struct IQ4 {
+  static constexpr int kBlockBytes = 136, kBoxes = 1, kPad = 16;  // pitch 1104
+  static constexpr bool kMinTerm = false, kRotated = false;
+};
+template <class Q> constexpr int box_blocks() { return kStageBlocks / Q::kBoxes; }
+template <class Q> constexpr int row_pitch() { return box_blocks<Q>() * Q::kBlockBytes + Q::kPad; }
+template <class Q> constexpr int box_bytes() { return kTileRows * row_pitch<Q>(); }
+template <class Q> constexpr int stage_bytes() { return Q::kBoxes * box_bytes<Q>(); }
 
 struct Smem {
   uint64_t full[kMaxStages], empty[kMaxStages];
@@ -59,18 +75,19 @@ static_assert(sizeof(Smem) <= kControlBytes, "control block overlaps the activat
 template <class Q, int NMAT, int XSPLIT> constexpr size_t fixed_bytes() {
   size_t frag = size_t(kChunkBlocks) * 16 * 32 * 8 * XSPLIT;
   size_t sums = Q::kMinTerm ? size_t(kChunkBlocks) * 32 * 8 : 0;
+  size_t scales = size_t(kChunkBlocks) * 8 * 4;
   size_t partial = size_t(2) * NMAT * kConsumerWarps * 128 * 4;
-  return kControlBytes + frag + sums + partial;
+  return kControlBytes + frag + sums + scales + partial;
 }
 
 // As many ring stages as fit beside the fragments in the 227 KB a CTA may use.
 template <class Q, int NMAT, int XSPLIT> constexpr int stage_count() {
-  int stages = int((size_t(227) * 1024 - fixed_bytes<Q, NMAT, XSPLIT>()) / Q::kStageBytes);
+  int stages = int((size_t(227) * 1024 - fixed_bytes<Q, NMAT, XSPLIT>()) / stage_bytes<Q>());
   return stages > kMaxStages ? kMaxStages : stages;
 }
 
 template <class Q, int NMAT, int XSPLIT> constexpr size_t smem_bytes() {
-  return fixed_bytes<Q, NMAT, XSPLIT>() + size_t(stage_count<Q, NMAT, XSPLIT>()) * Q::kStageBytes;
+  return fixed_bytes<Q, NMAT, XSPLIT>() + size_t(stage_count<Q, NMAT, XSPLIT>()) * stage_bytes<Q>();
 }
 
 __device__ __forceinline__ uint32_t lds_u32_unaligned(const uint8_t* p) {
@@ -98,7 +115,7 @@ __device__ __forceinline__ uint2 lds64(uint32_t address) {
 // `rot`, the byte offsets of the other three rotations), xsum the lane's min-term fragment.
 template <int XSPLIT>
 __device__ __forceinline__ void q4k_unit(uint32_t pA, uint32_t pB, int t, uint32_t xhi, uint32_t xlo, const int (&rot)[4], uint32_t xsum,
-                                         float (&total)[4]) {
+                                         float2 xs, float (&total)[4]) {
   const uint4 hA = lds128(pA), hB = lds128(pB);
   // 6-bit scales / mins of the 8 sub-blocks, four per word (scale_min_k4, quant_linear.metal:12-20).
   const uint32_t scA[2] = {hA.y & 0x3f3f3f3fu, (hA.w & 0x0f0f0f0fu) | ((hA.y >> 2) & 0x30303030u)};
@@ -167,10 +184,153 @@ __device__ __forceinline__ void q4k_unit(uint32_t pA, uint32_t pB, int t, uint32
     mma_16816(accm, a, b.x, b.y);
   }
   const float2 dA = __half22float2(*reinterpret_cast<const __half2*>(&hA.x)), dB = __half22float2(*reinterpret_cast<const __half2*>(&hB.x));
-  total[0] += dA.x * ((acc[0][0] + acc[1][0]) + (acc[2][0] + acc[3][0])) - dA.y * accm[0];
-  total[1] += dA.x * ((acc[0][1] + acc[1][1]) + (acc[2][1] + acc[3][1])) - dA.y * accm[1];
-  total[2] += dB.x * ((acc[0][2] + acc[1][2]) + (acc[2][2] + acc[3][2])) - dB.y * accm[2];
-  total[3] += dB.x * ((acc[0][3] + acc[1][3]) + (acc[2][3] + acc[3][3])) - dB.y * accm[3];
+  total[0] += xs.x * (dA.x * ((acc[0][0] + acc[1][0]) + (acc[2][0] + acc[3][0])) - dA.y * accm[0]);
+  total[1] += xs.y * (dA.x * ((acc[0][1] + acc[1][1]) + (acc[2][1] + acc[3][1])) - dA.y * accm[1]);
+  total[2] += xs.x * (dB.x * ((acc[0][2] + acc[1][2]) + (acc[2][2] + acc[3][2])) - dB.y * accm[2]);
+  total[3] += xs.y * (dB.x * ((acc[0][3] + acc[1][3]) + (acc[2][3] + acc[3][3])) - dB.y * accm[3]);
+}
+
+// ---- the formats whose sub-blocks are 32 wide ------------------------------------------------------------------
+// Fragment of one MMA from four quant bytes of the rows g and g+8: (base + byte) - base in fp16, base = 1024 + bias, exact.
+__device__ __forceinline__ void byte_fragment(uint32_t (&a)[4], uint32_t bytesA, uint32_t bytesB, uint32_t bias2) {
+  a[0] = hsub2_u32(__byte_perm(bytesA, 0x64u, 0x4140), bias2);
+  a[1] = hsub2_u32(__byte_perm(bytesB, 0x64u, 0x4140), bias2);
+  a[2] = hsub2_u32(__byte_perm(bytesA, 0x64u, 0x4342), bias2);
+  a[3] = hsub2_u32(__byte_perm(bytesB, 0x64u, 0x4342), bias2);
+}
+// Both MMAs (hi, lo) of fragment gi.
+template <int XSPLIT> __device__ __forceinline__ void mma_split(float (&acc)[4], const uint32_t (&a)[4], const uint2* xhi, const uint2* xlo, int at) {
+  uint2 b = xhi[at];
+  mma_16816(acc, a, b.x, b.y);
+  if (XSPLIT == 2) {
+    b = xlo[at];
+    mma_16816(acc, a, b.x, b.y);
+  }
+}
+__device__ __forceinline__ void add_scaled(float (&sum)[4], float sA, float sB, const float (&acc)[4]) {
+  sum[0] = fmaf(sA, acc[0], sum[0]), sum[1] = fmaf(sA, acc[1], sum[1]), sum[2] = fmaf(sB, acc[2], sum[2]), sum[3] = fmaf(sB, acc[3], sum[3]);
+}
+__device__ __forceinline__ void add_total(float (&total)[4], float2 xs, const float (&sum)[4]) {
+  total[0] = fmaf(xs.x, sum[0], total[0]), total[1] = fmaf(xs.y, sum[1], total[1]);
+  total[2] = fmaf(xs.x, sum[2], total[2]), total[3] = fmaf(xs.y, sum[3], total[3]);
+}
+__device__ __forceinline__ uint32_t lds_u32(const uint8_t* p) { return *reinterpret_cast<const uint32_t*>(p); }
+__device__ __forceinline__ float byte_of(uint32_t word, int i) { return float(__byte_perm(word, 0u, 0x4440 + i)); }
+
+// Q5_K (quant_linear.metal:50-67): fp16 d, dmin | 6-bit scales and mins | qh[32] | qs[128]. Element l of sub-block j has its
+// low nibble in qs[32 (j / 2) + l] (high half of the byte when j is odd) and its fifth bit in bit j of qh[l].
+template <int XSPLIT>
+__device__ __forceinline__ void q5k_unit(const uint8_t* pA, const uint8_t* pB, int lane, const uint2* xhi, const uint2* xlo, uint2 xsum, float2 xs,
+                                         float (&total)[4]) {
+  const int t = lane & 3;
+  const uint4 hA = *reinterpret_cast<const uint4*>(pA), hB = *reinterpret_cast<const uint4*>(pB);
+  const uint32_t scA[2] = {hA.y & 0x3f3f3f3fu, (hA.w & 0x0f0f0f0fu) | ((hA.y >> 2) & 0x30303030u)};
+  const uint32_t mnA[2] = {hA.z & 0x3f3f3f3fu, ((hA.w >> 4) & 0x0f0f0f0fu) | ((hA.z >> 2) & 0x30303030u)};
+  const uint32_t scB[2] = {hB.y & 0x3f3f3f3fu, (hB.w & 0x0f0f0f0fu) | ((hB.y >> 2) & 0x30303030u)};
+  const uint32_t mnB[2] = {hB.z & 0x3f3f3f3fu, ((hB.w >> 4) & 0x0f0f0f0fu) | ((hB.z >> 2) & 0x30303030u)};
+  constexpr uint32_t k1024 = 0x64006400u;
+  uint32_t highA[2], highB[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+    highA[u] = lds_u32(pA + 16 + 16 * u + 4 * t), highB[u] = lds_u32(pB + 16 + 16 * u + 4 * t);
+  float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t lowA[2], lowB[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      lowA[u] = lds_u32(pA + 48 + 32 * c + 16 * u + 4 * t), lowB[u] = lds_u32(pB + 48 + 32 * c + 16 * u + 4 * t);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int j = 2 * c + h;
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const uint32_t fifthA = (j < 4 ? highA[u] << (4 - j) : highA[u] >> (j - 4)) & 0x10101010u;
+        const uint32_t fifthB = (j < 4 ? highB[u] << (4 - j) : highB[u] >> (j - 4)) & 0x10101010u;
+        uint32_t a[4];
+        byte_fragment(a, ((h ? lowA[u] >> 4 : lowA[u]) & 0x0f0f0f0fu) | fifthA, ((h ? lowB[u] >> 4 : lowB[u]) & 0x0f0f0f0fu) | fifthB, k1024);
+        mma_split<XSPLIT>(acc, a, xhi, xlo, (2 * j + u) * 32 + lane);
+      }
+      add_scaled(sum, byte_of(scA[j >> 2], j & 3), byte_of(scB[j >> 2], j & 3), acc);
+    }
+  }
+  float accm[4] = {0.f, 0.f, 0.f, 0.f};
+  {
+    const uint32_t wordA = (t & 2) ? mnA[1] : mnA[0], wordB = (t & 2) ? mnB[1] : mnB[0];
+    const uint32_t pairA = (wordA >> ((t & 1) * 16)) & 0xffffu, pairB = (wordB >> ((t & 1) * 16)) & 0xffffu;
+    uint32_t a[4];
+    a[0] = a[2] = hsub2_u32(__byte_perm(pairA, 0x64u, 0x4140), k1024);
+    a[1] = a[3] = hsub2_u32(__byte_perm(pairB, 0x64u, 0x4140), k1024);
+    mma_16816(accm, a, xsum.x, xsum.y);
+  }
+  const float2 dA = __half22float2(*reinterpret_cast<const __half2*>(&hA.x)), dB = __half22float2(*reinterpret_cast<const __half2*>(&hB.x));
+  sum[0] = dA.x * sum[0] - dA.y * accm[0], sum[1] = dA.x * sum[1] - dA.y * accm[1];
+  sum[2] = dB.x * sum[2] - dB.y * accm[2], sum[3] = dB.x * sum[3] - dB.y * accm[3];
+  add_total(total, xs, sum);
+}
+
+// Q8_0 (quant_linear.metal:87-97): eight blocks of fp16 d | int8[32] stand for one super-block.
+template <int XSPLIT>
+__device__ __forceinline__ void q8_unit(const uint8_t* pA, const uint8_t* pB, int lane, const uint2* xhi, const uint2* xlo, float2 xs, float (&total)[4]) {
+  const int t = lane & 3;
+  constexpr uint32_t k1152 = 0x64806480u;
+  float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int at = 34 * j + 2 + 16 * u + 4 * t;  // word-aligned in odd blocks only
+      const uint32_t bytesA = (j & 1 ? lds_u32(pA + at) : lds_u32_unaligned(pA + at)) ^ 0x80808080u;
+      const uint32_t bytesB = (j & 1 ? lds_u32(pB + at) : lds_u32_unaligned(pB + at)) ^ 0x80808080u;
+      uint32_t a[4];
+      byte_fragment(a, bytesA, bytesB, k1152);
+      mma_split<XSPLIT>(acc, a, xhi, xlo, (2 * j + u) * 32 + lane);
+    }
+    add_scaled(sum, load_half_bits(pA + 34 * j), load_half_bits(pB + 34 * j), acc);
+  }
+  add_total(total, xs, sum);
+}
+
+// IQ4_XS (quant_linear.metal:99-115): fp16 d | scales_h u16 | scales_l[4] | qs[128]. Element l of sub-block j is the grid
+// value at the low (l < 16) or high nibble of qs[16 j + l % 16], times ls_j - 32.
+// Eight grid values of a word by byte permutes: `low` = grid values + 128 of the low nibbles of bytes 0..3 and of the high
+// ones, as the pairs (byte 0 low, byte 0 high, byte 1 low, byte 1 high) in x and those of bytes 2 and 3 in y.
+__device__ __forceinline__ uint2 iq4_lookup(uint32_t word) {
+  constexpr uint32_t k0 = 0x3f2d1801u, k1 = 0x766a5d4fu, k2 = 0xa6998d81u, k3 = 0xf1d9c5b5u;  // grid + 128, four per word
+  const uint32_t index = word & 0x77777777u, half = ((word >> 1) & 0x44444444u) | 0x32103210u;
+  uint2 out;
+  out.x = __byte_perm(__byte_perm(k0, k1, index), __byte_perm(k2, k3, index), half);
+  out.y = __byte_perm(__byte_perm(k0, k1, index >> 16), __byte_perm(k2, k3, index >> 16), half >> 16);
+  return out;
+}
+template <int XSPLIT>
+__device__ __forceinline__ void iq4_unit(const uint8_t* pA, const uint8_t* pB, int lane, const uint2* xhi, const uint2* xlo, float2 xs, float (&total)[4]) {
+  const int t = lane & 3;
+  constexpr uint32_t k1152 = 0x64806480u;
+  const uint2 hA = *reinterpret_cast<const uint2*>(pA), hB = *reinterpret_cast<const uint2*>(pB);
+  float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint2 qA = iq4_lookup(lds_u32(pA + 8 + 16 * j + 4 * t)), qB = iq4_lookup(lds_u32(pB + 8 + 16 * j + 4 * t));
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      uint32_t a[4];
+      a[0] = hsub2_u32(__byte_perm(qA.x, 0x64u, u ? 0x4341 : 0x4240), k1152);
+      a[1] = hsub2_u32(__byte_perm(qB.x, 0x64u, u ? 0x4341 : 0x4240), k1152);
+      a[2] = hsub2_u32(__byte_perm(qA.y, 0x64u, u ? 0x4341 : 0x4240), k1152);
+      a[3] = hsub2_u32(__byte_perm(qB.y, 0x64u, u ? 0x4341 : 0x4240), k1152);
+      mma_split<XSPLIT>(acc, a, xhi, xlo, (2 * j + u) * 32 + lane);
+    }
+    const int lsA = int((hA.y >> (4 * j)) & 15u) | int(((hA.x >> (16 + 2 * j)) & 3u) << 4);
+    const int lsB = int((hB.y >> (4 * j)) & 15u) | int(((hB.x >> (16 + 2 * j)) & 3u) << 4);
+    add_scaled(sum, float(lsA - 32), float(lsB - 32), acc);
+  }
+  const float dA = load_half_bits(pA), dB = load_half_bits(pB);
+  sum[0] *= dA, sum[1] *= dA, sum[2] *= dB, sum[3] *= dB;
+  add_total(total, xs, sum);
 }
 
 // ---- Q6_K: one 16-row x 256-k unit -------------------------------------------------------------
@@ -179,9 +339,10 @@ __device__ __forceinline__ void q4k_unit(uint32_t pA, uint32_t pB, int t, uint32
 // in qh[32*hh + l] >> 2s, and scale sc[r/16]. MMA gi covers elements [16gi, 16gi+16); lane t supplies
 // elements 16gi + 4t + {0,1,2,3}. Blocks are only 2-byte aligned, so words are fetched as two halves.
 template <int XSPLIT>
-__device__ __forceinline__ void q6k_unit(const uint8_t* pA, const uint8_t* pB, int lane, int hh, const uint2* xhi, const uint2* xlo,
+__device__ __forceinline__ void q6k_unit(const uint8_t* pA, const uint8_t* pB, int lane, int hh, const uint2* xhi, const uint2* xlo, float2 xs,
                                          float (&total)[4]) {
   const int t = lane & 3;
+  float sum[4] = {0.f, 0.f, 0.f, 0.f};
   const float dA = load_half_bits(pA + 208), dB = load_half_bits(pB + 208);
   constexpr uint32_t k1056 = 0x64206420u;
 #pragma unroll
@@ -208,13 +369,11 @@ __device__ __forceinline__ void q6k_unit(const uint8_t* pA, const uint8_t* pB, i
             mma_16816(acc, a, b.x, b.y);
           }
           const float sA = dA * float(int(reinterpret_cast<const int8_t*>(pA + 192)[gi])), sB = dB * float(int(reinterpret_cast<const int8_t*>(pB + 192)[gi]));
-          total[0] += sA * acc[0];
-          total[1] += sA * acc[1];
-          total[2] += sB * acc[2];
-          total[3] += sB * acc[3];
+          add_scaled(sum, sA, sB, acc);
         }
       }
     }
+  add_total(total, xs, sum);
 }
 
 __device__ __forceinline__ int find_segment(const GemvParams& p, int tile) {
@@ -231,7 +390,8 @@ template <class Q, int NMAT, int XSPLIT> __global__ void __launch_bounds__(kThre
   uint2* fragHi = reinterpret_cast<uint2*>(smemRaw + kControlBytes);
   uint2* fragLo = fragHi + (XSPLIT == 2 ? kChunkBlocks * 16 * 32 : 0);
   uint2* fragSum = fragHi + kChunkBlocks * 16 * 32 * XSPLIT;
-  float* partial = reinterpret_cast<float*>(fragSum + (Q::kMinTerm ? kChunkBlocks * 32 : 0));
+  float* xScale = reinterpret_cast<float*>(fragSum + (Q::kMinTerm ? kChunkBlocks * 32 : 0));  // [super-block][activation row]
+  float* partial = xScale + kChunkBlocks * 8;
   uint8_t* ring = reinterpret_cast<uint8_t*>(partial + 2 * NMAT * kConsumerWarps * 128);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -277,9 +437,12 @@ template <class Q, int NMAT, int XSPLIT> __global__ void __launch_bounds__(kThre
             // One tiled copy moves the whole 16-row x 8-super-block slab; columns past the end of a row are zero-filled
             // and still counted, so the transaction size is always the full box.
             if (lane == 0) {
-              mbar_arrive_expect_tx(&ctl.full[slot], uint32_t(Q::kStageBytes));
-              tma_load_2d(ring + size_t(slot) * Q::kStageBytes, &p.map[segment][mat], (chunk * (kChunkBlocks / kStageBlocks) + grp) * Q::kBlockBytes,
-                          int(row0), &ctl.full[slot]);
+              mbar_arrive_expect_tx(&ctl.full[slot], uint32_t(stage_bytes<Q>()));
+#pragma unroll
+              for (int box = 0; box < Q::kBoxes; ++box)
+                tma_load_2d(ring + size_t(slot) * stage_bytes<Q>() + box * box_bytes<Q>(), &p.map[segment][mat],
+                            ((chunk * (kChunkBlocks / kStageBlocks) + grp) * Q::kBoxes + box) * (box_blocks<Q>() * Q::kBlockBytes / 8), int(row0),
+                            &ctl.full[slot]);
             }
             __syncwarp();
           }
@@ -302,45 +465,63 @@ template <class Q, int NMAT, int XSPLIT> __global__ void __launch_bounds__(kThre
     const int chunkBlocks = min(kChunkBlocks, blocksPerRow - chunk * kChunkBlocks);
     const int groups = (chunkBlocks + kStageBlocks - 1) / kStageBlocks;
     const int k0 = chunk * kChunkBlocks * 256;
-    // Stage the activations of this K chunk in B-fragment order (hi / lo fp16 split). A warp takes a
-    // 64-value span of all 8 rows at a time: lane (row = lane/4, jj = lane%4) loads four float4 at
-    // 16*e + 4*jj, so each row contributes whole 64-byte pieces. Q4_K fragments are stored rotated by jj
-    // inside their 32-entry line, which makes both these writes and the MMA-time reads conflict-free.
-    for (int span = warp; span < chunkBlocks * 4; span += kConsumerWarps) {
-        const int row = lane >> 2, jj = lane & 3, sb = span >> 2, tq = span & 3;
-        float4 v[4];
+    // Stage the activations of this K chunk in B-fragment order (hi / lo fp16 split). A warp takes one super-block of all
+    // 8 rows at a time, in 64-value spans: lane (row = lane/4, jj = lane%4) loads four float4 of a span at 16*e + 4*jj,
+    // so each row contributes whole 64-byte pieces. Q4_K fragments are stored rotated by jj inside their 32-entry line,
+    // which makes both these writes and the MMA-time reads conflict-free.
+    for (int sb = warp; sb < chunkBlocks; sb += kConsumerWarps) {
+      const int row = lane >> 2, jj = lane & 3;
+      float4 v[4][4];
+      float largest = 0.f;
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          v[e] = row < p.m ? *reinterpret_cast<const float4*>(p.x + size_t(row) * p.ldx + k0 + 64 * span + 16 * e + 4 * jj)
-                           : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int tq = 0; tq < 4; ++tq)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
+          v[tq][e] = row < p.m ? *reinterpret_cast<const float4*>(p.x + size_t(row) * p.ldx + k0 + 256 * sb + 64 * tq + 16 * e + 4 * jj)
+                               : make_float4(0.f, 0.f, 0.f, 0.f);
+          largest = fmaxf(fmaxf(fmaxf(largest, fabsf(v[tq][e].x)), fmaxf(fabsf(v[tq][e].y), fabsf(v[tq][e].z))), fabsf(v[tq][e].w));
+        }
+      largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, 1));
+      largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, 2));
+      // the power of two that brings the row's largest value of this super-block into [512, 1024) (exponent field 136;
+      // sub-block sums then stay below 2^15), and its inverse
+      const int field = min(254, max(1, 263 - int(__float_as_uint(largest) >> 23)));
+      const float power = __uint_as_float(uint32_t(field) << 23);
+      if (jj == 0)
+        xScale[sb * 8 + row] = __uint_as_float(uint32_t(max(1, 254 - field)) << 23);
+#pragma unroll
+      for (int tq = 0; tq < 4; ++tq) {
+        float s[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float4 w = v[tq][e];
+          w.x *= power, w.y *= power, w.z *= power, w.w *= power;
           uint2 hi;
           float4 r;
           int slot;
-          if (Q::kMinTerm) {  // A pairs bytes (0,2) and (1,3) of a quant word
+          if (Q::kRotated) {  // A pairs bytes (0,2) and (1,3) of a quant word
             const int c = 2 * tq + (e & 1), i = ((c >> 2) * 4 + jj) * 2 + (e >> 1);
             slot = (sb * 16 + i) * 32 + ((row * 4 + (c & 3) + jj) & 31);
-            hi.x = pack_half2(v[e].x, v[e].z);
-            hi.y = pack_half2(v[e].y, v[e].w);
+            hi.x = pack_half2(w.x, w.z);
+            hi.y = pack_half2(w.y, w.w);
             const float2 f0 = __half22float2(*reinterpret_cast<__half2*>(&hi.x)), f1 = __half22float2(*reinterpret_cast<__half2*>(&hi.y));
-            r = make_float4(v[e].x - f0.x, v[e].z - f0.y, v[e].y - f1.x, v[e].w - f1.y);
+            r = make_float4(w.x - f0.x, w.z - f0.y, w.y - f1.x, w.w - f1.y);
           } else {
             slot = (sb * 16 + tq * 4 + e) * 32 + lane;
-            hi.x = pack_half2(v[e].x, v[e].y);
-            hi.y = pack_half2(v[e].z, v[e].w);
+            hi.x = pack_half2(w.x, w.y);
+            hi.y = pack_half2(w.z, w.w);
             const float2 f0 = __half22float2(*reinterpret_cast<__half2*>(&hi.x)), f1 = __half22float2(*reinterpret_cast<__half2*>(&hi.y));
-            r = make_float4(v[e].x - f0.x, v[e].y - f0.y, v[e].z - f1.x, v[e].w - f1.y);
+            r = make_float4(w.x - f0.x, w.y - f0.y, w.z - f1.x, w.w - f1.y);
           }
           fragHi[slot] = hi;
           if (XSPLIT == 2)
             fragLo[slot] = make_uint2(pack_half2(r.x, r.y), pack_half2(r.z, r.w));
+          if (Q::kMinTerm)  // sums of the two 32-value sub-blocks of this span, for the min term
+            s[e] = (w.x + w.y) + (w.z + w.w);
         }
-        if (Q::kMinTerm) {  // sums of the two 32-value sub-blocks of this span, for the min term
-          float s[4];
+        if (Q::kMinTerm) {
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            s[e] = (v[e].x + v[e].y) + (v[e].z + v[e].w);
             s[e] += __shfl_xor_sync(0xffffffffu, s[e], 1);
             s[e] += __shfl_xor_sync(0xffffffffu, s[e], 2);
           }
@@ -352,6 +533,7 @@ template <class Q, int NMAT, int XSPLIT> __global__ void __launch_bounds__(kThre
           }
         }
       }
+    }
     named_barrier(1, kConsumerWarps * kWarp);
 
     for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, ++tileCounter) {
@@ -386,17 +568,24 @@ template <class Q, int NMAT, int XSPLIT> __global__ void __launch_bounds__(kThre
           }
           const int count = min(kStageBlocks, chunkBlocks - grp * kStageBlocks);
           if (warp < count) {
-            const uint8_t* base = ring + size_t(slot) * Q::kStageBytes + warp * Q::kBlockBytes;
+            const uint8_t* base = ring + size_t(slot) * stage_bytes<Q>() + (warp / box_blocks<Q>()) * box_bytes<Q>() + (warp % box_blocks<Q>()) * Q::kBlockBytes;
+            const uint8_t *pA = base + g * row_pitch<Q>(), *pB = base + (g + 8) * row_pitch<Q>();
             const int sb = grp * kStageBlocks + warp;
-            if (Q::kMinTerm) {
-              const uint32_t rows = smem_u32(base);
-              q4k_unit<XSPLIT>(rows + g * Q::kRowStride, rows + (g + 8) * Q::kRowStride, t, fragHiAddress + sb * 4096, fragLoAddress + sb * 4096, rotation,
-                               fragSumAddress + sb * 256, total[mat]);
+            const float2 xs = *reinterpret_cast<const float2*>(xScale + sb * 8 + 2 * t);
+            const uint2 *hi = fragHi + sb * 512, *lo = fragLo + sb * 512;
+            if constexpr (std::is_same_v<Q, Q4K>) {
+              q4k_unit<XSPLIT>(smem_u32(pA), smem_u32(pB), t, fragHiAddress + sb * 4096, fragLoAddress + sb * 4096, rotation, fragSumAddress + sb * 256, xs,
+                               total[mat]);
+            } else if constexpr (std::is_same_v<Q, Q5K>) {
+              q5k_unit<XSPLIT>(pA, pB, lane, hi, lo, fragSum[sb * 32 + lane], xs, total[mat]);
+            } else if constexpr (std::is_same_v<Q, Q8>) {
+              q8_unit<XSPLIT>(pA, pB, lane, hi, lo, xs, total[mat]);
+            } else if constexpr (std::is_same_v<Q, IQ4>) {
+              iq4_unit<XSPLIT>(pA, pB, lane, hi, lo, xs, total[mat]);
             } else {
 #pragma unroll
               for (int half = 0; half < 2; ++half)
-                q6k_unit<XSPLIT>(base + g * Q::kRowStride, base + (g + 8) * Q::kRowStride, lane, half, fragHi + sb * 512, fragLo + sb * 512,
-                                 total[mat]);
+                q6k_unit<XSPLIT>(pA, pB, lane, half, hi, lo, xs, total[mat]);
             }
           }
           __syncwarp();
@@ -442,15 +631,33 @@ template <class Q, int NMAT, int XSPLIT> cudaError_t launch(const GemvParams& p,
 
 }  // namespace
 
-// type: ggml type id (12 = Q4_K, 14 = Q6_K); pair: gate/up fusion (two matrices, silu(a)*b epilogue).
-cudaError_t gemv_launch(int type, bool pair, int xsplit, const GemvParams& p, int sms, cudaStream_t stream) {
-  if (type == 12) {
-    if (pair)
-      return xsplit == 2 ? launch<Q4K, 2, 2>(p, sms, stream) : launch<Q4K, 2, 1>(p, sms, stream);
-    return xsplit == 2 ? launch<Q4K, 1, 2>(p, sms, stream) : launch<Q4K, 1, 1>(p, sms, stream);
+GemvBox gemv_box(int type) {
+  switch (type) {
+    case 8: return {Q8::kBlockBytes, box_blocks<Q8>(), Q8::kPad};
+    case 12: return {Q4K::kBlockBytes, box_blocks<Q4K>(), Q4K::kPad};
+    case 13: return {Q5K::kBlockBytes, box_blocks<Q5K>(), Q5K::kPad};
+    case 14: return {Q6K::kBlockBytes, box_blocks<Q6K>(), Q6K::kPad};
+    case 23: return {IQ4::kBlockBytes, box_blocks<IQ4>(), IQ4::kPad};
+    default: return {0, 0, 0};
   }
-  if (type == 14 && !pair)
-    return xsplit == 2 ? launch<Q6K, 1, 2>(p, sms, stream) : launch<Q6K, 1, 1>(p, sms, stream);
+}
+
+// type: ggml type id; pair: gate/up fusion (two matrices, silu(a)*b epilogue). Only Q4_K and Q6_K may drop the low half of
+// the activations (xsplit 1).
+cudaError_t gemv_launch(int type, bool pair, int xsplit, const GemvParams& p, int sms, cudaStream_t stream) {
+  switch (type) {
+    case 8: return pair ? launch<Q8, 2, 2>(p, sms, stream) : launch<Q8, 1, 2>(p, sms, stream);
+    case 12:
+      if (pair)
+        return xsplit == 2 ? launch<Q4K, 2, 2>(p, sms, stream) : launch<Q4K, 2, 1>(p, sms, stream);
+      return xsplit == 2 ? launch<Q4K, 1, 2>(p, sms, stream) : launch<Q4K, 1, 1>(p, sms, stream);
+    case 13: return pair ? launch<Q5K, 2, 2>(p, sms, stream) : launch<Q5K, 1, 2>(p, sms, stream);
+    case 14:
+      if (pair)
+        break;
+      return xsplit == 2 ? launch<Q6K, 1, 2>(p, sms, stream) : launch<Q6K, 1, 1>(p, sms, stream);
+    case 23: return pair ? launch<IQ4, 2, 2>(p, sms, stream) : launch<IQ4, 1, 2>(p, sms, stream);
+  }
   return cudaErrorInvalidValue;
 }
 

@@ -431,15 +431,16 @@ int infdev_dequant(infdev_ctx* ctx, int type, const void* blocks, int64_t count,
 // `supplied`: image of x to read instead of quantising it (integer kernel only).
 static int linear_run(infdev_ctx* ctx, int type, bool pair, int count, const void* const* w, const void* const* w2, const int64_t* n, int64_t k,
                       const float* x, int64_t m, float* const* y, const float* const* residual, const uint8_t* supplied) {
-  if (type != INFDEV_Q4_K && type != INFDEV_Q6_K)
-    return fail(ctx, INFDEV_E_ARGUMENT, "linear: weight type must be Q4_K or Q6_K");
-  if (pair && type != INFDEV_Q4_K)
-    return fail(ctx, INFDEV_E_ARGUMENT, "gate_up: only Q4_K pairs are supported");
+  const infdev::GemvBox box = infdev::gemv_box(type);
+  if (!box.blockBytes)
+    return fail(ctx, INFDEV_E_ARGUMENT, "linear: unsupported weight type " + std::to_string(type));
+  if (pair && type == INFDEV_Q6_K)
+    return fail(ctx, INFDEV_E_ARGUMENT, "gate_up: Q6_K pairs are not supported");
   if (count < 1 || count > 4 || m < 0 || k <= 0 || k % 256)
     return fail(ctx, INFDEV_E_ARGUMENT, "linear: need 1..4 matrices and k a positive multiple of 256");
   if (type == INFDEV_Q6_K && k % 2048)
     return fail(ctx, INFDEV_E_ARGUMENT, "linear: Q6_K rows must be 16-byte aligned (k a multiple of 2048)");
-  if (pair && k > 4096)
+  if (pair && k > infdev::kGemvPairMaxK)
     return fail(ctx, INFDEV_E_ARGUMENT, "gate_up: k must not exceed 4096");
   if (!aligned16(x) || (k % 4))
     return fail(ctx, INFDEV_E_ARGUMENT, "linear: activations must be 16-byte aligned");
@@ -494,17 +495,16 @@ static int linear_run(infdev_ctx* ctx, int type, bool pair, int count, const voi
   p.nseg = count;
   int tiles = 0;
   const bool integer = type == INFDEV_Q4_K && ctx->integerDecode && k <= 16384;
-  const int pad = integer ? infdev::kDecodePadBytes : 0;
+  const int boxBlocks = integer ? infdev::kGemvStageBlocks : box.blocks, pad = integer ? infdev::kDecodePadBytes : box.padBytes;
   for (int i = 0; i < count; ++i) {
     if (n[i] <= 0 || n[i] % 16 || !aligned16(w[i]) || (pair && !aligned16(w2[i])))
       return fail(ctx, INFDEV_E_ARGUMENT, "linear: n must be a positive multiple of 16 and weights 16-byte aligned");
     p.seg[i] = {static_cast<const uint8_t*>(w[i]), pair ? static_cast<const uint8_t*>(w2[i]) : nullptr, y[i], residual ? residual[i] : nullptr,
                 int(n[i]), int(n[i]), tiles};
-    const int blockBytes = type == INFDEV_Q4_K ? 144 : 210;
-    if (int r = weight_map(ctx, w[i], n[i], k, blockBytes, infdev::kGemvStageBlocks, infdev::kGemvTileRows, &p.map[i][0], pad))
+    if (int r = weight_map(ctx, w[i], n[i], k, box.blockBytes, boxBlocks, infdev::kGemvTileRows, &p.map[i][0], pad))
       return r;
     if (pair)
-      if (int r = weight_map(ctx, w2[i], n[i], k, blockBytes, infdev::kGemvStageBlocks, infdev::kGemvTileRows, &p.map[i][1], pad))
+      if (int r = weight_map(ctx, w2[i], n[i], k, box.blockBytes, boxBlocks, infdev::kGemvTileRows, &p.map[i][1], pad))
         return r;
     tiles += int(n[i] / 16);
   }
@@ -548,7 +548,17 @@ static int linear_common(infdev_ctx* ctx, int type, bool pair, int count, const 
   uint8_t* captured = take_capture(ctx);
   if (captured && (count != 1 || n[0] % 256))
     return fail(ctx, INFDEV_E_ARGUMENT, "linear: an image of the result needs a single matrix with n a multiple of 256");
-  if (infdev::format_supported(type)) {  // Q5_K, Q8_0, IQ4_XS: one plain launch per matrix and 8-row slice
+  // Q5_K, Q8_0, IQ4_XS: the tensor-core GEMV takes whole 16-row tiles whose rows a tiled copy can address, and gate / up
+  // pairs of one K chunk; any other shape goes to the plain kernel, one launch per matrix and 8-row slice.
+  bool plain = infdev::format_supported(type);
+  if (plain) {
+    const int64_t rowBytes = k / 256 * infdev::gemv_box(type).blockBytes;
+    bool tiled = rowBytes % 16 == 0 && (!pair || k <= infdev::kGemvPairMaxK);
+    for (int i = 0; i < count; ++i)
+      tiled = tiled && n[i] > 0 && n[i] % infdev::kGemvTileRows == 0 && aligned16(w[i]) && (!pair || aligned16(w2[i]));
+    plain = !tiled;
+  }
+  if (plain) {
     if (m < 0 || k <= 0 || k % 256 || !aligned16(x))
       return fail(ctx, INFDEV_E_ARGUMENT, "linear: k must be a positive multiple of 256 and the activations 16-byte aligned");
     for (int i = 0; i < count; ++i) {

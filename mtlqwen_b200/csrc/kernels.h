@@ -29,6 +29,7 @@ struct GemvParams {
 
 // Box geometry shared by the host encoder and the kernel.
 constexpr int kGemvStageBlocks = 8, kGemvTileRows = 16;
+constexpr int64_t kGemvPairMaxK = 4096;  // a gate / up pair is finished within one K chunk
 // The integer Q4_K kernel reads 32 bytes past the 8 super-blocks of a box row, which makes the row pitch in shared
 // memory 1184 = 32 (mod 128) bytes: the 32-byte pieces of consecutive rows that a warp reads in one load then fall
 // into different banks.
@@ -55,6 +56,12 @@ struct UmmaParams {
 
 cudaError_t umma_launch(bool pair, const UmmaParams& p, const float* x, int ldx, int sms, cudaStream_t stream);
 
+// What a tiled copy of the fp16 GEMV moves per row of a matrix of this type: `blocks` super-blocks of `blockBytes` (for
+// Q8_0: eight blocks) and `padBytes` more. blockBytes 0: not a type of that kernel.
+struct GemvBox {
+  int blockBytes, blocks, padBytes;
+};
+GemvBox gemv_box(int type);
 cudaError_t gemv_launch(int type, bool pair, int xsplit, const GemvParams& p, int sms, cudaStream_t stream);
 
 // Integer-MMA Q4_K decode GEMV over an activation image (q4k_decode.cu).

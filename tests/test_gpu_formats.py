@@ -47,6 +47,24 @@ def test_linear_matches_oracle(dev, name, qtype, n, k, m):
   assert rel_err(y.download(), oracle.linear(w, qtype, n, k, x, res)) < 1e-5
 
 
+@pytest.mark.parametrize("name,qtype", TYPES + [("q6k", D.Q6_K)])
+@pytest.mark.parametrize("n,k,m", [(16, 2048, 1), (2400, 2048, 3), (48, 10240, 8), (16, 256, 2), (32, 1536, 7), (160, 1280, 5), (24, 4096, 4)])
+def test_tensor_core_gemv_edges(dev, name, qtype, n, k, m):
+  """One tile, more tiles than SMs with a ragged last round, a last K chunk of one stage, rows shorter than a stage, and
+  shapes the tensor-core kernel leaves to the plain one (n not a multiple of 16, rows that are not 16-byte aligned). The
+  activations span what fp32 holds and fp16 does not: the kernel scales every (row, super-block) by a power of two."""
+  if qtype == D.Q6_K and (k % 2048 or n % 16):
+    pytest.skip("Q6_K takes rows of whole 2048-value spans and tiles of 16 rows")
+  w, x = synth.weight(qtype, n, k, 63), synth.activations(m, k, 64)
+  x[:, :256] *= 1.0e6
+  x[m - 1] *= 1.0e-9
+  y = dev.empty((m, n))
+  dev.linear(qtype, dev.array(w), n, k, dev.array(x), m, y)
+  got, want = y.download(), oracle.linear(w, qtype, n, k, x)
+  for row in range(m):  # row by row: their magnitudes differ by fifteen orders
+    assert rel_err(got[row], want[row]) < 1e-5, row
+
+
 @pytest.mark.parametrize("name,qtype", TYPES)
 def test_gate_up_matches_oracle(dev, name, qtype):
   n, k, m = 768, 4096, 5
