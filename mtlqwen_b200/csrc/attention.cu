@@ -2,7 +2,8 @@
 //
 // attention_prepare_kernel <- attention_prepare (attention.metal:14-50) + the cache append that the
 //                             reference does inside attention_scan (:126-133)
-// attention_scan_kernel    <- attention_scan   (attention.metal:103-183)
+// attention_scan_kernel    <- attention_scan   (attention.metal:103-183), for passes whose queries have one row each
+// attention_group_kernel   <- the same, for passes with prompt chunks or speculative rows
 // attention_reduce_kernel  <- attention_reduce (attention.metal:185-216)
 //
 // K/V pool of one layer: [physical block][4 kv heads][blockTokens][256] fp16, so the 16 tokens of a tile of
@@ -14,6 +15,7 @@
 // row depends only on how many tokens that row attends to, so a sequence gets the same arithmetic whether
 // it runs alone or batched. One CTA serves the four query heads that share a kv head, so K and V are read
 // once per group.
+#include <algorithm>
 #include <mutex>
 #include "act_image.cuh"
 #include "ops.h"
@@ -245,17 +247,280 @@ __global__ void __launch_bounds__(128, 6) attention_scan_kernel(const float* q, 
   }
 }
 
+// ---- rows of one query together: prompt chunks and speculative rows --------------------------------------------------
+// The scan above reads K and V once per row: 128 prompt rows behind 2000 tokens pull 1 GB through the L2 (170 us, and
+// 18 us to merge 32 splits of every row). Here up to 16 consecutive rows of a query share every K/V tile: a CTA holds the
+// 16 rows x 4 query heads of one kv head as 64 rows of the two contractions, and walks its piece of the context in tiles
+// of 64 tokens, softmax online. 8 warps = 4 heads x 2 halves: a warp scores 32 tokens of the tile, hands its weights to
+// its partner through shared memory and accumulates 128 of the 256 value dims for all 64. Operands as in the scan: fp16
+// keys and values, query and softmax weights as fp16 hi + lo, fp32 accumulation.
+// Bound by the mma.sync rate (4.2 G multiply-adds with both halves of q and p for 128 rows behind 1920, about 15 us).
+//
+// Work items (tile of rows, piece of context, kv head) are dealt to one CTA per SM; which exist only the device knows, so
+// a CTA finds its next item by a scan over the queries. The pieces of a tile follow from its context and from `most`, which
+// the host sets so that the items of the pass fill the SMs about once; a tile of few rows (decode rows that share a pass
+// with a prompt) is cut as finely as the caller's scratch allows.
+constexpr int kGroupRows = 16, kGroupTokens = 64, kGroupThreads = 256, kGroupPitch = kDim + 8, kWeightPitch = kGroupTokens + 8;
+
+struct GroupShared {
+  __half q[2][kGroup * kGroupRows][kGroupPitch];                         // hi, lo; row 16 * head + r
+  __half k[2][kGroupTokens][kGroupPitch], v[2][kGroupTokens][kGroupPitch];  // two buffers
+  __half p[2][kGroup * kGroupRows][kWeightPitch];                        // hi, lo
+  float exchange[2][kGroup * kGroupRows];
+};
+
+struct RowTile {
+  uint32_t start, rows, first, attended, slot;  // first: position of its first row; attended: context of its last row
+};
+
+__device__ __forceinline__ RowTile tile_of(const infdev_query& query, uint32_t index) {
+  RowTile tile;
+  tile.start = query.start + index * kGroupRows;
+  tile.rows = min(uint32_t(kGroupRows), query.count - index * kGroupRows);
+  tile.first = query.position + index * kGroupRows;
+  tile.attended = tile.first + tile.rows;
+  tile.slot = query.slot;
+  return tile;
+}
+
+// Pieces of a tile's context: at least 128 tokens, whole 64-token tiles.
+__device__ __forceinline__ uint32_t piece_tokens(uint32_t attended, uint32_t rows, uint32_t most, uint32_t maxSplits) {
+  const uint32_t wanted = max(1u, min((attended + 127u) / 128u, rows <= 4 ? maxSplits : most));
+  return ((attended + wanted - 1) / wanted + kGroupTokens - 1) / kGroupTokens * kGroupTokens;
+}
+__device__ __forceinline__ uint32_t piece_count(uint32_t attended, uint32_t piece) { return (attended + piece - 1) / piece; }
+
+// Work item `item` of the pass, found by one warp together; false when there are fewer.
+__device__ __forceinline__ bool find_item(const infdev_query* queries, int queryCount, uint32_t most, uint32_t maxSplits, uint32_t item, RowTile& tile,
+                                          uint32_t& split, uint32_t& piece) {
+  const uint32_t lane = threadIdx.x & 31;
+  for (int base = 0; base < queryCount; base += 32) {
+    uint32_t mine = 0, tiles = 0;
+    infdev_query query = {};
+    if (base + int(lane) < queryCount) {
+      query = queries[base + lane];
+      tiles = (query.count + kGroupRows - 1) / kGroupRows;
+      for (uint32_t t = 0; t < tiles; ++t) {
+        const RowTile each = tile_of(query, t);
+        mine += piece_count(each.attended, piece_tokens(each.attended, each.rows, most, maxSplits));
+      }
+    }
+    uint32_t inclusive = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t other = __shfl_up_sync(0xffffffffu, inclusive, o);
+      if (int(lane) >= o)
+        inclusive += other;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, inclusive, 31);
+    if (item >= total) {
+      item -= total;
+      continue;
+    }
+    const int owner = __ffs(__ballot_sync(0xffffffffu, inclusive > item)) - 1;
+    uint32_t found[7] = {};
+    if (int(lane) == owner) {
+      uint32_t local = item - (inclusive - mine);
+      for (uint32_t t = 0; t < tiles; ++t) {
+        const RowTile each = tile_of(query, t);
+        const uint32_t tokens = piece_tokens(each.attended, each.rows, most, maxSplits), count = piece_count(each.attended, tokens);
+        if (local < count) {
+          found[0] = each.start, found[1] = each.rows, found[2] = each.first, found[3] = each.attended, found[4] = each.slot, found[5] = local,
+          found[6] = tokens;
+          break;
+        }
+        local -= count;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 7; ++i)
+      found[i] = __shfl_sync(0xffffffffu, found[i], owner);
+    tile = {found[0], found[1], found[2], found[3], found[4]};
+    split = found[5], piece = found[6];
+    return true;
+  }
+  return false;
+}
+
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const __half* address) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(address)));
+}
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], const __half* address) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(smem_u32(address)));
+}
+// {a, b} as fp16 hi and lo pairs
+__device__ __forceinline__ uint2 split_pair(float a, float b) {
+  const uint32_t hi = pack_half2(a, b);
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+  return make_uint2(hi, pack_half2(a - f.x, b - f.y));
+}
+
+__global__ void __launch_bounds__(kGroupThreads, 1)
+    attention_group_kernel(const float* q, const __half* cacheK, const __half* cacheV, const infdev_query* queries, int queryCount, const int32_t* table,
+                           int tableStride, int blockTokens, uint32_t most, uint32_t maxSplits, float* partials) {
+  pdl_launch_dependents();
+  pdl_wait();
+  extern __shared__ __align__(16) uint8_t groupRaw[];
+  GroupShared& sh = *reinterpret_cast<GroupShared*>(groupRaw);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, head = warp & 3, half = warp >> 2, g = lane >> 2, t = lane & 3;
+  const int rowBase = head * kGroupRows;  // this warp's 16 rows of q, p and exchange
+  RowTile tile;
+  uint32_t split, piece;
+  for (uint32_t item = blockIdx.x; find_item(queries, queryCount, most, maxSplits, item / kKvHeads, tile, split, piece); item += gridDim.x) {
+    const uint32_t kvHead = item % kKvHeads, begin = split * piece, end = min(tile.attended, begin + piece);
+    const int32_t* slotTable = table + size_t(tile.slot) * tableStride;
+    auto fetch = [&](uint32_t from, int buffer) {  // a warp copies one token's 512 bytes at a time
+#pragma unroll
+      for (int c = 0; c < kGroupTokens / 8; ++c) {
+        const uint32_t token = c * 8 + warp, at = min(from + token, end - 1);
+        const uint32_t bytes = from + token < end ? 16u : 0u;  // zeros past the end
+        const size_t base = ((size_t(slotTable[at / blockTokens]) * kKvHeads + kvHead) * blockTokens + at % blockTokens) * kDim + lane * 8;
+        copy_async16(&sh.k[buffer][token][lane * 8], cacheK + base, bytes);
+        copy_async16(&sh.v[buffer][token][lane * 8], cacheV + base, bytes);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    __syncthreads();  // the item before this one is finished with the shared arrays
+    fetch(begin, 0);
+    // the 16 rows x 4 heads of q, hi and lo; rows past the tile's are zero
+    for (int i = threadIdx.x; i < kGroup * kGroupRows * (kDim / 4); i += kGroupThreads) {
+      const int row = i / (kDim / 4), d = i % (kDim / 4) * 4, r = row % kGroupRows, h = row / kGroupRows;
+      float4 value = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r < int(tile.rows))
+        value = *reinterpret_cast<const float4*>(q + (size_t(tile.start + r) * kQHeads + kvHead * kGroup + h) * kDim + d);
+      const uint2 a = split_pair(value.x, value.y), b = split_pair(value.z, value.w);
+      *reinterpret_cast<uint2*>(&sh.q[0][row][d]) = make_uint2(a.x, b.x);
+      *reinterpret_cast<uint2*>(&sh.q[1][row][d]) = make_uint2(a.y, b.y);
+    }
+    float maximum[2] = {-1.0e30f, -1.0e30f}, norm[2] = {0.f, 0.f}, acc[16][4];  // rows g and g + 8
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+    int buffer = 0;
+    for (uint32_t from = begin; from < end; from += kGroupTokens, buffer ^= 1) {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();  // the tile has landed, and everybody is done with the one before
+      if (from + kGroupTokens < end)
+        fetch(from + kGroupTokens, buffer ^ 1);
+      float score[4][4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        score[j][0] = score[j][1] = score[j][2] = score[j][3] = 0.f;
+#pragma unroll
+      for (int step = 0; step < kDim / 16; ++step) {
+        uint32_t hi[4], lo[4];
+        ldmatrix4(hi, &sh.q[0][rowBase + (lane & 15)][16 * step + 8 * (lane >> 4)]);
+        ldmatrix4(lo, &sh.q[1][rowBase + (lane & 15)][16 * step + 8 * (lane >> 4)]);
+#pragma unroll
+        for (int pair = 0; pair < 2; ++pair) {
+          uint32_t b[4];
+          ldmatrix4(b, &sh.k[buffer][32 * half + 16 * pair + 8 * (lane >> 4) + (lane & 7)][16 * step + 8 * ((lane >> 3) & 1)]);
+          mma_16816(score[2 * pair], hi, b[0], b[1]);
+          mma_16816(score[2 * pair + 1], hi, b[2], b[3]);
+          mma_16816(score[2 * pair], lo, b[0], b[1]);
+          mma_16816(score[2 * pair + 1], lo, b[2], b[3]);
+        }
+      }
+      // scale, causal mask, row maxima over both halves of the tile
+      float best[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t token = from + 32 * half + 8 * j + 2 * t + (i & 1), limit = min(end, tile.first + g + 8 * (i >> 1) + 1);
+          score[j][i] = token < limit ? score[j][i] * (1.0f / 16.0f) : -INFINITY;
+          best[i >> 1] = fmaxf(best[i >> 1], score[j][i]);
+        }
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        best[r] = fmaxf(best[r], __shfl_xor_sync(0xffffffffu, best[r], 1));
+        best[r] = fmaxf(best[r], __shfl_xor_sync(0xffffffffu, best[r], 2));
+        if (t == 0)
+          sh.exchange[half][rowBase + g + 8 * r] = best[r];
+      }
+      named_barrier(1 + head, 64);
+      float rescale[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float next = fmaxf(maximum[r], fmaxf(best[r], sh.exchange[half ^ 1][rowBase + g + 8 * r]));
+        rescale[r] = expf(maximum[r] - next);
+        maximum[r] = next;
+        norm[r] *= rescale[r];
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const float w0 = expf(score[j][2 * r] - maximum[r]), w1 = expf(score[j][2 * r + 1] - maximum[r]);
+          norm[r] += w0 + w1;
+          const uint2 w = split_pair(w0, w1);
+          *reinterpret_cast<uint32_t*>(&sh.p[0][rowBase + g + 8 * r][32 * half + 8 * j + 2 * t]) = w.x;
+          *reinterpret_cast<uint32_t*>(&sh.p[1][rowBase + g + 8 * r][32 * half + 8 * j + 2 * t]) = w.y;
+        }
+      named_barrier(1 + head, 64);  // both halves of the weights are there
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        acc[j][0] *= rescale[0], acc[j][1] *= rescale[0], acc[j][2] *= rescale[1], acc[j][3] *= rescale[1];
+#pragma unroll
+      for (int step = 0; step < kGroupTokens / 16; ++step) {
+        uint32_t hi[4], lo[4];
+        ldmatrix4(hi, &sh.p[0][rowBase + (lane & 15)][16 * step + 8 * (lane >> 4)]);
+        ldmatrix4(lo, &sh.p[1][rowBase + (lane & 15)][16 * step + 8 * (lane >> 4)]);
+#pragma unroll
+        for (int pair = 0; pair < 8; ++pair) {
+          uint32_t b[4];
+          ldmatrix4_trans(b, &sh.v[buffer][16 * step + (lane & 15)][128 * half + 16 * pair + 8 * (lane >> 4)]);
+          mma_16816(acc[2 * pair], hi, b[0], b[1]);
+          mma_16816(acc[2 * pair + 1], hi, b[2], b[3]);
+          mma_16816(acc[2 * pair], lo, b[0], b[1]);
+          mma_16816(acc[2 * pair + 1], lo, b[2], b[3]);
+        }
+      }
+    }
+    // the norm over both halves, then this piece's record of every live row
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      norm[r] += __shfl_xor_sync(0xffffffffu, norm[r], 1);
+      norm[r] += __shfl_xor_sync(0xffffffffu, norm[r], 2);
+      if (t == 0)
+        sh.exchange[half][rowBase + g + 8 * r] = norm[r];
+    }
+    named_barrier(1 + head, 64);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const uint32_t row = g + 8 * r;
+      if (row >= tile.rows)
+        continue;
+      float* record = partials + ((size_t(tile.start + row) * kQHeads + kvHead * kGroup + head) * maxSplits + split) * kPartialStride;
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        *reinterpret_cast<float2*>(record + 128 * half + 8 * j + 2 * t) = make_float2(acc[j][2 * r], acc[j][2 * r + 1]);
+      if (half == 0 && t == 0)
+        *reinterpret_cast<float2*>(record + kDim) = make_float2(maximum[r], sh.exchange[0][rowBase + row] + sh.exchange[1][rowBase + row]);
+    }
+  }
+}
+
 // grid (rows * 16), 256 threads: merge the splits, normalise, multiply by sigmoid(gate).
 // `image`, when not null, also receives the activation image of the output rows: a head is one 256-value block.
+// GROUPED: the splits are those of attention_group_kernel.
+template <bool GROUPED>
 __global__ void __launch_bounds__(256) attention_reduce_kernel(const float* partials, const float* qg, const infdev_query* queries, int queryCount,
-                                                               uint32_t maxSplits, float* out, uint8_t* image) {
+                                                               uint32_t most, uint32_t maxSplits, float* out, uint8_t* image) {
   pdl_launch_dependents();
   pdl_wait();
   const uint32_t headRow = blockIdx.x, row = headRow / kQHeads, dim = threadIdx.x;
   const infdev_query& info = query_of_row(queries, queryCount, row);
-  const uint32_t attended = info.position + (row - info.start) + 1;
-  uint32_t begin, end, count;
-  split_range(attended, maxSplits, 0, begin, end, count);
+  uint32_t count;
+  if (GROUPED) {
+    const RowTile tile = tile_of(info, (row - info.start) / kGroupRows);
+    count = piece_count(tile.attended, piece_tokens(tile.attended, tile.rows, most, maxSplits));
+  } else {
+    uint32_t begin, end;
+    split_range(info.position + (row - info.start) + 1, maxSplits, 0, begin, end, count);
+  }
   const float* src = partials + size_t(headRow) * maxSplits * kPartialStride;
   // Lane s of every warp fetches the running maximum and norm of split s (at most 32 splits) in one trip to the L2; the
   // weights of the splits then travel by shuffle, and the loop below has only independent loads, taken in split order
@@ -304,13 +569,29 @@ cudaError_t attention_prepare_launch(const float* qg, const float* rawK, const f
 
 cudaError_t attention_launch(const float* q, const float* qg, const void* cacheK, const void* cacheV, const infdev_query* queries,
                              int queryCount, const int32_t* table, int tableStride, int blockTokens, int64_t rows, uint32_t maxSplits, float* partials, float* out,
-                             uint8_t* image, cudaStream_t stream) {
+                             uint8_t* image, bool rowwise, int sms, cudaStream_t stream) {
   if (rows <= 0)
     return cudaSuccess;
-  launch_kernel(attention_scan_kernel, dim3(maxSplits, kKvHeads, unsigned(rows)), 128, 0, stream, q, static_cast<const __half*>(cacheK),
+  const uint32_t splits = std::min<uint32_t>(maxSplits, 32);  // the merge keeps one split per lane
+  if (rows > queryCount && !rowwise) {
+    // Some query has several rows. (One row each is the decode pass, where the scan is faster: no query rows to share a
+    // tile with, and six small CTAs per SM hide the copies that the group kernel's single CTA waits for.)
+    static PerDeviceOnce configured;
+    if (const cudaError_t e = configure_shared_memory(attention_group_kernel, sizeof(GroupShared), configured))
+      return e;
+    const int64_t tiles = std::max<int64_t>((rows + kGroupRows - 1) / kGroupRows, queryCount);
+    const uint32_t most = uint32_t(std::clamp<int64_t>(sms / (kKvHeads * tiles), 1, splits));
+    const int64_t items = (rows + queryCount) * kKvHeads * splits;  // no more than these
+    launch_kernel(attention_group_kernel, unsigned(std::min<int64_t>(items, sms)), kGroupThreads, sizeof(GroupShared), stream, q,
+                  static_cast<const __half*>(cacheK), static_cast<const __half*>(cacheV), queries, queryCount, table, tableStride, blockTokens, most, splits,
+                  partials);
+    launch_kernel(attention_reduce_kernel<true>, unsigned(rows * kQHeads), 256, 0, stream, partials, qg, queries, queryCount, most, splits, out, image);
+    return cudaGetLastError();
+  }
+  launch_kernel(attention_scan_kernel, dim3(splits, kKvHeads, unsigned(rows)), 128, 0, stream, q, static_cast<const __half*>(cacheK),
                                                                                        static_cast<const __half*>(cacheV), queries, queryCount, table,
-                                                                                       tableStride, blockTokens, maxSplits, partials);
-  launch_kernel(attention_reduce_kernel, unsigned(rows * kQHeads), 256, 0, stream, partials, qg, queries, queryCount, maxSplits, out, image);
+                                                                                       tableStride, blockTokens, splits, partials);
+  launch_kernel(attention_reduce_kernel<false>, unsigned(rows * kQHeads), 256, 0, stream, partials, qg, queries, queryCount, 0u, splits, out, image);
   return cudaGetLastError();
 }
 
@@ -351,7 +632,7 @@ cudaError_t attention_static_launch(const float* q, const float* qg, const void*
   launch_kernel(attention_scan_kernel, dim3(kStaticSplits, kKvHeads, unsigned(rows)), 128, 0, stream, q, static_cast<const __half*>(cacheK),
                                                                                           static_cast<const __half*>(cacheV), queries, queryCount, table,
                                                                                           tableStride, blockTokens, kStaticSplits, partials);
-  launch_kernel(attention_reduce_kernel, unsigned(rows * kQHeads), 256, 0, stream, partials, qg, queries, queryCount, kStaticSplits, out, nullptr);
+  launch_kernel(attention_reduce_kernel<false>, unsigned(rows * kQHeads), 256, 0, stream, partials, qg, queries, queryCount, 0u, uint32_t(kStaticSplits), out, nullptr);
   return cudaGetLastError();
 }
 

@@ -17,7 +17,7 @@
 
 struct infdev_ctx {
   int device = 0, sms = 0, xsplit = 2;
-  int umma = 1;  // tcgen05 GEMM for Q4_K launches of more than 8 activation rows: 0 off, 1 on
+  int umma = 1;  // tcgen05 GEMM for Q4_K launches of more than 8 activation rows, grouped attention rows: 0 off, 1 on
   int integerDecode = 1;     // Q4_K decode GEMV: 1 integer-MMA kernel over an activation image, 0 fp16-MMA kernel
   uint8_t* image = nullptr;  // activation image for the integer decode kernel (K up to 16384)
   int* imageCounters = nullptr;        // arrival counters of the kernels that write images block by block (zero between launches)
@@ -729,7 +729,7 @@ int infdev_attention(infdev_ctx* ctx, const float* q, const float* qg, const voi
   ctx->launches += 2;
   return check(ctx,
                infdev::attention_launch(q, qg, cacheK, cacheV, queries, queryCount, table, tableStride, blockTokens, rows, maxSplits, partials, out,
-                                        take_capture(ctx), ctx->stream),
+                                        take_capture(ctx), !ctx->umma, ctx->sms, ctx->stream),
                "attention");
 }
 

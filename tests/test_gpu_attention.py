@@ -112,6 +112,28 @@ def test_attention_shapes(dev, contexts, counts, block_tokens):
   assert run_attention(dev, rng, contexts, counts, block_tokens) < TOL
 
 
+@pytest.mark.parametrize("contexts,counts,block_tokens,max_splits", [
+  ([2], [2], 16, 32),  # the shortest group: two rows of a fresh sequence
+  ([16], [16], 16, 32), ([17], [17], 16, 32), ([15, 33], [15, 33], 16, 32),  # exactly one tile, one row more, one fewer
+  ([64, 65, 127], [3, 4, 5], 16, 32),  # context at the edges of the 64-token tiles, rows at the cut of the piece rule
+  ([4100, 900, 70], [1, 1, 16], 128, 32),  # decode rows with long contexts beside a prompt tile
+  ([1500, 2500], [100, 28], 128, 3),  # the caller's scratch bounds the pieces
+  ([130] * 8, [5] * 8, 128, 32),  # speculative rows of eight sequences
+])
+def test_rows_that_share_a_tile(dev, contexts, counts, block_tokens, max_splits):
+  contexts = [max(context, count) for context, count in zip(contexts, counts)]
+  rng = np.random.default_rng(sum(contexts) + 31 * len(counts))
+  assert run_attention(dev, rng, contexts, counts, block_tokens, max_splits) < 1e-5
+
+
+def test_switching_the_group_kernel_off_changes_rounding_only(dev):
+  dev.set_umma(0)
+  try:
+    assert run_attention(dev, np.random.default_rng(4), [700, 40], [90, 12], 128) < 1e-5
+  finally:
+    dev.set_umma(1)
+
+
 def test_attention_result_does_not_depend_on_batching(dev):
   """A row's split partition depends only on its own context: the output of a sequence's decode row inside an
   8-row pass equals, byte for byte, the output of the same row run alone on the same cache."""
