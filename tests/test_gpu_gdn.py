@@ -111,6 +111,12 @@ def test_gdn_mixed_pass_fresh_and_speculative(dev):
   assert run_layer(dev, rng, [1, 37, 5, 1, 128, 5, 2, 1], fresh=(1, 3), speculative=(2, 5)) < TOL
 
 
+def test_gdn_preparation_across_row_groups(dev):
+  """Query boundaries at every place of the eight-row groups the preparation kernel works in, and a ragged last group."""
+  rng = np.random.default_rng(8)
+  assert run_layer(dev, rng, [3, 1, 2, 9, 8, 17, 7, 4], fresh=(0, 4), speculative=(3, 7)) < 1e-4
+
+
 def test_gdn_single_query_edge_lengths(dev):
   rng = np.random.default_rng(4)
   for lengths in ([1], [2], [3], [4], [512]):
