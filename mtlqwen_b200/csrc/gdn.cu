@@ -44,7 +44,7 @@ __device__ __forceinline__ const infdev_query& query_of_row(const infdev_query* 
 constexpr int kConvRows = 8, kGateRows = 8, kGateHeads = 8;
 constexpr int kConvChannels = 4 * 256;  // per CTA
 
-__global__ void __launch_bounds__(256) gdn_prepare_kernel(const float* x, const float* wBeta, const float* wAlpha, const float* A, const float* dt,
+__global__ void __launch_bounds__(256, 2) gdn_prepare_kernel(const float* x, const float* wBeta, const float* wAlpha, const float* A, const float* dt,
                                                           const float* mixed, const float* w, const infdev_query* queries, int rows, int gateBlocks,
                                                           uint64_t stateOffset, uint64_t stateBytes, float* q, float* k, float* v, float* beta,
                                                           float* g) {
@@ -416,31 +416,187 @@ __global__ void __launch_bounds__(256, 2) delta_rule_kernel(const float* q, cons
 }
 
 // ---- chunked form for long prefill queries -----------------------------------------------------------
-// Replaces delta_rule_prefill (delta_rule.metal:19-253): 16 tokens per step instead of one. With S0 the state
-// before the chunk, d_t the decay of token t, G_t = d_0 ... d_t and R[t][i] = G_t / G_i, the recurrence of
-// delta_rule_kernel unrolls to
-//   delta_t = beta_t * (v_t - G_t * S0^T k_t - sum_{i<t} R[t][i] (k_i . k_t) delta_i)        (a unit lower-triangular system)
-//   o_t     = G_t * S0^T q_t + sum_{i<=t} R[t][i] (k_i . q_t) delta_i
-//   S       = G_15 * S0 + sum_i (G_15 / G_i) k_i delta_i^T
-// All in fp32 on the CUDA cores, like the sequential kernel (so both agree to rounding): the two S0 products cost what
-// 16 sequential steps cost, but a chunk needs 5 block-wide barriers instead of 64, which is what bounds a prefill query
-// (one CTA per head, 128 dependent steps per pass).
-// grid (32 value heads, queries), 256 threads, same state ownership as delta_rule_kernel; serves the non-speculative
-// queries of at least `chunkedFrom` tokens. A last chunk of fewer than 16 tokens is padded with tokens of beta = 0,
-// k = q = 0 and decay 1, which change nothing.
-constexpr int kChunk = 16;
-struct ChunkShared {
-  float k[kChunk][kHeadDim + 4], q[kChunk][kHeadDim + 4], v[kChunk][kHeadDim];  // rows of k, q padded: column reads over 16 rows hit 16 banks
-  float partialK[kChunk][8][kHeadDim], partialQ[kChunk][8][kHeadDim];  // per-warp partial S0^T k_t, S0^T q_t
-  float ks[kChunk][kHeadDim], qs[kChunk][kHeadDim];                    // S0^T k_t, S0^T q_t
-  float u[kChunk][kHeadDim], o[kChunk][kHeadDim];                      // (G_15 / G_t) delta_t, o_t
-  float kk[kChunk][kChunk], qk[kChunk][kChunk];                        // R[t][i] (k_i . k_t), R[t][i] (k_i . q_t)
-  float cumulative[kChunk], beta[kChunk];                              // log G_t, beta_t
+// Replaces delta_rule_prefill (delta_rule.metal:19-253): 16 tokens per step instead of one. With S the state before the
+// chunk, G_t = d_0 ... d_t the cumulated decay, R[t][i] = G_t / G_i and the unit lower-triangular
+// A[t][i] = beta_t R[t][i] (k_t . k_i) for i < t, the recurrence of delta_rule_kernel unrolls to
+//   delta  = A^-1 rhs,   rhs_t = beta_t * (v_t - G_t * S^T k_t)
+//   o_t    = G_t * S^T q_t + sum_{i<=t} R[t][i] (q_t . k_i) delta_i
+//   S      = G_15 * S + sum_i (G_15 / G_i) k_i delta_i^T
+// grid (32 value heads, queries), 8 + 4 warps; serves the non-speculative queries of at least `chunkedFrom` tokens. A last
+// chunk of fewer than 16 tokens is padded with tokens of beta = 0, k = q = v = 0 and decay 1, which change nothing.
+//
+// A query is a chain of chunks per head, so what counts is the time of one chunk. Everything that does not depend on S - the
+// normalised keys and queries, the gates, A^-1 and the weights of the second sum - is prepared by four warps of their own,
+// a chunk or two ahead, in two shared-memory buffers. The eight others hold S^T in registers, 16 value columns each: a warp
+// needs nothing from its neighbours until the norm of the output, because a value column's recurrence is its own. All
+// products run on the tensor cores; a warp's accumulators (value column x key dim, or x token) are at the same time, as they
+// lie in its registers, the A operand of the next product. Operands are split into fp16 hi + lo after scaling by a power of
+// two (fixed for keys and queries, by the largest value of the warp for S, rhs and delta), and the three products that matter
+// (hi hi, lo hi, hi lo) are accumulated in fp32: 22 bits of every operand, the error against the sequential fp32 form stays at its own rounding.
+// 156 HMMA per warp and chunk at 512 multiply-adds per clock and SM bound it to 2.7 us per chunk; the form before this one,
+// fp32 FMAs with eight partial sums per product through shared memory, took 19 us.
+constexpr int kChunk = 16, kComputeWarps = 8, kPrepareWarps = 4;
+constexpr int kChunkThreads = (kComputeWarps + kPrepareWarps) * kWarp;
+constexpr float kKeyUnit = 256.f, kSolveUnit = 16.f, kMixUnit = 256.f;  // fixed scales of the fp16 operands
+struct ChunkBuffer {
+  __half k[2][kChunk][kHeadDim + 8], q[2][kChunk][kHeadDim + 8];  // hi, lo of kKeyUnit x the normalised rows
+  __half solve[2][kChunk][kChunk + 8], mix[2][kChunk][kChunk + 8];  // hi, lo of kSolveUnit x A^-1 and kMixUnit x R (q . k)
+  float decay[kChunk], tail[kChunk], beta[kChunk];                // G_t, G_15 / G_t, beta_t
 };
+struct ChunkShared {
+  ChunkBuffer buffer[2];
+  float cumulative[kChunk], gateBeta[kChunk];  // of the chunk being prepared
+  float system[kChunk][kChunk + 1];
+  float squares[2][kComputeWarps][kChunk];
+};
+// named barriers: 1, 2 buffer filled; 3, 4 buffer free; 5 the preparing warps; 6 the computing warps
+__device__ __forceinline__ void chunk_ldmatrix(uint32_t (&r)[4], const __half* address) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(address)) : "memory");
+}
+__device__ __forceinline__ void chunk_ldmatrix_trans(uint32_t (&r)[4], const __half* address) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(smem_u32(address))
+               : "memory");
+}
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
+  hi = pack_half2(a, b);
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+  lo = pack_half2(a - f.x, b - f.y);
+}
+// 2^n that brings the warp's largest magnitude into [512, 1024), and 2^-n
+__device__ __forceinline__ float2 warp_unit(float largest) {
+  largest = warp_max(largest);
+  const int field = min(254, max(1, 263 - int(__float_as_uint(largest) >> 23)));
+  return make_float2(__uint_as_float(uint32_t(field) << 23), __uint_as_float(uint32_t(max(1, 254 - field)) << 23));
+}
+// The two 16 x 8 accumulators of 16 x 16 values (C fragments) x unit as the A operand, hi and lo.
+__device__ __forceinline__ void split_tile(const float (&c0)[4], const float (&c1)[4], float unit, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
+  split_pair(c0[0] * unit, c0[1] * unit, hi[0], lo[0]);
+  split_pair(c0[2] * unit, c0[3] * unit, hi[1], lo[1]);
+  split_pair(c1[0] * unit, c1[1] * unit, hi[2], lo[2]);
+  split_pair(c1[2] * unit, c1[3] * unit, hi[3], lo[3]);
+}
+// d0, d1 += A x B for the two n-tiles of B fragments bHi, bLo, as hi hi + lo hi + hi lo.
+__device__ __forceinline__ void mma_three(float (&d0)[4], float (&d1)[4], const uint32_t (&hi)[4], const uint32_t (&lo)[4], const uint32_t (&bHi)[4],
+                                          const uint32_t (&bLo)[4]) {
+  mma_16816(d0, hi, bHi[0], bHi[1]), mma_16816(d1, hi, bHi[2], bHi[3]);
+  mma_16816(d0, lo, bHi[0], bHi[1]), mma_16816(d1, lo, bHi[2], bHi[3]);
+  mma_16816(d0, hi, bLo[0], bLo[1]), mma_16816(d1, hi, bLo[2], bLo[3]);
+}
 
-__global__ void __launch_bounds__(256) delta_rule_chunked_kernel(const float* q, const float* k, const float* v, const float* g, const float* beta,
-                                                                 const float* z, const float* normWeight, const infdev_query* queries,
-                                                                 uint64_t stateOffset, float* out, uint32_t chunkedFrom) {
+// The four preparing warps: chunk after chunk into the two buffers.
+__device__ __forceinline__ void chunk_prepare(ChunkShared& sh, const infdev_query& info, const float* q, const float* k, const float* g, const float* beta,
+                                              int head) {
+  const int warp = (threadIdx.x >> 5) - kComputeWarps, lane = threadIdx.x & 31, keyHead = head % kKeyHeads;
+  const int tokenOfB = (lane & 7) + 8 * (lane >> 4), dimOfB = 8 * ((lane >> 3) & 1);  // ldmatrix rows of a B operand stored [n][k]
+  float4 nextQ[4], nextK[4];
+  float nextG = 0.f, nextBeta = 0.f;
+  auto load = [&](uint32_t first) {  // warp w: tokens 4w .. 4w + 3
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t token = first + 4 * warp + j;
+      nextQ[j] = nextK[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (token < info.count) {
+        const size_t at = (size_t(info.start + token) * kKeyHeads + keyHead) * kHeadDim + 4 * lane;
+        nextQ[j] = *reinterpret_cast<const float4*>(q + at), nextK[j] = *reinterpret_cast<const float4*>(k + at);
+      }
+    }
+    if (warp == 0) {
+      const bool live = lane < kChunk && first + lane < info.count;
+      nextG = live ? g[size_t(info.start + first + lane) * kValueHeads + head] : 0.f;
+      nextBeta = live ? beta[size_t(info.start + first + lane) * kValueHeads + head] : 0.f;
+    }
+  };
+  load(0);
+  uint32_t step = 0;
+  for (uint32_t first = 0; first < info.count; first += kChunk, ++step) {
+    ChunkBuffer& out = sh.buffer[step & 1];
+    if (step >= 2)
+      named_barrier(3 + (step & 1), kChunkThreads);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float4 a = nextQ[j], b = nextK[j];
+      const float qq = warp_sum(a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w), kk = warp_sum(b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w);
+      const float qn = rsqrtf(qq + 1.0e-6f) * 0.08838834764831845f * kKeyUnit, kn = rsqrtf(kk + 1.0e-6f) * kKeyUnit;
+      uint2 hi, lo;
+      split_pair(a.x * qn, a.y * qn, hi.x, lo.x), split_pair(a.z * qn, a.w * qn, hi.y, lo.y);
+      *reinterpret_cast<uint2*>(&out.q[0][4 * warp + j][4 * lane]) = hi, *reinterpret_cast<uint2*>(&out.q[1][4 * warp + j][4 * lane]) = lo;
+      split_pair(b.x * kn, b.y * kn, hi.x, lo.x), split_pair(b.z * kn, b.w * kn, hi.y, lo.y);
+      *reinterpret_cast<uint2*>(&out.k[0][4 * warp + j][4 * lane]) = hi, *reinterpret_cast<uint2*>(&out.k[1][4 * warp + j][4 * lane]) = lo;
+    }
+    if (warp == 0) {
+      float running = 0.f, mine = 0.f;
+#pragma unroll
+      for (int t = 0; t < kChunk; ++t) {
+        running += __shfl_sync(0xffffffffu, nextG, t);
+        mine = lane == t ? running : mine;
+      }
+      if (lane < kChunk) {
+        sh.cumulative[lane] = mine, sh.gateBeta[lane] = nextBeta;
+        out.decay[lane] = expf(mine), out.tail[lane] = expf(running - mine), out.beta[lane] = nextBeta;
+      }
+    }
+    load(first + kChunk);  // past the end: zeros
+    named_barrier(5, kPrepareWarps * kWarp);
+    if (warp < 2) {
+      // warp 0: k . k and the inverse of the triangular system; warp 1: q . k
+      float dot[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, low[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      const auto& left = warp == 0 ? out.k : out.q;
+#pragma unroll
+      for (int s = 0; s < kHeadDim / 16; ++s) {
+        uint32_t hi[4], lo[4], bHi[4], bLo[4];
+        chunk_ldmatrix(hi, &left[0][lane & 15][16 * s + 8 * (lane >> 4)]);
+        chunk_ldmatrix(lo, &left[1][lane & 15][16 * s + 8 * (lane >> 4)]);
+        chunk_ldmatrix(bHi, &out.k[0][tokenOfB][16 * s + dimOfB]);
+        chunk_ldmatrix(bLo, &out.k[1][tokenOfB][16 * s + dimOfB]);
+        mma_16816(dot[0], hi, bHi[0], bHi[1]), mma_16816(dot[1], hi, bHi[2], bHi[3]);
+        mma_16816(low[0], lo, bHi[0], bHi[1]), mma_16816(low[1], lo, bHi[2], bHi[3]);
+        mma_16816(low[0], hi, bLo[0], bLo[1]), mma_16816(low[1], hi, bLo[2], bLo[3]);
+      }
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int t = (lane >> 2) + 8 * (e >> 1), i = 8 * n + 2 * (lane & 3) + (e & 1);
+          const float value = (dot[n][e] + low[n][e]) * (1.0f / (kKeyUnit * kKeyUnit)) * expf(sh.cumulative[t] - sh.cumulative[i]);
+          if (warp == 0) {
+            sh.system[t][i] = i < t ? value * sh.gateBeta[t] : 0.f;
+          } else {
+            const float scaled = i <= t ? value * kMixUnit : 0.f;
+            const __half hi = __float2half_rn(scaled);
+            out.mix[0][t][i] = hi, out.mix[1][t][i] = __float2half_rn(scaled - __half2float(hi));
+          }
+        }
+      if (warp == 0) {
+        __syncwarp();
+        // column `lane` of the inverse by forward substitution (lanes 16 .. 31 repeat columns 0 .. 15)
+        const int column = lane & 15;
+        float x[kChunk];
+#pragma unroll
+        for (int t = 0; t < kChunk; ++t)
+          x[t] = t == column ? 1.f : 0.f;
+#pragma unroll
+        for (int i = 0; i < kChunk; ++i)
+#pragma unroll
+          for (int t = i + 1; t < kChunk; ++t)
+            x[t] = fmaf(-sh.system[t][i], x[i], x[t]);
+        if (lane < kChunk)
+#pragma unroll
+          for (int t = 0; t < kChunk; ++t) {
+            const float scaled = x[t] * kSolveUnit;
+            const __half hi = __float2half_rn(scaled);
+            out.solve[0][t][column] = hi, out.solve[1][t][column] = __float2half_rn(scaled - __half2float(hi));
+          }
+      }
+    }
+    named_barrier_arrive(1 + (step & 1), kChunkThreads);
+  }
+}
+
+__global__ void __launch_bounds__(kChunkThreads, 1)
+    delta_rule_chunked_kernel(const float* q, const float* k, const float* v, const float* g, const float* beta, const float* z, const float* normWeight,
+                              const infdev_query* queries, uint64_t stateOffset, float* out, uint32_t chunkedFrom) {
   pdl_launch_dependents();
   pdl_wait();
   const infdev_query info = queries[blockIdx.y];
@@ -448,152 +604,171 @@ __global__ void __launch_bounds__(256) delta_rule_chunked_kernel(const float* q,
     return;
   extern __shared__ __align__(16) uint8_t chunkRaw[];
   ChunkShared& sh = *reinterpret_cast<ChunkShared*>(chunkRaw);
-  const int head = blockIdx.x, keyHead = head % kKeyHeads, tid = threadIdx.x, part = tid >> 5, lane = tid & 31;
-
-  float4 S[16];
-  if (info.previous) {
-    const float4* src = reinterpret_cast<const float4*>(info.previous + stateOffset) + size_t(head) * kHeadDim * 32;
-#pragma unroll
-    for (int i = 0; i < 16; ++i)
-      S[i] = src[(part + 8 * i) * 32 + lane];
-  } else {
-#pragma unroll
-    for (int i = 0; i < 16; ++i)
-      S[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int head = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp >= kComputeWarps) {
+    chunk_prepare(sh, info, q, k, g, beta, head);
+    return;
   }
-
-  for (uint32_t first = 0; first < info.count; first += kChunk) {
-    const uint32_t live = min(uint32_t(kChunk), info.count - first);
-    // (a) normalised q (scaled by 1/sqrt(128)) and k, raw v, gates: warp w prepares tokens 2w and 2w+1
+  const int row = lane >> 2, t2 = 2 * (lane & 3), column = 16 * warp + row;  // value columns `column` and `column` + 8
+  const int tokenOfB = (lane & 7) + 8 * (lane >> 4), dimOfB = 8 * ((lane >> 3) & 1);
+  // S^T x unit: tile j holds key dims 8j + t2, + 1 of the two value columns
+  float S[kHeadDim / 8][4], inverse = 1.f;  // inverse of unit
+  const size_t state = size_t(head) * kHeadDim * kHeadDim + column;
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const uint32_t t = 2 * part + j;
-      float4 qv = make_float4(0.f, 0.f, 0.f, 0.f), kv = qv, vv = qv;
-      if (t < live) {
-        const size_t row = info.start + first + t;
-        qv = *reinterpret_cast<const float4*>(q + (row * kKeyHeads + keyHead) * kHeadDim + 4 * lane);
-        kv = *reinterpret_cast<const float4*>(k + (row * kKeyHeads + keyHead) * kHeadDim + 4 * lane);
-        vv = *reinterpret_cast<const float4*>(v + (row * kValueHeads + head) * kHeadDim + 4 * lane);
-      }
-      const float qq = warp_sum(qv.x * qv.x + qv.y * qv.y + qv.z * qv.z + qv.w * qv.w);
-      const float kq = warp_sum(kv.x * kv.x + kv.y * kv.y + kv.z * kv.z + kv.w * kv.w);
-      const float qn = rsqrtf(qq + 1.0e-6f) * 0.08838834764831845f, kn = rsqrtf(kq + 1.0e-6f);
-      *reinterpret_cast<float4*>(&sh.q[t][4 * lane]) = make_float4(qv.x * qn, qv.y * qn, qv.z * qn, qv.w * qn);
-      *reinterpret_cast<float4*>(&sh.k[t][4 * lane]) = make_float4(kv.x * kn, kv.y * kn, kv.z * kn, kv.w * kn);
-      *reinterpret_cast<float4*>(&sh.v[t][4 * lane]) = vv;
-    }
-    if (tid == 0) {
-      float running = 0.f;
-      for (uint32_t t = 0; t < kChunk; ++t) {
-        const size_t row = info.start + first + t;
-        running += t < live ? g[row * kValueHeads + head] : 0.f;
-        sh.cumulative[t] = running;
-        sh.beta[t] = t < live ? beta[row * kValueHeads + head] : 0.f;
-      }
-    }
-    __syncthreads();
-    // (b) per-warp partial products of the chunk's keys and queries with S0, and the token-by-token dot products
-#pragma unroll 2
-    for (int t = 0; t < kChunk; ++t) {
-      float4 pk = make_float4(0.f, 0.f, 0.f, 0.f), pq = pk;
+  for (int j = 0; j < kHeadDim / 8; ++j)
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const float kv = sh.k[t][part + 8 * i], qv = sh.q[t][part + 8 * i];
-        pk.x = fmaf(S[i].x, kv, pk.x), pk.y = fmaf(S[i].y, kv, pk.y), pk.z = fmaf(S[i].z, kv, pk.z), pk.w = fmaf(S[i].w, kv, pk.w);
-        pq.x = fmaf(S[i].x, qv, pq.x), pq.y = fmaf(S[i].y, qv, pq.y), pq.z = fmaf(S[i].z, qv, pq.z), pq.w = fmaf(S[i].w, qv, pq.w);
+    for (int e = 0; e < 4; ++e)
+      S[j][e] = info.previous ? reinterpret_cast<const float*>(info.previous + stateOffset)[state + (8 * j + t2 + (e & 1)) * kHeadDim + 8 * (e >> 1)] : 0.f;
+  float weight[2] = {0.f, 0.f};
+  if (z)
+    weight[0] = normWeight[column], weight[1] = normWeight[column + 8];
+  // element (n, e) of a token tile: token 8n + t2 + e % 2, value column + 8 (e / 2)
+  float value[2][4], gate[2][4];
+  auto load = [&](float (&into)[2][4], const float* from, uint32_t first) {
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint32_t token = first + 8 * n + t2 + (e & 1);
+        into[n][e] = token < info.count ? from[(size_t(info.start + token) * kValueHeads + head) * kHeadDim + column + 8 * (e >> 1)] : 0.f;
       }
-      *reinterpret_cast<float4*>(&sh.partialK[t][part][4 * lane]) = pk;
-      *reinterpret_cast<float4*>(&sh.partialQ[t][part][4 * lane]) = pq;
+  };
+  load(value, v, 0);
+  uint32_t step = 0;
+  for (uint32_t first = 0; first < info.count; first += kChunk, ++step) {
+    const ChunkBuffer& in = sh.buffer[step & 1];
+    if (z)
+      load(gate, z, first);
+    float largest = 0.f;
+#pragma unroll
+    for (int j = 0; j < kHeadDim / 8; ++j)
+      largest = fmaxf(fmaxf(fmaxf(largest, fabsf(S[j][0])), fmaxf(fabsf(S[j][1]), fabsf(S[j][2]))), fabsf(S[j][3]));
+    const float2 stateUnit = warp_unit(largest);
+    named_barrier(1 + (step & 1), kChunkThreads);
+    // S^T k and S^T q of the 16 tokens
+    float ks[2][4], qs[2][4];
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        ks[n][e] = qs[n][e] = 0.f;
+#pragma unroll
+    for (int s = 0; s < kHeadDim / 16; ++s) {
+      uint32_t hi[4], lo[4], bHi[4], bLo[4];
+      split_tile(S[2 * s], S[2 * s + 1], stateUnit.x, hi, lo);
+      chunk_ldmatrix(bHi, &in.k[0][tokenOfB][16 * s + dimOfB]);
+      chunk_ldmatrix(bLo, &in.k[1][tokenOfB][16 * s + dimOfB]);
+      mma_three(ks[0], ks[1], hi, lo, bHi, bLo);
+      chunk_ldmatrix(bHi, &in.q[0][tokenOfB][16 * s + dimOfB]);
+      chunk_ldmatrix(bLo, &in.q[1][tokenOfB][16 * s + dimOfB]);
+      mma_three(qs[0], qs[1], hi, lo, bHi, bLo);
     }
+    const float productUnit = stateUnit.y * inverse * (1.0f / kKeyUnit);
+    float decay[2][2];
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        decay[n][e] = in.decay[8 * n + t2 + e];
+    // rhs, delta = A^-1 rhs
+    float rhs[2][4], delta[2][4];
+    largest = 0.f;
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        rhs[n][e] = in.beta[8 * n + t2 + (e & 1)] * (value[n][e] - decay[n][e & 1] * (ks[n][e] * productUnit));
+        largest = fmaxf(largest, fabsf(rhs[n][e]));
+        delta[n][e] = 0.f;
+      }
+    load(value, v, first + kChunk);  // of the next chunk
+    uint32_t hi[4], lo[4], bHi[4], bLo[4];
+    float2 scale = warp_unit(largest);
+    split_tile(rhs[0], rhs[1], scale.x, hi, lo);
+    chunk_ldmatrix(bHi, &in.solve[0][tokenOfB][dimOfB]);
+    chunk_ldmatrix(bLo, &in.solve[1][tokenOfB][dimOfB]);
+    mma_three(delta[0], delta[1], hi, lo, bHi, bLo);
+    // outputs, and the state's update with (G_15 / G_i) delta_i
+    float mixed[2][4], update[2][4];
+    largest = 0.f;
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        delta[n][e] *= scale.y * (1.0f / kSolveUnit);
+        update[n][e] = delta[n][e] * in.tail[8 * n + t2 + (e & 1)];
+        largest = fmaxf(largest, fmaxf(fabsf(delta[n][e]), fabsf(update[n][e])));
+        mixed[n][e] = 0.f;
+      }
+    scale = warp_unit(largest);
+    split_tile(delta[0], delta[1], scale.x, hi, lo);
+    chunk_ldmatrix(bHi, &in.mix[0][tokenOfB][dimOfB]);
+    chunk_ldmatrix(bLo, &in.mix[1][tokenOfB][dimOfB]);
+    mma_three(mixed[0], mixed[1], hi, lo, bHi, bLo);
+    split_tile(update[0], update[1], scale.x, hi, lo);
     {
-      const int t = tid >> 4, i = tid & 15;  // one (t, i) pair per thread
-      float kk = 0.f, qk = 0.f;
-      if (i <= t) {
-#pragma unroll 8
-        for (int d = 0; d < kHeadDim; d += 4) {
-          const float4 a = *reinterpret_cast<const float4*>(&sh.k[i][d]), b = *reinterpret_cast<const float4*>(&sh.k[t][d]),
-                       c = *reinterpret_cast<const float4*>(&sh.q[t][d]);
-          kk += a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w;
-          qk += a.x * c.x + a.y * c.y + a.z * c.z + a.w * c.w;
+      const float rescale = in.decay[kChunk - 1] * scale.x * kKeyUnit * inverse;
+#pragma unroll
+      for (int j = 0; j < kHeadDim / 8; ++j)
+        S[j][0] *= rescale, S[j][1] *= rescale, S[j][2] *= rescale, S[j][3] *= rescale;
+      inverse = scale.y * (1.0f / kKeyUnit);
+    }
+#pragma unroll
+    for (int s = 0; s < kHeadDim / 16; ++s) {
+      chunk_ldmatrix_trans(bHi, &in.k[0][lane & 15][16 * s + 8 * (lane >> 4)]);
+      chunk_ldmatrix_trans(bLo, &in.k[1][lane & 15][16 * s + 8 * (lane >> 4)]);
+      mma_three(S[2 * s], S[2 * s + 1], hi, lo, bHi, bLo);
+    }
+    named_barrier_arrive(3 + (step & 1), kChunkThreads);  // the buffer may be refilled
+    // o, its gated norm over the head's 128 columns (gated_rms_norm_128), and the store
+    float o[2][4], squares[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        o[n][e] = decay[n][e & 1] * (qs[n][e] * productUnit) + mixed[n][e] * (scale.y * (1.0f / kMixUnit));
+        squares[n][e & 1] = fmaf(o[n][e], o[n][e], squares[n][e & 1]);
+      }
+    if (z) {
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          float sum = squares[n][e];
+#pragma unroll
+          for (int m = 4; m < 32; m <<= 1)
+            sum += __shfl_xor_sync(0xffffffffu, sum, m);
+          if (row == 0)
+            sh.squares[step & 1][warp][8 * n + t2 + e] = sum;
         }
-        const float ratio = expf(sh.cumulative[t] - sh.cumulative[i]);
-        kk *= ratio, qk *= ratio;
-      }
-      sh.kk[t][i] = i < t ? kk : 0.f;
-      sh.qk[t][i] = i <= t ? qk : 0.f;
-    }
-    __syncthreads();
-    // (c) sum the eight partials: 2048 values each for ks and qs, eight per thread
+      named_barrier(6, kComputeWarps * kWarp);  // two sets of sums in turn: nobody is two chunks behind
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int at = tid + 256 * j, t = at >> 7, d = at & 127;
-      float a = 0.f, b = 0.f;
+      for (int n = 0; n < 2; ++n)
 #pragma unroll
-      for (int w = 0; w < 8; ++w) {
-        a += sh.partialK[t][w][d];
-        b += sh.partialQ[t][w][d];
-      }
-      sh.ks[t][d] = a;
-      sh.qs[t][d] = b;
-    }
-    __syncthreads();
-    // (d) one thread per value column: forward substitution for delta, then the outputs
-    if (tid < kHeadDim) {
-      const float last = sh.cumulative[kChunk - 1];
-      float delta[kChunk];
+        for (int e = 0; e < 2; ++e) {
+          float sum = 0.f;
 #pragma unroll
-      for (int t = 0; t < kChunk; ++t) {
-        const float decay = expf(sh.cumulative[t]);
-        float r = sh.v[t][tid] - decay * sh.ks[t][tid], o = decay * sh.qs[t][tid];
-#pragma unroll
-        for (int i = 0; i < t; ++i) {
-          r = fmaf(-sh.kk[t][i], delta[i], r);
-          o = fmaf(sh.qk[t][i], delta[i], o);
+          for (int w = 0; w < kComputeWarps; ++w)
+            sum += sh.squares[step & 1][w][8 * n + t2 + e];
+          const float norm = rsqrtf(sum / float(kHeadDim) + 1.0e-6f);
+          o[n][e] = o[n][e] * norm * weight[0] * silu_f(gate[n][e]);
+          o[n][e + 2] = o[n][e + 2] * norm * weight[1] * silu_f(gate[n][e + 2]);
         }
-        delta[t] = r * sh.beta[t];
-        o = fmaf(sh.qk[t][t], delta[t], o);
-        sh.u[t][tid] = delta[t] * expf(last - sh.cumulative[t]);
-        sh.o[t][tid] = o;
-      }
-    }
-    __syncthreads();
-    // (e) new state, and the outputs of the chunk through the gated norm: warp w writes tokens 2w and 2w+1
-    {
-      const float decay = expf(sh.cumulative[kChunk - 1]);
-#pragma unroll
-      for (int i = 0; i < 16; ++i)
-        S[i].x *= decay, S[i].y *= decay, S[i].z *= decay, S[i].w *= decay;
-#pragma unroll 4
-      for (int t = 0; t < kChunk; ++t) {
-        const float4 u = *reinterpret_cast<const float4*>(&sh.u[t][4 * lane]);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float kv = sh.k[t][part + 8 * i];
-          S[i].x = fmaf(kv, u.x, S[i].x), S[i].y = fmaf(kv, u.y, S[i].y), S[i].z = fmaf(kv, u.z, S[i].z), S[i].w = fmaf(kv, u.w, S[i].w);
-        }
-      }
     }
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const uint32_t t = 2 * part + j;
-      if (t < live) {
-        const size_t at = ((info.start + first + t) * kValueHeads + head) * kHeadDim + 4 * lane;
-        float4 o = *reinterpret_cast<const float4*>(&sh.o[t][4 * lane]);
-        if (z) {  // gated_rms_norm_128
-          const float scale = rsqrtf(warp_sum(o.x * o.x + o.y * o.y + o.z * o.z + o.w * o.w) / float(kHeadDim) + 1.0e-6f);
-          const float4 w = *reinterpret_cast<const float4*>(normWeight + 4 * lane), gate = *reinterpret_cast<const float4*>(z + at);
-          o = make_float4(o.x * scale * w.x * silu_f(gate.x), o.y * scale * w.y * silu_f(gate.y), o.z * scale * w.z * silu_f(gate.z),
-                          o.w * scale * w.w * silu_f(gate.w));
-        }
-        *reinterpret_cast<float4*>(out + at) = o;
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint32_t token = first + 8 * n + t2 + (e & 1);
+        if (token < info.count)
+          out[(size_t(info.start + token) * kValueHeads + head) * kHeadDim + column + 8 * (e >> 1)] = o[n][e];
       }
-    }
-    __syncthreads();  // the chunk's shared arrays are rewritten by the next chunk
   }
-  float4* dst = reinterpret_cast<float4*>(info.next + stateOffset) + size_t(head) * kHeadDim * 32;
 #pragma unroll
-  for (int i = 0; i < 16; ++i)
-    dst[(part + 8 * i) * 32 + lane] = S[i];
+  for (int j = 0; j < kHeadDim / 8; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      reinterpret_cast<float*>(info.next + stateOffset)[state + (8 * j + t2 + (e & 1)) * kHeadDim + 8 * (e >> 1)] = S[j][e] * inverse;
 }
 
 }  // namespace
@@ -619,7 +794,7 @@ cudaError_t delta_rule_launch(const float* q, const float* k, const float* v, co
     static PerDeviceOnce configured;
     if (cudaError_t e = configure_shared_memory(delta_rule_chunked_kernel, sizeof(ChunkShared), configured))
       return e;
-    launch_kernel(delta_rule_chunked_kernel, dim3(kValueHeads, unsigned(queryCount)), 256, sizeof(ChunkShared), stream, q, k, v, g, beta, z, normWeight,
+    launch_kernel(delta_rule_chunked_kernel, dim3(kValueHeads, unsigned(queryCount)), kChunkThreads, sizeof(ChunkShared), stream, q, k, v, g, beta, z, normWeight,
                   queries, stateOffset, out, chunkedFrom);
   }
   launch_kernel(delta_rule_kernel<false>, dim3(kValueHeads, unsigned(queryCount)), 256, 0, stream, q, k, v, g, beta, z, normWeight, queries, stateOffset,
