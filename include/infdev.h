@@ -85,8 +85,9 @@ int infdev_event_record(infdev_ctx* ctx, void* event);
 float infdev_event_elapsed_ms(infdev_ctx* ctx, void* start, void* stop);
 /* Which quantised-linear kernel serves Q4_K matrices with n % 128 == 0 and k % 2048 == 0 when a launch has more than 8
  * activation rows (prefill chunks, speculative rows): 1 (default) = the tcgen05 / TMEM GEMM, 0 = the GEMV kernels in
- * slices of 8 rows, which compute every activation row on its own. Environment: INFENG_UMMA. With 0, infdev_attention also
- * treats every row on its own: otherwise, in a pass in which some query has several rows, up to 16 rows of a query share the
+ * slices of 8 rows, which compute every activation row on its own. Likewise for the other block types, whose launches of more
+ * than 8 rows decode a weight once for up to 40 rows (1) or go through the GEMV in slices (0). Environment: INFENG_UMMA. With 0,
+ * infdev_attention also treats every row on its own: otherwise, in a pass in which some query has several rows, up to 16 rows of a query share the
  * reading of K and V, and the rounding of a row's sums depends on how its query was cut into passes. */
 int infdev_set_umma(infdev_ctx* ctx, int enabled);
 /* Activation split of the fp16 tensor-core GEMV: 2 = hi+lo fp16 (fp32-accurate, default), 1 = hi only. */

@@ -24,7 +24,7 @@
 //  * Every mbarrier wait is bounded; on a timeout the kernel raises an abort flag, records a status code
 //    and all roles leave their loops.
 #include <type_traits>
-#include "common.cuh"
+#include "gemv_units.cuh"
 #include "kernels.h"
 
 namespace infdev {
@@ -88,10 +88,6 @@ template <class Q, int NMAT, int XSPLIT> constexpr int stage_count() {
 
 template <class Q, int NMAT, int XSPLIT> constexpr size_t smem_bytes() {
   return fixed_bytes<Q, NMAT, XSPLIT>() + size_t(stage_count<Q, NMAT, XSPLIT>()) * stage_bytes<Q>();
-}
-
-__device__ __forceinline__ uint32_t lds_u32_unaligned(const uint8_t* p) {
-  return uint32_t(*reinterpret_cast<const uint16_t*>(p)) | (uint32_t(*reinterpret_cast<const uint16_t*>(p + 2)) << 16);
 }
 
 // ---- Q4_K: one 16-row x 256-k unit -------------------------------------------------------------
@@ -190,191 +186,19 @@ __device__ __forceinline__ void q4k_unit(uint32_t pA, uint32_t pB, int t, uint32
   total[3] += xs.y * (dB.x * ((acc[0][3] + acc[1][3]) + (acc[2][3] + acc[3][3])) - dB.y * accm[3]);
 }
 
-// ---- the formats whose sub-blocks are 32 wide ------------------------------------------------------------------
-// Fragment of one MMA from four quant bytes of the rows g and g+8: (base + byte) - base in fp16, base = 1024 + bias, exact.
-__device__ __forceinline__ void byte_fragment(uint32_t (&a)[4], uint32_t bytesA, uint32_t bytesB, uint32_t bias2) {
-  a[0] = hsub2_u32(__byte_perm(bytesA, 0x64u, 0x4140), bias2);
-  a[1] = hsub2_u32(__byte_perm(bytesB, 0x64u, 0x4140), bias2);
-  a[2] = hsub2_u32(__byte_perm(bytesA, 0x64u, 0x4342), bias2);
-  a[3] = hsub2_u32(__byte_perm(bytesB, 0x64u, 0x4342), bias2);
-}
-// Both MMAs (hi, lo) of fragment gi.
-template <int XSPLIT> __device__ __forceinline__ void mma_split(float (&acc)[4], const uint32_t (&a)[4], const uint2* xhi, const uint2* xlo, int at) {
-  uint2 b = xhi[at];
-  mma_16816(acc, a, b.x, b.y);
-  if (XSPLIT == 2) {
-    b = xlo[at];
-    mma_16816(acc, a, b.x, b.y);
+// The activations of one super-block as the units of gemv_units.cuh read them: one tile of eight rows, hi and lo fragments apart.
+template <int XSPLIT> struct StagedRows {
+  const uint2 *hi, *lo;  // fragment 0, this lane's slot
+  uint2 minSums;
+  float2 powers;
+  static constexpr bool kSplit = XSPLIT == 2;
+  __device__ __forceinline__ uint4 fragment(int i, int) const {
+    const uint2 h = hi[i * 32], l = XSPLIT == 2 ? lo[i * 32] : make_uint2(0u, 0u);
+    return make_uint4(h.x, h.y, l.x, l.y);
   }
-}
-__device__ __forceinline__ void add_scaled(float (&sum)[4], float sA, float sB, const float (&acc)[4]) {
-  sum[0] = fmaf(sA, acc[0], sum[0]), sum[1] = fmaf(sA, acc[1], sum[1]), sum[2] = fmaf(sB, acc[2], sum[2]), sum[3] = fmaf(sB, acc[3], sum[3]);
-}
-__device__ __forceinline__ void add_total(float (&total)[4], float2 xs, const float (&sum)[4]) {
-  total[0] = fmaf(xs.x, sum[0], total[0]), total[1] = fmaf(xs.y, sum[1], total[1]);
-  total[2] = fmaf(xs.x, sum[2], total[2]), total[3] = fmaf(xs.y, sum[3], total[3]);
-}
-__device__ __forceinline__ uint32_t lds_u32(const uint8_t* p) { return *reinterpret_cast<const uint32_t*>(p); }
-__device__ __forceinline__ float byte_of(uint32_t word, int i) { return float(__byte_perm(word, 0u, 0x4440 + i)); }
-
-// Q5_K (quant_linear.metal:50-67): fp16 d, dmin | 6-bit scales and mins | qh[32] | qs[128]. Element l of sub-block j has its
-// low nibble in qs[32 (j / 2) + l] (high half of the byte when j is odd) and its fifth bit in bit j of qh[l].
-template <int XSPLIT>
-__device__ __forceinline__ void q5k_unit(const uint8_t* pA, const uint8_t* pB, int lane, const uint2* xhi, const uint2* xlo, uint2 xsum, float2 xs,
-                                         float (&total)[4]) {
-  const int t = lane & 3;
-  const uint4 hA = *reinterpret_cast<const uint4*>(pA), hB = *reinterpret_cast<const uint4*>(pB);
-  const uint32_t scA[2] = {hA.y & 0x3f3f3f3fu, (hA.w & 0x0f0f0f0fu) | ((hA.y >> 2) & 0x30303030u)};
-  const uint32_t mnA[2] = {hA.z & 0x3f3f3f3fu, ((hA.w >> 4) & 0x0f0f0f0fu) | ((hA.z >> 2) & 0x30303030u)};
-  const uint32_t scB[2] = {hB.y & 0x3f3f3f3fu, (hB.w & 0x0f0f0f0fu) | ((hB.y >> 2) & 0x30303030u)};
-  const uint32_t mnB[2] = {hB.z & 0x3f3f3f3fu, ((hB.w >> 4) & 0x0f0f0f0fu) | ((hB.z >> 2) & 0x30303030u)};
-  constexpr uint32_t k1024 = 0x64006400u;
-  uint32_t highA[2], highB[2];
-#pragma unroll
-  for (int u = 0; u < 2; ++u)
-    highA[u] = lds_u32(pA + 16 + 16 * u + 4 * t), highB[u] = lds_u32(pB + 16 + 16 * u + 4 * t);
-  float sum[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    uint32_t lowA[2], lowB[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-      lowA[u] = lds_u32(pA + 48 + 32 * c + 16 * u + 4 * t), lowB[u] = lds_u32(pB + 48 + 32 * c + 16 * u + 4 * t);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int j = 2 * c + h;
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const uint32_t fifthA = (j < 4 ? highA[u] << (4 - j) : highA[u] >> (j - 4)) & 0x10101010u;
-        const uint32_t fifthB = (j < 4 ? highB[u] << (4 - j) : highB[u] >> (j - 4)) & 0x10101010u;
-        uint32_t a[4];
-        byte_fragment(a, ((h ? lowA[u] >> 4 : lowA[u]) & 0x0f0f0f0fu) | fifthA, ((h ? lowB[u] >> 4 : lowB[u]) & 0x0f0f0f0fu) | fifthB, k1024);
-        mma_split<XSPLIT>(acc, a, xhi, xlo, (2 * j + u) * 32 + lane);
-      }
-      add_scaled(sum, byte_of(scA[j >> 2], j & 3), byte_of(scB[j >> 2], j & 3), acc);
-    }
-  }
-  float accm[4] = {0.f, 0.f, 0.f, 0.f};
-  {
-    const uint32_t wordA = (t & 2) ? mnA[1] : mnA[0], wordB = (t & 2) ? mnB[1] : mnB[0];
-    const uint32_t pairA = (wordA >> ((t & 1) * 16)) & 0xffffu, pairB = (wordB >> ((t & 1) * 16)) & 0xffffu;
-    uint32_t a[4];
-    a[0] = a[2] = hsub2_u32(__byte_perm(pairA, 0x64u, 0x4140), k1024);
-    a[1] = a[3] = hsub2_u32(__byte_perm(pairB, 0x64u, 0x4140), k1024);
-    mma_16816(accm, a, xsum.x, xsum.y);
-  }
-  const float2 dA = __half22float2(*reinterpret_cast<const __half2*>(&hA.x)), dB = __half22float2(*reinterpret_cast<const __half2*>(&hB.x));
-  sum[0] = dA.x * sum[0] - dA.y * accm[0], sum[1] = dA.x * sum[1] - dA.y * accm[1];
-  sum[2] = dB.x * sum[2] - dB.y * accm[2], sum[3] = dB.x * sum[3] - dB.y * accm[3];
-  add_total(total, xs, sum);
-}
-
-// Q8_0 (quant_linear.metal:87-97): eight blocks of fp16 d | int8[32] stand for one super-block.
-template <int XSPLIT>
-__device__ __forceinline__ void q8_unit(const uint8_t* pA, const uint8_t* pB, int lane, const uint2* xhi, const uint2* xlo, float2 xs, float (&total)[4]) {
-  const int t = lane & 3;
-  constexpr uint32_t k1152 = 0x64806480u;
-  float sum[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int at = 34 * j + 2 + 16 * u + 4 * t;  // word-aligned in odd blocks only
-      const uint32_t bytesA = (j & 1 ? lds_u32(pA + at) : lds_u32_unaligned(pA + at)) ^ 0x80808080u;
-      const uint32_t bytesB = (j & 1 ? lds_u32(pB + at) : lds_u32_unaligned(pB + at)) ^ 0x80808080u;
-      uint32_t a[4];
-      byte_fragment(a, bytesA, bytesB, k1152);
-      mma_split<XSPLIT>(acc, a, xhi, xlo, (2 * j + u) * 32 + lane);
-    }
-    add_scaled(sum, load_half_bits(pA + 34 * j), load_half_bits(pB + 34 * j), acc);
-  }
-  add_total(total, xs, sum);
-}
-
-// IQ4_XS (quant_linear.metal:99-115): fp16 d | scales_h u16 | scales_l[4] | qs[128]. Element l of sub-block j is the grid
-// value at the low (l < 16) or high nibble of qs[16 j + l % 16], times ls_j - 32.
-// Eight grid values of a word by byte permutes: `low` = grid values + 128 of the low nibbles of bytes 0..3 and of the high
-// ones, as the pairs (byte 0 low, byte 0 high, byte 1 low, byte 1 high) in x and those of bytes 2 and 3 in y.
-__device__ __forceinline__ uint2 iq4_lookup(uint32_t word) {
-  constexpr uint32_t k0 = 0x3f2d1801u, k1 = 0x766a5d4fu, k2 = 0xa6998d81u, k3 = 0xf1d9c5b5u;  // grid + 128, four per word
-  const uint32_t index = word & 0x77777777u, half = ((word >> 1) & 0x44444444u) | 0x32103210u;
-  uint2 out;
-  out.x = __byte_perm(__byte_perm(k0, k1, index), __byte_perm(k2, k3, index), half);
-  out.y = __byte_perm(__byte_perm(k0, k1, index >> 16), __byte_perm(k2, k3, index >> 16), half >> 16);
-  return out;
-}
-template <int XSPLIT>
-__device__ __forceinline__ void iq4_unit(const uint8_t* pA, const uint8_t* pB, int lane, const uint2* xhi, const uint2* xlo, float2 xs, float (&total)[4]) {
-  const int t = lane & 3;
-  constexpr uint32_t k1152 = 0x64806480u;
-  const uint2 hA = *reinterpret_cast<const uint2*>(pA), hB = *reinterpret_cast<const uint2*>(pB);
-  float sum[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const uint2 qA = iq4_lookup(lds_u32(pA + 8 + 16 * j + 4 * t)), qB = iq4_lookup(lds_u32(pB + 8 + 16 * j + 4 * t));
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      uint32_t a[4];
-      a[0] = hsub2_u32(__byte_perm(qA.x, 0x64u, u ? 0x4341 : 0x4240), k1152);
-      a[1] = hsub2_u32(__byte_perm(qB.x, 0x64u, u ? 0x4341 : 0x4240), k1152);
-      a[2] = hsub2_u32(__byte_perm(qA.y, 0x64u, u ? 0x4341 : 0x4240), k1152);
-      a[3] = hsub2_u32(__byte_perm(qB.y, 0x64u, u ? 0x4341 : 0x4240), k1152);
-      mma_split<XSPLIT>(acc, a, xhi, xlo, (2 * j + u) * 32 + lane);
-    }
-    const int lsA = int((hA.y >> (4 * j)) & 15u) | int(((hA.x >> (16 + 2 * j)) & 3u) << 4);
-    const int lsB = int((hB.y >> (4 * j)) & 15u) | int(((hB.x >> (16 + 2 * j)) & 3u) << 4);
-    add_scaled(sum, float(lsA - 32), float(lsB - 32), acc);
-  }
-  const float dA = load_half_bits(pA), dB = load_half_bits(pB);
-  sum[0] *= dA, sum[1] *= dA, sum[2] *= dB, sum[3] *= dB;
-  add_total(total, xs, sum);
-}
-
-// ---- Q6_K: one 16-row x 256-k unit -------------------------------------------------------------
-// Block layout (quant_linear.metal:69-85): ql[128] | qh[64] | int8 sc[16] | fp16 d. Element r = 128*hh + 32*s
-// + l has its low nibble in ql[64*hh + 32*(s&1) + l] (high half of the byte when s >= 2), its top two bits
-// in qh[32*hh + l] >> 2s, and scale sc[r/16]. MMA gi covers elements [16gi, 16gi+16); lane t supplies
-// elements 16gi + 4t + {0,1,2,3}. Blocks are only 2-byte aligned, so words are fetched as two halves.
-template <int XSPLIT>
-__device__ __forceinline__ void q6k_unit(const uint8_t* pA, const uint8_t* pB, int lane, int hh, const uint2* xhi, const uint2* xlo, float2 xs,
-                                         float (&total)[4]) {
-  const int t = lane & 3;
-  float sum[4] = {0.f, 0.f, 0.f, 0.f};
-  const float dA = load_half_bits(pA + 208), dB = load_half_bits(pB + 208);
-  constexpr uint32_t k1056 = 0x64206420u;
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const uint32_t hiA = lds_u32_unaligned(pA + 128 + 32 * hh + 16 * u + 4 * t), hiB = lds_u32_unaligned(pB + 128 + 32 * hh + 16 * u + 4 * t);
-#pragma unroll
-      for (int sl = 0; sl < 2; ++sl) {
-        const uint32_t loA = lds_u32_unaligned(pA + 64 * hh + 32 * sl + 16 * u + 4 * t), loB = lds_u32_unaligned(pB + 64 * hh + 32 * sl + 16 * u + 4 * t);
-#pragma unroll
-        for (int sh = 0; sh < 2; ++sh) {
-          const int s = sl + 2 * sh, gi = hh * 8 + s * 2 + u;
-          const uint32_t bytesA = ((sh ? loA >> 4 : loA) & 0x0f0f0f0fu) | (((hiA >> (2 * s)) & 0x03030303u) << 4);
-          const uint32_t bytesB = ((sh ? loB >> 4 : loB) & 0x0f0f0f0fu) | (((hiB >> (2 * s)) & 0x03030303u) << 4);
-          uint32_t a[4];
-          a[0] = hsub2_u32(__byte_perm(bytesA, 0x64u, 0x4140), k1056);
-          a[1] = hsub2_u32(__byte_perm(bytesB, 0x64u, 0x4140), k1056);
-          a[2] = hsub2_u32(__byte_perm(bytesA, 0x64u, 0x4342), k1056);
-          a[3] = hsub2_u32(__byte_perm(bytesB, 0x64u, 0x4342), k1056);
-          float acc[4] = {0.f, 0.f, 0.f, 0.f};
-          uint2 b = xhi[gi * 32 + lane];
-          mma_16816(acc, a, b.x, b.y);
-          if (XSPLIT == 2) {
-            b = xlo[gi * 32 + lane];
-            mma_16816(acc, a, b.x, b.y);
-          }
-          const float sA = dA * float(int(reinterpret_cast<const int8_t*>(pA + 192)[gi])), sB = dB * float(int(reinterpret_cast<const int8_t*>(pB + 192)[gi]));
-          add_scaled(sum, sA, sB, acc);
-        }
-      }
-    }
-  add_total(total, xs, sum);
-}
+  __device__ __forceinline__ float2 scales(int) const { return powers; }
+  __device__ __forceinline__ uint2 sums(int) const { return minSums; }
+};
 
 __device__ __forceinline__ int find_segment(const GemvParams& p, int tile) {
   int s = 0;
@@ -551,10 +375,10 @@ template <class Q, int NMAT, int XSPLIT> __global__ void __launch_bounds__(kThre
         else if (NMAT == 1 && seg.res)
           addend = seg.res[at];
       }
-      float total[NMAT][4];
+      float total[NMAT][1][4];
 #pragma unroll
       for (int mat = 0; mat < NMAT; ++mat)
-        total[mat][0] = total[mat][1] = total[mat][2] = total[mat][3] = 0.f;
+        clear(total[mat]);
 #pragma unroll
       for (int mat = 0; mat < NMAT; ++mat)
         for (int grp = 0; grp < groups; ++grp, ++it) {
@@ -572,20 +396,21 @@ template <class Q, int NMAT, int XSPLIT> __global__ void __launch_bounds__(kThre
             const uint8_t *pA = base + g * row_pitch<Q>(), *pB = base + (g + 8) * row_pitch<Q>();
             const int sb = grp * kStageBlocks + warp;
             const float2 xs = *reinterpret_cast<const float2*>(xScale + sb * 8 + 2 * t);
-            const uint2 *hi = fragHi + sb * 512, *lo = fragLo + sb * 512;
+            StagedRows<XSPLIT> rows{fragHi + sb * 512 + lane, fragLo + sb * 512 + lane, make_uint2(0u, 0u), xs};
             if constexpr (std::is_same_v<Q, Q4K>) {
               q4k_unit<XSPLIT>(smem_u32(pA), smem_u32(pB), t, fragHiAddress + sb * 4096, fragLoAddress + sb * 4096, rotation, fragSumAddress + sb * 256, xs,
-                               total[mat]);
+                               total[mat][0]);
             } else if constexpr (std::is_same_v<Q, Q5K>) {
-              q5k_unit<XSPLIT>(pA, pB, lane, hi, lo, fragSum[sb * 32 + lane], xs, total[mat]);
+              rows.minSums = fragSum[sb * 32 + lane];
+              q5k_unit(pA, pB, lane, rows, total[mat]);
             } else if constexpr (std::is_same_v<Q, Q8>) {
-              q8_unit<XSPLIT>(pA, pB, lane, hi, lo, xs, total[mat]);
+              q8_unit(pA, pB, lane, rows, total[mat]);
             } else if constexpr (std::is_same_v<Q, IQ4>) {
-              iq4_unit<XSPLIT>(pA, pB, lane, hi, lo, xs, total[mat]);
+              iq4_unit(pA, pB, lane, rows, total[mat]);
             } else {
 #pragma unroll
               for (int half = 0; half < 2; ++half)
-                q6k_unit<XSPLIT>(pA, pB, lane, half, hi, lo, xs, total[mat]);
+                q6k_unit(pA, pB, lane, half, rows, total[mat]);
             }
           }
           __syncwarp();
@@ -597,10 +422,10 @@ template <class Q, int NMAT, int XSPLIT> __global__ void __launch_bounds__(kThre
 #pragma unroll
       for (int mat = 0; mat < NMAT; ++mat) {
         float* dst = mine + (mat * kConsumerWarps + warp) * 128;
-        dst[(2 * t) * 16 + g] = total[mat][0];
-        dst[(2 * t + 1) * 16 + g] = total[mat][1];
-        dst[(2 * t) * 16 + g + 8] = total[mat][2];
-        dst[(2 * t + 1) * 16 + g + 8] = total[mat][3];
+        dst[(2 * t) * 16 + g] = total[mat][0][0];
+        dst[(2 * t + 1) * 16 + g] = total[mat][0][1];
+        dst[(2 * t) * 16 + g + 8] = total[mat][0][2];
+        dst[(2 * t + 1) * 16 + g + 8] = total[mat][0][3];
       }
       named_barrier(1, kConsumerWarps * kWarp);
       if (tid < 128) {

@@ -24,6 +24,8 @@ struct infdev_ctx {
   uint8_t* captureImage = nullptr;     // one-shot: where the next producer call writes the image of its result
   const uint8_t* supplyImage = nullptr;  // one-shot: image the next linear call reads instead of quantising x
   float* ummaPartial = nullptr;  // K-slice partial results of the tcgen05 prefill GEMM: [4][128][8192] floats, allocated on first use
+  uint8_t* wideImage = nullptr;  // activations laid out for the GEMM of the other block types
+  float* widePartial = nullptr;  // its K-slice partial results
   void* ummaActs = nullptr;  // fp16 activations laid out for the tcgen05 prefill GEMM (K up to 16384)
   std::atomic<uint64_t> launches{0};  // kernels launched through this context
   cudaStream_t stream = nullptr;
@@ -175,6 +177,8 @@ infdev_ctx* infdev_create(int device, char* error) {
       (e = cudaMalloc(reinterpret_cast<void**>(&ctx->imageCounters), infdev::kImageCounters * sizeof(int))) != cudaSuccess ||
       (e = cudaMemset(ctx->imageCounters, 0, infdev::kImageCounters * sizeof(int))) != cudaSuccess ||
       (e = cudaMalloc(&ctx->ummaActs, size_t(64) * infdev::kUmmaMaxActBytesPerBlock)) != cudaSuccess ||
+      (e = cudaMalloc(reinterpret_cast<void**>(&ctx->wideImage), infdev::kWideImageBytes)) != cudaSuccess ||
+      (e = cudaMalloc(reinterpret_cast<void**>(&ctx->widePartial), infdev::kWidePartialFloats * sizeof(float))) != cudaSuccess ||
       (e = cudaHostAlloc(reinterpret_cast<void**>(&ctx->statusHost), sizeof(int), cudaHostAllocDefault)) != cudaSuccess) {
     std::string text = std::string("context setup: ") + cudaGetErrorString(e);
     delete ctx;
@@ -196,6 +200,8 @@ void infdev_destroy(infdev_ctx* ctx) {
   cudaFree(ctx->imageCounters);
   cudaFree(ctx->ummaPartial);
   cudaFree(ctx->ummaActs);
+  cudaFree(ctx->wideImage);
+  cudaFree(ctx->widePartial);
   cudaFreeHost(ctx->statusHost);
   cudaEventDestroy(ctx->done);
   cudaStreamDestroy(ctx->stream);
@@ -488,6 +494,48 @@ static int linear_run(infdev_ctx* ctx, int type, bool pair, int count, const voi
       if (int r = check(ctx, infdev::umma_launch(pair, u, x + row * k, int(k), ctx->sms, ctx->stream), "umma launch"))
         return r;
       ctx->launches += u.splits > 1 ? 3 : 2;
+    }
+    return INFDEV_OK;
+  }
+  // More than 8 rows of the other types share one decode of the weights; infdev_set_umma(0) and one-sided activations keep the
+  // slices of 8 rows, whose sums do not depend on the row count.
+  const infdev::GemvBox wideBox = infdev::wide_box(type);
+  bool wide = ctx->umma && m > 8 && wideBox.blockBytes && k <= infdev::kWideMaxK && (type != INFDEV_Q6_K || ctx->xsplit == 2);
+  int64_t columns = 0;
+  for (int i = 0; i < count; ++i) {
+    wide = wide && n[i] > 0 && n[i] % 16 == 0 && aligned16(w[i]) && (!pair || aligned16(w2[i]));
+    columns += n[i];
+  }
+  columns *= pair ? 2 : 1;
+  wide = wide && columns < (int64_t(1) << 30) && (!pair || (count == 1 && size_t(columns) * infdev::kWideMaxRows <= infdev::kWidePartialFloats));
+  if (wide) {
+    infdev::WideParams p{};
+    p.nseg = pair ? 2 : count;
+    p.pair = pair;
+    for (int i = 0; i < p.nseg; ++i) {
+      const int at = pair ? 0 : i;
+      const void* weights = pair && i ? w2[0] : w[at];
+      p.seg[i] = {static_cast<const uint8_t*>(weights), nullptr, y[at], residual ? residual[at] : nullptr, int(n[at]), int(n[at]), p.tiles};
+      if (int r = weight_map(ctx, weights, n[at], k, wideBox.blockBytes, 1, infdev::kGemvTileRows, &p.map[i], wideBox.padBytes))
+        return r;
+      p.tiles += int(n[at] / 16);
+    }
+    p.blocks = int(k / 256), p.pitch = int(columns);
+    p.image = ctx->wideImage, p.partial = ctx->widePartial, p.status = ctx->status;
+    for (int64_t row = 0; row < m;) {
+      // groups of 128 rows; a rest of up to 8 rows joins the group before it, halved
+      const int64_t left = m - row, take = left <= infdev::kWideMaxRows ? left : left <= infdev::kWideMaxRows + 8 ? (left + 15) / 16 * 8 : infdev::kWideMaxRows;
+      p.m = int(take);
+      for (int i = 0; i < p.nseg; ++i) {
+        const int at = pair ? 0 : i;
+        p.seg[i].y = y[at] + row * n[at];
+        p.seg[i].res = residual && residual[at] ? residual[at] + row * n[at] : nullptr;
+      }
+      int launches = 0;
+      if (int r = check(ctx, infdev::wide_launch(type, p, x + row * k, int(k), ctx->sms, ctx->stream, &launches), "wide linear launch"))
+        return r;
+      ctx->launches += launches;
+      row += take;
     }
     return INFDEV_OK;
   }

@@ -64,6 +64,27 @@ struct GemvBox {
 GemvBox gemv_box(int type);
 cudaError_t gemv_launch(int type, bool pair, int xsplit, const GemvParams& p, int sms, cudaStream_t stream);
 
+// ---- 9 to 128 rows of Q5_K, Q6_K, Q8_0, IQ4_XS (gemv_wide.cu) ----
+constexpr int kWideMaxRows = 128, kWideMaxK = 16384, kWideTileBytes = 16 * 32 * 16 + 32 * 8 + 8 * 4;  // image of 256 activations x 8 rows
+constexpr size_t kWideImageBytes = size_t(kWideMaxK / 256) * (kWideMaxRows / 8) * kWideTileBytes;
+constexpr size_t kWidePartialFloats = size_t(4) * 128 * 8192;
+
+struct WideParams {
+  alignas(64) CUtensorMap map[4];  // box = wide_box() of one super-block x 16 rows
+  GemvSeg seg[4];        // a pair is two segments, gate and up, with one result
+  int nseg, tiles;       // tiles of 16 weight rows
+  bool pair;             // y of the first segment = silu(gate) * up
+  int m, blocks, pitch;  // activation rows, super-blocks of K, weight rows of all segments
+  int groups, slices;    // row groups and K slices that different CTAs take (set by wide_launch)
+  const uint8_t* image;  // kWideImageBytes
+  float* partial;        // kWidePartialFloats, [slices][m][pitch]: results that wide_reduce_kernel finishes
+  int* status;
+};
+
+GemvBox wide_box(int type);
+// p.m rows of x, `ldx` floats apart (a multiple of 4); a pair needs m x pitch <= kWidePartialFloats.
+cudaError_t wide_launch(int type, const WideParams& p, const float* x, int ldx, int sms, cudaStream_t stream, int* launches);
+
 // Integer-MMA Q4_K decode GEMV over an activation image (q4k_decode.cu).
 cudaError_t q4k_decode_launch(bool pair, const GemvParams& p, int sms, cudaStream_t stream);
 // fp32 activations [m][ldx] -> image of k/256 blocks; rows m..7 are zero-filled.

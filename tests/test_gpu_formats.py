@@ -74,6 +74,41 @@ def test_gate_up_matches_oracle(dev, name, qtype):
   assert rel_err(y.download(), oracle.gate_up(wg, wu, qtype, n, k, x)) < 1e-5
 
 
+WIDE_TYPES = [*TYPES, ("q6_k", D.Q6_K)]
+
+
+@pytest.mark.parametrize("m,n,k", [(9, 16, 2048), (16, 4096, 4096), (17, 208, 6144), (24, 1024, 2048), (33, 48, 12288), (40, 2512, 4096), (43, 96, 2048),
+                                   (56, 160, 4096), (64, 4096, 4096), (65, 16, 2048), (128, 1040, 12288), (131, 64, 4096), (137, 32, 2048),
+                                   (15, 21008, 2048), (40, 21008, 2048)])
+@pytest.mark.parametrize("name,qtype", WIDE_TYPES)
+def test_many_rows_share_a_decode(dev, name, qtype, m, n, k):
+  """9 rows and up: every tile count, the last tile of a row group partly filled, tiles fewer and several times more than all warps, K in
+  one chunk, several chunks and several slices; with a residual that the result overwrites. 22-bit activations, exact quants
+  and fp32 sums as with up to eight rows, so the bound is that of the calls above."""
+  w, x, y = synth.weight(qtype, n, k, 90), synth.activations(m, k, 91), synth.activations(m, n, 92)
+  x[m - 1] *= 1.0e6
+  x[m // 2] *= 1.0e-9
+  buffer = dev.array(y)
+  dev.linear(qtype, dev.array(w), n, k, dev.array(x), m, buffer, buffer)
+  got, want = buffer.download() - y, oracle.linear(w, qtype, n, k, x)
+  # adding the residual rounds to its own last place: 1.2e-7 of it beside the products' bound
+  for row in range(m):
+    assert np.linalg.norm(got[row] - want[row]) < 1e-5 * np.linalg.norm(want[row]) + 2.4e-7 * np.linalg.norm(y[row]), row
+
+
+@pytest.mark.parametrize("m", [11, 40, 100, 128])
+@pytest.mark.parametrize("name,qtype", TYPES)
+def test_many_rows_of_a_pair_and_of_a_group(dev, name, qtype, m):
+  n, k = 768, 4096
+  wg, wu, x = synth.weight(qtype, n, k, 93), synth.weight(qtype, n, k, 94), synth.activations(m, k, 95)
+  y, z = dev.empty((m, n)), dev.empty((m, n))
+  dev.gate_up(qtype, dev.array(wg), dev.array(wu), n, k, dev.array(x), m, y)
+  assert rel_err(y.download(), oracle.gate_up(wg, wu, qtype, n, k, x)) < 1e-5
+  dev.linear_group(qtype, [dev.array(wg), dev.array(wu)], [n, n], k, dev.array(x), m, [y, z])
+  assert rel_err(y.download(), oracle.linear(wg, qtype, n, k, x)) < 1e-5
+  assert rel_err(z.download(), oracle.linear(wu, qtype, n, k, x)) < 1e-5
+
+
 @pytest.mark.parametrize("name,qtype", TYPES)
 def test_embedding_rows_are_the_oracle_rows(dev, name, qtype):
   n, k, ids = 96, 4096, np.array([0, 95, 7, 7, 41], np.int32)
