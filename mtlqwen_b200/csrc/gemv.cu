@@ -408,9 +408,7 @@ template <class Q, int NMAT, int XSPLIT> __global__ void __launch_bounds__(kThre
             } else if constexpr (std::is_same_v<Q, IQ4>) {
               iq4_unit(pA, pB, lane, rows, total[mat]);
             } else {
-#pragma unroll
-              for (int half = 0; half < 2; ++half)
-                q6k_unit(pA, pB, lane, half, rows, total[mat]);
+              q6k_unit(pA, pB, lane, rows, total[mat]);
             }
           }
           __syncwarp();

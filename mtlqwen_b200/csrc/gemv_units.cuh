@@ -187,12 +187,14 @@ template <int NT, class B> __device__ __forceinline__ void iq4_unit(const uint8_
 // in qh[32*hh + l] >> 2s, and scale sc[r/16]. MMA gi covers elements [16gi, 16gi+16); lane t supplies
 // elements 16gi + 4t + {0,1,2,3}. Blocks are only 2-byte aligned, so words are fetched as two halves.
 template <int NT, class B>
-__device__ __forceinline__ void q6k_unit(const uint8_t* pA, const uint8_t* pB, int lane, int hh, const B& b, float (&total)[NT][4]) {
+__device__ __forceinline__ void q6k_unit(const uint8_t* pA, const uint8_t* pB, int lane, const B& b, float (&total)[NT][4]) {
   const int t = lane & 3;
   float sum[NT][4];
   clear(sum);
   const float dA = load_half_bits(pA + 208), dB = load_half_bits(pB + 208);
   constexpr uint32_t k1056 = 0x64206420u;
+#pragma unroll(NT > 2 ? 1 : 2)
+  for (int hh = 0; hh < 2; ++hh) {
 #pragma unroll(NT > 3 ? 1 : 2)
     for (int u = 0; u < 2; ++u) {
       const uint32_t hiA = lds_u32_unaligned(pA + 128 + 32 * hh + 16 * u + 4 * t), hiB = lds_u32_unaligned(pB + 128 + 32 * hh + 16 * u + 4 * t);
@@ -211,6 +213,7 @@ __device__ __forceinline__ void q6k_unit(const uint8_t* pA, const uint8_t* pB, i
         }
       }
     }
+  }
   add_totals(total, b, sum);
 }
 

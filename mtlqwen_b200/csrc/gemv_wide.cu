@@ -18,9 +18,11 @@
 //
 // What bounds it: shared memory and the tensor pipe together. A group of 16 k x 16 weights x 8 rows is 16 cycles of MMA and 16
 // cycles of a scheduler's share of the fragment reads; with four tiles a unit (16 rows x 256 k) takes a scheduler 1.0 to 1.3
-// us of which the MMAs are 0.57. Slices of eight rows against this kernel: Q6_K output head 248320 x 4096, 16 rows 481 -> 300
-// us, 40 rows 1180 -> 730 us; projections of a layer of mixed types, 16 rows 176 -> 132 us, 40 rows 440 -> 230 us, 128 rows
-// 1410 -> 530 us. At nine rows the two are level (layer: 135 against 130 us), which is why it starts there.
+// us of which the MMAs are 0.57. Slices of eight rows against this kernel: Q6_K output head 248320 x 4096, 16 rows 481 -> 307
+// us, 40 rows 1180 -> 790 us; projections of a layer of mixed types, 16 rows 176 -> 135 us, 40 rows 440 -> 241 us, 128 rows
+// 1410 -> 577 us. At nine rows 176 -> 123 us for the layer, which is why it starts there. A chunk's sum is added to what
+// rests in the result at the chunk's end: fetching that first and adding on top hid the latency (530 us at 128 rows) but lost
+// accuracy (Q6_K, K = 12288: 2.0e-7 against fp64; 1.3e-7 now, 1.4e-7 for the slices).
 #include <algorithm>
 #include <type_traits>
 #include "gemv_units.cuh"
@@ -268,16 +270,6 @@ template <class Q, int NT> __global__ void __launch_bounds__(kThreads, 1) wide_k
         const float* const before = chunk > 0 ? y : parked ? nullptr : seg.res;
         float total[NT][4];
         clear(total);
-        if (before) {
-#pragma unroll
-          for (int n = 0; n < NT; ++n)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int row = row0 + 8 * n + (i & 1);
-              if (row < m)
-                total[n][i] = before[size_t(row) * ldy + column + 8 * (i >> 1)];
-            }
-        }
 #pragma unroll 1
         for (int j = 0; j < count; ++j, ++used) {
           const uint32_t slot = used % kDepth;
@@ -296,15 +288,21 @@ template <class Q, int NT> __global__ void __launch_bounds__(kThreads, 1) wide_k
           } else if constexpr (std::is_same_v<Q, IQ4>) {
             iq4_unit(pA, pB, lane, rows, total);
           } else {
-#pragma unroll(NT > 2 ? 1 : 2)
-            for (int half = 0; half < 2; ++half)
-              q6k_unit(pA, pB, lane, half, rows, total);
+            q6k_unit(pA, pB, lane, rows, total);
           }
           __syncwarp();
           if (lane == 0)
             mbar_arrive(&ctl.empty[slot][warp]);
         }
         if (ok) {
+#pragma unroll
+          for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {  // added here, not at the start: a chunk's own sum is rounded on a finer grid
+              const int row = row0 + 8 * n + (i & 1);
+              if (before && row < m)
+                total[n][i] += before[size_t(row) * ldy + column + 8 * (i >> 1)];
+            }
 #pragma unroll
           for (int n = 0; n < NT; ++n)
 #pragma unroll
@@ -392,7 +390,7 @@ template <class Q> cudaError_t launch(const WideParams& params, const float* x, 
   const int groupTiles = (tiles + p.groups - 1) / p.groups;
   p.slices = slices(p, groupTiles, sms);
   const int warps = p.groups * groupTiles * p.blocks;
-  launch_kernel(wide_prepare_kernel, (warps + 3) / 4, 128, 0, stream, x, ldx, p.m, p.groups * groupTiles, groupTiles, p.blocks,
+  launch_kernel<1>(wide_prepare_kernel, (warps + 3) / 4, 128, 0, stream, x, ldx, p.m, p.groups * groupTiles, groupTiles, p.blocks,
                 const_cast<uint8_t*>(p.image));
   cudaError_t e = cudaErrorInvalidValue;
   switch (groupTiles) {
@@ -403,7 +401,7 @@ template <class Q> cudaError_t launch(const WideParams& params, const float* x, 
   }
   *launches = 2;
   if (e == cudaSuccess && (p.pair || p.slices > 1)) {
-    launch_kernel(wide_reduce_kernel, unsigned((size_t(p.m) * p.pitch / (p.pair ? 8 : 4) + 255) / 256), 256, 0, stream, p);
+    launch_kernel<1>(wide_reduce_kernel, unsigned((size_t(p.m) * p.pitch / (p.pair ? 8 : 4) + 255) / 256), 256, 0, stream, p);
     *launches = 3;
     e = cudaGetLastError();
   }
