@@ -285,16 +285,17 @@ __device__ __forceinline__ RowTile tile_of(const infdev_query& query, uint32_t i
   return tile;
 }
 
-// Pieces of a tile's context: at least 128 tokens, whole 64-token tiles.
+// Pieces of a tile's context: whole 64-token tiles.
 __device__ __forceinline__ uint32_t piece_tokens(uint32_t attended, uint32_t rows, uint32_t most, uint32_t maxSplits) {
-  const uint32_t wanted = max(1u, min((attended + 127u) / 128u, rows <= 4 ? maxSplits : most));
+  const uint32_t wanted = max(1u, min((attended + kGroupTokens - 1) / kGroupTokens, rows <= 4 ? maxSplits : most));
   return ((attended + wanted - 1) / wanted + kGroupTokens - 1) / kGroupTokens * kGroupTokens;
 }
 __device__ __forceinline__ uint32_t piece_count(uint32_t attended, uint32_t piece) { return (attended + piece - 1) / piece; }
 
-// Work item `item` of the pass, found by one warp together; false when there are fewer.
+// Work item `item` of the pass, found by one warp together; false when there are fewer. `items`: how many there are, where one
+// round over the queries tells.
 __device__ __forceinline__ bool find_item(const infdev_query* queries, int queryCount, uint32_t most, uint32_t maxSplits, uint32_t item, RowTile& tile,
-                                          uint32_t& split, uint32_t& piece) {
+                                          uint32_t& split, uint32_t& piece, uint32_t& items) {
   const uint32_t lane = threadIdx.x & 31;
   for (int base = 0; base < queryCount; base += 32) {
     uint32_t mine = 0, tiles = 0;
@@ -315,6 +316,7 @@ __device__ __forceinline__ bool find_item(const infdev_query* queries, int query
         inclusive += other;
     }
     const uint32_t total = __shfl_sync(0xffffffffu, inclusive, 31);
+    items = queryCount <= 32 ? total : 0xffffffffu;
     if (item >= total) {
       item -= total;
       continue;
@@ -369,8 +371,9 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, head = warp & 3, half = warp >> 2, g = lane >> 2, t = lane & 3;
   const int rowBase = head * kGroupRows;  // this warp's 16 rows of q, p and exchange
   RowTile tile;
-  uint32_t split, piece;
-  for (uint32_t item = blockIdx.x; find_item(queries, queryCount, most, maxSplits, item / kKvHeads, tile, split, piece); item += gridDim.x) {
+  uint32_t split, piece, items = 0xffffffffu;
+  for (uint32_t item = blockIdx.x;
+       item / kKvHeads < items && find_item(queries, queryCount, most, maxSplits, item / kKvHeads, tile, split, piece, items); item += gridDim.x) {
     const uint32_t kvHead = item % kKvHeads, begin = split * piece, end = min(tile.attended, begin + piece);
     const int32_t* slotTable = table + size_t(tile.slot) * tableStride;
     auto fetch = [&](uint32_t from, int buffer) {  // a warp copies one token's 512 bytes at a time
@@ -385,14 +388,20 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
     __syncthreads();  // the item before this one is finished with the shared arrays
+    // the 16 rows x 4 heads of q, hi and lo; rows past the tile's are zero. All loads are in flight before the first is used.
+    constexpr int kQuads = kGroup * kGroupRows * (kDim / 4) / kGroupThreads;
+    float4 value[kQuads];
+#pragma unroll
+    for (int i = 0; i < kQuads; ++i) {
+      const int at = i * kGroupThreads + threadIdx.x, row = at / (kDim / 4), d = at % (kDim / 4) * 4, r = row % kGroupRows, h = row / kGroupRows;
+      value[i] = r < int(tile.rows) ? *reinterpret_cast<const float4*>(q + (size_t(tile.start + r) * kQHeads + kvHead * kGroup + h) * kDim + d)
+                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     fetch(begin, 0);
-    // the 16 rows x 4 heads of q, hi and lo; rows past the tile's are zero
-    for (int i = threadIdx.x; i < kGroup * kGroupRows * (kDim / 4); i += kGroupThreads) {
-      const int row = i / (kDim / 4), d = i % (kDim / 4) * 4, r = row % kGroupRows, h = row / kGroupRows;
-      float4 value = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (r < int(tile.rows))
-        value = *reinterpret_cast<const float4*>(q + (size_t(tile.start + r) * kQHeads + kvHead * kGroup + h) * kDim + d);
-      const uint2 a = split_pair(value.x, value.y), b = split_pair(value.z, value.w);
+#pragma unroll
+    for (int i = 0; i < kQuads; ++i) {
+      const int at = i * kGroupThreads + threadIdx.x, row = at / (kDim / 4), d = at % (kDim / 4) * 4;
+      const uint2 a = split_pair(value[i].x, value[i].y), b = split_pair(value[i].z, value[i].w);
       *reinterpret_cast<uint2*>(&sh.q[0][row][d]) = make_uint2(a.x, b.x);
       *reinterpret_cast<uint2*>(&sh.q[1][row][d]) = make_uint2(a.y, b.y);
     }
@@ -417,6 +426,8 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
         ldmatrix4(lo, &sh.q[1][rowBase + (lane & 15)][16 * step + 8 * (lane >> 4)]);
 #pragma unroll
         for (int pair = 0; pair < 2; ++pair) {
+          if (from + 32 * half + 16 * pair >= end)  // past the piece: these scores are masked below
+            continue;
           uint32_t b[4];
           ldmatrix4(b, &sh.k[buffer][32 * half + 16 * pair + 8 * (lane >> 4) + (lane & 7)][16 * step + 8 * ((lane >> 3) & 1)]);
           mma_16816(score[2 * pair], hi, b[0], b[1]);
@@ -467,6 +478,8 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
         acc[j][0] *= rescale[0], acc[j][1] *= rescale[0], acc[j][2] *= rescale[1], acc[j][3] *= rescale[1];
 #pragma unroll
       for (int step = 0; step < kGroupTokens / 16; ++step) {
+        if (from + 16 * step >= end)  // weights of zero
+          break;
         uint32_t hi[4], lo[4];
         ldmatrix4(hi, &sh.p[0][rowBase + (lane & 15)][16 * step + 8 * (lane >> 4)]);
         ldmatrix4(lo, &sh.p[1][rowBase + (lane & 15)][16 * step + 8 * (lane >> 4)]);
@@ -575,7 +588,13 @@ cudaError_t attention_launch(const float* q, const float* qg, const void* cacheK
   if (rows <= 0)
     return cudaSuccess;
   const uint32_t splits = std::min<uint32_t>(maxSplits, 32);  // the merge keeps one split per lane
-  if (rows > queryCount && !rowwise) {
+  // The group kernel takes passes whose queries have five rows or more on average, unless no context of the pass can be long
+  // (the table has no room for it): with r rows a query, its longer chain costs 2 us where r x context is below about 4096 (8
+  // rows of 128 tokens 18.7 against 16.7 us for prepare and attention), from there on it is level or faster (8 rows of 2008
+  // tokens 20.8 against 29.1, 16 of 616 22.8 against 23.6, 16 of 2016 22.8 against 39.4, 64 of 128 24.0 against 28.0).
+  const int64_t capacity = int64_t(tableStride) * blockTokens;
+  const bool grouped = rows >= 32 * int64_t(queryCount) || (rows >= 5 * int64_t(queryCount) && rows * capacity >= 4096 * int64_t(queryCount));
+  if (grouped && !rowwise) {
     // Some query has several rows. (One row each is the decode pass, where the scan is faster: no query rows to share a
     // tile with, and six small CTAs per SM hide the copies that the group kernel's single CTA waits for.)
     static PerDeviceOnce configured;
@@ -584,10 +603,10 @@ cudaError_t attention_launch(const float* q, const float* qg, const void* cacheK
     const int64_t tiles = std::max<int64_t>((rows + kGroupRows - 1) / kGroupRows, queryCount);
     const uint32_t most = uint32_t(std::clamp<int64_t>(sms / (kKvHeads * tiles), 1, splits));
     const int64_t items = (rows + queryCount) * kKvHeads * splits;  // no more than these
-    launch_kernel(attention_group_kernel, unsigned(std::min<int64_t>(items, sms)), kGroupThreads, sizeof(GroupShared), stream, q,
+    launch_kernel<2>(attention_group_kernel, unsigned(std::min<int64_t>(items, sms)), kGroupThreads, sizeof(GroupShared), stream, q,
                   static_cast<const __half*>(cacheK), static_cast<const __half*>(cacheV), queries, queryCount, table, tableStride, blockTokens, most, splits,
                   partials);
-    launch_kernel(attention_reduce_kernel<true>, unsigned(rows * kQHeads), 256, 0, stream, partials, qg, queries, queryCount, most, splits, out, image);
+    launch_kernel<2>(attention_reduce_kernel<true>, unsigned(rows * kQHeads), 256, 0, stream, partials, qg, queries, queryCount, most, splits, out, image);
     return cudaGetLastError();
   }
   launch_kernel(attention_scan_kernel, dim3(splits, kKvHeads, unsigned(rows)), 128, 0, stream, q, static_cast<const __half*>(cacheK),

@@ -126,6 +126,17 @@ def test_rows_that_share_a_tile(dev, contexts, counts, block_tokens, max_splits)
   assert run_attention(dev, rng, contexts, counts, block_tokens, max_splits) < 1e-5
 
 
+@pytest.mark.parametrize("contexts,counts,block_tokens,max_splits", [
+  ([32], [32], 16, 32), ([33], [33], 16, 32), ([40, 47], [40, 24], 16, 32),  # short contexts, 32 rows a query
+  ([16, 1500], [16, 5], 16, 32), ([17, 1500], [17, 6], 16, 32),  # one tile exactly and one row more, in a pass with a long context
+  ([64, 65, 80, 81, 127, 1600], [3, 4, 5, 5, 5, 12], 16, 32),  # pieces that end at every 16-token step of a tile
+  ([20], [20], 16, 32), ([204], [20], 16, 32), ([205], [20], 16, 32), ([300, 300], [5, 4], 16, 32),  # either side of the rule that picks the kernel
+])
+def test_rows_that_share_a_tile_where_the_rule_takes_them(dev, contexts, counts, block_tokens, max_splits):
+  rng = np.random.default_rng(sum(contexts) + 31 * len(counts))
+  assert run_attention(dev, rng, contexts, counts, block_tokens, max_splits) < 1e-5
+
+
 def test_switching_the_group_kernel_off_changes_rounding_only(dev):
   dev.set_umma(0)
   try:

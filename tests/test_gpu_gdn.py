@@ -117,6 +117,13 @@ def test_gdn_preparation_across_row_groups(dev):
   assert run_layer(dev, rng, [3, 1, 2, 9, 8, 17, 7, 4], fresh=(0, 4), speculative=(3, 7)) < 1e-4
 
 
+@pytest.mark.parametrize("lengths", [[1], [15], [33, 1, 30], [33, 1, 31], [3, 60, 2, 9, 8, 17, 7, 4]])
+def test_gdn_preparation_at_the_line_between_its_forms(dev, lengths):
+  """Up to 64 rows a thread has one row and a CTA one head, from 65 on eight of each."""
+  rng = np.random.default_rng(sum(lengths))
+  assert run_layer(dev, rng, lengths, speculative=(1,) if len(lengths) > 2 else ()) < 1e-4
+
+
 def test_gdn_single_query_edge_lengths(dev):
   rng = np.random.default_rng(4)
   for lengths in ([1], [2], [3], [4], [512]):
