@@ -56,35 +56,40 @@ template <int NMAT> constexpr size_t smem_bytes() { return fixed_bytes<NMAT>() +
 __device__ __forceinline__ uint4 lds128(const uint8_t* p) { return *reinterpret_cast<const uint4*>(p); }
 __device__ __forceinline__ uint2 lds64(const uint8_t* p) { return *reinterpret_cast<const uint2*>(p); }
 
-// D(16x8,s32) = A(16x32,u8,row) * B(32x8,s8 or u8,col)
+// D(16x8,s32) += A(16x32,u8,row) * B(32x8,s8 or u8,col)
 __device__ __forceinline__ void imma_u8s8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-               : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ void imma_u8u8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-               : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// What one lane keeps of the image of one super-block (act_image.cuh) while its warp walks the tiles: lane
-// (g = lane/4, t = lane%4) holds, per sub-block j, the B fragments of activation row g, quarter t: registers b0, b1 of
-// the high-byte MMA in x, y and of the low-byte MMA in z, w.
+// What one lane keeps of the image of one super-block (act_image.cuh) while its warp walks the tiles. With eight activation
+// rows the eight columns of an MMA are the rows. With ROWS = 1 or 2 they are (row, sub-block) pairs: column c stands for
+// row c % ROWS and, of every 8 / ROWS consecutive sub-blocks, for sub-block c / ROWS, and the B operand of a sub-block is zero
+// in the other columns. The MMAs of 8 / ROWS sub-blocks then share one accumulator, and a sub-block scale multiplies
+// every result once instead of leaving columns empty.
+// Lane (g = lane/4, t = lane%4) holds, per sub-block j, the B fragments of column g, quarter t: registers b0, b1 of the
+// high-byte MMA in x, y and of the low-byte MMA in z, w.
 struct Fragments {
   uint4 quant[8];
   uint2 sums;    // min-term fragment: fp16 pairs of S_j / 32, high halves in x, low halves in y
-  uint2 scales;  // fp32 bits of the activation scales of rows 2t and 2t+1
+  uint2 scales;  // fp32 bits of the activation scales of the rows of columns 2t and 2t+1
 };
 
-__device__ __forceinline__ Fragments load_fragments(const uint8_t* block, int lane) {
+template <int ROWS> __device__ __forceinline__ Fragments load_fragments(const uint8_t* block, int lane) {
+  constexpr int kShare = 8 / ROWS;
   Fragments f;
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll
   for (int j = 0; j < 8; ++j)
-    f.quant[j] = *reinterpret_cast<const uint4*>(block + j * 512 + g * 64 + t * 16);
+    f.quant[j] = g / ROWS == j % kShare ? *reinterpret_cast<const uint4*>(block + j * 512 + (g % ROWS) * 64 + t * 16) : make_uint4(0, 0, 0, 0);
   f.sums = *reinterpret_cast<const uint2*>(block + kImageSumOffset + lane * 8);
-  f.scales = *reinterpret_cast<const uint2*>(block + kImageScaleOffset + t * 8);
+  f.scales = *reinterpret_cast<const uint2*>(block + kImageScaleOffset + (2 * t % ROWS) * 4);
   return f;
 }
 
@@ -93,7 +98,11 @@ __device__ __forceinline__ Fragments load_fragments(const uint8_t* block, int la
 // nibbles the same values of sub-block 2c+1 (GGUF layout as read by dequant_tile, quant_linear.metal:39-46). The four
 // bytes of a word fill four consecutive summation slots of the MMA, which is the order the image stores the
 // activations in.
-__device__ __forceinline__ void q4k_unit(const uint8_t* pA, const uint8_t* pB, int t, const Fragments& f, float (&total)[4]) {
+// The integer sums are exact, and with fewer than eight rows they are completed over the lanes of a row before they are
+// rounded to fp32, so that a row has the same bits whatever ROWS. Only lanes with 2t < ROWS then hold results.
+template <int ROWS> __device__ __forceinline__ void q4k_unit(const uint8_t* pA, const uint8_t* pB, int t, const Fragments& f, float (&total)[4]) {
+  static_assert(ROWS == 1 || ROWS == 2 || ROWS == 8, "scale selection");
+  constexpr int kShare = 8 / ROWS;
   const uint4 hA = lds128(pA), hB = lds128(pB);
   // 6-bit scales / mins of the 8 sub-blocks, four per word (scale_min_k4, quant_linear.metal:12-20).
   const uint32_t scA[2] = {hA.y & 0x3f3f3f3fu, (hA.w & 0x0f0f0f0fu) | ((hA.y >> 2) & 0x30303030u)};
@@ -103,29 +112,53 @@ __device__ __forceinline__ void q4k_unit(const uint8_t* pA, const uint8_t* pB, i
   // 16 x the sum over the 8 sub-blocks of scale * (integer dot product), separately for the low and the high activation
   // byte: |low| <= 16 * 8 * 63 * 15 * 32 * 255 < 2^30 and |high| <= 16 * 8 * 63 * 15 * 32 * 128 both stay inside int32.
   int sumLow[4] = {0, 0, 0, 0}, sumHigh[4] = {0, 0, 0, 0};
+  int high[4], low[4];
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     const uint2 qA = lds64(pA + 16 + 32 * c + 8 * t), qB = lds64(pB + 16 + 32 * c + 8 * t);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int j = 2 * c + h;
+      const int j = 2 * c + h, set = ROWS == 2 ? j / kShare : 0;
       uint32_t a[4];
       // Low nibbles as they are, high nibbles in place as 16 q (still a byte); the sub-block scale of the low ones is
       // taken 16-fold instead, and the common factor leaves with d at the end.
       const uint32_t mask = h == 0 ? 0x0f0f0f0fu : 0xf0f0f0f0u;
       a[0] = qA.x & mask, a[1] = qB.x & mask, a[2] = qA.y & mask, a[3] = qB.y & mask;
       const uint4 b = f.quant[j];
-      int high[4], low[4];
+      if (j % kShare == 0)
+        high[0] = high[1] = high[2] = high[3] = low[0] = low[1] = low[2] = low[3] = 0;
       imma_u8s8(high, a, b.x, b.y);
       imma_u8u8(low, a, b.z, b.w);
-      const int byteA = int(__byte_perm(scA[j >> 2], 0u, 0x4440 + (j & 3))), byteB = int(__byte_perm(scB[j >> 2], 0u, 0x4440 + (j & 3)));
-      const int sA = h == 0 ? byteA * 16 : byteA, sB = h == 0 ? byteB * 16 : byteB;
+      if (j % kShare != kShare - 1)
+        continue;
+      if (ROWS == 1) {  // columns 2t and 2t + 1 are the sub-blocks of those numbers
+        const uint32_t pairA = (t & 2 ? scA[1] : scA[0]) >> (16 * (t & 1)), pairB = (t & 2 ? scB[1] : scB[0]) >> (16 * (t & 1));
+        const int evenA = int(pairA & 0xffu) * 16, oddA = int(pairA >> 8 & 0xffu), evenB = int(pairB & 0xffu) * 16, oddB = int(pairB >> 8 & 0xffu);
+        sumLow[0] = evenA * low[0] + oddA * low[1], sumHigh[0] = evenA * high[0] + oddA * high[1];
+        sumLow[2] = evenB * low[2] + oddB * low[3], sumHigh[2] = evenB * high[2] + oddB * high[3];
+        continue;
+      }
+      int sA, sB;
+      if (ROWS == 8) {
+        const int byteA = int(__byte_perm(scA[j >> 2], 0u, 0x4440 + (j & 3))), byteB = int(__byte_perm(scB[j >> 2], 0u, 0x4440 + (j & 3)));
+        sA = h == 0 ? byteA * 16 : byteA, sB = h == 0 ? byteB * 16 : byteB;
+      } else {  // sub-block 4 * set + t; even ones hold low nibbles
+        const int fold = t & 1 ? 0 : 4;
+        sA = int(scA[set] >> (8 * t) & 0xffu) << fold, sB = int(scB[set] >> (8 * t) & 0xffu) << fold;
+      }
       sumLow[0] += sA * low[0], sumHigh[0] += sA * high[0];
       sumLow[1] += sA * low[1], sumHigh[1] += sA * high[1];
       sumLow[2] += sB * low[2], sumHigh[2] += sB * high[2];
       sumLow[3] += sB * low[3], sumHigh[3] += sB * high[3];
     }
   }
+#pragma unroll
+  for (int lanes = 1; ROWS < 8 && lanes < 4; lanes *= 2)
+#pragma unroll
+    for (int i = 0; i < 4; i += ROWS == 1 ? 2 : 1) {
+      sumLow[i] += __shfl_xor_sync(0xffffffffu, sumLow[i], lanes);
+      sumHigh[i] += __shfl_xor_sync(0xffffffffu, sumHigh[i], lanes);
+    }
   // min term: sum_j m_j * S_j / 32; summation slots 0..7 carry the fp16 high halves of the sums, 8..15 the low halves.
   float accm[4] = {0.f, 0.f, 0.f, 0.f};
   {
@@ -141,9 +174,11 @@ __device__ __forceinline__ void q4k_unit(const uint8_t* pA, const uint8_t* pB, i
   const float2 dA = __half22float2(*reinterpret_cast<const __half2*>(&hA.x)), dB = __half22float2(*reinterpret_cast<const __half2*>(&hB.x));
   const float mA = 32.f * dA.y, mB = 32.f * dB.y, sixteenthA = 0.0625f * dA.x, sixteenthB = 0.0625f * dB.x;
   total[0] += xs0 * (sixteenthA * fmaf(float(sumHigh[0]), 256.f, float(sumLow[0])) - mA * accm[0]);
-  total[1] += xs1 * (sixteenthA * fmaf(float(sumHigh[1]), 256.f, float(sumLow[1])) - mA * accm[1]);
+  if (ROWS > 1)
+    total[1] += xs1 * (sixteenthA * fmaf(float(sumHigh[1]), 256.f, float(sumLow[1])) - mA * accm[1]);
   total[2] += xs0 * (sixteenthB * fmaf(float(sumHigh[2]), 256.f, float(sumLow[2])) - mB * accm[2]);
-  total[3] += xs1 * (sixteenthB * fmaf(float(sumHigh[3]), 256.f, float(sumLow[3])) - mB * accm[3]);
+  if (ROWS > 1)
+    total[3] += xs1 * (sixteenthB * fmaf(float(sumHigh[3]), 256.f, float(sumLow[3])) - mB * accm[3]);
 }
 
 __device__ __forceinline__ int find_segment(const GemvParams& p, int tile) {
@@ -153,7 +188,7 @@ __device__ __forceinline__ int find_segment(const GemvParams& p, int tile) {
   return s;
 }
 
-template <int NMAT> __global__ void __launch_bounds__(kThreads, 1) q4k_decode_kernel(const __grid_constant__ GemvParams p) {
+template <int NMAT, int ROWS> __global__ void __launch_bounds__(kThreads, 1) q4k_decode_kernel(const __grid_constant__ GemvParams p) {
   constexpr int kStages = stage_count<NMAT>();
   extern __shared__ __align__(128) uint8_t smemRaw[];
   Control& ctl = *reinterpret_cast<Control*>(smemRaw);
@@ -293,7 +328,7 @@ template <int NMAT> __global__ void __launch_bounds__(kThreads, 1) q4k_decode_ke
     const bool live = myBlock < chunkBlocks;
     Fragments fragments;
     if (live)
-      fragments = load_fragments(p.image + size_t(chunk * kChunkBlocks + myBlock) * kImageBlockBytes, lane);
+      fragments = load_fragments<ROWS>(p.image + size_t(chunk * kChunkBlocks + myBlock) * kImageBlockBytes, lane);
     int buffer = 0;
     for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, buffer = buffer == kFinisherWarps - 1 ? 0 : buffer + 1) {
       float total[NMAT][4];
@@ -317,9 +352,9 @@ template <int NMAT> __global__ void __launch_bounds__(kThreads, 1) q4k_decode_ke
         if (live) {
           const uint8_t* rows = ring + slot * kStageBytes + laneRow;
           if (NMAT == 2 && mat)
-            q4k_unit(rows, rows + 8 * kRowPitch, t, fragments, total[NMAT - 1]);
+            q4k_unit<ROWS>(rows, rows + 8 * kRowPitch, t, fragments, total[NMAT - 1]);
           else
-            q4k_unit(rows, rows + 8 * kRowPitch, t, fragments, total[0]);
+            q4k_unit<ROWS>(rows, rows + 8 * kRowPitch, t, fragments, total[0]);
         }
         __syncwarp();
         if (lane == 0)
@@ -364,25 +399,34 @@ __global__ void __launch_bounds__(256) activation_image_kernel(const float* x, i
   image_store_block(out, row, lane, v);
 }
 
-template <int NMAT> cudaError_t launch(const GemvParams& p, int sms, cudaStream_t stream) {
+template <int NMAT, int ROWS> cudaError_t launch(const GemvParams& p, int sms, cudaStream_t stream) {
   static PerDeviceOnce configured;
   constexpr size_t bytes = smem_bytes<NMAT>();
-  if (cudaError_t e = configure_shared_memory(q4k_decode_kernel<NMAT>, bytes, configured))
+  if (cudaError_t e = configure_shared_memory(q4k_decode_kernel<NMAT, ROWS>, bytes, configured))
     return e;
   const int grid = p.tiles < sms ? p.tiles : sms;
-  launch_kernel<1>(q4k_decode_kernel<NMAT>, grid, kThreads, bytes, stream, p);
+  launch_kernel<1>(q4k_decode_kernel<NMAT, ROWS>, grid, kThreads, bytes, stream, p);
   return cudaGetLastError();
+}
+
+// One or two rows pay for their own columns only: 12288 x 4096 with its image launch 12.5 -> 11.0 us at one row, 11.5 at two;
+// all projections of a layer 54.4 -> 48.8 and 52.7 us. Four rows in two sub-blocks a column set measured 56.4 us against 55.0
+// (the fragments and eight sums of two sets spill at 96 registers), so three rows and more take the plain columns.
+template <int NMAT> cudaError_t launch_rows(const GemvParams& p, int sms, cudaStream_t stream) {
+  return p.m <= 1   ? launch<NMAT, 1>(p, sms, stream)
+         : p.m == 2 ? launch<NMAT, 2>(p, sms, stream)
+                    : launch<NMAT, 8>(p, sms, stream);
 }
 
 }  // namespace
 
 cudaError_t q4k_decode_launch(bool pair, const GemvParams& p, int sms, cudaStream_t stream) {
-  return pair ? launch<2>(p, sms, stream) : launch<1>(p, sms, stream);
+  return pair ? launch_rows<2>(p, sms, stream) : launch_rows<1>(p, sms, stream);
 }
 
 cudaError_t activation_image_launch(const float* x, int ldx, int m, int k, uint8_t* image, cudaStream_t stream) {
   const int blocks = k / 256;
-  launch_kernel<2>(activation_image_kernel, (blocks * kImageRows + 7) / 8, 256, 0, stream, x, ldx, m, blocks, image);
+  launch_kernel<1>(activation_image_kernel, (blocks * kImageRows + 7) / 8, 256, 0, stream, x, ldx, m, blocks, image);
   return cudaGetLastError();
 }
 

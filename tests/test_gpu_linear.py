@@ -213,3 +213,23 @@ def test_embedding_and_rms_norm(dev):
   y = dev.empty((rows, k))
   dev.rms_norm(dev.array(x), dev.array(w), rows, k, y)
   assert rel_err(y.download(), oracle.rms_norm(x, w)) < 1e-5
+
+
+@pytest.mark.parametrize("n,k", [(16, 256), (48, 4096), (2400, 2048), (160, 12288)])
+def test_a_row_has_the_same_bits_in_every_width(dev, n, k):
+  """One and two rows put several sub-blocks into the columns of an MMA; their sums are integers, completed before they are
+  rounded, so a row alone, in a pair or among eight gives the same bits (and those match the oracle)."""
+  w, x = synth.weight(D.Q4_K, n, k, 51), synth.activations(8, k, 52)
+  alone = {m: run_linear(dev, D.Q4_K, n, k, m, 0, x=x[:m].copy(), w=w) for m in (1, 2, 3, 8)}
+  for m, (got, want) in alone.items():
+    assert rel_err(got, want) < 2e-4
+    assert got.tobytes() == alone[8][0][:m].tobytes(), m
+
+
+@pytest.mark.parametrize("m", [1, 2])
+def test_gate_up_of_one_and_two_rows(dev, m):
+  n, k = 272, 4096
+  wg, wu, x = synth.weight(D.Q4_K, n, k, 53), synth.weight(D.Q4_K, n, k, 54), synth.activations(m, k, 55)
+  y = dev.empty((m, n))
+  dev.gate_up(D.Q4_K, dev.array(wg), dev.array(wu), n, k, dev.array(x), m, y)
+  assert rel_err(y.download(), oracle.gate_up(wg, wu, D.Q4_K, n, k, x)) < 2e-4
