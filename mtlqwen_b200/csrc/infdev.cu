@@ -44,7 +44,7 @@ namespace infdev {
 int pdl_mode() {
   static const int mode = [] {
     const char* env = std::getenv("INFENG_PDL");
-    return env ? std::atoi(env) : 2;
+    return env ? std::atoi(env) : 3;
   }();
   return mode;
 }

@@ -441,13 +441,13 @@ template <int NMAT> cudaError_t launch_tiles(const UmmaParams& params, const flo
   // per super-block instead of 64 KB and spends a third of the tensor time.
   UmmaParams p = params;
   p.actRows = (p.m + 15) / 16 * 16;
-  launch_kernel(umma_prepare_rows_kernel, dim3(p.k / 256, p.actRows / 8), 256, 0, stream, x, ldx, p.m, p.actRows,
+  launch_kernel<1>(umma_prepare_rows_kernel, dim3(p.k / 256, p.actRows / 8), 256, 0, stream, x, ldx, p.m, p.actRows,
                 reinterpret_cast<__half*>(const_cast<uint8_t*>(p.acts)));
   const int items = p.tiles * p.splits, grid = items < sms ? items : sms;
   launch_kernel<1>(umma_linear_kernel<NMAT>, grid, kThreads, kSharedBytes, stream, p);
   if (p.splits > 1) {
     const size_t count = size_t(p.m) * p.seg[0].ldy;
-    launch_kernel(umma_reduce_kernel, unsigned((count / 4 + 255) / 256), 256, 0, stream, p.partial, p.splits, count, p.seg[0].res, p.seg[0].y);
+    launch_kernel<1>(umma_reduce_kernel, unsigned((count / 4 + 255) / 256), 256, 0, stream, p.partial, p.splits, count, p.seg[0].res, p.seg[0].y);
   }
   return cudaGetLastError();
 }
