@@ -273,6 +273,10 @@ template <class Q, int NMAT, int XSPLIT> __global__ void __launch_bounds__(kThre
         }
       }
     }
+    if (lane == 0)  // no copy may be in flight when the CTA ends, whoever gave up
+      for (uint32_t i = it > uint32_t(kStages) ? it - kStages : 0; i < it; ++i)
+        mbar_wait_bounded(&ctl.full[i % kStages], (i / kStages) & 1, abortFlag);
+    __syncwarp();
     pdl_wait();  // every thread of every kernel waits, so completion stays transitive along the stream
     return;
   }

@@ -47,7 +47,9 @@ static_assert(sizeof(Control) <= kControlBytes, "control block overlaps the part
 template <int NMAT> constexpr size_t fixed_bytes() { return kControlBytes + size_t(kFinisherWarps) * NMAT * kConsumerWarps * 128 * 4; }
 template <int NMAT> constexpr int stage_count() {
   int stages = int((size_t(227) * 1024 - fixed_bytes<NMAT>()) / kStageBytes);
-  return stages > kMaxStages ? kMaxStages : stages;
+  // Even, so that a slot always belongs to the same half of the consumers: a half that ran ahead in a slot of the other one could
+  // find the parity of the phase before last and read the slot ahead of its own copy.
+  return (stages > kMaxStages ? kMaxStages : stages) / 2 * 2;
 }
 template <int NMAT> constexpr size_t smem_bytes() { return fixed_bytes<NMAT>() + size_t(stage_count<NMAT>()) * kStageBytes; }
 
@@ -245,6 +247,9 @@ template <int NMAT, int ROWS> __global__ void __launch_bounds__(kThreads, 1) q4k
           }
         }
       }
+      // no copy may be in flight when the CTA ends, whoever gave up
+      for (uint32_t i = it > uint32_t(kStages) ? it - kStages : 0; i < it; ++i)
+        mbar_wait_bounded(&ctl.full[i % kStages], (i / kStages) & 1, abortFlag);
     }
     __syncwarp();
     pdl_wait();  // every thread of every kernel waits, so completion stays transitive along the stream

@@ -15,9 +15,9 @@
 // TMEM lane quadrant each), 12..15 = epilogue. Every mbarrier wait is bounded; on a timeout the kernel raises an abort
 // flag, records a status code, and every role leaves its loops.
 // The fp16 activations of a super-block are 64 KB, so weight slabs and activations travel through separate rings, the
-// activations in two halves of eight k-steps each: 3 slab stages + 5 half stages keep two and a half super-blocks in
-// flight. The producer warp first asks the L2 for the whole tile (and the next one of this CTA) with bulk prefetches,
-// which need no shared memory, so that three 18 KB slab copies in flight are enough.
+// activations in two halves of eight k-steps each: 4 slab stages + 4 half stages. The producer warp first asks the L2 for the
+// whole tile (and the next one of this CTA) with bulk prefetches, which need no shared memory, so that few 18 KB slab copies
+// in flight are enough.
 // The kernel is launched programmatically dependent on the kernel that lays out the activations: set-up, the
 // prefetches and the first weight slab run while that one is still at work, and only the activation copies and the
 // epilogue wait for it.
@@ -33,7 +33,10 @@ constexpr int kRows = kUmmaTileRows;      // weight rows per tile = TMEM lanes
 constexpr int kActs = 128;                // most activation rows per launch; the MMA N is the live rows rounded up to 16
 constexpr int kSlabBytes = kRows * 144;   // 18,432
 constexpr int kThreads = 512;
-constexpr int kStages = 3, kActStages = 5;
+// An even number of slab slots: a slot then always belongs to the same dequant group. With three, a group could find the parity of
+// the phase before last in a slot whose slab for the other group had not landed yet, and read it ahead of its own copy.
+constexpr int kStages = 4, kActStages = 4;
+static_assert(kStages % 2 == 0, "a slot serves one dequant group");
 constexpr int kActHalfBytes = 8 * kActs * 16 * 2;  // ring stage: 8 k-steps x [128 x 16] fp16; a launch of N rows uses N x 256 of it
 // kind::f16 instruction descriptor: fp32 accumulate, fp16 A and B, both K-major, M = 128
 __device__ __forceinline__ uint32_t instruction_descriptor(int n) { return (1u << 4) | (uint32_t(n >> 3) << 17) | (uint32_t(kRows >> 4) << 24); }
@@ -199,7 +202,7 @@ template <int NMAT> __global__ void __launch_bounds__(kThreads, 1) umma_linear_k
     if (int(blockIdx.x) < items)
       prefetch(blockIdx.x);
     const uint32_t halfBytes = uint32_t(p.actRows) * 256;  // 8 k-steps x [actRows x 16] fp16
-    uint32_t it = 0;
+    uint32_t it = 0, slabs = 0, halves = 0;  // slabs, halves: copies issued
     bool ok = true, waited = false;
     for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
       if (item + int(gridDim.x) < items)
@@ -218,6 +221,7 @@ template <int NMAT> __global__ void __launch_bounds__(kThreads, 1) umma_linear_k
             if (ok) {
               mbar_arrive_expect_tx(&ctl.full[slot], kSlabBytes);
               tma_load_2d(ring + size_t(slot) * kSlabBytes, &p.map[segment][mat], sb * 18, row0, &ctl.full[slot]);
+              ++slabs;
             }
             if (!waited) {  // the activations are the preceding kernel's output
               pdl_wait();
@@ -230,6 +234,7 @@ template <int NMAT> __global__ void __launch_bounds__(kThreads, 1) umma_linear_k
               if (ok) {
                 mbar_arrive_expect_tx(&ctl.actFull[actSlot], halfBytes);
                 bulk_load(actRing + size_t(actSlot) * kActHalfBytes, p.acts + (size_t(sb) * 2 + h) * halfBytes, halfBytes, &ctl.actFull[actSlot]);
+                ++halves;
               }
             }
             if (!ok) {
@@ -239,6 +244,13 @@ template <int NMAT> __global__ void __launch_bounds__(kThreads, 1) umma_linear_k
           }
           ok = __shfl_sync(0xffffffffu, ok, 0);
         }
+    }
+    // no copy may be in flight when the CTA ends, whoever gave up
+    if (lane == 0) {
+      for (uint32_t i = slabs > uint32_t(kStages) ? slabs - kStages : 0; i < slabs; ++i)
+        mbar_wait_bounded(&ctl.full[i % kStages], (i / kStages) & 1, abortFlag);
+      for (uint32_t i = halves > uint32_t(kActStages) ? halves - kActStages : 0; i < halves; ++i)
+        mbar_wait_bounded(&ctl.actFull[i % kActStages], (i / kActStages) & 1, abortFlag);
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (lane 0) ----------------

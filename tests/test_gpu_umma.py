@@ -74,3 +74,26 @@ def test_prefill_k_slices(umma):
   assert umma.launch_count - before == 3
   umma.linear(D.Q4_K, w, n, k, x, m, b, res)
   assert a.download().tobytes() == b.download().tobytes()
+
+
+def test_every_sm_streaming_a_matrix_larger_than_the_l2(umma):
+  """148 tiles of 64 super-blocks, 174 MB of weights: slabs land out of order, and a dequant group must not take an earlier
+  group's slab for its own. Against the GEMV in slices of eight rows, several times over."""
+  n, k, m = 18944, 16384, 128
+  w = umma.array(np.tile(synth.weight(D.Q4_K, n // 64, k, 950), (64, 1)))
+  x = umma.array(synth.activations(m, k, 951))
+  want, got = umma.empty((m, n)), umma.empty((m, n))
+  umma.set_umma(0)
+  try:
+    umma.linear(D.Q4_K, w, n, k, x, m, want)
+    umma.commit()
+  finally:
+    umma.set_umma(1)
+  first = None
+  for _ in range(8):
+    umma.linear(D.Q4_K, w, n, k, x, m, got)
+    umma.commit()
+    result = got.download()
+    first = result if first is None else first
+    assert result.tobytes() == first.tobytes()
+  assert rel_err(first, want.download()) < TOL
