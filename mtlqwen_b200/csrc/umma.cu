@@ -21,8 +21,8 @@
 // The kernel is launched programmatically dependent on the kernel that lays out the activations: set-up, the
 // prefetches and the first weight slab run while that one is still at work, and only the activation copies and the
 // epilogue wait for it.
-// Measured at 12288 x 4096 x 128 rows: 1.18 us per super-block (the 16 MMAs of a super-block keep the tensor pipe busy
-// for about two thirds of that), 31 us per call of which 4 us are the layout kernel; 96 tiles occupy 96 of 148 SMs.
+// Measured at 128 rows: 0.93 us per super-block, of which the 16 MMAs are 0.55 (64 cycles each; 11 at 16 rows, 0.84 us per
+// super-block), the rest the dequantisation; 96 tiles (n = 12288) occupy 96 of 148 SMs.
 #include "common.cuh"
 #include "kernels.h"
 
@@ -62,6 +62,14 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t columns) {
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t base, uint32_t columns) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(columns) : "memory");
+}
+// One lane of the calling warp. In code under `lane == 0` the compiler must expect several active lanes and wraps every MMA,
+// whose operands are uniform registers, in a loop over them: 93 cycles an instruction whatever its size. Under elect.sync it
+// knows that there is one.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t elected;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
+  return elected != 0;
 }
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -152,7 +160,7 @@ template <int NMAT> __global__ void __launch_bounds__(kThreads, 1) umma_linear_k
   uint8_t* actRing = ring + size_t(kStages) * kSlabBytes;  // halves of a super-block's activations
 
   pdl_launch_dependents();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   // With p.splits > 1 (one matrix) the work items are (tile, K slice) pairs, so that a matrix of few 128-row tiles still
   // fills the GPU; `blocksPerRow` is then the super-blocks of one slice. One accumulator buffer per (item, matrix).
   const int blocksPerRow = p.k / 256 / p.splits, items = p.tiles * p.splits;
@@ -253,8 +261,8 @@ template <int NMAT> __global__ void __launch_bounds__(kThreads, 1) umma_linear_k
         mbar_wait_bounded(&ctl.actFull[i % kActStages], (i / kActStages) & 1, abortFlag);
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer (lane 0) ----------------
-    if (lane == 0) {
+    // ---------------- MMA issuer (one lane) ----------------
+    if (elect_one()) {
       uint32_t it = 0, unit = 0;
       bool ok = true;
       const uint32_t instruction = instruction_descriptor(p.actRows), stepBytes = uint32_t(p.actRows) * 32;
