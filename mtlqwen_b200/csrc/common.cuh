@@ -74,6 +74,15 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// One lane of the calling warp, for instructions that one thread issues and whose operands are uniform registers (tcgen05.mma,
+// bulk and tiled copies). In code under `lane == 0` the compiler must expect several active lanes and wraps such an
+// instruction in a loop over them (93 cycles for an MMA whatever its size); under elect.sync it knows that there is one.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t elected;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
+  return elected != 0;
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
