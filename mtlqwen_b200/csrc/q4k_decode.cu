@@ -197,7 +197,7 @@ template <int NMAT, int ROWS> __global__ void __launch_bounds__(kThreads, 1) q4k
   float* partial = reinterpret_cast<float*>(smemRaw + kControlBytes);
   uint8_t* ring = reinterpret_cast<uint8_t*>(partial + kFinisherWarps * NMAT * kConsumerWarps * 128);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int blocksPerRow = p.k / 256;
   const int chunks = (blocksPerRow + kChunkBlocks - 1) / kChunkBlocks;
 
@@ -220,7 +220,7 @@ template <int NMAT, int ROWS> __global__ void __launch_bounds__(kThreads, 1) q4k
   if (warp == kProducerWarp) {
     // ---- producer (one thread): weight slabs into the ring. The weights do not depend on the kernels before this
     // one, so the ring fills while they finish.
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (int chunk = 0; chunk < chunks && ok; ++chunk) {
