@@ -18,11 +18,13 @@
 //
 // What bounds it: shared memory and the tensor pipe together. A group of 16 k x 16 weights x 8 rows is 16 cycles of MMA and 16
 // cycles of a scheduler's share of the fragment reads; with four tiles a unit (16 rows x 256 k) takes a scheduler 1.0 to 1.3
-// us of which the MMAs are 0.57. Slices of eight rows against this kernel: Q6_K output head 248320 x 4096, 16 rows 481 -> 307
-// us, 40 rows 1180 -> 790 us; projections of a layer of mixed types, 16 rows 176 -> 135 us, 40 rows 440 -> 241 us, 128 rows
-// 1410 -> 577 us. At nine rows 176 -> 123 us for the layer, which is why it starts there. A chunk's sum is added to what
+// us of which the MMAs are 0.57. Slices of eight rows against this kernel: Q6_K output head 248320 x 4096, 16 rows 481 -> 304
+// us, 40 rows 1180 -> 650 us; projections of a layer of mixed types, 16 rows 176 -> 126 us, 40 rows 440 -> 216 us, 128 rows
+// 1410 -> 544 us. At nine rows 176 -> 119 us for the layer, which is why it starts there. A chunk's sum is added to what
 // rests in the result at the chunk's end: fetching that first and adding on top hid the latency (530 us at 128 rows) but lost
-// accuracy (Q6_K, K = 12288: 2.0e-7 against fp64; 1.3e-7 now, 1.4e-7 for the slices).
+// accuracy (Q6_K, K = 12288: 2.0e-7 against fp64; 1.3e-7 now, 1.4e-7 for the slices). The warp index is made warp-uniform for
+// the compiler (__shfl_sync): without it the roles' addresses take registers of every lane and five tiles spilled (40 rows of
+// the head 790 us).
 #include <algorithm>
 #include <type_traits>
 #include "gemv_units.cuh"
@@ -170,7 +172,7 @@ template <class Q, int NT> __global__ void __launch_bounds__(kThreads, 1) wide_k
   uint8_t* image = smem + kControlBytes;
   uint8_t* ring = image + resident_bytes<Q, NT>();  // [kDepth][warp]
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   if (tid == 0) {
     for (int s = 0; s < kDepth * kConsumerWarps; ++s) {
       mbar_init(&ctl.full[s / kConsumerWarps][s % kConsumerWarps], 1);
