@@ -126,7 +126,7 @@ template <int NT, class B> __device__ __forceinline__ void q8_unit(const uint8_t
   constexpr uint32_t k1152 = 0x64806480u;
   float sum[NT][4];
   clear(sum);
-#pragma unroll(NT > 3 ? 2 : NT > 2 ? 4 : 8)
+#pragma unroll(NT > 4 ? 2 : NT > 2 ? 4 : 8)
   for (int j = 0; j < 8; ++j) {
     uint32_t a[2][4];
 #pragma unroll
@@ -159,7 +159,7 @@ template <int NT, class B> __device__ __forceinline__ void iq4_unit(const uint8_
   const uint2 hA = *reinterpret_cast<const uint2*>(pA), hB = *reinterpret_cast<const uint2*>(pB);
   float sum[NT][4];
   clear(sum);
-#pragma unroll(NT > 3 ? 2 : NT > 2 ? 4 : 8)
+#pragma unroll(NT > 4 ? 2 : NT > 2 ? 4 : 8)
   for (int j = 0; j < 8; ++j) {
     const uint2 qA = iq4_lookup(lds_u32(pA + 8 + 16 * j + 4 * t)), qB = iq4_lookup(lds_u32(pB + 8 + 16 * j + 4 * t));
     uint32_t a[2][4];
@@ -195,7 +195,7 @@ __device__ __forceinline__ void q6k_unit(const uint8_t* pA, const uint8_t* pB, i
   constexpr uint32_t k1056 = 0x64206420u;
 #pragma unroll(NT > 2 ? 1 : 2)
   for (int hh = 0; hh < 2; ++hh) {
-#pragma unroll(NT > 3 ? 1 : 2)
+#pragma unroll(NT > 4 ? 1 : 2)
     for (int u = 0; u < 2; ++u) {
       const uint32_t hiA = lds_u32_unaligned(pA + 128 + 32 * hh + 16 * u + 4 * t), hiB = lds_u32_unaligned(pB + 128 + 32 * hh + 16 * u + 4 * t);
 #pragma unroll
