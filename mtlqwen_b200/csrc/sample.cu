@@ -468,7 +468,7 @@ cudaError_t sample_launch(const float* logits, int vocab, infdev_query* queries,
                           cudaStream_t stream) {
   if (count <= 0)
     return cudaSuccess;
-  launch_kernel(sample_kernel, dim3(kClusterCtas, unsigned(count)), kClusterThreads, 0, stream, logits, vocab, queries, mode, tokens);
+  launch_kernel<2>(sample_kernel, dim3(kClusterCtas, unsigned(count)), kClusterThreads, 0, stream, logits, vocab, queries, mode, tokens);
   return cudaGetLastError();
 }
 

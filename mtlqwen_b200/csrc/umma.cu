@@ -216,10 +216,10 @@ template <int NMAT, int GROUPS> __global__ void __launch_bounds__(kThreads<GROUP
       while (segment + 1 < p.nseg && tile >= p.seg[segment + 1].tile0)
         ++segment;
       const int row0 = (tile - p.seg[segment].tile0) * kRows;
-      for (int mat = 0; mat < NMAT && ok; ++mat)
-        for (int sb = firstBlock; sb < firstBlock + blocksPerRow && ok; ++sb, ++it) {
-          const uint32_t slot = it % kStages, round = it / kStages;
-          if (lane == 0) {
+      if (elect_one())  // the same lane every time: it keeps the counters
+        for (int mat = 0; mat < NMAT && ok; ++mat)
+          for (int sb = firstBlock; sb < firstBlock + blocksPerRow && ok; ++sb, ++it) {
+            const uint32_t slot = it % kStages, round = it / kStages;
             if (round > 0)
               ok = mbar_wait_bounded(&ctl.slotFree[slot], (round - 1) & 1, abortFlag);
             if (ok) {
@@ -246,11 +246,10 @@ template <int NMAT, int GROUPS> __global__ void __launch_bounds__(kThreads<GROUP
               atomicExch(p.status, kStatusBarrierTimeout);
             }
           }
-          ok = __shfl_sync(0xffffffffu, ok, 0);
-        }
+      ok = __all_sync(0xffffffffu, ok);
     }
     // no copy may be in flight when the CTA ends, whoever gave up
-    if (lane == 0) {
+    if (elect_one()) {
       for (uint32_t i = slabs > uint32_t(kStages) ? slabs - kStages : 0; i < slabs; ++i)
         mbar_wait_bounded(&ctl.full[i % kStages], (i / kStages) & 1, abortFlag);
       for (uint32_t i = halves > uint32_t(kActStages) ? halves - kActStages : 0; i < halves; ++i)
