@@ -597,12 +597,27 @@ __device__ __forceinline__ void chunk_prepare(ChunkShared& sh, const infdev_quer
   }
 }
 
+// Which query the CTAs of row `rank` of the grid take: the one with the rank-th largest count, so that the longest chains start
+// first and the short ones fill the SMs that are left over (eight queries of 59 to 493 rows, 256 CTAs on 148 SMs: 323 us in
+// the order of the pass, 281 us sorted). Every lane of a warp calls; beyond 32 queries the order of the pass stays.
+__device__ __forceinline__ uint32_t query_by_length(const infdev_query* queries, uint32_t count, uint32_t rank) {
+  if (count > 32)
+    return rank;
+  const uint32_t lane = threadIdx.x & 31, mine = lane < count ? queries[lane].count : 0u;
+  uint32_t before = 0;
+  for (uint32_t j = 0; j < count; ++j) {
+    const uint32_t other = __shfl_sync(0xffffffffu, mine, j);
+    before += other > mine || (other == mine && j < lane) ? 1u : 0u;
+  }
+  return uint32_t(__ffs(__ballot_sync(0xffffffffu, lane < count && before == rank)) - 1);
+}
+
 __global__ void __launch_bounds__(kChunkThreads, 1)
     delta_rule_chunked_kernel(const float* q, const float* k, const float* v, const float* g, const float* beta, const float* z, const float* normWeight,
                               const infdev_query* queries, uint64_t stateOffset, float* out, uint32_t chunkedFrom) {
   pdl_launch_dependents();
   pdl_wait();
-  const infdev_query info = queries[blockIdx.y];
+  const infdev_query info = queries[query_by_length(queries, gridDim.y, blockIdx.y)];
   if (info.state != kUnbound || info.count < chunkedFrom)  // delta_rule_kernel takes this query
     return;
   extern __shared__ __align__(16) uint8_t chunkRaw[];
@@ -804,10 +819,10 @@ cudaError_t delta_rule_launch(const float* q, const float* k, const float* v, co
     static PerDeviceOnce configured;
     if (cudaError_t e = configure_shared_memory(delta_rule_chunked_kernel, sizeof(ChunkShared), configured))
       return e;
-    launch_kernel(delta_rule_chunked_kernel, dim3(kValueHeads, unsigned(queryCount)), kChunkThreads, sizeof(ChunkShared), stream, q, k, v, g, beta, z, normWeight,
+    launch_kernel<2>(delta_rule_chunked_kernel, dim3(kValueHeads, unsigned(queryCount)), kChunkThreads, sizeof(ChunkShared), stream, q, k, v, g, beta, z, normWeight,
                   queries, stateOffset, out, chunkedFrom);
   }
-  launch_kernel(delta_rule_kernel<false>, dim3(kValueHeads, unsigned(queryCount)), 256, 0, stream, q, k, v, g, beta, z, normWeight, queries, stateOffset,
+  launch_kernel<2>(delta_rule_kernel<false>, dim3(kValueHeads, unsigned(queryCount)), 256, 0, stream, q, k, v, g, beta, z, normWeight, queries, stateOffset,
                 stateBytes, out, image, counters, chunkedFrom, GdnInputs{});
   return cudaGetLastError();
 }
