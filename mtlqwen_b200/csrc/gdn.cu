@@ -822,7 +822,9 @@ cudaError_t delta_rule_launch(const float* q, const float* k, const float* v, co
     launch_kernel<2>(delta_rule_chunked_kernel, dim3(kValueHeads, unsigned(queryCount)), kChunkThreads, sizeof(ChunkShared), stream, q, k, v, g, beta, z, normWeight,
                   queries, stateOffset, out, chunkedFrom);
   }
-  launch_kernel<2>(delta_rule_kernel<false>, dim3(kValueHeads, unsigned(queryCount)), 256, 0, stream, q, k, v, g, beta, z, normWeight, queries, stateOffset,
+  // Not launched early: its CTAs would be placed around those of the kernels before it, two on an SM, and the token-by-token chain
+  // of short queries runs slower for it (12 rows: 37.5 against 31.0 us; passes that the chunked kernel takes lose 1 us).
+  launch_kernel(delta_rule_kernel<false>, dim3(kValueHeads, unsigned(queryCount)), 256, 0, stream, q, k, v, g, beta, z, normWeight, queries, stateOffset,
                 stateBytes, out, image, counters, chunkedFrom, GdnInputs{});
   return cudaGetLastError();
 }
