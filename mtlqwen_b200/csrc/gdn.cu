@@ -467,11 +467,12 @@ __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint3
   const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
   lo = pack_half2(a - f.x, b - f.y);
 }
-// 2^n that brings the warp's largest magnitude into [512, 1024), and 2^-n
+// 2^n that brings the warp's largest magnitude into [512, 1024), and 2^-n. Both are normal numbers, whatever the magnitude is:
+// the exponent fields lie in 1 .. 253 (all zero: 2^126 and 2^-126).
 __device__ __forceinline__ float2 warp_unit(float largest) {
   largest = warp_max(largest);
-  const int field = min(254, max(1, 263 - int(__float_as_uint(largest) >> 23)));
-  return make_float2(__uint_as_float(uint32_t(field) << 23), __uint_as_float(uint32_t(max(1, 254 - field)) << 23));
+  const int field = min(253, max(1, 263 - int(__float_as_uint(largest) >> 23)));
+  return make_float2(__uint_as_float(uint32_t(field) << 23), __uint_as_float(uint32_t(254 - field) << 23));
 }
 // The two 16 x 8 accumulators of 16 x 16 values (C fragments) x unit as the A operand, hi and lo.
 __device__ __forceinline__ void split_tile(const float (&c0)[4], const float (&c1)[4], float unit, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
@@ -629,8 +630,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
   }
   const int row = lane >> 2, t2 = 2 * (lane & 3), column = 16 * warp + row;  // value columns `column` and `column` + 8
   const int tokenOfB = (lane & 7) + 8 * (lane >> 4), dimOfB = 8 * ((lane >> 3) & 1);
-  // S^T x unit: tile j holds key dims 8j + t2, + 1 of the two value columns
-  float S[kHeadDim / 8][4], inverse = 1.f;  // inverse of unit
+  float S[kHeadDim / 8][4];  // S^T: tile j holds key dims 8j + t2, + 1 of the two value columns
   const size_t state = size_t(head) * kHeadDim * kHeadDim + column;
 #pragma unroll
   for (int j = 0; j < kHeadDim / 8; ++j)
@@ -681,7 +681,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
       chunk_ldmatrix(bLo, &in.q[1][tokenOfB][16 * s + dimOfB]);
       mma_three(qs[0], qs[1], hi, lo, bHi, bLo);
     }
-    const float productUnit = stateUnit.y * inverse * (1.0f / kKeyUnit);
+    const float productUnit = stateUnit.y * (1.0f / kKeyUnit);
     float decay[2][2];
 #pragma unroll
     for (int n = 0; n < 2; ++n)
@@ -724,18 +724,18 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
     chunk_ldmatrix(bLo, &in.mix[1][tokenOfB][dimOfB]);
     mma_three(mixed[0], mixed[1], hi, lo, bHi, bLo);
     split_tile(update[0], update[1], scale.x, hi, lo);
-    {
-      const float rescale = in.decay[kChunk - 1] * scale.x * kKeyUnit * inverse;
-#pragma unroll
-      for (int j = 0; j < kHeadDim / 8; ++j)
-        S[j][0] *= rescale, S[j][1] *= rescale, S[j][2] *= rescale, S[j][3] *= rescale;
-      inverse = scale.y * (1.0f / kKeyUnit);
-    }
+    // The sum over the tokens starts from zero and is scaled before it meets the state, which stays in units of its own: deltas
+    // may be zero or any number of powers of two smaller than the state (beta = 0, value columns without weights).
+    const float stateDecay = in.decay[kChunk - 1], updateUnit = scale.y * (1.0f / kKeyUnit);
 #pragma unroll
     for (int s = 0; s < kHeadDim / 16; ++s) {
+      float added[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
       chunk_ldmatrix_trans(bHi, &in.k[0][lane & 15][16 * s + 8 * (lane >> 4)]);
       chunk_ldmatrix_trans(bLo, &in.k[1][lane & 15][16 * s + 8 * (lane >> 4)]);
-      mma_three(S[2 * s], S[2 * s + 1], hi, lo, bHi, bLo);
+      mma_three(added[0], added[1], hi, lo, bHi, bLo);
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        S[2 * s][e] = fmaf(added[0][e], updateUnit, S[2 * s][e] * stateDecay), S[2 * s + 1][e] = fmaf(added[1][e], updateUnit, S[2 * s + 1][e] * stateDecay);
     }
     named_barrier_arrive(3 + (step & 1), kChunkThreads);  // the buffer may be refilled
     // o, its gated norm over the head's 128 columns (gated_rms_norm_128), and the store
@@ -786,7 +786,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
   for (int j = 0; j < kHeadDim / 8; ++j)
 #pragma unroll
     for (int e = 0; e < 4; ++e)
-      reinterpret_cast<float*>(info.next + stateOffset)[state + (8 * j + t2 + (e & 1)) * kHeadDim + 8 * (e >> 1)] = S[j][e] * inverse;
+      reinterpret_cast<float*>(info.next + stateOffset)[state + (8 * j + t2 + (e & 1)) * kHeadDim + 8 * (e >> 1)] = S[j][e];
 }
 
 }  // namespace

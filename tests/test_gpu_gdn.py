@@ -150,6 +150,50 @@ def test_gdn_chunked_agrees_with_sequential(dev):
   assert a < TOL and b < TOL and abs(a - b) < 2e-4
 
 
+def run_rule(dev, q, k, v, g, beta, S0, prefill=True):
+  """One query through the recurrence alone (no preparation, no gated norm): outputs and the final state."""
+  T = v.shape[0]
+  previous, next_, out = dev.array(S0.astype(np.float32)), dev.empty((32, 128, 128)), dev.empty((T, 32, 128))
+  info = D.Query()
+  info.previous, info.next, info.start, info.count, info.position, info.slot, info.state = previous.ptr, next_.ptr, 0, T, 77, 0, D.UNBOUND
+  inputs = [dev.array(np.asarray(a, np.float32)) for a in (q, k, v, g, beta)]
+  dev.delta_rule(*inputs, None, None, dev.queries([info]), 1, 0, LAYER, out, prefill=prefill)
+  dev.commit()
+  return out.download(), next_.download()
+
+
+def rule_inputs(rng, T, decay=0.05):
+  g = -decay * rng.uniform(0.2, 1.8, (T, 32))
+  return [rng.standard_normal((T, 16, 128)), rng.standard_normal((T, 16, 128)), rng.standard_normal((T, 32, 128)), g, rng.uniform(0.1, 0.9, (T, 32)),
+          0.5 * rng.standard_normal((32, 128, 128))]
+
+
+@pytest.mark.parametrize("what", ["beta 0, no decay", "fresh state, v 0", "a block of 16 columns", "one column", "a chunk of zeros behind others", "deltas of 1e-36",
+                                  "everything 0"])
+def test_chunk_whose_deltas_are_zero_leaves_the_state_alone(dev, what):
+  """The chunked form scales deltas to the range of fp16: zero ones, or ones far below the state, must not disturb the state."""
+  rng = np.random.default_rng(20)
+  q, k, v, g, beta, S = rule_inputs(rng, 50)
+  if what == "beta 0, no decay":
+    beta[16:], g[16:] = 0.0, 0.0
+  elif what == "fresh state, v 0":
+    S[:], v[:] = 0.0, 0.0
+  elif what == "a block of 16 columns":
+    S[:, :, 32:48], v[:, :, 32:48] = 0.0, 0.0
+  elif what == "one column":
+    S[:, :, 77], v[:, :, 77] = 0.0, 0.0
+  elif what == "a chunk of zeros behind others":
+    q[16:32], k[16:32], v[16:32] = 0.0, 0.0, 0.0
+  elif what == "deltas of 1e-36":
+    beta[:] *= 1e-36
+  else:
+    q[:], k[:], v[:], g[:], beta[:], S[:] = 0.0, 0.0, 0.0, 0.0, 0.0, 0.0
+  out, state = run_rule(dev, q, k, v, g, beta, S)
+  want_out, want_state, _ = oracle.delta_rule(q, k, v, g, beta, S)
+  assert np.isfinite(out).all() and np.isfinite(state).all()
+  assert rel_err(out, want_out) < 1e-5 and rel_err(state, want_state) < 1e-5
+
+
 def test_prefill_variant_refuses_an_image(dev):
   dev.image_capture(dev.empty(dev.image_bytes(8, 4096), np.uint8))
   with pytest.raises(RuntimeError, match="no image"):
