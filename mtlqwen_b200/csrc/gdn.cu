@@ -448,7 +448,9 @@ struct ChunkBuffer {
 };
 struct ChunkShared {
   ChunkBuffer buffer[2];
-  float cumulative[kChunk], gateBeta[kChunk];  // of the chunk being prepared
+  // of the chunk being prepared, two sets in turn: warp 1 reads one while warp 0 may already write the next chunk's, and a set
+  // comes up again only behind the barrier that frees its buffer
+  float cumulative[2][kChunk], gateBeta[2][kChunk];
   float system[kChunk][kChunk + 1];
   float squares[2][kComputeWarps][kChunk];
 };
@@ -537,7 +539,7 @@ __device__ __forceinline__ void chunk_prepare(ChunkShared& sh, const infdev_quer
         mine = lane == t ? running : mine;
       }
       if (lane < kChunk) {
-        sh.cumulative[lane] = mine, sh.gateBeta[lane] = nextBeta;
+        sh.cumulative[step & 1][lane] = mine, sh.gateBeta[step & 1][lane] = nextBeta;
         out.decay[lane] = expf(mine), out.tail[lane] = expf(running - mine), out.beta[lane] = nextBeta;
       }
     }
@@ -563,9 +565,9 @@ __device__ __forceinline__ void chunk_prepare(ChunkShared& sh, const infdev_quer
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int t = (lane >> 2) + 8 * (e >> 1), i = 8 * n + 2 * (lane & 3) + (e & 1);
-          const float value = (dot[n][e] + low[n][e]) * (1.0f / (kKeyUnit * kKeyUnit)) * expf(sh.cumulative[t] - sh.cumulative[i]);
+          const float value = (dot[n][e] + low[n][e]) * (1.0f / (kKeyUnit * kKeyUnit)) * expf(sh.cumulative[step & 1][t] - sh.cumulative[step & 1][i]);
           if (warp == 0) {
-            sh.system[t][i] = i < t ? value * sh.gateBeta[t] : 0.f;
+            sh.system[t][i] = i < t ? value * sh.gateBeta[step & 1][t] : 0.f;
           } else {
             const float scaled = i <= t ? value * kMixUnit : 0.f;
             const __half hi = __float2half_rn(scaled);

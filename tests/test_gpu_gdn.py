@@ -194,6 +194,22 @@ def test_chunk_whose_deltas_are_zero_leaves_the_state_alone(dev, what):
   assert rel_err(out, want_out) < 1e-5 and rel_err(state, want_state) < 1e-5
 
 
+@pytest.mark.parametrize("T", [17, 32, 33, 49])
+def test_first_chunks_have_their_own_decays(dev, T):
+  """The preparation of the second chunk may start while the first one's weights are still being formed. Decays of the two differ
+  by e^8 here, so that weights formed with the wrong ones would show; and every run gives the same bits."""
+  rng = np.random.default_rng(T)
+  q, k, v, g, beta, S = rule_inputs(rng, T)
+  g[:16], g[16:] = -0.01, -0.5
+  want, want_state, _ = oracle.delta_rule(q, k, v, g, beta, S)
+  first = None
+  for _ in range(20):
+    out, state = run_rule(dev, q, k, v, g, beta, S)
+    assert rel_err(out, want) < 1e-5 and rel_err(state, want_state) < 1e-5
+    first = first or (out.tobytes(), state.tobytes())
+    assert first == (out.tobytes(), state.tobytes())
+
+
 def test_prefill_variant_refuses_an_image(dev):
   dev.image_capture(dev.empty(dev.image_bytes(8, 4096), np.uint8))
   with pytest.raises(RuntimeError, match="no image"):
