@@ -175,7 +175,8 @@ int infdev_gdn_decode(infdev_ctx* ctx, const float* x, const float* mixed, const
                       int queryCount, uint64_t convStateOffset, uint64_t stateOffset, uint64_t stateBytes, float* out);
 /* The same for a pass that holds prefill chunks: non-speculative queries of at least 16 tokens take the chunked form
  * (16 tokens per step, the role of delta_rule_prefill, delta_rule.metal:19-253), every other query the sequential one.
- * Results agree with infdev_delta_rule to fp32 rounding. Two launches; no image of the result (a pending
+ * Products run on the tensor cores over split operands (22 to 24 bits), sums in fp32: against fp64 the results are off by about
+ * 2e-7, those of infdev_delta_rule by 1e-7. Two launches; no image of the result (a pending
  * infdev_image_capture makes the call fail). */
 int infdev_delta_rule_prefill(infdev_ctx* ctx, const float* q, const float* k, const float* v, const float* g, const float* beta, const float* z,
                               const float* normWeight, const infdev_query* queries, int queryCount, uint64_t stateOffset, uint64_t stateBytes,

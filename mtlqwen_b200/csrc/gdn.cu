@@ -9,6 +9,7 @@
 // CTA (256 threads x 64 values): it is read from HBM once, updated for every token of the query, and
 // written once (or once per token for speculative queries, whose every row must stay selectable). The
 // reference makes two passes over the state in device memory per token (delta_rule.metal:320-333, 351-360).
+#include <cuda_bf16.h>
 #include "act_image.cuh"
 #include "kernels.h"
 #include "ops.h"
@@ -433,29 +434,41 @@ __global__ void __launch_bounds__(256, 2) delta_rule_kernel(const float* q, cons
 // a chunk or two ahead, in two shared-memory buffers. The eight others hold S^T in registers, 16 value columns each: a warp
 // needs nothing from its neighbours until the norm of the output, because a value column's recurrence is its own. All
 // products run on the tensor cores; a warp's accumulators (value column x key dim, or x token) are at the same time, as they
-// lie in its registers, the A operand of the next product. Operands are split into fp16 hi + lo after scaling by a power of
-// two (fixed for keys and queries, by the largest value of the warp for S, rhs and delta), and the three products that matter
-// (hi hi, lo hi, hi lo) are accumulated in fp32: 22 bits of every operand, the error against the sequential fp32 form stays at its own rounding.
-// 156 HMMA per warp and chunk at 512 multiply-adds per clock and SM bound it to 2.7 us per chunk; the form before this one,
-// fp32 FMAs with eight partial sums per product through shared memory, took 19 us.
+// lie in its registers, the A operand of the next product.
+//
+// Precision. Keys, queries, S and the update of S are split into fp16 hi + lo after scaling by a power of two (fixed for keys
+// and queries, whose norm is at most 1; by the largest value of each value column for the others), and the three products that
+// matter (lo hi, hi lo, hi hi) are formed. A^-1, the weights of the second sum, rhs and delta span whatever the decays and the
+// values span, so they are split into three bf16 parts (24 bits and the exponents of fp32) and six products. The tensor cores
+// cut off what does not fit their accumulator instead of rounding it, so no sum is carried through them: every product of 16
+// terms starts from zero and is added with a rounded fp32 addition. Decays are cumulated in double precision, because their
+// logarithms reach hundreds while differences of neighbours matter to the last bit. Against fp64, with gates, values and states
+// as a model has them, 512 tokens: outputs 1.8e-7, state 1.4e-7 (2-norms); the fp32 chunk form before it 2.1e-7 and 4.7e-7,
+// token by token 1.1e-7 and 0.7e-7. One scale for the 16 columns of a warp, fp16 parts throughout and sums carried in the
+// accumulators gave 4.1e-7 and 5.4e-7, and lost value columns far below their neighbours; they took 278 us for eight queries
+// of 59 to 493 rows, this form 315 us.
+// A chunk takes about 4.8 us (one query of 512 rows: 32 chunks, 177 us with the preparation); its 168 MMAs per warp are 1.4 us
+// of them at the measured 8.06 cycles per MMA and scheduler, the rest is the chain of products that wait for each other. The
+// fp32 form, FMAs with eight partial sums per product through shared memory, took 12 us.
 constexpr int kChunk = 16, kComputeWarps = 8, kPrepareWarps = 4;
 constexpr int kChunkThreads = (kComputeWarps + kPrepareWarps) * kWarp;
-constexpr float kKeyUnit = 256.f, kSolveUnit = 16.f, kMixUnit = 256.f;  // fixed scales of the fp16 operands
+constexpr float kKeyUnit = 256.f;  // fixed scale of the normalised keys and queries
 struct ChunkBuffer {
   __half k[2][kChunk][kHeadDim + 8], q[2][kChunk][kHeadDim + 8];  // hi, lo of kKeyUnit x the normalised rows
-  __half solve[2][kChunk][kChunk + 8], mix[2][kChunk][kChunk + 8];  // hi, lo of kSolveUnit x A^-1 and kMixUnit x R (q . k)
+  __nv_bfloat16 solve[3][kChunk][kChunk + 8], mix[3][kChunk][kChunk + 8];  // three parts of A^-1 and R (q . k)
   float decay[kChunk], tail[kChunk], beta[kChunk];                // G_t, G_15 / G_t, beta_t
 };
 struct ChunkShared {
   ChunkBuffer buffer[2];
   // of the chunk being prepared, two sets in turn: warp 1 reads one while warp 0 may already write the next chunk's, and a set
   // comes up again only behind the barrier that frees its buffer
-  float cumulative[2][kChunk], gateBeta[2][kChunk];
+  double cumulative[2][kChunk];
+  float gateBeta[2][kChunk];
   float system[kChunk][kChunk + 1];
   float squares[2][kComputeWarps][kChunk];
 };
 // named barriers: 1, 2 buffer filled; 3, 4 buffer free; 5 the preparing warps; 6 the computing warps
-__device__ __forceinline__ void chunk_ldmatrix(uint32_t (&r)[4], const __half* address) {
+__device__ __forceinline__ void chunk_ldmatrix(uint32_t (&r)[4], const void* address) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(address)) : "memory");
 }
 __device__ __forceinline__ void chunk_ldmatrix_trans(uint32_t (&r)[4], const __half* address) {
@@ -469,26 +482,84 @@ __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint3
   const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
   lo = pack_half2(a - f.x, b - f.y);
 }
-// 2^n that brings the warp's largest magnitude into [512, 1024), and 2^-n. Both are normal numbers, whatever the magnitude is:
-// the exponent fields lie in 1 .. 253 (all zero: 2^126 and 2^-126).
-__device__ __forceinline__ float2 warp_unit(float largest) {
-  largest = warp_max(largest);
+// a, b as three bf16 pairs, largest first
+__device__ __forceinline__ void split_three(float a, float b, uint32_t (&part)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const __nv_bfloat162 pair = __floats2bfloat162_rn(a, b);
+    part[i] = *reinterpret_cast<const uint32_t*>(&pair);
+    a -= __low2float(pair), b -= __high2float(pair);
+  }
+}
+// 2^n that brings a value column's largest magnitude into [512, 1024), and 2^-n; the column's values lie in the four lanes of a
+// quad. Both are normal numbers, whatever the magnitude is: the exponent fields lie in 1 .. 253 (all zero: 2^126 and 2^-126).
+__device__ __forceinline__ float2 column_unit(float largest) {
+  largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, 1));
+  largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, 2));
   const int field = min(253, max(1, 263 - int(__float_as_uint(largest) >> 23)));
   return make_float2(__uint_as_float(uint32_t(field) << 23), __uint_as_float(uint32_t(254 - field) << 23));
 }
-// The two 16 x 8 accumulators of 16 x 16 values (C fragments) x unit as the A operand, hi and lo.
-__device__ __forceinline__ void split_tile(const float (&c0)[4], const float (&c1)[4], float unit, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
+// The two 16 x 8 accumulators of 16 x 16 values (C fragments) x their columns' units as the A operand, hi and lo.
+__device__ __forceinline__ void split_tile(const float (&c0)[4], const float (&c1)[4], float unit, float unit8, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
   split_pair(c0[0] * unit, c0[1] * unit, hi[0], lo[0]);
-  split_pair(c0[2] * unit, c0[3] * unit, hi[1], lo[1]);
+  split_pair(c0[2] * unit8, c0[3] * unit8, hi[1], lo[1]);
   split_pair(c1[0] * unit, c1[1] * unit, hi[2], lo[2]);
-  split_pair(c1[2] * unit, c1[3] * unit, hi[3], lo[3]);
+  split_pair(c1[2] * unit8, c1[3] * unit8, hi[3], lo[3]);
 }
-// d0, d1 += A x B for the two n-tiles of B fragments bHi, bLo, as hi hi + lo hi + hi lo.
-__device__ __forceinline__ void mma_three(float (&d0)[4], float (&d1)[4], const uint32_t (&hi)[4], const uint32_t (&lo)[4], const uint32_t (&bHi)[4],
+// d = A x B for the two n-tiles of B fragments bHi, bLo, as lo hi + hi lo + hi hi.
+__device__ __forceinline__ void mma_three(float (&d)[2][4], const uint32_t (&hi)[4], const uint32_t (&lo)[4], const uint32_t (&bHi)[4],
                                           const uint32_t (&bLo)[4]) {
-  mma_16816(d0, hi, bHi[0], bHi[1]), mma_16816(d1, hi, bHi[2], bHi[3]);
-  mma_16816(d0, lo, bHi[0], bHi[1]), mma_16816(d1, lo, bHi[2], bHi[3]);
-  mma_16816(d0, hi, bLo[0], bLo[1]), mma_16816(d1, hi, bLo[2], bLo[3]);
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    d[0][e] = d[1][e] = 0.f;
+  mma_16816(d[0], lo, bHi[0], bHi[1]), mma_16816(d[1], lo, bHi[2], bHi[3]);
+  mma_16816(d[0], hi, bLo[0], bLo[1]), mma_16816(d[1], hi, bLo[2], bLo[3]);
+  mma_16816(d[0], hi, bHi[0], bHi[1]), mma_16816(d[1], hi, bHi[2], bHi[3]);
+}
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// d = the 16 x 16 values c (C fragments, 16 value columns x 16 tokens) x B^T, B [3][token][token] in shared memory; all the
+// products of three parts by three that reach 24 bits, summed by their order of magnitude.
+__device__ __forceinline__ void token_product(float (&d)[2][4], const float (&c)[2][4], const __nv_bfloat16 (&b)[3][kChunk][kChunk + 8], int row, int column) {
+  uint32_t a[3][4], fragment[3][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    uint32_t part[3];
+    split_three(c[i >> 1][2 * (i & 1)], c[i >> 1][2 * (i & 1) + 1], part);
+    a[0][i] = part[0], a[1][i] = part[1], a[2][i] = part[2];
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    chunk_ldmatrix(fragment[i], &b[i][row][column]);
+  float sum[3][2][4] = {};  // by order of magnitude
+#pragma unroll
+  for (int order = 2; order >= 0; --order)
+#pragma unroll
+    for (int i = 0; i <= order; ++i)
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+        mma_bf16(sum[order][n], a[i], fragment[order - i][2 * n], fragment[order - i][2 * n + 1]);
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      d[n][e] = sum[0][n][e] + (sum[1][n][e] + sum[2][n][e]);
+}
+// e^x rounded from more digits than a float x has: cumulated log decays of hundreds would lose all but a few of e^x.
+__device__ __forceinline__ float exp_of(double x) {
+  const float hi = float(x), lo = x == double(hi) ? 0.f : float(x - double(hi)), e = expf(hi);
+  return e < INFINITY ? fmaf(e, lo, e) : e;
+}
+
+__device__ __forceinline__ void store_three(__nv_bfloat16 (&to)[3][kChunk][kChunk + 8], int t, int i, float value) {
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+    to[p][t][i] = __float2bfloat16_rn(value);
+    value -= __bfloat162float(to[p][t][i]);
+  }
 }
 
 // The four preparing warps: chunk after chunk into the two buffers.
@@ -532,22 +603,22 @@ __device__ __forceinline__ void chunk_prepare(ChunkShared& sh, const infdev_quer
       *reinterpret_cast<uint2*>(&out.k[0][4 * warp + j][4 * lane]) = hi, *reinterpret_cast<uint2*>(&out.k[1][4 * warp + j][4 * lane]) = lo;
     }
     if (warp == 0) {
-      float running = 0.f, mine = 0.f;
+      double running = 0.0, mine = 0.0;
 #pragma unroll
       for (int t = 0; t < kChunk; ++t) {
-        running += __shfl_sync(0xffffffffu, nextG, t);
+        running += double(__shfl_sync(0xffffffffu, nextG, t));
         mine = lane == t ? running : mine;
       }
       if (lane < kChunk) {
         sh.cumulative[step & 1][lane] = mine, sh.gateBeta[step & 1][lane] = nextBeta;
-        out.decay[lane] = expf(mine), out.tail[lane] = expf(running - mine), out.beta[lane] = nextBeta;
+        out.decay[lane] = exp_of(mine), out.tail[lane] = exp_of(running - mine), out.beta[lane] = nextBeta;
       }
     }
     load(first + kChunk);  // past the end: zeros
     named_barrier(5, kPrepareWarps * kWarp);
     if (warp < 2) {
       // warp 0: k . k and the inverse of the triangular system; warp 1: q . k
-      float dot[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, low[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      float dot[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
       const auto& left = warp == 0 ? out.k : out.q;
 #pragma unroll
       for (int s = 0; s < kHeadDim / 16; ++s) {
@@ -556,22 +627,22 @@ __device__ __forceinline__ void chunk_prepare(ChunkShared& sh, const infdev_quer
         chunk_ldmatrix(lo, &left[1][lane & 15][16 * s + 8 * (lane >> 4)]);
         chunk_ldmatrix(bHi, &out.k[0][tokenOfB][16 * s + dimOfB]);
         chunk_ldmatrix(bLo, &out.k[1][tokenOfB][16 * s + dimOfB]);
-        mma_16816(dot[0], hi, bHi[0], bHi[1]), mma_16816(dot[1], hi, bHi[2], bHi[3]);
-        mma_16816(low[0], lo, bHi[0], bHi[1]), mma_16816(low[1], lo, bHi[2], bHi[3]);
-        mma_16816(low[0], hi, bLo[0], bLo[1]), mma_16816(low[1], hi, bLo[2], bLo[3]);
+        float part[2][4];
+        mma_three(part, hi, lo, bHi, bLo);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          dot[0][e] += part[0][e], dot[1][e] += part[1][e];
       }
 #pragma unroll
       for (int n = 0; n < 2; ++n)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int t = (lane >> 2) + 8 * (e >> 1), i = 8 * n + 2 * (lane & 3) + (e & 1);
-          const float value = (dot[n][e] + low[n][e]) * (1.0f / (kKeyUnit * kKeyUnit)) * expf(sh.cumulative[step & 1][t] - sh.cumulative[step & 1][i]);
+          const float value = dot[n][e] * (1.0f / (kKeyUnit * kKeyUnit)) * exp_of(sh.cumulative[step & 1][t] - sh.cumulative[step & 1][i]);
           if (warp == 0) {
             sh.system[t][i] = i < t ? value * sh.gateBeta[step & 1][t] : 0.f;
           } else {
-            const float scaled = i <= t ? value * kMixUnit : 0.f;
-            const __half hi = __float2half_rn(scaled);
-            out.mix[0][t][i] = hi, out.mix[1][t][i] = __float2half_rn(scaled - __half2float(hi));
+            store_three(out.mix, t, i, i <= t ? value : 0.f);
           }
         }
       if (warp == 0) {
@@ -590,9 +661,7 @@ __device__ __forceinline__ void chunk_prepare(ChunkShared& sh, const infdev_quer
         if (lane < kChunk)
 #pragma unroll
           for (int t = 0; t < kChunk; ++t) {
-            const float scaled = x[t] * kSolveUnit;
-            const __half hi = __float2half_rn(scaled);
-            out.solve[0][t][column] = hi, out.solve[1][t][column] = __float2half_rn(scaled - __half2float(hi));
+            store_three(out.solve, t, column, x[t]);
           }
       }
     }
@@ -659,11 +728,13 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
     const ChunkBuffer& in = sh.buffer[step & 1];
     if (z)
       load(gate, z, first);
-    float largest = 0.f;
+    float largest[2] = {0.f, 0.f};
 #pragma unroll
     for (int j = 0; j < kHeadDim / 8; ++j)
-      largest = fmaxf(fmaxf(fmaxf(largest, fabsf(S[j][0])), fmaxf(fabsf(S[j][1]), fabsf(S[j][2]))), fabsf(S[j][3]));
-    const float2 stateUnit = warp_unit(largest);
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        largest[e >> 1] = fmaxf(largest[e >> 1], fabsf(S[j][e]));
+    const float2 unit = column_unit(largest[0]), unit8 = column_unit(largest[1]);
     named_barrier(1 + (step & 1), kChunkThreads);
     // S^T k and S^T q of the 16 tokens
     float ks[2][4], qs[2][4];
@@ -675,15 +746,22 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
 #pragma unroll
     for (int s = 0; s < kHeadDim / 16; ++s) {
       uint32_t hi[4], lo[4], bHi[4], bLo[4];
-      split_tile(S[2 * s], S[2 * s + 1], stateUnit.x, hi, lo);
+      float part[2][4];
+      split_tile(S[2 * s], S[2 * s + 1], unit.x, unit8.x, hi, lo);
       chunk_ldmatrix(bHi, &in.k[0][tokenOfB][16 * s + dimOfB]);
       chunk_ldmatrix(bLo, &in.k[1][tokenOfB][16 * s + dimOfB]);
-      mma_three(ks[0], ks[1], hi, lo, bHi, bLo);
+      mma_three(part, hi, lo, bHi, bLo);
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        ks[0][e] += part[0][e], ks[1][e] += part[1][e];
       chunk_ldmatrix(bHi, &in.q[0][tokenOfB][16 * s + dimOfB]);
       chunk_ldmatrix(bLo, &in.q[1][tokenOfB][16 * s + dimOfB]);
-      mma_three(qs[0], qs[1], hi, lo, bHi, bLo);
+      mma_three(part, hi, lo, bHi, bLo);
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        qs[0][e] += part[0][e], qs[1][e] += part[1][e];
     }
-    const float productUnit = stateUnit.y * (1.0f / kKeyUnit);
+    const float productUnit[2] = {unit.y * (1.0f / kKeyUnit), unit8.y * (1.0f / kKeyUnit)};
     float decay[2][2];
 #pragma unroll
     for (int n = 0; n < 2; ++n)
@@ -692,52 +770,42 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
         decay[n][e] = in.decay[8 * n + t2 + e];
     // rhs, delta = A^-1 rhs
     float rhs[2][4], delta[2][4];
-    largest = 0.f;
 #pragma unroll
     for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        rhs[n][e] = in.beta[8 * n + t2 + (e & 1)] * (value[n][e] - decay[n][e & 1] * (ks[n][e] * productUnit));
-        largest = fmaxf(largest, fabsf(rhs[n][e]));
-        delta[n][e] = 0.f;
-      }
-    load(value, v, first + kChunk);  // of the next chunk
-    uint32_t hi[4], lo[4], bHi[4], bLo[4];
-    float2 scale = warp_unit(largest);
-    split_tile(rhs[0], rhs[1], scale.x, hi, lo);
-    chunk_ldmatrix(bHi, &in.solve[0][tokenOfB][dimOfB]);
-    chunk_ldmatrix(bLo, &in.solve[1][tokenOfB][dimOfB]);
-    mma_three(delta[0], delta[1], hi, lo, bHi, bLo);
-    // outputs, and the state's update with (G_15 / G_i) delta_i
-    float mixed[2][4], update[2][4];
-    largest = 0.f;
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        delta[n][e] *= scale.y * (1.0f / kSolveUnit);
-        update[n][e] = delta[n][e] * in.tail[8 * n + t2 + (e & 1)];
-        largest = fmaxf(largest, fmaxf(fabsf(delta[n][e]), fabsf(update[n][e])));
-        mixed[n][e] = 0.f;
-      }
-    scale = warp_unit(largest);
-    split_tile(delta[0], delta[1], scale.x, hi, lo);
-    chunk_ldmatrix(bHi, &in.mix[0][tokenOfB][dimOfB]);
-    chunk_ldmatrix(bLo, &in.mix[1][tokenOfB][dimOfB]);
-    mma_three(mixed[0], mixed[1], hi, lo, bHi, bLo);
-    split_tile(update[0], update[1], scale.x, hi, lo);
-    // The sum over the tokens starts from zero and is scaled before it meets the state, which stays in units of its own: deltas
-    // may be zero or any number of powers of two smaller than the state (beta = 0, value columns without weights).
-    const float stateDecay = in.decay[kChunk - 1], updateUnit = scale.y * (1.0f / kKeyUnit);
-#pragma unroll
-    for (int s = 0; s < kHeadDim / 16; ++s) {
-      float added[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-      chunk_ldmatrix_trans(bHi, &in.k[0][lane & 15][16 * s + 8 * (lane >> 4)]);
-      chunk_ldmatrix_trans(bLo, &in.k[1][lane & 15][16 * s + 8 * (lane >> 4)]);
-      mma_three(added[0], added[1], hi, lo, bHi, bLo);
 #pragma unroll
       for (int e = 0; e < 4; ++e)
-        S[2 * s][e] = fmaf(added[0][e], updateUnit, S[2 * s][e] * stateDecay), S[2 * s + 1][e] = fmaf(added[1][e], updateUnit, S[2 * s + 1][e] * stateDecay);
+        rhs[n][e] = in.beta[8 * n + t2 + (e & 1)] * (value[n][e] - decay[n][e & 1] * (ks[n][e] * productUnit[e >> 1]));
+    load(value, v, first + kChunk);  // of the next chunk
+    token_product(delta, rhs, in.solve, tokenOfB, dimOfB);
+    // outputs, and the state's update with (G_15 / G_i) delta_i
+    float mixed[2][4];
+    token_product(mixed, delta, in.mix, tokenOfB, dimOfB);
+    largest[0] = largest[1] = 0.f;
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        delta[n][e] *= in.tail[8 * n + t2 + (e & 1)];
+        largest[e >> 1] = fmaxf(largest[e >> 1], fabsf(delta[n][e]));
+      }
+    const float2 scale = column_unit(largest[0]), scale8 = column_unit(largest[1]);
+    uint32_t hi[4], lo[4];
+    split_tile(delta[0], delta[1], scale.x, scale8.x, hi, lo);
+    // The sum over the tokens starts from zero and is scaled before it meets the state, which stays in units of its own: deltas
+    // may be zero or any number of powers of two smaller than the state (beta = 0, value columns without weights).
+    const float stateDecay = in.decay[kChunk - 1], updateUnit[2] = {scale.y * (1.0f / kKeyUnit), scale8.y * (1.0f / kKeyUnit)};
+#pragma unroll
+    for (int s = 0; s < kHeadDim / 16; ++s) {
+      uint32_t bHi[4], bLo[4];
+      float added[2][4];
+      chunk_ldmatrix_trans(bHi, &in.k[0][lane & 15][16 * s + 8 * (lane >> 4)]);
+      chunk_ldmatrix_trans(bLo, &in.k[1][lane & 15][16 * s + 8 * (lane >> 4)]);
+      mma_three(added, hi, lo, bHi, bLo);
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          S[2 * s + n][e] = fmaf(added[n][e], updateUnit[e >> 1], S[2 * s + n][e] * stateDecay);
     }
     named_barrier_arrive(3 + (step & 1), kChunkThreads);  // the buffer may be refilled
     // o, its gated norm over the head's 128 columns (gated_rms_norm_128), and the store
@@ -746,7 +814,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
     for (int n = 0; n < 2; ++n)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        o[n][e] = decay[n][e & 1] * (qs[n][e] * productUnit) + mixed[n][e] * (scale.y * (1.0f / kMixUnit));
+        o[n][e] = decay[n][e & 1] * (qs[n][e] * productUnit[e >> 1]) + mixed[n][e];
         squares[n][e & 1] = fmaf(o[n][e], o[n][e], squares[n][e & 1]);
       }
     if (z) {

@@ -144,7 +144,8 @@ def test_gdn_chunked_mixed_pass(dev):
 
 
 def test_gdn_chunked_agrees_with_sequential(dev):
-  """Both forms are fp32 on the CUDA cores and must agree far inside the tolerance against the oracle."""
+  """One form is fp32 on the CUDA cores, the other split operands on the tensor cores; both must lie far inside the tolerance
+  against the oracle. How close the second one is to fp64: test_chunked_precision."""
   a = run_layer(dev, np.random.default_rng(6), [100, 64], prefill=False)
   b = run_layer(dev, np.random.default_rng(6), [100, 64], prefill=True)
   assert a < TOL and b < TOL and abs(a - b) < 2e-4
@@ -192,6 +193,50 @@ def test_chunk_whose_deltas_are_zero_leaves_the_state_alone(dev, what):
   want_out, want_state, _ = oracle.delta_rule(q, k, v, g, beta, S)
   assert np.isfinite(out).all() and np.isfinite(state).all()
   assert rel_err(out, want_out) < 1e-5 and rel_err(state, want_state) < 1e-5
+
+
+def rule_in_fp64(q, k, v, g, beta, S):
+  q, k, v, g, beta, S = (np.asarray(a, np.float32).astype(np.float64) for a in (q, k, v, g, beta, S))
+  heads = np.arange(32) % 16
+  q = q / np.sqrt((q * q).sum(-1, keepdims=True) + 1e-6) / np.sqrt(128.0)
+  k = k / np.sqrt((k * k).sum(-1, keepdims=True) + 1e-6)
+  out = []
+  for t in range(v.shape[0]):
+    S = S * np.exp(g[t])[:, None, None]
+    delta = (v[t] - np.einsum("hk,hkv->hv", k[t][heads], S)) * beta[t][:, None]
+    S = S + k[t][heads][:, :, None] * delta[:, None, :]
+    out.append(np.einsum("hk,hkv->hv", q[t][heads], S))
+  return np.stack(out), S
+
+
+def norm_err(got, want, axes=None):
+  return np.sqrt(((got - want)**2).sum(axes) / (want**2).sum(axes)).max()
+
+
+@pytest.mark.parametrize("what", ["as in a model", "little decay", "columns of very different size", "tokens of very different size"])
+def test_chunked_precision(dev, what):
+  """Against fp64. Operands are rounded to 22 bits or better (2^-23 of two factors, 2.4e-7 when nothing averages out) and sums to
+  fp32: 3e-7 over all, an outer bound of 2e-6 for a value column of its own, whatever its neighbours hold."""
+  rng = np.random.default_rng(70)
+  T = 160
+  q, k, v, g, beta, S = rule_inputs(rng, T, decay=1e-3 if what == "little decay" else 0.2)
+  S *= 0.02
+  if what == "as in a model":
+    g = -np.log1p(np.exp(rng.standard_normal((T, 32)))) * rng.uniform(1, 16, 32)
+  elif what == "columns of very different size":
+    size = np.exp(4 * rng.standard_normal((32, 128)))
+    v, S = v * size, S * size[:, None, :]
+  elif what == "tokens of very different size":
+    g = -np.log1p(np.exp(rng.standard_normal((T, 32)))) * rng.uniform(1, 16, 32)
+    v = v * np.exp(4 * rng.standard_normal((T, 1, 1)))
+  out, state = run_rule(dev, q, k, v, g, beta, S)
+  want_out, want_state = rule_in_fp64(q, k, v, g, beta, S)
+  assert norm_err(state, want_state) < 3e-7 and norm_err(state, want_state, 1) < 2e-6
+  if what == "tokens of very different size":
+    # an output that is a small difference of large terms keeps few digits in any fp32 form (1.6e-4 of its own size with plain FMAs)
+    assert norm_err(out, want_out, 2) < 1e-3
+  else:
+    assert norm_err(out, want_out) < 3e-7
 
 
 @pytest.mark.parametrize("T", [17, 32, 33, 49])
