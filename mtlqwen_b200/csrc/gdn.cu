@@ -453,9 +453,10 @@ __global__ void __launch_bounds__(256, 2) delta_rule_kernel(const float* q, cons
 constexpr int kChunk = 16, kComputeWarps = 8, kPrepareWarps = 4;
 constexpr int kChunkThreads = (kComputeWarps + kPrepareWarps) * kWarp;
 constexpr float kKeyUnit = 256.f;  // fixed scale of the normalised keys and queries
+using TokenMatrix = __nv_bfloat16[3][kChunk][kChunk + 8];  // lower triangular, [part][token][token]
 struct ChunkBuffer {
   __half k[2][kChunk][kHeadDim + 8], q[2][kChunk][kHeadDim + 8];  // hi, lo of kKeyUnit x the normalised rows
-  __nv_bfloat16 solve[3][kChunk][kChunk + 8], mix[3][kChunk][kChunk + 8];  // three parts of A^-1 and R (q . k)
+  TokenMatrix solve, mix;  // three parts of A^-1 and R (q . k)
   float decay[kChunk], tail[kChunk], beta[kChunk];                // G_t, G_15 / G_t, beta_t
 };
 struct ChunkShared {
@@ -521,9 +522,42 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// d = the 16 x 16 values c (C fragments, 16 value columns x 16 tokens) x B^T, B [3][token][token] in shared memory; all the
-// products of three parts by three that reach 24 bits, summed by their order of magnitude.
-__device__ __forceinline__ void token_product(float (&d)[2][4], const float (&c)[2][4], const __nv_bfloat16 (&b)[3][kChunk][kChunk + 8], int row, int column) {
+// token_product without the products with the matrix's zeros; values: this lane's eight of c (element 4n + e), then of d.
+__device__ __forceinline__ void token_sums(const TokenMatrix& b, float (&values)[8]) {
+  const int lane = threadIdx.x & 31, t2 = 2 * (lane & 3);
+  float sum[8] = {};
+#pragma unroll 1
+  for (int from = 0; from < kChunk; ++from) {
+    const int source = (lane & ~3) + ((from & 7) >> 1), element = 4 * (from >> 3) + (from & 1);
+    const float value[2] = {__shfl_sync(0xffffffffu, values[element], source), __shfl_sync(0xffffffffu, values[element + 2], source)};
+    for (int i = 0; i < 8; ++i) {
+      const int token = 8 * (i >> 2) + t2 + (i & 1);
+      if (from <= token)
+        sum[i] = fmaf((__bfloat162float(b[2][token][from]) + __bfloat162float(b[1][token][from])) + __bfloat162float(b[0][token][from]), value[(i >> 1) & 1],
+                      sum[i]);
+    }
+  }
+  for (int i = 0; i < 8; ++i)
+    values[i] = sum[i];
+}
+// d = the 16 x 16 values c (C fragments, 16 value columns x 16 tokens) x B^T; all the products of three parts by three that
+// reach 24 bits, summed by their order of magnitude.
+__device__ __forceinline__ void token_product(float (&d)[2][4], const float (&c)[2][4], const TokenMatrix& b, int row, int column) {
+  float finite = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    finite = fmaf(c[i >> 2][i & 3], 0.f, finite);
+  if (__any_sync(0xffffffffu, !(finite == 0.f))) {  // times the zeros it would reach the tokens before it
+    float values[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      values[i] = c[i >> 2][i & 3];
+    token_sums(b, values);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      d[i >> 2][i & 3] = values[i];
+    return;
+  }
   uint32_t a[3][4], fragment[3][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -554,7 +588,7 @@ __device__ __forceinline__ float exp_of(double x) {
   return e < INFINITY ? fmaf(e, lo, e) : e;
 }
 
-__device__ __forceinline__ void store_three(__nv_bfloat16 (&to)[3][kChunk][kChunk + 8], int t, int i, float value) {
+__device__ __forceinline__ void store_three(TokenMatrix& to, int t, int i, float value) {
 #pragma unroll
   for (int p = 0; p < 3; ++p) {
     to[p][t][i] = __float2bfloat16_rn(value);
@@ -695,10 +729,14 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
   extern __shared__ __align__(16) uint8_t chunkRaw[];
   ChunkShared& sh = *reinterpret_cast<ChunkShared*>(chunkRaw);
   const int head = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // The computing warps hold more than a third of the registers each: 2 x 192 + 120 = 3 x 168 a thread, of the 168 that the launch
+  // bounds give all three groups of four warps.
   if (warp >= kComputeWarps) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 120;");
     chunk_prepare(sh, info, q, k, g, beta, head);
     return;
   }
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 192;");
   const int row = lane >> 2, t2 = 2 * (lane & 3), column = 16 * warp + row;  // value columns `column` and `column` + 8
   const int tokenOfB = (lane & 7) + 8 * (lane >> 4), dimOfB = 8 * ((lane >> 3) & 1);
   float S[kHeadDim / 8][4];  // S^T: tile j holds key dims 8j + t2, + 1 of the two value columns

@@ -255,6 +255,31 @@ def test_first_chunks_have_their_own_decays(dev, T):
     assert first == (out.tobytes(), state.tobytes())
 
 
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("where", ["v", "k", "q", "g", "beta"])
+def test_tokens_before_one_that_is_not_finite_do_not_notice(dev, where, value):
+  """The chunked form computes 16 tokens together; the ones before a broken one must come out as if it were not there."""
+  rng = np.random.default_rng(60)
+  q, k, v, g, beta, S = rule_inputs(rng, 45)
+  clean, _, _ = oracle.delta_rule(q, k, v, g, beta, S)
+  token = 27
+  if where == "v":
+    v[token, 5, 33] = value
+  elif where in ("k", "q"):
+    (k if where == "k" else q)[token, 5, 33] = value
+  else:
+    (g if where == "g" else beta)[token, 5] = value
+  out, _ = run_rule(dev, q, k, v, g, beta, S)
+  assert rel_err(out[:token], clean[:token]) < 1e-5
+  others = [h for h in range(32) if h % 16 != 5]
+  assert rel_err(out[:, others], clean[:, others]) < 1e-5
+  if where == "v":  # one value column of one head
+    columns = [c for c in range(128) if c != 33]
+    assert rel_err(out[:, 5][:, columns], clean[:, 5][:, columns]) < 1e-5 and not np.isfinite(out[token:, 5, 33]).any()
+  elif where != "g" or value != -np.inf:  # (a decay of zero leaves the token itself finite)
+    assert not np.isfinite(out[token, 5]).any()
+
+
 def test_prefill_variant_refuses_an_image(dev):
   dev.image_capture(dev.empty(dev.image_bytes(8, 4096), np.uint8))
   with pytest.raises(RuntimeError, match="no image"):
