@@ -311,19 +311,14 @@ template <class Q, int NMAT, int XSPLIT> __global__ void __launch_bounds__(kThre
         }
       largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, 1));
       largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, 2));
-      // the power of two that brings the row's largest value of this super-block into [512, 1024) (exponent field 136;
-      // sub-block sums then stay below 2^15), and its inverse
-      const int field = min(254, max(1, 263 - int(__float_as_uint(largest) >> 23)));
-      const float power = __uint_as_float(uint32_t(field) << 23);
+      const float2 power = activation_power(largest);
       if (jj == 0)
-        xScale[sb * 8 + row] = __uint_as_float(uint32_t(max(1, 254 - field)) << 23);
-#pragma unroll
-      for (int tq = 0; tq < 4; ++tq) {
+        xScale[sb * 8 + row] = largest != INFINITY ? power.y : INFINITY;
+      auto store = [&](int tq, const float4 (&span)[4]) {  // four scaled float4 of a 64-value span
         float s[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          float4 w = v[tq][e];
-          w.x *= power, w.y *= power, w.z *= power, w.w *= power;
+          const float4 w = span[e];
           uint2 hi;
           float4 r;
           int slot;
@@ -359,6 +354,25 @@ template <class Q, int NMAT, int XSPLIT> __global__ void __launch_bounds__(kThre
             const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
             fragSum[sb * 32 + row * 4 + tq] = make_uint2(hi, pack_half2(s0 - f.x, s1 - f.y));
           }
+        }
+      };
+#pragma unroll
+      for (int tq = 0; tq < 4; ++tq) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          v[tq][e].x *= power.x, v[tq][e].y *= power.x, v[tq][e].z *= power.x, v[tq][e].w *= power.x;
+        store(tq, v[tq]);
+      }
+      if (__any_sync(0xffffffffu, largest == INFINITY)) {  // once more, from memory: out of the way of the ordinary case
+#pragma unroll 1
+        for (int tq = 0; tq < 4; ++tq) {
+          float4 span[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            span[e] = scaled_with_infinities(row < p.m ? *reinterpret_cast<const float4*>(p.x + size_t(row) * p.ldx + k0 + 256 * sb + 64 * tq + 16 * e + 4 * jj)
+                                                       : make_float4(0.f, 0.f, 0.f, 0.f),
+                                             largest, power.x);
+          store(tq, span);
         }
       }
     }

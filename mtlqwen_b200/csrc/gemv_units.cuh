@@ -11,6 +11,20 @@
 
 namespace infdev {
 
+// The power of two that brings a row's largest activation of a super-block into [512, 1024) (exponent field 136; sub-block sums
+// then stay below 2^15), and its inverse. Both are normal numbers, whatever the magnitude is: the fields lie in 1 .. 253.
+__device__ __forceinline__ float2 activation_power(float largest) {
+  const int field = min(253, max(1, 263 - int(__float_as_uint(largest) >> 23)));
+  return make_float2(__uint_as_float(uint32_t(field) << 23), __uint_as_float(uint32_t(254 - field) << 23));
+}
+// Four activations scaled, for a super-block in which some row has an infinite one: in such a row infinite values stand as +-512
+// and finite ones as zero, and infinity takes the place of the power's inverse, so that products come out as +-infinity with the
+// sign of the weight (the hi + lo halves of an infinity would be infinity - infinity). NaN stays NaN.
+__device__ __forceinline__ float4 scaled_with_infinities(const float4& v, float largest, float power) {
+  auto scaled = [&](float x) { return largest != INFINITY ? x * power : fabsf(x) == INFINITY ? copysignf(512.f, x) : x * 0.f; };
+  return make_float4(scaled(v.x), scaled(v.y), scaled(v.z), scaled(v.w));
+}
+
 __device__ __forceinline__ uint32_t lds_u32_unaligned(const uint8_t* p) {
   return uint32_t(*reinterpret_cast<const uint16_t*>(p)) | (uint32_t(*reinterpret_cast<const uint16_t*>(p + 2)) << 16);
 }

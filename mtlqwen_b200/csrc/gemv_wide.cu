@@ -115,17 +115,14 @@ __global__ void __launch_bounds__(128) wide_prepare_kernel(const float* x, int l
     }
   largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, 1));
   largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, 2));
-  const int field = min(254, max(1, 263 - int(__float_as_uint(largest) >> 23)));
-  const float power = __uint_as_float(uint32_t(field) << 23);
+  const float2 power = activation_power(largest);
   if (jj == 0)
-    powers[row] = __uint_as_float(uint32_t(max(1, 254 - field)) << 23);
-#pragma unroll
-  for (int tq = 0; tq < 4; ++tq) {
+    powers[row] = largest != INFINITY ? power.y : INFINITY;
+  auto store = [&](int tq, const float4 (&span)[4]) {  // four scaled float4 of a 64-value span
     float s[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      float4 w = v[tq][e];
-      w.x *= power, w.y *= power, w.z *= power, w.w *= power;
+      const float4 w = span[e];
       uint4 b;
       b.x = pack_half2(w.x, w.y), b.y = pack_half2(w.z, w.w);
       const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&b.x)), f1 = __half22float2(*reinterpret_cast<const __half2*>(&b.y));
@@ -140,6 +137,25 @@ __global__ void __launch_bounds__(128) wide_prepare_kernel(const float* x, int l
       const uint32_t hi = pack_half2(s0, s1);
       const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
       sums[row * 4 + tq] = make_uint2(hi, pack_half2(s0 - f.x, s1 - f.y));
+    }
+  };
+#pragma unroll
+  for (int tq = 0; tq < 4; ++tq) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      v[tq][e].x *= power.x, v[tq][e].y *= power.x, v[tq][e].z *= power.x, v[tq][e].w *= power.x;
+    store(tq, v[tq]);
+  }
+  if (__any_sync(0xffffffffu, largest == INFINITY)) {  // once more, from memory: out of the way of the ordinary case
+#pragma unroll 1
+    for (int tq = 0; tq < 4; ++tq) {
+      float4 span[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        span[e] = scaled_with_infinities(source < m ? *reinterpret_cast<const float4*>(x + size_t(source) * ldx + 256 * sb + 64 * tq + 16 * e + 4 * jj)
+                                                    : make_float4(0.f, 0.f, 0.f, 0.f),
+                                         largest, power.x);
+      store(tq, span);
     }
   }
 }

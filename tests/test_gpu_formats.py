@@ -96,6 +96,25 @@ def test_many_rows_share_a_decode(dev, name, qtype, m, n, k):
     assert np.linalg.norm(got[row] - want[row]) < 1e-5 * np.linalg.norm(want[row]) + 2.4e-7 * np.linalg.norm(y[row]), row
 
 
+@pytest.mark.parametrize("m", [3, 8, 9, 40])
+@pytest.mark.parametrize("name,qtype", WIDE_TYPES)
+def test_activations_at_the_ends_of_the_range(dev, name, qtype, m):
+  """Rows that fp32 only just holds, whose power of two and its inverse must stay normal numbers; and rows with one infinite
+  activation, whose results are infinite with the sign of its weight, beside finite rows that must not notice."""
+  n, k = 64, 4096
+  w, x = synth.weight(qtype, n, k, 97), synth.activations(m, k, 98)
+  x[0] *= 3.0e-37
+  x[1, 300] = np.inf
+  x[2, 4095], x[2, 100] = -np.inf, 1.0e30
+  y = dev.empty((m, n))
+  dev.linear(qtype, dev.array(w), n, k, dev.array(x), m, y)
+  with np.errstate(all="ignore"):
+    got, want = y.download(), oracle.linear(w, qtype, n, k, x)
+  assert not np.isfinite(want[1:3]).any() and np.array_equal(got[1:3], want[1:3], equal_nan=True)
+  for row in [0, *range(3, m)]:
+    assert rel_err(got[row], want[row]) < 1e-5, row
+
+
 @pytest.mark.parametrize("m", [11, 40, 100, 128])
 @pytest.mark.parametrize("name,qtype", TYPES)
 def test_many_rows_of_a_pair_and_of_a_group(dev, name, qtype, m):
