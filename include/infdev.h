@@ -8,7 +8,9 @@
  *
  * Return convention: 0 on success, a negative INFDEV_E_* code otherwise; the text of the last failure
  * of a context is available from infdev_error(). Launches are asynchronous on the context's stream and
- * execute in call order, like the reference's barrier-after-every-dispatch encoder (device.hpp:132).
+ * execute in call order, like the reference's barrier-after-every-dispatch encoder (device.hpp:132). Weights alone may be
+ * fetched while the call before still runs: a call that writes them must be a copy, infdev_fill or infdev_dequant, or be
+ * followed by infdev_commit before they are used.
  */
 #ifndef INFDEV_H
 #define INFDEV_H
@@ -92,6 +94,12 @@ float infdev_event_elapsed_ms(infdev_ctx* ctx, void* start, void* stop);
 int infdev_set_umma(infdev_ctx* ctx, int enabled);
 /* Activation split of the fp16 tensor-core GEMV: 2 = hi+lo fp16 (fp32-accurate, default), 1 = hi only. */
 int infdev_set_xsplit(infdev_ctx* ctx, int xsplit);
+/* 1: the caller promises that the query table and the `previous` records that infdev_gdn_decode reads are complete before the
+ * call that precedes it on the stream starts: written before an infdev_commit, or before an infdev_upload, _download, _copy,
+ * _fill, _gather_tokens or _embedding call that lies between, each of which starts only when everything before it has ended.
+ * The kernel then fetches them while that preceding call still runs. 0 (default): they are read in turn, and a step may
+ * follow the step that wrote its records with anything or nothing in between. */
+int infdev_set_settled_records(infdev_ctx* ctx, int settled);
 /* Q4_K GEMV for up to 8 rows per launch: 1 (default) = integer-MMA kernel over activations quantised to 16 bits per
  * 256-value block (error at most 1.6e-5 of the block maximum), 0 = the fp16-MMA kernel. Q6_K always takes the
  * fp16-MMA kernel. Environment: INFENG_INTEGER_DECODE. */

@@ -185,10 +185,13 @@ __global__ void __launch_bounds__(256, 2) gdn_prepare_kernel(const float* x, con
 // What bounds a decode launch is latency, not bytes: all 256 CTAs are resident at once, so the time is the longest
 // dependent chain of one CTA. The kernel therefore asks for everything up front and keeps block-wide barriers to two per
 // token:
-//  * before griddepcontrol.wait (these depend on nothing the preceding kernel writes): the gate-projection rows of the
-//    head, the conv weights and taps go to shared memory with cp.async (no registers held while in flight), then the 64
-//    KB state goes to registers; after the wait the token's input row follows. The small operands, which hit the L2,
-//    arrive and are consumed while the state is still on its way from HBM.
+//  * before griddepcontrol.wait, like the weights of every kernel here, the gate-projection rows of the head go to shared
+//    memory with cp.async (no registers held while in flight). So do the conv weights and taps, and the 64 KB state goes
+//    to registers: before the wait too where the caller vouches that the preceding kernel writes neither table nor records
+//    (`ahead`), else right after it (one call after the other, 4.3 MB a sequence in the L2: one sequence 5.1 us with and 6.1
+//    without, four 6.9 and 7.4, eight 8.6 and 9.7; 6.4, 9.1 and 10.3 with the gate rows behind the wait as well). The
+//    token's input row follows after the wait. The small operands, which hit the L2, arrive and are consumed while the
+//    state is still on its way from HBM.
 //  * after the first barrier every thread derives the q / k norms and the two gates itself from the partial sums
 //    (redundantly; a second barrier to broadcast them costs more than 256 threads repeating a few instructions);
 //  * after the second barrier (partial products with the state) every warp sums the eight partials of its own four
@@ -219,10 +222,20 @@ __global__ void __launch_bounds__(256, 2) delta_rule_kernel(const float* q, cons
                                                          uint64_t stateOffset, uint64_t stateBytes, float* out, uint8_t* image, int* counters,
                                                          uint32_t chunkedFrom, GdnInputs in) {
   pdl_launch_dependents();
-  // The weights never change. The query table and the state records were written by the first kernels of this pass and
-  // by the pass before it: when only the GEMV kernels and their followers are launched early, those have completed
-  // before the preceding kernel could start, and both may be read ahead of the wait. When every kernel of the pass is
-  // launched early nothing bounds how far ahead this one runs, and it waits first.
+  // A kernel that is launched early lets its successor go before its own wait, so with a few small ones in a row this one can
+  // start while the kernel three or four before it, say the step that writes these records, still runs. The caller knows
+  // whether one of the kernels between is not launched early and so bounds how far ahead this one gets.
+  extern __shared__ float4 stageRaw[];
+  GdnStage& stage = *reinterpret_cast<GdnStage*>(stageRaw);
+  if (FUSED) {
+    const float4* wb = reinterpret_cast<const float4*>(in.wBeta + size_t(blockIdx.x) * 4096);
+    const float4* wa = reinterpret_cast<const float4*>(in.wAlpha + size_t(blockIdx.x) * 4096);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      cp_async16(&stage.wBeta[threadIdx.x + 256 * i], wb + threadIdx.x + 256 * i);
+      cp_async16(&stage.wAlpha[threadIdx.x + 256 * i], wa + threadIdx.x + 256 * i);
+    }
+  }
   if (!in.ahead)
     pdl_wait();
   const infdev_query info = queries[blockIdx.y];
@@ -230,21 +243,12 @@ __global__ void __launch_bounds__(256, 2) delta_rule_kernel(const float* q, cons
   const bool speculative = info.state != kUnbound;
   if (chunkedFrom && !speculative && info.count >= chunkedFrom)  // delta_rule_chunked_kernel takes this query
     return;
-  extern __shared__ float4 stageRaw[];
-  GdnStage& stage = *reinterpret_cast<GdnStage*>(stageRaw);
   __shared__ float qraw[kHeadDim], kraw[kHeadDim], vraw[kHeadDim], red[12], dots[8];
   __shared__ float4 partialPred[8][32], partialQ[8][32];
   const int channels[3] = {keyHead * kHeadDim + (tid & 127), 2048 + keyHead * kHeadDim + (tid & 127), 4096 + head * kHeadDim + (tid & 127)};
   float headA = 0.f, headDt = 0.f;
 
   if (FUSED) {
-    const float4* wb = reinterpret_cast<const float4*>(in.wBeta + size_t(head) * 4096);
-    const float4* wa = reinterpret_cast<const float4*>(in.wAlpha + size_t(head) * 4096);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      cp_async16(&stage.wBeta[tid + 256 * i], wb + tid + 256 * i);
-      cp_async16(&stage.wAlpha[tid + 256 * i], wa + tid + 256 * i);
-    }
     if (tid < kHeadDim) {
       const float4* taps = reinterpret_cast<const float4*>(info.previous + in.convStateOffset);
 #pragma unroll
@@ -940,14 +944,14 @@ cudaError_t delta_rule_launch(const float* q, const float* k, const float* v, co
 cudaError_t gdn_decode_launch(const float* x, const float* mixed, const float* wBeta, const float* wAlpha, const float* A, const float* dt,
                               const float* convWeight, const float* z, const float* normWeight, const infdev_query* queries, int queryCount,
                               uint64_t convStateOffset, uint64_t stateOffset, uint64_t stateBytes, float* out, uint8_t* image, int* counters,
-                              cudaStream_t stream) {
+                              bool ahead, cudaStream_t stream) {
   if (queryCount <= 0)
     return cudaSuccess;
   static PerDeviceOnce configured;
   if (cudaError_t e = configure_shared_memory(delta_rule_kernel<true>, sizeof(GdnStage), configured))
     return e;
   launch_kernel<1>(delta_rule_kernel<true>, dim3(kValueHeads, unsigned(queryCount)), 256, sizeof(GdnStage), stream, nullptr, nullptr, nullptr, nullptr, nullptr, z, normWeight,
-                   queries, stateOffset, stateBytes, out, image, counters, 0u, GdnInputs{x, wBeta, wAlpha, A, dt, mixed, convWeight, convStateOffset, pdl_mode() != 1});
+                   queries, stateOffset, stateBytes, out, image, counters, 0u, GdnInputs{x, wBeta, wAlpha, A, dt, mixed, convWeight, convStateOffset, ahead && pdl_mode() != 1});
   return cudaGetLastError();
 }
 

@@ -18,6 +18,7 @@
 struct infdev_ctx {
   int device = 0, sms = 0, xsplit = 2;
   int umma = 1;  // tcgen05 GEMM for Q4_K launches of more than 8 activation rows, grouped attention rows: 0 off, 1 on
+  bool settledRecords = false;  // infdev_gdn_decode may read its records ahead of its turn
   int integerDecode = 1;     // Q4_K decode GEMV: 1 integer-MMA kernel over an activation image, 0 fp16-MMA kernel
   uint8_t* image = nullptr;  // activation image for the integer decode kernel (K up to 16384)
   int* imageCounters = nullptr;        // arrival counters of the kernels that write images block by block (zero between launches)
@@ -389,6 +390,11 @@ int infdev_set_xsplit(infdev_ctx* ctx, int xsplit) {
   return INFDEV_OK;
 }
 
+int infdev_set_settled_records(infdev_ctx* ctx, int settled) {
+  ctx->settledRecords = settled != 0;
+  return INFDEV_OK;
+}
+
 int infdev_graph_begin(infdev_ctx* ctx) {
   Bind bind(ctx);
   ctx->captureStart = ctx->launches.load();
@@ -702,7 +708,7 @@ int infdev_gdn_decode(infdev_ctx* ctx, const float* x, const float* mixed, const
   ctx->launches += 1;
   return check(ctx,
                infdev::gdn_decode_launch(x, mixed, wBeta, wAlpha, ssmA, ssmDt, convWeight, z, normWeight, queries, queryCount, convStateOffset, stateOffset,
-                                         stateBytes, out, take_capture(ctx), ctx->imageCounters, ctx->stream),
+                                         stateBytes, out, take_capture(ctx), ctx->imageCounters, ctx->settledRecords, ctx->stream),
                "gdn_decode");
 }
 

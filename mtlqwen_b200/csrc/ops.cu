@@ -39,8 +39,7 @@ __device__ __forceinline__ float dequant_q6k_element(const uint8_t* b, int r) {
 }
 
 template <int TYPE> __global__ void dequant_kernel(const uint8_t* blocks, int64_t count, float* out) {
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_wait();  // nobody is let go early: the result may be a weight, which kernels fetch before their own wait
   constexpr int bytes = TYPE == 12 ? 144 : 210;
   const int64_t block = blockIdx.x;
   if (block >= count)
@@ -296,6 +295,7 @@ cudaError_t gather_tokens_launch(const infdev_query* queries, int queryCount, co
                                  const int32_t* proposals, uint32_t mode, int32_t* rowTokens, cudaStream_t stream) {
   if (queryCount <= 0)
     return cudaSuccess;
+  // This and the embedding stay out of the early launches: infdev_set_settled_records counts on them.
   launch_kernel(gather_tokens_kernel, queryCount, 128, 0, stream, queries, queryCount, requestData, capacity, proposals, mode, rowTokens);
   return cudaGetLastError();
 }

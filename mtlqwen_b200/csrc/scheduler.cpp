@@ -188,6 +188,9 @@ Engine::Engine(const std::filesystem::path& path, uint32_t context, const std::f
   batchInvariant = environment("INFENG_BATCH_INVARIANT", 0) != 0;
   if (batchInvariant)
     infdev_set_umma(device.ctx, 0);
+  // Every pass gathers its tokens and embeds them before its first layer, and no kernel of a pass writes a record that a later
+  // layer of the same pass reads.
+  infdev_set_settled_records(device.ctx, 1);
   // The reference sizes the physical pool for one sequence of maximum context (engine.cpp:86); INFENG_KV_BLOCKS overrides.
   const uint32_t perSlot = (context + blockTokens - 1) / blockTokens;
   blocks.resize(environment("INFENG_KV_BLOCKS", perSlot));

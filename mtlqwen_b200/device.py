@@ -55,6 +55,7 @@ def library():
     "infdev_event_record": (i32, (vp, vp)),
     "infdev_event_elapsed_ms": (ctypes.c_float, (vp, vp, vp)),
     "infdev_set_xsplit": (i32, (vp, i32)),
+    "infdev_set_settled_records": (i32, (vp, i32)),
     "infdev_set_integer_decode": (i32, (vp, i32)),
     "infdev_image_bytes": (ctypes.c_size_t, (i64, i64)),
     "infdev_quantize": (i32, (vp, vp, i64, i64, vp)),
@@ -185,6 +186,10 @@ class Device:
 
   def set_xsplit(self, xsplit):
     self.check(self.lib.infdev_set_xsplit(self.ctx, xsplit))
+
+  def set_settled_records(self, settled):
+    """Lets gdn_decode read its query table and records ahead of its turn (see infdev_set_settled_records)."""
+    self.check(self.lib.infdev_set_settled_records(self.ctx, int(settled)))
 
   def set_integer_decode(self, enabled):
     self.check(self.lib.infdev_set_integer_decode(self.ctx, int(enabled)))

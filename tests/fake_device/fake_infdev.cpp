@@ -104,6 +104,7 @@ size_t infdev_image_bytes(int64_t rows, int64_t k) { return size_t((rows + 7) / 
 int infdev_image_capture(infdev_ctx*, uint8_t*) { return 0; }
 int infdev_image_supply(infdev_ctx*, const uint8_t*) { return 0; }
 int infdev_set_umma(infdev_ctx*, int) { return 0; }
+int infdev_set_settled_records(infdev_ctx*, int) { return 0; }
 size_t infdev_attention_scratch_bytes(int64_t rows, uint32_t maxSplits) { return size_t(rows) * 16 * maxSplits * 260 * sizeof(float); }
 
 int infdev_linear(infdev_ctx* ctx, int, const void*, int64_t, int64_t, const float*, int64_t, float*, const float*) { return ++ctx->launches, 0; }

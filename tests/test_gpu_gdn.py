@@ -4,7 +4,7 @@ import pytest
 
 import oracle
 from mtlqwen_b200 import device as D
-from mtlqwen_b200.testing import images
+from mtlqwen_b200.testing import images, synth
 
 pytestmark = pytest.mark.gpu
 TOL = 1e-3  # BASELINE: GDN outputs within 1e-3 relative error in fp32 accumulation
@@ -278,6 +278,58 @@ def test_tokens_before_one_that_is_not_finite_do_not_notice(dev, where, value):
     assert rel_err(out[:, 5][:, columns], clean[:, 5][:, columns]) < 1e-5 and not np.isfinite(out[token:, 5, 33]).any()
   elif where != "g" or value != -np.inf:  # (a decay of zero leaves the token itself finite)
     assert not np.isfinite(out[token, 5]).any()
+
+
+@pytest.mark.parametrize("between", ["nothing", "rms_norm", "linear"])
+def test_steps_follow_each_other_without_a_commit(dev, between):
+  """Each decode step reads the records that the step before it wrote, two sets in turn. What lies between two steps lets its
+  successor start early; the step must still wait for its records."""
+  rng = np.random.default_rng(30)
+  w = {name: dev.array(value) for name, value in layer_weights(rng).items()}
+  nq, steps = 3, 12
+  x, mixed, z = (dev.array(rng.standard_normal((nq, width)).astype(np.float32)) for width in (4096, 8192, 4096))
+  norm, small = dev.array(np.ones(4096, np.float32)), dev.array(synth.weight(D.Q4_K, 16, 4096, 31))
+  start = np.concatenate([rng.standard_normal((nq, 8192 * 4)), 0.01 * rng.standard_normal((nq, 32 * 128 * 128))], axis=1).astype(np.float32)
+  scratch, y, out = dev.empty((nq, 4096)), dev.empty((nq, 16)), dev.empty((nq, 32, 128))
+
+  def run(commit):
+    records = [dev.array(start), dev.empty((nq, LAYER // 4))]
+    tables = []
+    for turn in range(2):
+      queries = []
+      for i in range(nq):
+        q = D.Query()
+        q.previous, q.next = records[turn].ptr + i * LAYER, records[1 - turn].ptr + i * LAYER
+        q.start, q.count, q.position, q.slot, q.state = i, 1, 77, i, D.UNBOUND
+        queries.append(q)
+      tables.append(dev.queries(queries))
+    for step in range(steps):
+      dev.gdn_decode(x, mixed, w["w_beta"], w["w_alpha"], w["ssm_a"], w["ssm_dt"], w["conv"], z, w["norm"], tables[step % 2], nq, 0, D.CONV_STATE_BYTES,
+                     LAYER, out)
+      if between == "rms_norm":
+        dev.rms_norm(x, norm, nq, 4096, scratch)
+      elif between == "linear":
+        dev.linear(D.Q4_K, small, 16, 4096, x, nq, y)
+      if commit:
+        dev.commit()
+    dev.commit()
+    return out.download().tobytes(), records[steps % 2].download().tobytes()
+
+  want = run(True)
+  for _ in range(5):
+    assert run(False) == want
+
+
+def test_settled_records_give_the_same_bits(dev):
+  lengths, a, b = [1, 3, 1, 2], [], []
+  run_layer(dev, np.random.default_rng(32), lengths, speculative=(1, ), fused=True, outputs=a)
+  dev.set_settled_records(1)  # every input was uploaded and committed before the step
+  try:
+    run_layer(dev, np.random.default_rng(32), lengths, speculative=(1, ), fused=True, outputs=b)
+  finally:
+    dev.set_settled_records(0)
+  for x, y in zip(a, b):
+    assert x.tobytes() == y.tobytes()
 
 
 def test_prefill_variant_refuses_an_image(dev):
