@@ -594,7 +594,8 @@ cudaError_t attention_launch(const float* q, const float* qg, const void* cacheK
   // tokens 20.8 against 29.1, 16 of 616 22.8 against 23.6, 16 of 2016 22.8 against 39.4, 64 of 128 24.0 against 28.0).
   const int64_t capacity = int64_t(tableStride) * blockTokens;
   const bool grouped = rows >= 32 * int64_t(queryCount) || (rows >= 5 * int64_t(queryCount) && rows * capacity >= 4096 * int64_t(queryCount));
-  if (grouped && !rowwise) {
+  // The group kernel copies q in pieces of 16 bytes, the scan in pieces of 8.
+  if (grouped && !rowwise && reinterpret_cast<uintptr_t>(q) % 16 == 0) {
     // Some query has several rows. (One row each is the decode pass, where the scan is faster: no query rows to share a
     // tile with, and six small CTAs per SM hide the copies that the group kernel's single CTA waits for.)
     static PerDeviceOnce configured;

@@ -44,10 +44,15 @@ __device__ __forceinline__ const infdev_query& query_of_row(const infdev_query* 
 //    where reading and writing everything once takes 30). State layout: conv taps fp32 [8192][4] at record + stateOffset.
 // CONV_ROWS rows per thread and GATE_HEADS heads per CTA: 8 and 8 where the rows alone fill the GPU, 1 and 1 for short prompt
 // pieces, which have too few CTAs otherwise and wait for one thread's chain of rows (the sums are the same either way).
+// ALIGNED: mixed, convWeight, q, k and v lie on 16-byte boundaries; without, they are read and written value by value.
 constexpr int kGateRows = 8, kFewPrepareRows = 64;
 constexpr int kConvChannels = 4 * 256;  // per CTA
 
-template <int CONV_ROWS, int GATE_HEADS>
+template <bool ALIGNED> __device__ __forceinline__ float4 load_four(const float* p) {
+  return ALIGNED ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+
+template <int CONV_ROWS, int GATE_HEADS, bool ALIGNED>
 __global__ void __launch_bounds__(256, 2) gdn_prepare_kernel(const float* x, const float* wBeta, const float* wAlpha, const float* A, const float* dt,
                                                           const float* mixed, const float* w, const infdev_query* queries, int rows, int gateBlocks,
                                                           uint64_t stateOffset, uint64_t stateBytes, float* q, float* k, float* v, float* beta,
@@ -111,11 +116,11 @@ __global__ void __launch_bounds__(256, 2) gdn_prepare_kernel(const float* x, con
 #pragma unroll
   for (int i = 0; i < CONV_ROWS; ++i)
     if (row0 + i < last)
-      input[i] = *reinterpret_cast<const float4*>(mixed + size_t(row0 + i) * kChannels + c);
+      input[i] = load_four<ALIGNED>(mixed + size_t(row0 + i) * kChannels + c);
   float4 weight[4];  // of the thread's four channels, oldest tap first
 #pragma unroll
   for (int j = 0; j < 4; ++j)
-    weight[j] = *reinterpret_cast<const float4*>(w + size_t(c + j) * 4);
+    weight[j] = load_four<ALIGNED>(w + size_t(c + j) * 4);
   float* const out = c < 2048 ? q + c : c < 4096 ? k + (c - 2048) : v + (c - 4096);
   const size_t pitch = c < 4096 ? 2048 : 4096;
   const infdev_query* info = &query_of_row(queries, uint32_t(row0));
@@ -138,12 +143,12 @@ __global__ void __launch_bounds__(256, 2) gdn_prepare_kernel(const float* x, con
       if (p < 3)
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          taps[j] = info->previous ? *reinterpret_cast<const float4*>(prev + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+          taps[j] = info->previous ? load_four<ALIGNED>(prev + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
         const int position = p - 3 + r;  // tap position + 4 of the record (1 .. 3) when negative
         if (position >= 0)
-          window[r] = *reinterpret_cast<const float4*>(mixed + size_t(info->start + position) * kChannels + c);
+          window[r] = load_four<ALIGNED>(mixed + size_t(info->start + position) * kChannels + c);
         else if (position == -3)
           window[r] = make_float4(taps[0].y, taps[1].y, taps[2].y, taps[3].y);
         else if (position == -2)
@@ -157,9 +162,14 @@ __global__ void __launch_bounds__(256, 2) gdn_prepare_kernel(const float* x, con
     auto tap = [](const float4& weights, float a, float b, float d, float e) {
       return silu_f(fmaf(e, weights.w, fmaf(d, weights.z, fmaf(b, weights.y, fmaf(a, weights.x, 0.f)))));
     };
-    *reinterpret_cast<float4*>(out + size_t(row) * pitch) =
+    const float4 result =
         make_float4(tap(weight[0], window[0].x, window[1].x, window[2].x, now.x), tap(weight[1], window[0].y, window[1].y, window[2].y, now.y),
                     tap(weight[2], window[0].z, window[1].z, window[2].z, now.z), tap(weight[3], window[0].w, window[1].w, window[2].w, now.w));
+    float* const to = out + size_t(row) * pitch;
+    if (ALIGNED)
+      *reinterpret_cast<float4*>(to) = result;
+    else
+      to[0] = result.x, to[1] = result.y, to[2] = result.z, to[3] = result.w;
     const bool speculative = info->state != kUnbound;
     if (speculative || p + 1 == int(info->count)) {
       float4* state = reinterpret_cast<float4*>(info->next + stateOffset + (speculative ? uint64_t(p) * stateBytes : 0)) + c;
@@ -915,10 +925,16 @@ cudaError_t gdn_prepare_launch(const float* x, const float* mixed, const float* 
                      stateOffset, stateBytes, q, k, v, beta, g);
   };
   // With the delta rule after it: 2 rows 17.2 against 22.2 us, 16 rows 19.7 against 25.3, 64 rows level, 96 rows 47.1 against 45.3.
-  if (rows <= kFewPrepareRows)
-    launch(gdn_prepare_kernel<1, 1>, 1, 1);
+  // A caller's views may start at any float.
+  uintptr_t addresses = 0;
+  for (const float* p : {mixed, convWeight, static_cast<const float*>(q), static_cast<const float*>(k), static_cast<const float*>(v)})
+    addresses |= reinterpret_cast<uintptr_t>(p);
+  if (addresses & 15)
+    launch(gdn_prepare_kernel<1, 1, false>, 1, 1);
+  else if (rows <= kFewPrepareRows)
+    launch(gdn_prepare_kernel<1, 1, true>, 1, 1);
   else
-    launch(gdn_prepare_kernel<8, 8>, 8, 8);
+    launch(gdn_prepare_kernel<8, 8, true>, 8, 8);
   return cudaGetLastError();
 }
 

@@ -145,6 +145,26 @@ def test_switching_the_group_kernel_off_changes_rounding_only(dev):
     dev.set_umma(1)
 
 
+def test_queries_that_lie_on_an_odd_multiple_of_eight_bytes(dev):
+  """The kernel for the rows of a prompt copies 16 bytes of q at a time; a q that starts between two such places is served row by row."""
+  rng = np.random.default_rng(50)
+  rows, context, block_tokens = 40, 100, 16
+  table = dev.array(np.arange(7, dtype=np.int32))
+  keys, values = (dev.array(rng.standard_normal((7, 4, block_tokens, 256)).astype(np.float16).view(np.uint16)) for _ in range(2))
+  q, qg = rng.standard_normal((rows, 16, 256)).astype(np.float32), dev.array(rng.standard_normal((rows, 16, 512)).astype(np.float32))
+  info = D.Query()
+  info.start, info.count, info.position, info.slot, info.state = 0, rows, context - rows, 0, D.UNBOUND
+  results = []
+  for offset in (0, 2):
+    buffer = dev.array(np.concatenate([np.zeros(offset, np.float32), q.reshape(-1), np.zeros(8, np.float32)]))
+    view = type("View", (), {"ptr": buffer.ptr + 4 * offset})
+    out, partials = dev.empty((rows, 16, 256)), dev.empty(dev.attention_scratch_bytes(rows, 32) // 4)
+    dev.attention(view, qg, keys, values, dev.queries([info]), 1, rows, table, 7, block_tokens, 32, partials, out)
+    dev.commit()
+    results.append(out.download())
+  assert rel_err(results[1], results[0]) < 1e-5
+
+
 def test_attention_result_does_not_depend_on_batching(dev):
   """A row's split partition depends only on its own context: the output of a sequence's decode row inside an
   8-row pass equals, byte for byte, the output of the same row run alone on the same cache."""

@@ -280,6 +280,53 @@ def test_tokens_before_one_that_is_not_finite_do_not_notice(dev, where, value):
     assert not np.isfinite(out[token, 5]).any()
 
 
+class View:
+  """`count` floats of a buffer from float number `offset` on."""
+
+  def __init__(self, dev, values=None, count=0, offset=1):
+    self.count, self.offset = count if values is None else values.size, offset
+    whole = np.zeros(self.count + 8, np.float32)
+    if values is not None:
+      whole[offset:offset + self.count] = values.reshape(-1)
+    self.buffer = dev.array(whole)
+    self.ptr = self.buffer.ptr + 4 * offset
+
+  def download(self):
+    return self.buffer.download()[self.offset:self.offset + self.count]
+
+
+@pytest.mark.parametrize("lengths", [[1], [5, 2, 40], [100, 3]])
+@pytest.mark.parametrize("unaligned", ["mixed", "conv", "q", "k", "v"])
+def test_preparation_takes_views_at_any_float(dev, lengths, unaligned):
+  rng = np.random.default_rng(40)
+  rows, nq = sum(lengths), len(lengths)
+  w = layer_weights(rng)
+  x, mixed = rng.standard_normal((rows, 4096)).astype(np.float32), rng.standard_normal((rows, 8192)).astype(np.float32)
+  previous = dev.array(rng.standard_normal((nq, LAYER // 4)).astype(np.float32))
+  fixed = {name: dev.array(w[name]) for name in ("w_beta", "w_alpha", "ssm_a", "ssm_dt")}
+
+  def run(offsets):
+    next_ = dev.empty((nq, LAYER // 4))
+    queries, start = [], 0
+    for i, count in enumerate(lengths):
+      q = D.Query()
+      q.previous, q.next = previous.ptr + i * LAYER, next_.ptr + i * LAYER
+      q.start, q.count, q.position, q.slot, q.state = start, count, 77, i, D.UNBOUND
+      queries.append(q)
+      start += count
+    at = lambda name: offsets.get(name, 0)
+    out = [View(dev, count=rows * 2048, offset=at("q")), View(dev, count=rows * 2048, offset=at("k")), View(dev, count=rows * 4096, offset=at("v"))]
+    beta, g = dev.empty((rows, 32)), dev.empty((rows, 32))
+    dev.gdn_prepare(dev.array(x), View(dev, mixed, offset=at("mixed")), fixed["w_beta"], fixed["w_alpha"], fixed["ssm_a"], fixed["ssm_dt"],
+                    View(dev, w["conv"], offset=at("conv")), dev.queries(queries), nq, rows, 0, LAYER, *out, beta, g)
+    dev.commit()
+    return [buffer.download().tobytes() for buffer in (*out, beta, g, next_)]
+
+  want = run({})
+  for offset in (1, 2, 3):
+    assert run({unaligned: offset}) == want
+
+
 @pytest.mark.parametrize("between", ["nothing", "rms_norm", "linear"])
 def test_steps_follow_each_other_without_a_commit(dev, between):
   """Each decode step reads the records that the step before it wrote, two sets in turn. What lies between two steps lets its
