@@ -67,7 +67,7 @@ struct SampleShared {
   int sortedIndex[2 * kMostWanted];
   double chunkSum[kChunks];
   uint32_t histogram[256];
-  uint32_t count, prefix, remaining, ties;
+  uint32_t count, prefix, remaining;
   float threshold;
   int owner;
   double before;
@@ -94,12 +94,12 @@ __device__ __forceinline__ bool ahead(float va, int ia, float vb, int ib) { retu
 
 // The wanted largest of logit / temperature, ties by the earliest index, by a radix select over the order-preserving
 // integer image, for rows with too many equal logits for the cluster's collection. One CTA; leaves the (unsorted) set in
-// sh.value / sh.index and returns its size.
+// sh.value / sh.index and returns its size. A logit that is not a number belongs to no set, as in the cluster's collection.
 __device__ uint32_t radix_candidates(SampleShared& sh, const float* row, int vocab, float temperature, uint32_t wanted) {
   const int tid = threadIdx.x;
   __syncthreads();
   if (tid == 0)
-    sh.prefix = 0, sh.remaining = wanted, sh.count = 0, sh.ties = 0;
+    sh.prefix = 0, sh.remaining = wanted, sh.count = 0;
   for (int pass = 0; pass < 4; ++pass) {
     const int shift = 24 - 8 * pass;
     if (tid < 256)
@@ -107,8 +107,9 @@ __device__ uint32_t radix_candidates(SampleShared& sh, const float* row, int voc
     __syncthreads();
     const uint32_t prefix = sh.prefix, prefixMask = pass ? (0xffffffffu << (shift + 8)) : 0u;
     for (int j = tid; j < vocab; j += kClusterThreads) {
-      const uint32_t key = sortable(row[j] / temperature);
-      if ((key & prefixMask) == prefix)
+      const float value = row[j] / temperature;
+      const uint32_t key = sortable(value);
+      if (value == value && (key & prefixMask) == prefix)
         atomicAdd(&sh.histogram[(key >> shift) & 255u], 1u);
     }
     __syncthreads();
@@ -130,7 +131,7 @@ __device__ uint32_t radix_candidates(SampleShared& sh, const float* row, int voc
   const uint32_t threshold = sh.prefix;
   for (int j = tid; j < vocab; j += kClusterThreads) {
     const float value = row[j] / temperature;
-    if (sortable(value) > threshold) {
+    if (value == value && sortable(value) > threshold) {
       const uint32_t at = atomicAdd(&sh.count, 1u);
       if (at < uint32_t(kMostWanted))
         sh.value[at] = value, sh.index[at] = j;
@@ -141,7 +142,7 @@ __device__ uint32_t radix_candidates(SampleShared& sh, const float* row, int voc
     uint32_t count = min(sh.count, uint32_t(kMostWanted)), need = sh.remaining;
     for (int j = 0; j < vocab && need && count < uint32_t(kMostWanted); ++j) {  // serial scan in index order
       const float value = row[j] / temperature;
-      if (sortable(value) == threshold) {
+      if (value == value && sortable(value) == threshold) {
         sh.value[count] = value, sh.index[count] = j;
         ++count;
         --need;

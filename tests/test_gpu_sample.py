@@ -102,6 +102,21 @@ def test_more_ties_than_the_collection_holds(dev):
   assert tokens.download().tolist() == expected(logits, queries)
 
 
+@pytest.mark.parametrize("value", [np.nan, -np.nan])
+def test_nan_logits_beside_more_ties_than_the_collection_holds(dev, value):
+  """A NaN takes part in no comparison: the row samples as if it were not there, also where ties send it through the radix select."""
+  logits = np.full((1, VOCAB), -5.0, np.float32)
+  logits[0, 5000:8000], logits[0, 100000] = 2.0, 3.0
+  clean = logits.copy()
+  clean[0, [3, 700, 6001]], logits[0, [3, 700, 6001]] = -1.0e30, value
+  for seed in range(8):
+    queries, count = make_queries([(1.5, 1.0, 40, 1)])
+    queries[0].seed = seed
+    tokens = dev.empty(count, np.int32)
+    dev.sample(dev.array(logits), VOCAB, dev.queries(queries), len(queries), count, 0, tokens)
+    assert tokens.download().tolist() == expected(clean, queries)
+
+
 # ---- draft verification on the device against the host loop of the reference ----
 def host_acceptance(samples, speculative, sampled, proposals, draft_width, stops):
   """runtime/engine.cpp:205-216 for one query: returns (accepted, emitted, stopped)."""
