@@ -2,8 +2,9 @@
 //
 // attention_prepare_kernel <- attention_prepare (attention.metal:14-50) + the cache append that the
 //                             reference does inside attention_scan (:126-133)
-// attention_scan_kernel    <- attention_scan   (attention.metal:103-183), for passes whose queries have one row each
-// attention_group_kernel   <- the same, for passes with prompt chunks or speculative rows
+// attention_scan_kernel    <- attention_scan   (attention.metal:103-183), row by row: queries of one row, and passes whose
+//                             queries have few rows on average
+// attention_group_kernel   <- the same, for the queries of several rows of the other passes
 // attention_reduce_kernel  <- attention_reduce (attention.metal:185-216)
 //
 // K/V pool of one layer: [physical block][4 kv heads][blockTokens][256] fp16, so the 16 tokens of a tile of
@@ -11,10 +12,10 @@
 // reaches the same effect through Metal sparse-buffer page mappings, device.cpp:147-198).
 //
 // Split-K: the reference uses max(1, 8/rows) splits (forward.cpp:92), which leaves a 148-SM part idle on a
-// long single-row context and makes the reduction order depend on the batch. Here the number of splits of a
-// row depends only on how many tokens that row attends to, so a sequence gets the same arithmetic whether
-// it runs alone or batched. One CTA serves the four query heads that share a kv head, so K and V are read
-// once per group.
+// long single-row context and makes the reduction order depend on the batch. Here the number of splits of a decode
+// row depends only on how many tokens that row attends to, so a sequence that decodes gets the same arithmetic whether
+// it runs alone, batched or beside a prompt (the rows of a prompt or a draft do not: see attention_launch). One CTA
+// serves the four query heads that share a kv head, so K and V are read once per group.
 #include <algorithm>
 #include <mutex>
 #include "act_image.cuh"
@@ -103,14 +104,31 @@ __device__ __forceinline__ void copy_async16(void* dst, const void* src, uint32_
 // chain of load latencies. Both contractions run on the tensor cores as m16n8k16 with fp16 operands split hi + lo where
 // they are not fp16 already: warp 0 scores the tile's 16 tokens for the four query heads of the group, then warp w
 // accumulates the weighted values of dims 64w .. 64w+63 for all four heads.
+// SINGLES: grid (maxSplits + 1, 4 kv heads, queries), for the queries of one row of a pass whose other queries the group kernel
+// takes, beside that kernel: launched after it and early, it reads nothing that kernel writes and does not wait for it. The
+// group kernel lets it start only after its own wait, so what the kernels before both wrote is there; the fence keeps this
+// CTA's reads behind. One CTA does wait, so that the end of this kernel still means the end of all before it.
+template <bool SINGLES>
 __global__ void __launch_bounds__(128, 6) attention_scan_kernel(const float* q, const __half* cacheK, const __half* cacheV,
                                                                 const infdev_query* queries, int queryCount, const int32_t* table, int tableStride,
                                                                 int blockTokens, uint32_t maxSplits, float* partials) {
   pdl_launch_dependents();
-  pdl_wait();
-  const uint32_t split = blockIdx.x, kvHead = blockIdx.y, row = blockIdx.z;
+  const uint32_t split = blockIdx.x, kvHead = blockIdx.y;
+  if (!SINGLES) {
+    pdl_wait();
+  } else {
+    if (split == maxSplits) {
+      if (!kvHead && !blockIdx.z)
+        pdl_wait();
+      return;
+    }
+    __threadfence();
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const infdev_query& info = query_of_row(queries, queryCount, row);
+  const infdev_query& info = SINGLES ? queries[blockIdx.z] : query_of_row(queries, queryCount, blockIdx.z);
+  if (SINGLES && info.count != 1)
+    return;
+  const uint32_t row = SINGLES ? info.start : blockIdx.z;
   const uint32_t attended = info.position + (row - info.start) + 1;
   uint32_t begin, end, count;
   split_range(attended, maxSplits, split, begin, end, count);
@@ -260,8 +278,10 @@ __global__ void __launch_bounds__(128, 6) attention_scan_kernel(const float* q, 
 //
 // Work items (tile of rows, piece of context, kv head) are dealt to one CTA per SM; which exist only the device knows, so
 // a CTA finds its next item by a scan over the queries. The pieces of a tile follow from its context and from `most`, which
-// the host sets so that the items of the pass fill the SMs about once; a tile of few rows (decode rows that share a pass
-// with a prompt) is cut as finely as the caller's scratch allows.
+// the host sets so that the items of the pass fill the SMs about once; a tile of few rows (speculative rows that share a pass
+// with a prompt) is cut as finely as the caller's scratch allows. Queries of one row are no items: the arithmetic of 16 rows
+// for one made them the longest part of a pass (seven decode rows of 4000 tokens beside a prompt of 121 rows 97 us, 47 with
+// the scan beside this kernel, 63 with all rows in the scan; seven of 32000 tokens 518, 194 and 198).
 constexpr int kGroupRows = 16, kGroupTokens = 64, kGroupThreads = 256, kGroupPitch = kDim + 8, kWeightPitch = kGroupTokens + 8;
 
 struct GroupShared {
@@ -274,6 +294,8 @@ struct GroupShared {
 struct RowTile {
   uint32_t start, rows, first, attended, slot;  // first: position of its first row; attended: context of its last row
 };
+
+__device__ __forceinline__ uint32_t tiles_of(const infdev_query& query) { return query.count > 1 ? (query.count + kGroupRows - 1) / kGroupRows : 0u; }
 
 __device__ __forceinline__ RowTile tile_of(const infdev_query& query, uint32_t index) {
   RowTile tile;
@@ -302,7 +324,7 @@ __device__ __forceinline__ bool find_item(const infdev_query* queries, int query
     infdev_query query = {};
     if (base + int(lane) < queryCount) {
       query = queries[base + lane];
-      tiles = (query.count + kGroupRows - 1) / kGroupRows;
+      tiles = tiles_of(query);
       for (uint32_t t = 0; t < tiles; ++t) {
         const RowTile each = tile_of(query, t);
         mine += piece_count(each.attended, piece_tokens(each.attended, each.rows, most, maxSplits));
@@ -364,8 +386,8 @@ __device__ __forceinline__ uint2 split_pair(float a, float b) {
 __global__ void __launch_bounds__(kGroupThreads, 1)
     attention_group_kernel(const float* q, const __half* cacheK, const __half* cacheV, const infdev_query* queries, int queryCount, const int32_t* table,
                            int tableStride, int blockTokens, uint32_t most, uint32_t maxSplits, float* partials) {
+  pdl_wait();  // first: the scan of the queries of one row starts beside this kernel and relies on it
   pdl_launch_dependents();
-  pdl_wait();
   extern __shared__ __align__(16) uint8_t groupRaw[];
   GroupShared& sh = *reinterpret_cast<GroupShared*>(groupRaw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, head = warp & 3, half = warp >> 2, g = lane >> 2, t = lane & 3;
@@ -520,7 +542,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
 
 // grid (rows * 16), 256 threads: merge the splits, normalise, multiply by sigmoid(gate).
 // `image`, when not null, also receives the activation image of the output rows: a head is one 256-value block.
-// GROUPED: the splits are those of attention_group_kernel.
+// GROUPED: the splits of a row whose query has several are those of attention_group_kernel.
 template <bool GROUPED>
 __global__ void __launch_bounds__(256) attention_reduce_kernel(const float* partials, const float* qg, const infdev_query* queries, int queryCount,
                                                                uint32_t most, uint32_t maxSplits, float* out, uint8_t* image) {
@@ -529,7 +551,7 @@ __global__ void __launch_bounds__(256) attention_reduce_kernel(const float* part
   const uint32_t headRow = blockIdx.x, row = headRow / kQHeads, dim = threadIdx.x;
   const infdev_query& info = query_of_row(queries, queryCount, row);
   uint32_t count;
-  if (GROUPED) {
+  if (GROUPED && info.count > 1) {
     const RowTile tile = tile_of(info, (row - info.start) / kGroupRows);
     count = piece_count(tile.attended, piece_tokens(tile.attended, tile.rows, most, maxSplits));
   } else {
@@ -584,9 +606,11 @@ cudaError_t attention_prepare_launch(const float* qg, const float* rawK, const f
 
 cudaError_t attention_launch(const float* q, const float* qg, const void* cacheK, const void* cacheV, const infdev_query* queries,
                              int queryCount, const int32_t* table, int tableStride, int blockTokens, int64_t rows, uint32_t maxSplits, float* partials, float* out,
-                             uint8_t* image, bool rowwise, int sms, cudaStream_t stream) {
+                             uint8_t* image, bool rowwise, int sms, cudaStream_t stream, int* launches) {
+  *launches = 0;
   if (rows <= 0)
     return cudaSuccess;
+  *launches = 2;
   const uint32_t splits = std::min<uint32_t>(maxSplits, 32);  // the merge keeps one split per lane
   // The group kernel takes passes whose queries have five rows or more on average, unless no context of the pass can be long
   // (the table has no room for it): with r rows a query, its longer chain costs 2 us where r x context is below about 4096 (8
@@ -596,8 +620,6 @@ cudaError_t attention_launch(const float* q, const float* qg, const void* cacheK
   const bool grouped = rows >= 32 * int64_t(queryCount) || (rows >= 5 * int64_t(queryCount) && rows * capacity >= 4096 * int64_t(queryCount));
   // The group kernel copies q in pieces of 16 bytes, the scan in pieces of 8.
   if (grouped && !rowwise && reinterpret_cast<uintptr_t>(q) % 16 == 0) {
-    // Some query has several rows. (One row each is the decode pass, where the scan is faster: no query rows to share a
-    // tile with, and six small CTAs per SM hide the copies that the group kernel's single CTA waits for.)
     static PerDeviceOnce configured;
     if (const cudaError_t e = configure_shared_memory(attention_group_kernel, sizeof(GroupShared), configured))
       return e;
@@ -607,10 +629,26 @@ cudaError_t attention_launch(const float* q, const float* qg, const void* cacheK
     launch_kernel<2>(attention_group_kernel, unsigned(std::min<int64_t>(items, sms)), kGroupThreads, sizeof(GroupShared), stream, q,
                   static_cast<const __half*>(cacheK), static_cast<const __half*>(cacheV), queries, queryCount, table, tableStride, blockTokens, most, splits,
                   partials);
+    // Queries of one row stay with the scan, which is faster there: no query rows to share a tile with, and six small CTAs per
+    // SM hide the copies that the group kernel's single CTA waits for. Which queries they are only the device knows; with a
+    // single query there are none.
+    if (queryCount > 1) {
+      *launches = 3;
+      // Its CTAs start on the SMs that the group kernel leaves first: shared memory that nobody uses spreads the few of a pass with
+      // few queries over all SMs (one row of 32000 tokens beside a prompt: six on an SM 124 us, one 89).
+      constexpr size_t kSmShared = 228 * 1024, kScanShared = sizeof(float) * kGroup * kTile + sizeof(__half) * 2 * 2 * kTile * (kDim + 8) + 1024;
+      static PerDeviceOnce scanConfigured;
+      if (const cudaError_t e = configure_shared_memory(attention_scan_kernel<true>, kSmShared / 2 - kScanShared + 256, scanConfigured))
+        return e;
+      const size_t perSm = std::clamp<size_t>((splits * kKvHeads * size_t(queryCount - 1) + sms - 1) / sms, 1, 6);
+      const size_t spread = perSm < 6 ? kSmShared / (perSm + 1) - kScanShared + 256 : 0;
+      launch_kernel<2>(attention_scan_kernel<true>, dim3(splits + 1, kKvHeads, unsigned(queryCount)), 128, spread, stream, q, static_cast<const __half*>(cacheK),
+                       static_cast<const __half*>(cacheV), queries, queryCount, table, tableStride, blockTokens, splits, partials);
+    }
     launch_kernel<2>(attention_reduce_kernel<true>, unsigned(rows * kQHeads), 256, 0, stream, partials, qg, queries, queryCount, most, splits, out, image);
     return cudaGetLastError();
   }
-  launch_kernel(attention_scan_kernel, dim3(splits, kKvHeads, unsigned(rows)), 128, 0, stream, q, static_cast<const __half*>(cacheK),
+  launch_kernel(attention_scan_kernel<false>, dim3(splits, kKvHeads, unsigned(rows)), 128, 0, stream, q, static_cast<const __half*>(cacheK),
                                                                                        static_cast<const __half*>(cacheV), queries, queryCount, table,
                                                                                        tableStride, blockTokens, splits, partials);
   launch_kernel(attention_reduce_kernel<false>, unsigned(rows * kQHeads), 256, 0, stream, partials, qg, queries, queryCount, 0u, splits, out, image);
@@ -651,7 +689,7 @@ cudaError_t attention_static_launch(const float* q, const float* qg, const void*
   }
   // Nothing has to start at zero: the reduction reads exactly the (row, head, split) records that the scan of the
   // same call wrote; whatever an earlier call left in the array is never read.
-  launch_kernel(attention_scan_kernel, dim3(kStaticSplits, kKvHeads, unsigned(rows)), 128, 0, stream, q, static_cast<const __half*>(cacheK),
+  launch_kernel(attention_scan_kernel<false>, dim3(kStaticSplits, kKvHeads, unsigned(rows)), 128, 0, stream, q, static_cast<const __half*>(cacheK),
                                                                                           static_cast<const __half*>(cacheV), queries, queryCount, table,
                                                                                           tableStride, blockTokens, kStaticSplits, partials);
   launch_kernel(attention_reduce_kernel<false>, unsigned(rows * kQHeads), 256, 0, stream, partials, qg, queries, queryCount, 0u, uint32_t(kStaticSplits), out, nullptr);

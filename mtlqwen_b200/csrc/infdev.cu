@@ -780,11 +780,11 @@ int infdev_attention(infdev_ctx* ctx, const float* q, const float* qg, const voi
     return fail(ctx, INFDEV_E_ARGUMENT, "attention: rows without queries");
   if (blockTokens <= 0 || blockTokens % 16 || maxSplits < 1 || maxSplits > 64)
     return fail(ctx, INFDEV_E_ARGUMENT, "attention: blockTokens must be a multiple of 16 and maxSplits in 1..64");
-  ctx->launches += 2;
-  return check(ctx,
-               infdev::attention_launch(q, qg, cacheK, cacheV, queries, queryCount, table, tableStride, blockTokens, rows, maxSplits, partials, out,
-                                        take_capture(ctx), !ctx->umma, ctx->sms, ctx->stream),
-               "attention");
+  int launches = 0;
+  const cudaError_t e = infdev::attention_launch(q, qg, cacheK, cacheV, queries, queryCount, table, tableStride, blockTokens, rows, maxSplits, partials, out,
+                                                 take_capture(ctx), !ctx->umma, ctx->sms, ctx->stream, &launches);
+  ctx->launches += launches;
+  return check(ctx, e, "attention");
 }
 
 int infdev_mtp_fuse(infdev_ctx* ctx, const float* embedding, const float* hidden, const infdev_query* queries, int queryCount, const float* enorm,

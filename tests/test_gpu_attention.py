@@ -165,6 +165,35 @@ def test_queries_that_lie_on_an_odd_multiple_of_eight_bytes(dev):
   assert rel_err(results[1], results[0]) < 1e-5
 
 
+@pytest.mark.parametrize("prompt", [60, 128])
+def test_decode_rows_beside_a_prompt_have_the_bits_of_a_decode_pass(dev, prompt):
+  """Rows of one token stay with the row-by-row kernel when a prompt chunk shares their pass."""
+  rng = np.random.default_rng(51)
+  contexts, block_tokens, stride = [3000, 1, 700, 64], 16, 256
+  blocks = len(contexts) * stride + -(-prompt // block_tokens)
+  table = dev.array(np.concatenate([rng.permutation(blocks), np.zeros(5 * stride - blocks)]).astype(np.int32))
+  keys, values = (dev.array(rng.standard_normal((blocks, 4, block_tokens, 256)).astype(np.float16).view(np.uint16)) for _ in range(2))
+  rows = len(contexts) + prompt
+  q, qg = rng.standard_normal((rows, 16, 256)).astype(np.float32), rng.standard_normal((rows, 16, 512)).astype(np.float32)
+
+  def run(counts):
+    queries, start, positions = [], 0, [c - 1 for c in contexts] + [0]
+    for slot, count in enumerate(counts):
+      info = D.Query()
+      info.start, info.count, info.position, info.slot, info.state = start, count, positions[slot], slot, D.UNBOUND
+      queries.append(info)
+      start += count
+    out, partials = dev.empty((start, 16, 256)), dev.empty(dev.attention_scratch_bytes(start, 32) // 4)
+    dev.attention(dev.array(q[:start]), dev.array(qg[:start]), keys, values, dev.queries(queries), len(queries), start, table, stride, block_tokens, 32,
+                  partials, out)
+    dev.commit()
+    return out.download()
+
+  alone = run([1] * 4)
+  for _ in range(3):
+    assert run([1] * 4 + [prompt])[:4].tobytes() == alone.tobytes()
+
+
 def test_attention_result_does_not_depend_on_batching(dev):
   """A row's split partition depends only on its own context: the output of a sequence's decode row inside an
   8-row pass equals, byte for byte, the output of the same row run alone on the same cache."""
