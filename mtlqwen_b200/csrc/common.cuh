@@ -30,19 +30,31 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // of the decode attention takes SMs from the scan it waits for (142 -> 163 us for eight long contexts).
 int pdl_mode();
 
-template <int EARLY = 0, class... Params, class... Args>
-cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, dim3 block, size_t sharedBytes, cudaStream_t stream, Args&&... args) {
+// `cluster`: CTAs of a cluster along x, 0 for a kernel without.
+template <int EARLY, class... Params, class... Args>
+cudaError_t launch_clusters(unsigned cluster, void (*kernel)(Params...), dim3 grid, dim3 block, size_t sharedBytes, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
   config.blockDim = block;
   config.dynamicSmemBytes = sharedBytes;
   config.stream = stream;
-  cudaLaunchAttribute attribute[1];
-  attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attribute[2];
   config.attrs = attribute;
-  config.numAttrs = (pdl_mode() == 1 || (pdl_mode() == 2 && EARLY == 1) || (pdl_mode() == 3 && EARLY >= 1)) ? 1 : 0;
+  if (pdl_mode() == 1 || (pdl_mode() == 2 && EARLY == 1) || (pdl_mode() == 3 && EARLY >= 1)) {
+    attribute[config.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute[config.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster) {
+    attribute[config.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attribute[config.numAttrs].val.clusterDim.x = cluster;
+    attribute[config.numAttrs].val.clusterDim.y = attribute[config.numAttrs].val.clusterDim.z = 1;
+    ++config.numAttrs;
+  }
   return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+template <int EARLY = 0, class... Params, class... Args>
+cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, dim3 block, size_t sharedBytes, cudaStream_t stream, Args&&... args) {
+  return launch_clusters<EARLY>(0, kernel, grid, block, sharedBytes, stream, static_cast<Args&&>(args)...);
 }
 
 // A kernel's opt-in to more than 48 KB of dynamic shared memory is a property of the (kernel, device) pair, and one

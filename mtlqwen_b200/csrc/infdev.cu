@@ -820,7 +820,7 @@ int infdev_sample(infdev_ctx* ctx, const float* logits, int64_t vocab, infdev_qu
   Bind bind(ctx);
   (void)queryCount;
   ctx->launches += 1;
-  return check(ctx, infdev::sample_launch(logits, int(vocab), queries, count, mode, tokens, ctx->stream), "sample");
+  return check(ctx, infdev::sample_launch(logits, int(vocab), queries, count, mode, tokens, ctx->sms, ctx->stream), "sample");
 }
 
 int infdev_pack_queries(infdev_ctx* ctx, const infdev_query* in, int count, int drafting, uint32_t draftWidth, const uint64_t* statePrevious,

@@ -43,7 +43,7 @@ cudaError_t attention_static_launch(const float* q, const float* qg, const void*
                                     int queryCount, const int32_t* table, int tableStride, int blockTokens, int64_t rows, int device, float* out,
                                     cudaStream_t stream);
 int attention_static_max_rows();
-cudaError_t sample_launch(const float* logits, int vocab, infdev_query* queries, int64_t count, uint32_t mode, int32_t* tokens,
+cudaError_t sample_launch(const float* logits, int vocab, infdev_query* queries, int64_t count, uint32_t mode, int32_t* tokens, int sms,
                           cudaStream_t stream);
 cudaError_t pack_queries_launch(const infdev_query* in, int count, int drafting, uint32_t draftWidth, const uint64_t* statePrevious,
                                 const uint64_t* stateNext, uint64_t candidateBase, uint64_t stateBytes, infdev_query* out, uint32_t* meta,

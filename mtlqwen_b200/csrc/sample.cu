@@ -1,7 +1,7 @@
 // On-GPU sampling, query packing and draft verification.
 //
 // sample_kernel <- sample_logits (native_ops.metal:122-224). The reference runs the temperature path on one
-// thread (a serial insertion sort over 248,320 logits); here a cluster of eight CTAs finds the top-k set, and only the
+// thread (a serial insertion sort over 248,320 logits); here a cluster of CTAs finds the top-k set, and only the
 // final <= 64-step softmax / top-p / inverse-CDF walk is serial, in exactly the reference's order.
 // RNG: Philox4x32-10 keyed by the slot seed, counter = absolute index of the sampled token in its sequence,
 // so a sequence draws the same variates whether it runs alone, batched or speculatively (the reference
@@ -40,44 +40,51 @@ __device__ __forceinline__ uint32_t sortable(float v) {
   return bits ^ ((bits & 0x80000000u) ? 0xffffffffu : 0x80000000u);
 }
 
-// ---- one row of logits, eight CTAs ----------------------------------------------------------------------------------
-// grid (8, count), clusters of 8 CTAs of 512 threads: a cluster samples one row, each CTA looks at an eighth of the
+// ---- one row of logits, a cluster of up to eight CTAs -----------------------------------------------------------------
+// grid (C, count), clusters of C = 1, 2, 4 or 8 CTAs of 512 threads: a cluster samples one row, each CTA looks at a C-th of the
 // vocabulary and the results meet in the shared memory of the cluster's first CTA. A row is 1 MB that the output head
 // has just left in the L2, so what bounds it is how many SMs ask for it and how often; one CTA per row needed 20 us for
 // the argmax of eight rows of 248320 logits and 361 us for their top-40 (five walks over the row, and a histogram whose
-// shared-memory atomics nearly all hit the few bins that hold the exponents of ordinary logits). Norm, output head and
-// top-40 of eight rows went from 599 to 265 us, of which the output head is 245.
+// shared-memory atomics nearly all hit the few bins that hold the exponents of ordinary logits). C: see sample_launch.
 //
-// Top-k without a histogram: the cluster's 128 warps hold 128 disjoint parts of the row, so the wanted-th largest of
-// their 128 maxima has at least `wanted` logits at or above it and can serve as a threshold; a second walk collects what
-// reaches it (about 50 logits for a top-40 of random ones), and the exact order among those, value then index, is found
-// by counting. Ties can make the collection arbitrarily large; when it does not fit, the first CTA walks the row by
-// itself with a radix select (radix_candidates below).
-constexpr int kClusterCtas = 8, kClusterThreads = 512, kClusterWarps = kClusterThreads / kWarp;
+// Top-k without a histogram: the cluster's threads fall into 128 groups that hold 128 disjoint parts of the row, so the
+// wanted-th largest of their 128 maxima has at least `wanted` logits at or above it and can serve as a threshold; a second walk
+// collects what reaches it (about 50 logits for a top-40 of random ones), and the exact order among those, value then index, is
+// found by counting. Divisions by the temperature are left to the few logits near the threshold. Equal logits can make that
+// collection arbitrarily large: a row whose mask leaves few logits has its threshold among the masked ones. The first walk
+// therefore counts the logits that equal their part's maximum; where too many equal the threshold, only what lies above it is
+// collected, each warp looks for the first equal ones of a contiguous piece of the row, and the earliest of them fill the set up
+// (ten logits of 248320 left by a mask, eight rows: 32 us; 548 with one CTA and a radix select). Where the collection does
+// not fit all the same, the first CTA walks the row by itself with that select (radix_candidates below).
+constexpr int kMaxClusterCtas = 8, kClusterThreads = 512, kClusterWarps = kClusterThreads / kWarp;
+constexpr int kParts = 128;         // disjoint parts whose maxima the threshold is taken from
 constexpr int kCandidates = 2048;   // collected logits that fit
+constexpr int kMostTied = 256;      // more at the threshold than these stay out of the collection (ranking all of 1003 took 40 us)
 constexpr int kMostWanted = 64;
-constexpr int kChunks = 1024;       // plain temperature sampling sums the row in this many contiguous pieces
+constexpr int kChunks = 128;        // plain temperature sampling sums the row in this many contiguous pieces per CTA
 
 struct SampleShared {
-  float maxima[kClusterCtas * kClusterWarps];
-  int indices[kClusterCtas * kClusterWarps];
+  float maxima[kParts];  // of the parts; of the warps for the argmax
+  int indices[kParts];
   float value[kCandidates];
   int index[kCandidates];
   float sortedValue[2 * kMostWanted], weight[kMostWanted];
   int sortedIndex[2 * kMostWanted];
-  double chunkSum[kChunks];
+  int tie[kClusterWarps][kMostWanted], tieCount[kClusterWarps];  // the first logits equal to the threshold in this warp's piece
+  double chunkSum[kMaxClusterCtas * kChunks];
   uint32_t histogram[256];
-  uint32_t count, prefix, remaining;
+  uint32_t equals[kParts];  // logits of the part that equal its maximum
+  uint32_t count, prefix, remaining, tied;
   float threshold;
   int owner;
   double before;
 };
 
 // Calls f(logit, index) for this thread's logits of the CTA's part of the row, in ascending order of the index.
-template <class F> __device__ __forceinline__ void for_part(const float* row, int vocab, uint32_t part, F f) {
+template <class F> __device__ __forceinline__ void for_part(const float* row, int vocab, uint32_t part, uint32_t ctas, F f) {
   if (vocab % 4 == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
     const float4* row4 = reinterpret_cast<const float4*>(row);
-    const int quads = vocab / 4, per = (quads + kClusterCtas - 1) / kClusterCtas, last = min(quads, int(part + 1) * per);
+    const int quads = vocab / 4, per = (quads + int(ctas) - 1) / int(ctas), last = min(quads, int(part + 1) * per);
 #pragma unroll 4
     for (int j = int(part) * per + int(threadIdx.x); j < last; j += kClusterThreads) {
       const float4 v = row4[j];
@@ -85,7 +92,7 @@ template <class F> __device__ __forceinline__ void for_part(const float* row, in
     }
     return;
   }
-  const int per = (vocab + kClusterCtas - 1) / kClusterCtas, last = min(vocab, int(part + 1) * per);
+  const int per = (vocab + int(ctas) - 1) / int(ctas), last = min(vocab, int(part + 1) * per);
   for (int j = int(part) * per + int(threadIdx.x); j < last; j += kClusterThreads)
     f(row[j], j);
 }
@@ -156,16 +163,16 @@ __device__ uint32_t radix_candidates(SampleShared& sh, const float* row, int voc
 
 // mode 0: target sampling; mode 1: MTP drafting (always argmax, and bumps the drafter query's position,
 // native_ops.metal:128-129).
-__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads, 1)
+__global__ void __launch_bounds__(kClusterThreads, 1)
     sample_kernel(const float* logits, int vocab, infdev_query* queries, uint32_t mode, int32_t* tokens) {
   __shared__ SampleShared sh;
   cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   pdl_launch_dependents();
-  const uint32_t i = blockIdx.y, part = cluster.block_rank();
+  const uint32_t i = blockIdx.y, part = cluster.block_rank(), ctas = cluster.num_blocks();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   SampleShared& first = *cluster.map_shared_rank(&sh, 0);
   if (tid == 0)
-    sh.count = 0;
+    sh.count = 0, sh.tied = 0;
   cluster.sync();  // every CTA of the cluster runs, and the first one's counter is zero
   pdl_wait();
   const infdev_query info = query_of_logit(queries, i);
@@ -175,7 +182,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
     // first-index argmax (native_ops.metal:137-158)
     float best = -INFINITY;
     int index = 0;
-    for_part(row, vocab, part, [&](float v, int j) {
+    for_part(row, vocab, part, ctas, [&](float v, int j) {
       if (v > best)
         best = v, index = j;
     });
@@ -191,8 +198,8 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
     cluster.sync();
     if (part || warp)
       return;
-    best = sh.maxima[lane], index = sh.indices[lane];
-    for (int w = lane + 32; w < kClusterCtas * kClusterWarps; w += 32)
+    best = -INFINITY, index = 0;
+    for (int w = lane; w < int(ctas) * kClusterWarps; w += 32)
       if (ahead(sh.maxima[w], sh.indices[w], best, index))
         best = sh.maxima[w], index = sh.indices[w];
 #pragma unroll
@@ -216,12 +223,24 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
 
   const float temperature = info.temperature;
   const float random = philox_uniform(info.seed, uint64_t(info.position) + info.count - info.samples + (i - info.logit) + 1);
-  // every warp's maximum of logit / temperature, for every CTA of the cluster
+  // the maximum of every part (4 x ctas lanes) and how many logits equal it, for every CTA of the cluster
   float maximum = -INFINITY;
-  for_part(row, vocab, part, [&](float v, int) { maximum = fmaxf(maximum, v / temperature); });
-  maximum = warp_max(maximum);
-  if (lane < kClusterCtas)
-    cluster.map_shared_rank(&sh, lane)->maxima[part * kClusterWarps + warp] = maximum;
+  uint32_t equals = 0;
+  for_part(row, vocab, part, ctas, [&](float v, int) {
+    equals = v > maximum ? 1u : equals + (v == maximum ? 1u : 0u);
+    maximum = fmaxf(maximum, v);
+  });
+  const uint32_t lanes = 4 * ctas, mine = (part * kClusterThreads + tid) / lanes;
+  const float own = maximum;
+  for (uint32_t o = lanes / 2; o; o >>= 1)
+    maximum = fmaxf(maximum, __shfl_xor_sync(0xffffffffu, maximum, o));
+  equals = own == maximum ? equals : 0u;
+  for (uint32_t o = lanes / 2; o; o >>= 1)
+    equals += __shfl_xor_sync(0xffffffffu, equals, o);
+  if (lane % lanes < ctas) {
+    SampleShared& to = *cluster.map_shared_rank(&sh, lane % lanes);
+    to.maxima[mine] = maximum, to.equals[mine] = equals;
+  }
   cluster.sync();
 
   if (info.topK == 0) {
@@ -229,9 +248,9 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
     // double precision in contiguous chunks, 128 of them per CTA and one at a time per warp; the first CTA finds the chunk
     // in which the cumulative sum passes the target and walks that one in vocabulary order.
     maximum = fmaxf(fmaxf(sh.maxima[lane], sh.maxima[lane + 32]), fmaxf(sh.maxima[lane + 64], sh.maxima[lane + 96]));
-    maximum = warp_max(maximum);
-    const int chunk = (vocab + kChunks - 1) / kChunks;
-    for (int c = int(part) * (kChunks / kClusterCtas) + warp; c < int(part + 1) * (kChunks / kClusterCtas); c += kClusterWarps) {
+    maximum = warp_max(maximum) / temperature;
+    const int chunks = int(ctas) * kChunks, chunk = (vocab + chunks - 1) / chunks;
+    for (int c = int(part) * kChunks + warp; c < int(part + 1) * kChunks; c += kClusterWarps) {
       double sum = 0.0;
       for (int j = c * chunk + lane; j < min(vocab, (c + 1) * chunk); j += 32)
         sum += double(expf(row[j] / temperature - maximum));
@@ -244,11 +263,13 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
     cluster.sync();
     if (part || warp)
       return;
-    // lane l holds the sum of its 32 consecutive chunks; exclusive scan over the lanes
-    double mine = 0.0;
-    for (int c = 0; c < kChunks / 32; ++c)
-      mine += sh.chunkSum[lane * (kChunks / 32) + c];
-    double inclusive = mine;
+    // lane l holds the sum of its consecutive chunks; exclusive scan over the lanes
+    const int perLane = chunks / 32;
+    double lanes32 = 0.0;
+#pragma unroll 4
+    for (int c = 0; c < perLane; ++c)
+      lanes32 += sh.chunkSum[lane * perLane + c];
+    double inclusive = lanes32;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const double other = __shfl_up_sync(0xffffffffu, inclusive, o);
@@ -259,9 +280,9 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
     const uint32_t reached = __ballot_sync(0xffffffffu, inclusive >= target);
     const int ownerLane = reached ? __ffs(reached) - 1 : 31;
     if (lane == ownerLane) {
-      double cumulative = inclusive - mine;
-      int owner = lane * (kChunks / 32);
-      const int end = owner + kChunks / 32 - 1;
+      double cumulative = inclusive - lanes32;
+      int owner = lane * perLane;
+      const int end = owner + perLane - 1;
       for (; owner < end && cumulative + sh.chunkSum[owner] < target; ++owner)
         cumulative += sh.chunkSum[owner];
       sh.owner = owner, sh.before = cumulative;
@@ -293,31 +314,81 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
 
   // ---- top-k (<= 64) ----
   const uint32_t wanted = min(uint32_t(info.topK), uint32_t(kMostWanted));
-  if (tid < kClusterCtas * kClusterWarps) {
-    const float own = sh.maxima[tid];
+  if (tid < kParts) {
+    const float limit = sh.maxima[tid];
     uint32_t above = 0, level = 0;
 #pragma unroll 8
-    for (int w = 0; w < kClusterCtas * kClusterWarps; ++w) {
-      above += sh.maxima[w] > own ? 1u : 0u;
-      level += sh.maxima[w] >= own ? 1u : 0u;
+    for (int w = 0; w < kParts; ++w) {
+      above += sh.maxima[w] > limit ? 1u : 0u;
+      level += sh.maxima[w] >= limit ? 1u : 0u;
     }
-    if (above < wanted && wanted <= level)  // equal maxima all write the same value
-      sh.threshold = own;
+    if (above < wanted && wanted <= level)  // the parts whose maximum is the threshold, which all write it
+      sh.threshold = limit, atomicAdd(&sh.tied, sh.equals[tid]);
   }
   __syncthreads();
-  const float threshold = sh.threshold;
-  for_part(row, vocab, part, [&](float v, int j) {
+  const float threshold = sh.threshold / temperature;
+  // A quotient reaches the threshold's only if its logit comes within rounding of it (or if the quotients overflow).
+  const float slack = fmaxf(fmaxf(fabsf(sh.threshold) * 1.0e-6f, 1.0e-36f), temperature * 1.0e-44f), near = fabsf(threshold) < INFINITY ? sh.threshold - slack : -INFINITY;
+  const bool ties = sh.tied <= uint32_t(kMostTied);  // the collection holds what equals the threshold too
+  for_part(row, vocab, part, ctas, [&](float v, int j) {
+    if (!(v >= near))
+      return;
     const float value = v / temperature;
-    if (value >= threshold) {
+    if (ties ? value >= threshold : value > threshold) {
       const uint32_t at = atomicAdd(&first.count, 1u);
       if (at < uint32_t(kCandidates))
         first.value[at] = value, first.index[at] = j;
     }
   });
   cluster.sync();
+  if (ties && part)
+    return;
+  uint32_t count = first.count;
+  if (!ties && count < wanted) {
+    // every warp: the first logits of its contiguous piece that equal the threshold, no more than are missing
+    const uint32_t missing = wanted - count;
+    const int pieces = int(ctas) * kClusterWarps, per = (vocab + pieces - 1) / pieces, from = (int(part) * kClusterWarps + warp) * per, to = min(vocab, from + per);
+    uint32_t have = 0;
+    for (int base = from; base < to && have < missing; base += 4 * kWarp) {
+      float value[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int j = base + kWarp * e + lane;
+        value[e] = j < to ? row[j] / temperature : NAN;
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint32_t equal = __ballot_sync(0xffffffffu, value[e] == threshold), before = have + __popc(equal & ((1u << lane) - 1u));
+        if (value[e] == threshold && before < missing)
+          sh.tie[warp][before] = base + kWarp * e + lane;
+        have += __popc(equal);
+      }
+    }
+    if (lane == 0)
+      sh.tieCount[warp] = int(min(have, missing));
+    cluster.sync();
+    if (part == 0 && warp == 0) {
+      // the pieces in the order of the vocabulary
+      uint32_t filled = 0;
+      for (uint32_t rank = 0; rank < ctas && filled < missing; ++rank) {
+        const SampleShared& other = *cluster.map_shared_rank(&sh, rank);
+        for (int w = 0; w < kClusterWarps && filled < missing; ++w) {
+          const uint32_t take = min(uint32_t(other.tieCount[w]), missing - filled);
+          for (uint32_t e = lane; e < take; e += kWarp)
+            sh.value[count + filled + e] = threshold, sh.index[count + filled + e] = other.tie[w][e];
+          filled += take;
+        }
+      }
+      if (lane == 0)
+        sh.count = count + filled;
+    }
+    cluster.sync();  // the others' lists have been read
+    count = sh.count;  // of use in the first CTA
+  } else if (!ties) {
+    cluster.sync();  // all have read the first CTA's count
+  }
   if (part)
     return;
-  uint32_t count = sh.count;
   if (count > uint32_t(kCandidates))
     count = radix_candidates(sh, row, vocab, temperature, wanted);
   // the exact order: value descending, index ascending
@@ -465,12 +536,17 @@ __global__ void __launch_bounds__(256) commit_states_kernel(const infdev_query* 
 
 }  // namespace
 
-cudaError_t sample_launch(const float* logits, int vocab, infdev_query* queries, int64_t count, uint32_t mode, int32_t* tokens,
+cudaError_t sample_launch(const float* logits, int vocab, infdev_query* queries, int64_t count, uint32_t mode, int32_t* tokens, int sms,
                           cudaStream_t stream) {
   if (count <= 0)
     return cudaSuccess;
-  launch_kernel<2>(sample_kernel, dim3(kClusterCtas, unsigned(count)), kClusterThreads, 0, stream, logits, vocab, queries, mode, tokens);
-  return cudaGetLastError();
+  // As many CTAs for a row as leave every one an SM of its own and a float4 per thread: 40 rows of 248320 logits with eight CTAs
+  // each 24.5 us (argmax) and 66.8 (top-40), with two 14.8 and 38.6; eight rows with eight CTAs each 5.9 and 17.5, 1003 logits a
+  // row 53 us with eight (most warps had none, and the threshold let everything through), 9 with one.
+  unsigned ctas = kMaxClusterCtas;
+  while (ctas > 1 && (count * int64_t(ctas) > sms || vocab < int(ctas) * kClusterThreads * 4))
+    ctas /= 2;
+  return launch_clusters<2>(ctas, sample_kernel, dim3(ctas, unsigned(count)), kClusterThreads, 0, stream, logits, vocab, queries, mode, tokens);
 }
 
 cudaError_t pack_queries_launch(const infdev_query* in, int count, int drafting, uint32_t draftWidth, const uint64_t* statePrevious,

@@ -102,6 +102,46 @@ def test_more_ties_than_the_collection_holds(dev):
   assert tokens.download().tolist() == expected(logits, queries)
 
 
+@pytest.mark.parametrize("rows,vocab", [(18, 16384), (19, 16384), (37, 8200), (40, 8192), (75, 4096), (150, 4099), (3, 4095), (2, 130)])
+def test_every_number_of_ctas_for_a_row(dev, rows, vocab):
+  """Rows share the SMs: eight CTAs for a row of a few, four, two, one of many, and no more than the vocabulary keeps busy."""
+  rng = np.random.default_rng(rows)
+  logits = (2.0 * rng.standard_normal((rows, vocab))).astype(np.float32)
+  params = [(0.0, 1.0, 0, 1), (0.7, 0.9, 40, 1), (1.3, 1.0, 64, 1), (1.0, 0.8, 1, 1), (0.9, 1.0, 0, 1)]
+  queries, count = make_queries([params[i % len(params)] for i in range(rows)])
+  tokens = dev.empty(count, np.int32)
+  dev.sample(dev.array(logits), vocab, dev.queries(queries), len(queries), count, 0, tokens)
+  assert tokens.download().tolist() == expected(logits, queries)
+
+
+@pytest.mark.parametrize("masked", [-np.inf, np.finfo(np.float32).min, -1.0e9])
+@pytest.mark.parametrize("temperature", [0.7, 1.0, 1.5])
+@pytest.mark.parametrize("live", [0, 3, 200])
+def test_masked_rows(dev, masked, temperature, live):
+  """A mask leaves few logits, or none: the threshold is the masked value itself (or its overflow), and the earliest equal ones
+  fill the set up."""
+  rng = np.random.default_rng(live)
+  vocab = 20000
+  logits = np.full((5, vocab), masked, np.float32)
+  for row in logits:
+    where = rng.choice(vocab, live, replace=False)
+    row[where] = rng.standard_normal(live)
+  queries, count = make_queries([(temperature, 1.0, 40, 1), (temperature, 0.9, 64, 1), (temperature, 0.0, 8, 1), (temperature, 1.0, 1, 1), (0.0, 1.0, 0, 1)])
+  tokens = dev.empty(count, np.int32)
+  dev.sample(dev.array(logits), vocab, dev.queries(queries), len(queries), count, 0, tokens)
+  assert tokens.download().tolist() == expected(logits, queries)
+
+
+@pytest.mark.parametrize("step", [0.5, 1.0, 4.0])
+def test_coarse_logits_tie_everywhere(dev, step):
+  rng = np.random.default_rng(9)
+  logits = (step * np.round(1.5 * rng.standard_normal((6, VOCAB)) / step)).astype(np.float32)
+  queries, count = make_queries([(0.7, 0.9, 40, 1), (1.0, 1.0, 64, 1), (1.9, 1.0, 5, 1), (0.3, 1.0, 1, 1), (3.0, 1.0, 64, 1), (0.0, 1.0, 0, 1)])
+  tokens = dev.empty(count, np.int32)
+  dev.sample(dev.array(logits), VOCAB, dev.queries(queries), len(queries), count, 0, tokens)
+  assert tokens.download().tolist() == expected(logits, queries)
+
+
 @pytest.mark.parametrize("value", [np.nan, -np.nan])
 def test_nan_logits_beside_more_ties_than_the_collection_holds(dev, value):
   """A NaN takes part in no comparison: the row samples as if it were not there, also where ties send it through the radix select."""
