@@ -373,8 +373,11 @@ __global__ void __launch_bounds__(256) wide_reduce_kernel(const __grid_constant_
   y[0] = sum.x, y[1] = sum.y, y[2] = sum.z, y[3] = sum.w;
 }
 
-// Slices of K, and CTAs: what the busiest scheduler of an SM has to do (rounds of tiles x super-blocks, decode plus MMAs) plus
-// what a reduction of the slices costs (a launch, and every partial result written and read).
+// Slices of K, and CTAs: what the fullest CTA has to do, plus what a reduction of the slices costs (every partial result written
+// and read). A round of up to four tiles puts one warp on a scheduler, which then waits for its own copies and products; a round
+// of eight takes two such warps' issue slots. Fitted to every slice count of 616 shapes (four types, 16 to 20480 weight rows,
+// K 2048 to 12288, 9 to 128 rows): 1.2 % above the best count on average, where a model without the idle schedulers' share
+// lost 10.5 % (Q6_K 4096 x 4096 with 16 rows in one slice 19.5 us, in four 13.5; the slices of eight rows 16.5).
 int slices(const WideParams& p, int tilesPerGroup, int sms) {
   int best = 1;
   double least = 0;
@@ -382,9 +385,10 @@ int slices(const WideParams& p, int tilesPerGroup, int sms) {
     const int ctas = sms / (p.groups * s);
     if (ctas < 1 || ((s > 1 || p.pair) && size_t(s) * p.m * p.pitch > kWidePartialFloats))
       break;
-    const int rounds = ((p.tiles + ctas - 1) / ctas + 3) / 4;
-    const double unit = 0.25 + 0.075 * tilesPerGroup;  // microseconds a scheduler needs for 16 weight rows x 256 k
-    const double cost = rounds * double((p.blocks + s - 1) / s) * unit + (s > 1 ? 3.0 + s * double(p.m) * p.pitch * 8 / 4e6 : 0.0);
+    const int perCta = (p.tiles + ctas - 1) / ctas, rest = perCta % kConsumerWarps;
+    const double busy = 0.15 + 0.1 * tilesPerGroup, lone = 0.2 + 0.1 * tilesPerGroup;  // microseconds for 16 weight rows x 256 k
+    const double block = perCta / kConsumerWarps * 2 * busy + (rest == 0 ? 0.0 : rest <= kConsumerWarps / 2 ? lone : 2 * busy);
+    const double cost = block * ((p.blocks + s - 1) / s) + (s > 1 ? s * double(p.m) * p.pitch * 8 / 2e7 : 0.0);
     if (s == 1 || cost < least)
       least = cost, best = s;
   }

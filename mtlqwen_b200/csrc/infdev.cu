@@ -513,6 +513,9 @@ static int linear_run(infdev_ctx* ctx, int type, bool pair, int count, const voi
     columns += n[i];
   }
   columns *= pair ? 2 : 1;
+  // Two slices of small matrices are two launches at the least a launch takes, the shared decode is three: 16 to 1024 x 2048 with
+  // 9 to 16 rows 7.8 against 9.8 us; with twice the K 11.7 against 9.8.
+  wide = wide && (m > 16 || k > 2048 || columns / 16 > ctx->sms);
   wide = wide && columns < (int64_t(1) << 30) && (!pair || (count == 1 && size_t(columns) * infdev::kWideMaxRows <= infdev::kWidePartialFloats));
   if (wide) {
     infdev::WideParams p{};

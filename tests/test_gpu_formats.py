@@ -96,6 +96,18 @@ def test_many_rows_share_a_decode(dev, name, qtype, m, n, k):
     assert np.linalg.norm(got[row] - want[row]) < 1e-5 * np.linalg.norm(want[row]) + 2.4e-7 * np.linalg.norm(y[row]), row
 
 
+@pytest.mark.parametrize("m,n,k", [(16, 2368, 2048), (16, 2384, 2048), (17, 32, 2048), (9, 32, 4096), (16, 32, 2304)])
+@pytest.mark.parametrize("name,qtype", WIDE_TYPES)
+def test_either_side_of_the_line_to_the_slices(dev, name, qtype, m, n, k):
+  """Up to 16 rows of a matrix with few tiles and K of 2048 at the most go through the GEMV in two slices."""
+  if qtype == D.Q6_K and k % 2048:
+    pytest.skip("Q6_K takes rows of whole 2048-value spans")
+  w, x = synth.weight(qtype, n, k, 87), synth.activations(m, k, 88)
+  y = dev.empty((m, n))
+  dev.linear(qtype, dev.array(w), n, k, dev.array(x), m, y)
+  assert rel_err(y.download(), oracle.linear(w, qtype, n, k, x)) < 1e-5
+
+
 @pytest.mark.parametrize("m", [3, 8, 9, 40])
 @pytest.mark.parametrize("name,qtype", WIDE_TYPES)
 def test_activations_at_the_ends_of_the_range(dev, name, qtype, m):
