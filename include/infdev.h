@@ -89,8 +89,10 @@ float infdev_event_elapsed_ms(infdev_ctx* ctx, void* start, void* stop);
  * activation rows (prefill chunks, speculative rows): 1 (default) = the tcgen05 / TMEM GEMM, 0 = the GEMV kernels in
  * slices of 8 rows, which compute every activation row on its own. Likewise for the other block types, whose launches of more
  * than 8 rows decode a weight once for up to 40 rows (1) or go through the GEMV in slices (0). Environment: INFENG_UMMA. With 0,
- * infdev_attention also treats every row on its own: otherwise, in a pass in which some query has several rows, up to 16 rows of a query share the
- * reading of K and V, and the rounding of a row's sums depends on how its query was cut into passes. */
+ * infdev_attention also treats every row on its own. Otherwise, in a pass of 32 rows a query or more on average (of five, where
+ * rows a query times the tokens that a table row can hold reach 4096), up to 16 rows of a query of several share the reading
+ * of K and V, and the rounding of such a row's sums depends on its query's other rows and on how much else is in the pass; a
+ * query of one row keeps the arithmetic that it has alone. */
 int infdev_set_umma(infdev_ctx* ctx, int enabled);
 /* Activation split of the fp16 tensor-core GEMV: 2 = hi+lo fp16 (fp32-accurate, default), 1 = hi only. */
 int infdev_set_xsplit(infdev_ctx* ctx, int xsplit);
@@ -138,7 +140,8 @@ int infdev_dequant(infdev_ctx* ctx, int type, const void* blocks, int64_t count,
  * linear_decode_q4_k[_add] (quant_linear.metal:245-327), linear_decode_q6_k[_add] (:436-512) and, for
  * m > 8, linear_prefill (:151-233). x, y, residual fp32 row-major; residual may alias y or be null.
  * Q5_K, Q8_0 and IQ4_XS matrices (linear_decode_q5_k, linear_decode_q8_0, :329-434, 514-570; the types the real
- * Qwen3.5 files mix in) are served by a plain dequantise-and-multiply kernel: correct, not tuned. */
+ * Qwen3.5 files mix in) take the tensor-core kernels where n is a multiple of 16 and rows are multiples of 16 bytes, a
+ * plain dequantise-and-multiply kernel otherwise. */
 int infdev_linear(infdev_ctx* ctx, int type, const void* w, int64_t n, int64_t k, const float* x, int64_t m, float* y, const float* residual);
 /* Up to four weight matrices sharing x in one launch (the q/k/v and qkv/z projections of Ops::decoder,
  * forward.cpp:86-88, 98). */

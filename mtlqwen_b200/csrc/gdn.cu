@@ -460,8 +460,8 @@ __global__ void __launch_bounds__(256, 2) delta_rule_kernel(const float* q, cons
 // as a model has them, 512 tokens: outputs 1.8e-7, state 1.4e-7 (2-norms); the fp32 chunk form before it 2.1e-7 and 4.7e-7,
 // token by token 1.1e-7 and 0.7e-7. One scale for the 16 columns of a warp, fp16 parts throughout and sums carried in the
 // accumulators gave 4.1e-7 and 5.4e-7, and lost value columns far below their neighbours; they took 278 us for eight queries
-// of 59 to 493 rows, this form 315 us.
-// A chunk takes about 4.8 us (one query of 512 rows: 32 chunks, 177 us with the preparation); its 168 MMAs per warp are 1.4 us
+// of 59 to 493 rows, this form 311 us.
+// A chunk takes about 4.7 us (one query of 512 rows: 32 chunks, 173 us with the preparation); its 168 MMAs per warp are 1.4 us
 // of them at the measured 8.06 cycles per MMA and scheduler, the rest is the chain of products that wait for each other. The
 // fp32 form, FMAs with eight partial sums per product through shared memory, took 12 us.
 constexpr int kChunk = 16, kComputeWarps = 8, kPrepareWarps = 4;
@@ -718,8 +718,8 @@ __device__ __forceinline__ void chunk_prepare(ChunkShared& sh, const infdev_quer
 }
 
 // Which query the CTAs of row `rank` of the grid take: the one with the rank-th largest count, so that the longest chains start
-// first and the short ones fill the SMs that are left over (eight queries of 59 to 493 rows, 256 CTAs on 148 SMs: 323 us in
-// the order of the pass, 281 us sorted). Every lane of a warp calls; beyond 32 queries the order of the pass stays.
+// first and the short ones fill the SMs that are left over (eight queries of 59 to 493 rows, 256 CTAs on 148 SMs, with a
+// chunk of 4.2 us: 323 us in the order of the pass, 281 us sorted). Every lane of a warp calls; beyond 32 queries the order of the pass stays.
 __device__ __forceinline__ uint32_t query_by_length(const infdev_query* queries, uint32_t count, uint32_t rank) {
   if (count > 32)
     return rank;
