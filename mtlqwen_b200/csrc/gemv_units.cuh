@@ -5,7 +5,7 @@
 // kSplit) in z and w; b.scales(tile) are the powers of two of the rows 2t and 2t + 1; b.sums(tile) is the fragment of the
 // sub-block sums (Q5_K). NT tiles share a decoded fragment. From three tiles on the loops over sub-blocks are unrolled less:
 // loads hoisted over a whole unit push registers to local memory, which these kernels' shared-memory carve-out leaves no L1
-// for (Q6_K, 40 rows: 755 -> 690 us).
+// for (9 % of the time of Q6_K with 40 rows).
 #pragma once
 #include "common.cuh"
 
@@ -54,13 +54,34 @@ template <int NT> __device__ __forceinline__ void clear(float (&sum)[NT][4]) {
     sum[tile][0] = sum[tile][1] = sum[tile][2] = sum[tile][3] = 0.f;
 }
 // sum[tile] += scale * (the fragments a[0 .. F) times the activations of fragments first .. first + F). The MMAs of one half
-// over all tiles come before those of the other, so that no two neighbours depend on each other.
-template <int F, int NT, class B>
+// over all tiles come before those of the other, so that no two neighbours depend on each other. LOW_FIRST: the low halves of
+// all fragments before the high ones. An accumulator cuts off at its own magnitude with every product that is added, and that
+// of the low halves is 2^-11 of the others': half as many cuts. Q5_K needs it, whose values have not been centred yet (K =
+// 2048, against fp64: 1.4e-7 with it, 1.85e-7 without, 1.5e-7 for the plain fp32 kernel); the other types are at 1.2e-7 to
+// 1.5e-7 without, and it costs 3 to 8 % at 9 to 24 rows.
+template <bool LOW_FIRST, int F, int NT, class B>
 __device__ __forceinline__ void scaled_products(float (&sum)[NT][4], const uint32_t (&a)[F][4], const B& b, int first, float sA, float sB) {
   float acc[NT][4];
   clear(acc);
+  if (LOW_FIRST) {
+    uint2 high[F][NT];
 #pragma unroll
-  for (int f = 0; f < F; ++f) {
+    for (int f = 0; f < F; ++f)
+#pragma unroll
+      for (int tile = 0; tile < NT; ++tile) {
+        const uint4 x = b.fragment(first + f, tile);
+        high[f][tile] = make_uint2(x.x, x.y);
+        if (B::kSplit)
+          mma_16816(acc[tile], a[f], x.z, x.w);
+      }
+#pragma unroll
+    for (int f = 0; f < F; ++f)
+#pragma unroll
+      for (int tile = 0; tile < NT; ++tile)
+        mma_16816(acc[tile], a[f], high[f][tile].x, high[f][tile].y);
+  }
+#pragma unroll
+  for (int f = 0; f < (LOW_FIRST ? 0 : F); ++f) {
     uint4 x[NT];
 #pragma unroll
     for (int tile = 0; tile < NT; ++tile)
@@ -114,7 +135,7 @@ template <int NT, class B> __device__ __forceinline__ void q5k_unit(const uint8_
         byte_fragment(a[u], ((h ? lowA[u] >> 4 : lowA[u]) & 0x0f0f0f0fu) | fifthA, ((h ? lowB[u] >> 4 : lowB[u]) & 0x0f0f0f0fu) | fifthB, k1024);
       }
       const uint32_t wordA = (c < 2 ? scA[0] : scA[1]) >> (16 * (c & 1)), wordB = (c < 2 ? scB[0] : scB[1]) >> (16 * (c & 1));
-      scaled_products(sum, a, b, 2 * j, byte_of(wordA, h), byte_of(wordB, h));
+      scaled_products<true>(sum, a, b, 2 * j, byte_of(wordA, h), byte_of(wordB, h));
     }
   }
   const float2 dA = __half22float2(*reinterpret_cast<const __half2*>(&hA.x)), dB = __half22float2(*reinterpret_cast<const __half2*>(&hB.x));
@@ -150,7 +171,7 @@ template <int NT, class B> __device__ __forceinline__ void q8_unit(const uint8_t
       const uint32_t bytesB = (j & 1 ? lds_u32(pB + at) : lds_u32_unaligned(pB + at)) ^ 0x80808080u;
       byte_fragment(a[u], bytesA, bytesB, k1152);
     }
-    scaled_products(sum, a, b, 2 * j, load_half_bits(pA + 34 * j), load_half_bits(pB + 34 * j));
+    scaled_products<false>(sum, a, b, 2 * j, load_half_bits(pA + 34 * j), load_half_bits(pB + 34 * j));
   }
   add_totals(total, b, sum);
 }
@@ -186,7 +207,7 @@ template <int NT, class B> __device__ __forceinline__ void iq4_unit(const uint8_
     }
     const int lsA = int((hA.y >> (4 * j)) & 15u) | int(((hA.x >> (16 + 2 * j)) & 3u) << 4);
     const int lsB = int((hB.y >> (4 * j)) & 15u) | int(((hB.x >> (16 + 2 * j)) & 3u) << 4);
-    scaled_products(sum, a, b, 2 * j, float(lsA - 32), float(lsB - 32));
+    scaled_products<false>(sum, a, b, 2 * j, float(lsA - 32), float(lsB - 32));
   }
   const float dA = load_half_bits(pA), dB = load_half_bits(pB);
 #pragma unroll
@@ -223,7 +244,7 @@ __device__ __forceinline__ void q6k_unit(const uint8_t* pA, const uint8_t* pB, i
           uint32_t a[1][4];
           byte_fragment(a[0], bytesA, bytesB, k1056);
           const float sA = dA * float(int(reinterpret_cast<const int8_t*>(pA + 192)[gi])), sB = dB * float(int(reinterpret_cast<const int8_t*>(pB + 192)[gi]));
-          scaled_products(sum, a, b, gi, sA, sB);
+          scaled_products<false>(sum, a, b, gi, sA, sB);
         }
       }
     }
