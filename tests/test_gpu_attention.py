@@ -145,6 +145,37 @@ def test_switching_the_group_kernel_off_changes_rounding_only(dev):
     dev.set_umma(1)
 
 
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+@pytest.mark.parametrize("context,rows,token", [(40, 40, 39), (40, 40, 17), (200, 64, 150), (300, 33, 299), (90, 48, 60), (90, 48, 3)])
+def test_rows_before_a_value_that_is_not_finite_do_not_notice(dev, context, rows, token, value):
+  """The rows of a prompt share tiles of K and V: a row must not see a broken value of a token behind it."""
+  rng = np.random.default_rng(token)
+  block_tokens, stride = 16, 256
+  table = dev.array(np.concatenate([rng.permutation(24), np.zeros(stride - 24)]).astype(np.int32))
+  keys, values = (rng.standard_normal((24, 4, block_tokens, 256)).astype(np.float16) for _ in range(2))
+  q, qg = rng.standard_normal((rows, 16, 256)).astype(np.float32), dev.array(rng.standard_normal((rows, 16, 512)).astype(np.float32))
+  info = D.Query()
+  info.start, info.count, info.position, info.slot, info.state = 0, rows, context - rows, 0, D.UNBOUND
+
+  def run(values):
+    out, partials = dev.empty((rows, 16, 256)), dev.empty(dev.attention_scratch_bytes(rows, 32) // 4)
+    dev.attention(dev.array(q), qg, dev.array(keys.view(np.uint16)), dev.array(values.view(np.uint16)), dev.queries([info]), 1, rows, table, stride, block_tokens,
+                  32, partials, out)
+    dev.commit()
+    return out.download()
+
+  clean = run(values)
+  broken = values.copy()
+  block = table.download()[token // block_tokens]
+  broken[block, 1, token % block_tokens, [7, 200]] = value  # kv head 1: query heads 4 .. 7
+  got = run(broken)
+  first = max(0, token - (context - rows))  # the first row that attends to the token
+  hit = np.zeros_like(clean, bool)
+  hit[first:, 4:8, 7] = hit[first:, 4:8, 200] = True
+  assert not np.isfinite(got[hit]).any()
+  assert got[~hit].tobytes() == clean[~hit].tobytes()
+
+
 def test_queries_that_lie_on_an_odd_multiple_of_eight_bytes(dev):
   """The kernel for the rows of a prompt copies 16 bytes of q at a time; a q that starts between two such places is served row by row."""
   rng = np.random.default_rng(50)
