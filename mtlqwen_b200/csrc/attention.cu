@@ -272,9 +272,11 @@ __global__ void __launch_bounds__(128, 6) attention_scan_kernel(const float* q, 
 // of 64 tokens, softmax online. 8 warps = 4 heads x 2 halves: a warp scores 32 tokens of the tile, hands its weights to
 // its partner through shared memory and accumulates 128 of the 256 value dims for all 64. Operands as in the scan: fp16
 // keys and values, query and softmax weights as fp16 hi + lo, fp32 accumulation.
-// Bound by the rate of mma.sync (4.2 G multiply-adds with both halves of q and p for 128 rows behind 1920 take 38 us at 512
-// per clock and SM): sixteen warps instead of eight measured 66 instead of 61 us for the whole call, and two groups of four
-// warps with tiles and softmax of their own, nothing exchanged, the same 61.
+// 128 rows behind 1920 tokens are 4.2 G multiply-adds with both halves of q and p, 14 us at the 1016 per clock and SM of
+// mma.sync; the kernel takes about 38, because with two warps a scheduler the products, the fragment reads and the exchange
+// between the halves wait for each other (tensor pipe 42 % of the active cycles, 0.29 issued per cycle and scheduler). In an
+// earlier form sixteen warps instead of eight measured 66 instead of 61 us for the whole call, and two groups of four warps
+// with tiles and softmax of their own, nothing exchanged, the same 61.
 //
 // Work items (tile of rows, piece of context, kv head) are dealt to one CTA per SM; which exist only the device knows, so
 // a CTA finds its next item by a scan over the queries. The pieces of a tile follow from its context and from `most`, which
