@@ -15,6 +15,14 @@
 #include "kernels.h"
 #include "ops.h"
 
+namespace infdev {
+struct NormRequest {
+  const float* weight = nullptr;  // null: none
+  float* normalised = nullptr;
+  bool store = false;
+};
+}  // namespace infdev
+
 struct infdev_ctx {
   int device = 0, sms = 0, xsplit = 2;
   int umma = 1;  // tcgen05 GEMM for Q4_K launches of more than 8 activation rows, grouped attention rows: 0 off, 1 on
@@ -24,6 +32,7 @@ struct infdev_ctx {
   int* imageCounters = nullptr;        // arrival counters of the kernels that write images block by block (zero between launches)
   uint8_t* captureImage = nullptr;     // one-shot: where the next producer call writes the image of its result
   const uint8_t* supplyImage = nullptr;  // one-shot: image the next linear call reads instead of quantising x
+  infdev::NormRequest norm;              // one-shot: the next linear call's activations are the RMS norm of its x
   float* ummaPartial = nullptr;  // K-slice partial results of the tcgen05 prefill GEMM: [4][128][8192] floats, allocated on first use
   uint8_t* wideImage = nullptr;  // activations laid out for the GEMM of the other block types
   float* widePartial = nullptr;  // its K-slice partial results
@@ -81,6 +90,12 @@ const uint8_t* take_supply(infdev_ctx* ctx) {
   const uint8_t* image = ctx->supplyImage;
   ctx->supplyImage = nullptr;
   return image;
+}
+
+infdev::NormRequest take_norm(infdev_ctx* ctx) {
+  const infdev::NormRequest norm = ctx->norm;
+  ctx->norm = {};
+  return norm;
 }
 
 using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -378,6 +393,13 @@ int infdev_image_supply(infdev_ctx* ctx, const uint8_t* image) {
   return INFDEV_OK;
 }
 
+int infdev_norm_supply(infdev_ctx* ctx, const float* w, float* normalised, int store) {
+  if (!w || !normalised || !aligned16(w) || !aligned16(normalised))
+    return fail(ctx, INFDEV_E_ARGUMENT, "norm_supply: weights and scratch must be given, 16-byte aligned");
+  ctx->norm = {w, normalised, store != 0};
+  return INFDEV_OK;
+}
+
 int infdev_set_integer_decode(infdev_ctx* ctx, int enabled) {
   ctx->integerDecode = enabled != 0;
   return INFDEV_OK;
@@ -442,7 +464,7 @@ int infdev_dequant(infdev_ctx* ctx, int type, const void* blocks, int64_t count,
 
 // `supplied`: image of x to read instead of quantising it (integer kernel only).
 static int linear_run(infdev_ctx* ctx, int type, bool pair, int count, const void* const* w, const void* const* w2, const int64_t* n, int64_t k,
-                      const float* x, int64_t m, float* const* y, const float* const* residual, const uint8_t* supplied) {
+                      const float* x, int64_t m, float* const* y, const float* const* residual, const uint8_t* supplied, const infdev::NormRequest& norm) {
   const infdev::GemvBox box = infdev::gemv_box(type);
   if (!box.blockBytes)
     return fail(ctx, INFDEV_E_ARGUMENT, "linear: unsupported weight type " + std::to_string(type));
@@ -578,8 +600,15 @@ static int linear_run(infdev_ctx* ctx, int type, bool pair, int count, const voi
       p.seg[i].res = residual && residual[i] ? residual[i] + row * n[i] : nullptr;
     }
     if (integer) {
-      if (supplied) {  // 8-row slices of k/256 blocks
+      if (norm.weight) {
+        p.norm = norm.weight, p.normalised = norm.store ? norm.normalised + row * k : nullptr;
+      } else if (supplied) {  // 8-row slices of k/256 blocks
         p.image = supplied + size_t(row / 8) * size_t(k / 256) * infdev::kActivationImageBlockBytes;
+      } else if (p.m * k <= 32768 && (p.m <= 4 || p.tiles > ctx->sms)) {
+        // Every CTA quantises the activations itself, where reading 128 KB or less takes no longer than a launch more: 12288 x 4096 with
+        // its own image 9.7 (one row) and 11.2 us (eight), without 7.6 and 10.6; 4096 x 12288 9.5 and 11.5, without 8.7 and
+        // 13.7; 1024 x 4096, which is a start and an end only, 3.6 and 4.1, without 2.7 and 4.4.
+        p.image = nullptr;
       } else {
         p.image = ctx->image;
         if (int r = check(ctx, infdev::activation_image_launch(p.x, p.ldx, p.m, p.k, ctx->image, ctx->stream), "activation image"))
@@ -603,6 +632,18 @@ static int linear_common(infdev_ctx* ctx, int type, bool pair, int count, const 
   Bind bind(ctx);
   const uint8_t* supplied = take_supply(ctx);
   uint8_t* captured = take_capture(ctx);
+  infdev::NormRequest norm = take_norm(ctx);
+  if (norm.weight && (supplied || k != infdev::kGemvNormK))
+    return fail(ctx, INFDEV_E_ARGUMENT, "linear: normalised activations need k = 4096 and no image");
+  if (norm.weight && (m > 8 || type != INFDEV_Q4_K || !ctx->integerDecode)) {  // not on the way into the GEMV
+    if (!aligned16(x))
+      return fail(ctx, INFDEV_E_ARGUMENT, "linear: activations must be 16-byte aligned");
+    if (int r = check(ctx, infdev::rms_norm_launch(x, norm.weight, nullptr, m, k, norm.normalised, nullptr, ctx->stream), "rms_norm"))
+      return r;
+    ++ctx->launches;
+    x = norm.normalised;
+    norm = {};
+  }
   if (captured && (count != 1 || n[0] % 256))
     return fail(ctx, INFDEV_E_ARGUMENT, "linear: an image of the result needs a single matrix with n a multiple of 256");
   // Q5_K, Q8_0, IQ4_XS: the tensor-core GEMV takes whole 16-row tiles whose rows a tiled copy can address, and gate / up
@@ -626,7 +667,7 @@ static int linear_common(infdev_ctx* ctx, int type, bool pair, int count, const 
     }
     return captured ? quantize_rows(ctx, y[0], m, n[0], captured) : INFDEV_OK;
   }
-  if (int r = linear_run(ctx, type, pair, count, w, w2, n, k, x, m, y, residual, supplied))
+  if (int r = linear_run(ctx, type, pair, count, w, w2, n, k, x, m, y, residual, supplied, norm))
     return r;
   // A GEMV tile is 16 outputs wide, a 256-value image block spans 16 tiles on different SMs: the image of the result
   // takes a launch of its own.

@@ -22,13 +22,18 @@ struct GemvParams {
   GemvSeg seg[4];
   int nseg, tiles;
   const float* x;  // [m][ldx] fp32, rows 16-byte aligned
-  const uint8_t* image;  // quantised activations (act_image.cuh) of all k/256 blocks, for the integer Q4_K kernel
+  // The integer Q4_K kernel takes the quantised activations (act_image.cuh) of all k/256 blocks from `image`, or quantises x itself
+  // where that is null. Then, with k = kGemvNormK, `norm` makes the activations rmsnorm(x) * norm, stored in `normalised` if not null.
+  const uint8_t* image;
+  const float* norm;
+  float* normalised;  // [m][k]
   int ldx, m, k;
   int* status;
 };
 
 // Box geometry shared by the host encoder and the kernel.
 constexpr int kGemvStageBlocks = 8, kGemvTileRows = 16;
+constexpr int64_t kGemvNormK = 4096;     // a normalised row is one K chunk
 constexpr int64_t kGemvPairMaxK = 4096;  // a gate / up pair is finished within one K chunk
 // The integer Q4_K kernel reads 32 bytes past the 8 super-blocks of a box row, which makes the row pitch in shared
 // memory 1184 = 32 (mod 128) bytes: the 32-byte pieces of consecutive rows that a warp reads in one load then fall

@@ -16,7 +16,7 @@
 // shared memory is read for the weights only, which is what bounds the rate of this kernel (the activation fragments
 // of a unit are 4 KB against 2.3 KB of weights). Every wait on an mbarrier is bounded and ends in an abort flag plus a
 // device status code.
-#include "act_image.cuh"
+#include "q4k_units.cuh"
 #include "kernels.h"
 
 namespace infdev {
@@ -28,13 +28,8 @@ constexpr int kFinisherWarps = 3;  // each sums the consumers' partial results o
 constexpr int kProducerWarp = kConsumerWarps + kFinisherWarps;  // 16 + 3 + 1 warps: five on each scheduler
 constexpr int kThreads = (kProducerWarp + 1) * kWarp;
 constexpr int kChunkBlocks = 16;  // super-blocks of K per pass over the tiles: two slabs, one per half
-constexpr int kStageBlocks = kGemvStageBlocks;
-constexpr int kTileRows = kGemvTileRows;
 constexpr int kMaxStages = 12;
-constexpr int kBlockBytes = 144;
-constexpr int kRowPitch = kStageBlocks * kBlockBytes + kDecodePadBytes;  // 1184
-constexpr int kStageBytes = kTileRows * kRowPitch;                       // 18,944
-static_assert(kChunkBlocks == 2 * kStageBlocks, "a consumer warp's super-block within a chunk is fixed by its half");
+static_assert(kChunkBlocks == 2 * kGemvStageBlocks, "a consumer warp's super-block within a chunk is fixed by its half");
 
 struct Control {
   uint64_t full[kMaxStages], empty[kMaxStages];
@@ -42,146 +37,17 @@ struct Control {
   int abort;
 };
 constexpr int kControlBytes = 256;
+constexpr int kSquaresBytes = kConsumerWarps * kImageRows * 4;
 static_assert(sizeof(Control) <= kControlBytes, "control block overlaps the partial sums");
 
-template <int NMAT> constexpr size_t fixed_bytes() { return kControlBytes + size_t(kFinisherWarps) * NMAT * kConsumerWarps * 128 * 4; }
+template <int NMAT> constexpr size_t fixed_bytes() { return kControlBytes + kSquaresBytes + size_t(kFinisherWarps) * NMAT * kConsumerWarps * 128 * 4; }
 template <int NMAT> constexpr int stage_count() {
-  int stages = int((size_t(227) * 1024 - fixed_bytes<NMAT>()) / kStageBytes);
+  int stages = int((size_t(227) * 1024 - fixed_bytes<NMAT>()) / kQ4StageBytes);
   // Even, so that a slot always belongs to the same half of the consumers: a half that ran ahead in a slot of the other one could
   // find the parity of the phase before last and read the slot ahead of its own copy.
   return (stages > kMaxStages ? kMaxStages : stages) / 2 * 2;
 }
-template <int NMAT> constexpr size_t smem_bytes() { return fixed_bytes<NMAT>() + size_t(stage_count<NMAT>()) * kStageBytes; }
-
-// Ordinary loads (not volatile asm): the compiler may hoist and interleave them with the MMAs, but not move them
-// above the mbarrier wait, which clobbers memory.
-__device__ __forceinline__ uint4 lds128(const uint8_t* p) { return *reinterpret_cast<const uint4*>(p); }
-__device__ __forceinline__ uint2 lds64(const uint8_t* p) { return *reinterpret_cast<const uint2*>(p); }
-
-// D(16x8,s32) += A(16x32,u8,row) * B(32x8,s8 or u8,col)
-__device__ __forceinline__ void imma_u8s8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void imma_u8u8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// What one lane keeps of the image of one super-block (act_image.cuh) while its warp walks the tiles. With eight activation
-// rows the eight columns of an MMA are the rows. With ROWS = 1 or 2 they are (row, sub-block) pairs: column c stands for
-// row c % ROWS and, of every 8 / ROWS consecutive sub-blocks, for sub-block c / ROWS, and the B operand of a sub-block is zero
-// in the other columns. The MMAs of 8 / ROWS sub-blocks then share one accumulator, and a sub-block scale multiplies
-// every result once instead of leaving columns empty.
-// Lane (g = lane/4, t = lane%4) holds, per sub-block j, the B fragments of column g, quarter t: registers b0, b1 of the
-// high-byte MMA in x, y and of the low-byte MMA in z, w.
-struct Fragments {
-  uint4 quant[8];
-  uint2 sums;    // min-term fragment: fp16 pairs of S_j / 32, high halves in x, low halves in y
-  uint2 scales;  // fp32 bits of the activation scales of the rows of columns 2t and 2t+1
-};
-
-template <int ROWS> __device__ __forceinline__ Fragments load_fragments(const uint8_t* block, int lane) {
-  constexpr int kShare = 8 / ROWS;
-  Fragments f;
-  const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int j = 0; j < 8; ++j)
-    f.quant[j] = g / ROWS == j % kShare ? *reinterpret_cast<const uint4*>(block + j * 512 + (g % ROWS) * 64 + t * 16) : make_uint4(0, 0, 0, 0);
-  f.sums = *reinterpret_cast<const uint2*>(block + kImageSumOffset + lane * 8);
-  f.scales = *reinterpret_cast<const uint2*>(block + kImageScaleOffset + (2 * t % ROWS) * 4);
-  return f;
-}
-
-// One 16-row x 256-k unit. Lane (g, t) owns weight rows g and g+8 (shared-memory addresses pA, pB) and, in each
-// 32-byte quant chunk c, bytes 8t .. 8t+7: their low nibbles are values 8t .. 8t+7 of sub-block 2c, their high
-// nibbles the same values of sub-block 2c+1 (GGUF layout as read by dequant_tile, quant_linear.metal:39-46). The four
-// bytes of a word fill four consecutive summation slots of the MMA, which is the order the image stores the
-// activations in.
-// The integer sums are exact, and with fewer than eight rows they are completed over the lanes of a row before they are
-// rounded to fp32, so that a row has the same bits whatever ROWS. Only lanes with 2t < ROWS then hold results.
-template <int ROWS> __device__ __forceinline__ void q4k_unit(const uint8_t* pA, const uint8_t* pB, int t, const Fragments& f, float (&total)[4]) {
-  static_assert(ROWS == 1 || ROWS == 2 || ROWS == 8, "scale selection");
-  constexpr int kShare = 8 / ROWS;
-  const uint4 hA = lds128(pA), hB = lds128(pB);
-  // 6-bit scales / mins of the 8 sub-blocks, four per word (scale_min_k4, quant_linear.metal:12-20).
-  const uint32_t scA[2] = {hA.y & 0x3f3f3f3fu, (hA.w & 0x0f0f0f0fu) | ((hA.y >> 2) & 0x30303030u)};
-  const uint32_t mnA[2] = {hA.z & 0x3f3f3f3fu, ((hA.w >> 4) & 0x0f0f0f0fu) | ((hA.z >> 2) & 0x30303030u)};
-  const uint32_t scB[2] = {hB.y & 0x3f3f3f3fu, (hB.w & 0x0f0f0f0fu) | ((hB.y >> 2) & 0x30303030u)};
-  const uint32_t mnB[2] = {hB.z & 0x3f3f3f3fu, ((hB.w >> 4) & 0x0f0f0f0fu) | ((hB.z >> 2) & 0x30303030u)};
-  // 16 x the sum over the 8 sub-blocks of scale * (integer dot product), separately for the low and the high activation
-  // byte: |low| <= 16 * 8 * 63 * 15 * 32 * 255 < 2^30 and |high| <= 16 * 8 * 63 * 15 * 32 * 128 both stay inside int32.
-  int sumLow[4] = {0, 0, 0, 0}, sumHigh[4] = {0, 0, 0, 0};
-  int high[4], low[4];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const uint2 qA = lds64(pA + 16 + 32 * c + 8 * t), qB = lds64(pB + 16 + 32 * c + 8 * t);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int j = 2 * c + h, set = ROWS == 2 ? j / kShare : 0;
-      uint32_t a[4];
-      // Low nibbles as they are, high nibbles in place as 16 q (still a byte); the sub-block scale of the low ones is
-      // taken 16-fold instead, and the common factor leaves with d at the end.
-      const uint32_t mask = h == 0 ? 0x0f0f0f0fu : 0xf0f0f0f0u;
-      a[0] = qA.x & mask, a[1] = qB.x & mask, a[2] = qA.y & mask, a[3] = qB.y & mask;
-      const uint4 b = f.quant[j];
-      if (j % kShare == 0)
-        high[0] = high[1] = high[2] = high[3] = low[0] = low[1] = low[2] = low[3] = 0;
-      imma_u8s8(high, a, b.x, b.y);
-      imma_u8u8(low, a, b.z, b.w);
-      if (j % kShare != kShare - 1)
-        continue;
-      if (ROWS == 1) {  // columns 2t and 2t + 1 are the sub-blocks of those numbers
-        const uint32_t pairA = (t & 2 ? scA[1] : scA[0]) >> (16 * (t & 1)), pairB = (t & 2 ? scB[1] : scB[0]) >> (16 * (t & 1));
-        const int evenA = int(pairA & 0xffu) * 16, oddA = int(pairA >> 8 & 0xffu), evenB = int(pairB & 0xffu) * 16, oddB = int(pairB >> 8 & 0xffu);
-        sumLow[0] = evenA * low[0] + oddA * low[1], sumHigh[0] = evenA * high[0] + oddA * high[1];
-        sumLow[2] = evenB * low[2] + oddB * low[3], sumHigh[2] = evenB * high[2] + oddB * high[3];
-        continue;
-      }
-      int sA, sB;
-      if (ROWS == 8) {
-        const int byteA = int(__byte_perm(scA[j >> 2], 0u, 0x4440 + (j & 3))), byteB = int(__byte_perm(scB[j >> 2], 0u, 0x4440 + (j & 3)));
-        sA = h == 0 ? byteA * 16 : byteA, sB = h == 0 ? byteB * 16 : byteB;
-      } else {  // sub-block 4 * set + t; even ones hold low nibbles
-        const int fold = t & 1 ? 0 : 4;
-        sA = int(scA[set] >> (8 * t) & 0xffu) << fold, sB = int(scB[set] >> (8 * t) & 0xffu) << fold;
-      }
-      sumLow[0] += sA * low[0], sumHigh[0] += sA * high[0];
-      sumLow[1] += sA * low[1], sumHigh[1] += sA * high[1];
-      sumLow[2] += sB * low[2], sumHigh[2] += sB * high[2];
-      sumLow[3] += sB * low[3], sumHigh[3] += sB * high[3];
-    }
-  }
-#pragma unroll
-  for (int lanes = 1; ROWS < 8 && lanes < 4; lanes *= 2)
-#pragma unroll
-    for (int i = 0; i < 4; i += ROWS == 1 ? 2 : 1) {
-      sumLow[i] += __shfl_xor_sync(0xffffffffu, sumLow[i], lanes);
-      sumHigh[i] += __shfl_xor_sync(0xffffffffu, sumHigh[i], lanes);
-    }
-  // min term: sum_j m_j * S_j / 32; summation slots 0..7 carry the fp16 high halves of the sums, 8..15 the low halves.
-  float accm[4] = {0.f, 0.f, 0.f, 0.f};
-  {
-    constexpr uint32_t k1024 = 0x64006400u;
-    const uint32_t wordA = (t & 2) ? mnA[1] : mnA[0], wordB = (t & 2) ? mnB[1] : mnB[0];
-    const uint32_t pairA = (wordA >> ((t & 1) * 16)) & 0xffffu, pairB = (wordB >> ((t & 1) * 16)) & 0xffffu;
-    uint32_t a[4];
-    a[0] = a[2] = hsub2_u32(__byte_perm(pairA, 0x64u, 0x4140), k1024);
-    a[1] = a[3] = hsub2_u32(__byte_perm(pairB, 0x64u, 0x4140), k1024);
-    mma_16816(accm, a, f.sums.x, f.sums.y);
-  }
-  const float xs0 = __uint_as_float(f.scales.x), xs1 = __uint_as_float(f.scales.y);
-  const float2 dA = __half22float2(*reinterpret_cast<const __half2*>(&hA.x)), dB = __half22float2(*reinterpret_cast<const __half2*>(&hB.x));
-  const float mA = 32.f * dA.y, mB = 32.f * dB.y, sixteenthA = 0.0625f * dA.x, sixteenthB = 0.0625f * dB.x;
-  total[0] += xs0 * (sixteenthA * fmaf(float(sumHigh[0]), 256.f, float(sumLow[0])) - mA * accm[0]);
-  if (ROWS > 1)
-    total[1] += xs1 * (sixteenthA * fmaf(float(sumHigh[1]), 256.f, float(sumLow[1])) - mA * accm[1]);
-  total[2] += xs0 * (sixteenthB * fmaf(float(sumHigh[2]), 256.f, float(sumLow[2])) - mB * accm[2]);
-  if (ROWS > 1)
-    total[3] += xs1 * (sixteenthB * fmaf(float(sumHigh[3]), 256.f, float(sumLow[3])) - mB * accm[3]);
-}
+template <int NMAT> constexpr size_t smem_bytes() { return fixed_bytes<NMAT>() + size_t(stage_count<NMAT>()) * kQ4StageBytes; }
 
 __device__ __forceinline__ int find_segment(const GemvParams& p, int tile) {
   int s = 0;
@@ -194,7 +60,8 @@ template <int NMAT, int ROWS> __global__ void __launch_bounds__(kThreads, 1) q4k
   constexpr int kStages = stage_count<NMAT>();
   extern __shared__ __align__(128) uint8_t smemRaw[];
   Control& ctl = *reinterpret_cast<Control*>(smemRaw);
-  float* partial = reinterpret_cast<float*>(smemRaw + kControlBytes);
+  float* squaresOfBlock = reinterpret_cast<float*>(smemRaw + kControlBytes);  // [super-block][row]
+  float* partial = reinterpret_cast<float*>(smemRaw + kControlBytes + kSquaresBytes);
   uint8_t* ring = reinterpret_cast<uint8_t*>(partial + kFinisherWarps * NMAT * kConsumerWarps * 128);
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -225,10 +92,10 @@ template <int NMAT, int ROWS> __global__ void __launch_bounds__(kThreads, 1) q4k
       bool ok = true;
       for (int chunk = 0; chunk < chunks && ok; ++chunk) {
         const int chunkBlocks = min(kChunkBlocks, blocksPerRow - chunk * kChunkBlocks);
-        const int groups = (chunkBlocks + kStageBlocks - 1) / kStageBlocks;
+        const int groups = (chunkBlocks + kGemvStageBlocks - 1) / kGemvStageBlocks;
         for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x) {
           const int segment = find_segment(p, tile);
-          const int row0 = (tile - p.seg[segment].tile0) * kTileRows;
+          const int row0 = (tile - p.seg[segment].tile0) * kGemvTileRows;
           for (int mat = 0; mat < NMAT && ok; ++mat) {
             for (int grp = 0; grp < groups; ++grp, ++it) {
               const uint32_t slot = it % kStages, round = it / kStages;
@@ -240,8 +107,8 @@ template <int NMAT, int ROWS> __global__ void __launch_bounds__(kThreads, 1) q4k
               }
               // One tiled copy moves the whole slab; bytes past the end of a row are zero-filled and still counted, so
               // the transaction size is always the full box.
-              mbar_arrive_expect_tx(&ctl.full[slot], uint32_t(kStageBytes));
-              tma_load_2d(ring + size_t(slot) * kStageBytes, &p.map[segment][mat], (chunk * (kChunkBlocks / kStageBlocks) + grp) * (kStageBlocks * kBlockBytes / 8),
+              mbar_arrive_expect_tx(&ctl.full[slot], uint32_t(kQ4StageBytes));
+              tma_load_2d(ring + size_t(slot) * kQ4StageBytes, &p.map[segment][mat], (chunk * (kChunkBlocks / kGemvStageBlocks) + grp) * (kGemvStageBlocks * kQ4BlockBytes / 8),
                           row0, &ctl.full[slot]);
             }
           }
@@ -278,7 +145,7 @@ template <int NMAT, int ROWS> __global__ void __launch_bounds__(kThreads, 1) q4k
 #pragma unroll
         for (int r = 0; r < 2; ++r)
           if (2 * t + r < p.m) {
-            const size_t at = size_t(2 * t + r) * seg.ldy + size_t(tile - seg.tile0) * kTileRows + g;
+            const size_t at = size_t(2 * t + r) * seg.ldy + size_t(tile - seg.tile0) * kGemvTileRows + g;
             destination[r] = seg.y + at;
             if (NMAT == 1 && chunk > 0)
               addend[r] = destination[r][0], addend[2 + r] = destination[r][8];
@@ -318,22 +185,28 @@ template <int NMAT, int ROWS> __global__ void __launch_bounds__(kThreads, 1) q4k
   }
 
   // ---- consumers ----
-  pdl_wait();  // the image comes from the kernels before this one
+  pdl_wait();  // the activations come from the kernels before this one
   const int g = lane >> 2, t = lane & 3, half = warp / kStageWarps, unit = warp % kStageWarps;
-  const int laneRow = g * kRowPitch + unit * kBlockBytes;
+  const int laneRow = g * kQ4RowPitch + unit * kQ4BlockBytes;
   uint32_t it = 0, mine = half, slot = half, phase = 0;
   uint32_t bufferState = 0;  // bit b: parity of the next use of partial-sum buffer b; bit 4 + b: it has been used before
   for (int chunk = 0; chunk < chunks; ++chunk) {
     const int chunkBlocks = min(kChunkBlocks, blocksPerRow - chunk * kChunkBlocks);
-    const int groups = (chunkBlocks + kStageBlocks - 1) / kStageBlocks;
+    const int groups = (chunkBlocks + kGemvStageBlocks - 1) / kGemvStageBlocks;
     // With two slabs per tile the stages of a tile alternate between the halves (a chunk starts at an even stage,
     // only the last chunk of a row can be a single slab), with one slab every stage is slab 0: either way this warp
     // meets the same super-block in every tile of the chunk.
-    const int myBlock = (groups == 2 ? half * kStageBlocks : 0) + unit;
+    const int myBlock = (groups == 2 ? half * kGemvStageBlocks : 0) + unit;
     const bool live = myBlock < chunkBlocks;
     Fragments fragments;
+    float squares;
     if (live)
-      fragments = load_fragments<ROWS>(p.image + size_t(chunk * kChunkBlocks + myBlock) * kImageBlockBytes, lane);
+      fragments = p.image ? load_fragments<ROWS>(p.image + size_t(chunk * kChunkBlocks + myBlock) * kImageBlockBytes, lane)
+                          : quantize_fragments<ROWS>(p.x + size_t(chunk * kChunkBlocks + myBlock) * 256, p.ldx, p.m,
+                                                     p.norm ? p.norm + myBlock * 256 : nullptr, lane, squares);
+    if (p.norm)  // one chunk of 16 super-blocks
+      normalise_fragments<ROWS>(fragments, squares, squaresOfBlock, myBlock, p.m, p.x, p.ldx, p.norm,
+                                myBlock % int(gridDim.x) == int(blockIdx.x) ? p.normalised : nullptr, lane);
     int buffer = 0;
     for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, buffer = buffer == kFinisherWarps - 1 ? 0 : buffer + 1) {
       float total[NMAT][4];
@@ -355,11 +228,11 @@ template <int NMAT, int ROWS> __global__ void __launch_bounds__(kThreads, 1) q4k
           break;
         }
         if (live) {
-          const uint8_t* rows = ring + slot * kStageBytes + laneRow;
+          const uint8_t* rows = ring + slot * kQ4StageBytes + laneRow;
           if (NMAT == 2 && mat)
-            q4k_unit<ROWS>(rows, rows + 8 * kRowPitch, t, fragments, total[NMAT - 1]);
+            q4k_unit<ROWS>(rows, rows + 8 * kQ4RowPitch, t, fragments, total[NMAT - 1]);
           else
-            q4k_unit<ROWS>(rows, rows + 8 * kRowPitch, t, fragments, total[0]);
+            q4k_unit<ROWS>(rows, rows + 8 * kQ4RowPitch, t, fragments, total[0]);
         }
         __syncwarp();
         if (lane == 0)

@@ -61,6 +61,7 @@ def library():
     "infdev_quantize": (i32, (vp, vp, i64, i64, vp)),
     "infdev_image_capture": (i32, (vp, vp)),
     "infdev_image_supply": (i32, (vp, vp)),
+    "infdev_norm_supply": (i32, (vp, f32p, f32p, i32)),
     "infdev_set_umma": (i32, (vp, i32)),
     "infdev_graph_begin": (i32, (vp, )),
     "infdev_graph_end": (vp, (vp, )),
@@ -208,6 +209,10 @@ class Device:
   def image_supply(self, image):
     """The next linear call reads this image instead of quantising its activations."""
     self.check(self.lib.infdev_image_supply(self.ctx, image.ptr))
+
+  def norm_supply(self, w, normalised, store=False):
+    """The next linear call takes the RMS norm of its x as activations; store leaves the normalised rows in `normalised`."""
+    self.check(self.lib.infdev_norm_supply(self.ctx, w.ptr, normalised.ptr, int(store)))
 
   # ---- kernels ----
   def dequant(self, qtype, blocks, count, out):
