@@ -16,8 +16,8 @@
 // shared memory is read for the weights only, which is what bounds the rate of this kernel (the activation fragments
 // of a unit are 4 KB against 2.3 KB of weights). Every wait on an mbarrier is bounded and ends in an abort flag plus a
 // device status code.
+#include "gemv_ring.cuh"
 #include "q4k_units.cuh"
-#include "kernels.h"
 
 namespace infdev {
 namespace {
@@ -28,19 +28,11 @@ constexpr int kFinisherWarps = 3;  // each sums the consumers' partial results o
 constexpr int kProducerWarp = kConsumerWarps + kFinisherWarps;  // 16 + 3 + 1 warps: five on each scheduler
 constexpr int kThreads = (kProducerWarp + 1) * kWarp;
 constexpr int kChunkBlocks = 16;  // super-blocks of K per pass over the tiles: two slabs, one per half
-constexpr int kMaxStages = 12;
 static_assert(kChunkBlocks == 2 * kGemvStageBlocks, "a consumer warp's super-block within a chunk is fixed by its half");
 
-struct Control {
-  uint64_t full[kMaxStages], empty[kMaxStages];
-  uint64_t partialReady[kFinisherWarps], partialFree[kFinisherWarps];  // per partial-sum buffer: consumers -> its finisher and back
-  int abort;
-};
-constexpr int kControlBytes = 256;
 constexpr int kSquaresBytes = kConsumerWarps * kImageRows * 4;
-static_assert(sizeof(Control) <= kControlBytes, "control block overlaps the partial sums");
 
-template <int NMAT> constexpr size_t fixed_bytes() { return kControlBytes + kSquaresBytes + size_t(kFinisherWarps) * NMAT * kConsumerWarps * 128 * 4; }
+template <int NMAT> constexpr size_t fixed_bytes() { return kRingControlBytes + kSquaresBytes + size_t(kFinisherWarps) * NMAT * kConsumerWarps * 128 * 4; }
 template <int NMAT> constexpr int stage_count() {
   int stages = int((size_t(227) * 1024 - fixed_bytes<NMAT>()) / kQ4StageBytes);
   // Even, so that a slot always belongs to the same half of the consumers: a half that ran ahead in a slot of the other one could
@@ -49,19 +41,12 @@ template <int NMAT> constexpr int stage_count() {
 }
 template <int NMAT> constexpr size_t smem_bytes() { return fixed_bytes<NMAT>() + size_t(stage_count<NMAT>()) * kQ4StageBytes; }
 
-__device__ __forceinline__ int find_segment(const GemvParams& p, int tile) {
-  int s = 0;
-  while (s + 1 < p.nseg && tile >= p.seg[s + 1].tile0)
-    ++s;
-  return s;
-}
-
 template <int NMAT, int ROWS> __global__ void __launch_bounds__(kThreads, 1) q4k_decode_kernel(const __grid_constant__ GemvParams p) {
   constexpr int kStages = stage_count<NMAT>();
   extern __shared__ __align__(128) uint8_t smemRaw[];
-  Control& ctl = *reinterpret_cast<Control*>(smemRaw);
-  float* squaresOfBlock = reinterpret_cast<float*>(smemRaw + kControlBytes);  // [super-block][row]
-  float* partial = reinterpret_cast<float*>(smemRaw + kControlBytes + kSquaresBytes);
+  RingControl& ctl = *reinterpret_cast<RingControl*>(smemRaw);
+  float* squaresOfBlock = reinterpret_cast<float*>(smemRaw + kRingControlBytes);  // [super-block][row]
+  float* partial = reinterpret_cast<float*>(smemRaw + kRingControlBytes + kSquaresBytes);
   uint8_t* ring = reinterpret_cast<uint8_t*>(partial + kFinisherWarps * NMAT * kConsumerWarps * 128);
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -123,64 +108,10 @@ template <int NMAT, int ROWS> __global__ void __launch_bounds__(kThreads, 1) q4k
     return;
   }
 
-  // The partial sums of a tile go through one of three buffers, taken in turn within a K chunk, and each buffer has
-  // its own finisher warp and two mbarriers: partialReady[b] "every consumer warp has stored its partial sums" and
-  // partialFree[b] "the finisher has read them", which a consumer tests before it stores into the buffer again.
-  // Nobody waits for a warp of its own role, each barrier is watched phase by phase by the same warps, and a tile of
-  // the result has the same finisher in every K chunk, so the sum over the earlier chunks it adds is its own store.
   if (warp >= kConsumerWarps) {
-    // ---- finishers: four elements of a tile's 16 x 8 result per lane ----
+    // ---- finishers ----
     pdl_wait();
-    const int buffer = warp - kConsumerWarps;
-    uint32_t uses = 0;
-    for (int chunk = 0; chunk < chunks; ++chunk)
-      for (int tile = blockIdx.x + buffer * gridDim.x; tile < p.tiles; tile += kFinisherWarps * gridDim.x, ++uses) {
-        // Lane (g = lane/4, t = lane%4) sums what the same lane of every consumer warp holds: weight rows g and g+8 for
-        // activation rows 2t and 2t+1. What is added to them (the residual, or the sum over the earlier K chunks) is
-        // fetched before the wait.
-        const GemvSeg& seg = p.nseg == 1 ? p.seg[0] : p.seg[find_segment(p, tile)];
-        const int g = lane >> 2, t = lane & 3;
-        float* destination[2] = {nullptr, nullptr};  // activation rows 2t, 2t+1 at weight row g; g + 8 is 8 floats on
-        float addend[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int r = 0; r < 2; ++r)
-          if (2 * t + r < p.m) {
-            const size_t at = size_t(2 * t + r) * seg.ldy + size_t(tile - seg.tile0) * kGemvTileRows + g;
-            destination[r] = seg.y + at;
-            if (NMAT == 1 && chunk > 0)
-              addend[r] = destination[r][0], addend[2 + r] = destination[r][8];
-            else if (NMAT == 1 && seg.res)
-              addend[r] = seg.res[at], addend[2 + r] = seg.res[at + 8];
-          }
-        const float4* sums = reinterpret_cast<const float4*>(partial + size_t(buffer) * NMAT * kConsumerWarps * 128) + lane;
-        if (!mbar_wait_bounded(&ctl.partialReady[buffer], uses & 1, abortFlag)) {
-          *abortFlag = 1;
-          atomicExch(p.status, kStatusBarrierTimeout);
-          return;
-        }
-        float4 sum[NMAT];
-#pragma unroll
-        for (int mat = 0; mat < NMAT; ++mat) {
-          float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;  // two chains in a fixed order: the result does not depend on timing
-#pragma unroll
-          for (int w = 0; w < kConsumerWarps; w += 2) {
-            const float4 u = sums[(mat * kConsumerWarps + w) * 32], v = sums[(mat * kConsumerWarps + w + 1) * 32];
-            a.x += u.x, a.y += u.y, a.z += u.z, a.w += u.w;
-            b.x += v.x, b.y += v.y, b.z += v.z, b.w += v.w;
-          }
-          sum[mat] = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
-        }
-        __syncwarp();
-        if (lane == 0)
-          mbar_arrive(&ctl.partialFree[buffer]);
-        const float4 first = sum[0], second = sum[NMAT - 1];
-        const float lowRows[2] = {NMAT == 2 ? silu_f(first.x) * second.x : first.x + addend[0], NMAT == 2 ? silu_f(first.y) * second.y : first.y + addend[1]};
-        const float highRows[2] = {NMAT == 2 ? silu_f(first.z) * second.z : first.z + addend[2], NMAT == 2 ? silu_f(first.w) * second.w : first.w + addend[3]};
-#pragma unroll
-        for (int r = 0; r < 2; ++r)
-          if (destination[r])
-            destination[r][0] = lowRows[r], destination[r][8] = highRows[r];
-      }
+    finish_tiles<NMAT, kConsumerWarps, kFinisherWarps>(p, ctl, partial, warp - kConsumerWarps, chunks, lane);
     return;
   }
 

@@ -68,7 +68,7 @@ template <int ROWS> __device__ __forceinline__ Fragments quantize_fragments(cons
   for (int i = 0; i < ROWS; ++i) {
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
     if (row < m)
-      a = __ldcg(reinterpret_cast<const float4*>(src + i * kShare * 32)), b = __ldcg(reinterpret_cast<const float4*>(src + i * kShare * 32 + 4));
+      a = *reinterpret_cast<const float4*>(src + i * kShare * 32), b = *reinterpret_cast<const float4*>(src + i * kShare * 32 + 4);
     v[i][0] = a.x, v[i][1] = a.y, v[i][2] = a.z, v[i][3] = a.w, v[i][4] = b.x, v[i][5] = b.y, v[i][6] = b.z, v[i][7] = b.w;
   }
   squares = 0.f;
@@ -200,7 +200,7 @@ __device__ __forceinline__ void normalise_fragments(Fragments& f, float squares,
       const size_t at = size_t(block) * 256 + lane * 8;
 #pragma unroll
       for (int e = 0; e < 8; e += 4) {
-        const float4 a = __ldcg(reinterpret_cast<const float4*>(x + size_t(row) * ldx + at + e)), w = *reinterpret_cast<const float4*>(norm + at + e);
+        const float4 a = *reinterpret_cast<const float4*>(x + size_t(row) * ldx + at + e), w = *reinterpret_cast<const float4*>(norm + at + e);
         *reinterpret_cast<float4*>(normalised + size_t(row) * kGemvNormK + at + e) =
             make_float4(a.x * mine * w.x, a.y * mine * w.y, a.z * mine * w.z, a.w * mine * w.w);
       }
