@@ -15,12 +15,11 @@
 // four, one TMEM lane quadrant each), the last four = epilogue. Every mbarrier wait is bounded; on a timeout the kernel raises an abort
 // flag, records a status code, and every role leaves its loops.
 // The fp16 activations of a super-block are 64 KB, so weight slabs and activations travel through separate rings, the
-// activations in two halves of eight k-steps each: 4 slab stages + 4 half stages. The producer warp first asks the L2 for the
-// whole tile (and the next one of this CTA) with bulk prefetches, which need no shared memory, so that few 18 KB slab copies
-// in flight are enough.
-// The kernel is launched programmatically dependent on the kernel that lays out the activations: set-up, the
-// prefetches and the first weight slab run while that one is still at work, and only the activation copies and the
-// epilogue wait for it.
+// activations in two halves of eight k-steps each: 4 slab stages + 4 half stages. Bulk prefetches of whole tiles into the L2, which
+// the producer once began with, got in the way of the copies (18944 x 16384 with 9 rows 71.9 -> 64.6 us without them, with 128 rows
+// 92.0 -> 84.3; all projections of a layer 88.3 -> 82.1 and 121.7 -> 112.9).
+// The kernel is launched programmatically dependent on the kernel that lays out the activations: set-up and the first
+// weight slab run while that one is still at work, and only the activation copies and the epilogue wait for it.
 // Measured: about 0.8 us per super-block, of which the 16 MMAs are 0.55 at 128 rows (64 cycles each; 11 at 16 rows), bounded by
 // the dequantisation; 96 tiles (n = 12288) occupy 96 of 148 SMs.
 #include "common.cuh"
@@ -53,10 +52,6 @@ struct Control {
 constexpr int kControlBytes = 512;
 static_assert(sizeof(Control) <= kControlBytes, "control block too large");
 constexpr size_t kSharedBytes = 1024 + kControlBytes + size_t(kStages) * kSlabBytes + size_t(kActStages) * kActHalfBytes;
-
-__device__ __forceinline__ void prefetch_l2(const void* address, uint32_t bytes) {  // 16-byte aligned, bytes a multiple of 16
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(address), "r"(bytes) : "memory");
-}
 
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t columns) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(columns) : "memory");
@@ -190,27 +185,10 @@ template <int NMAT, int GROUPS> __global__ void __launch_bounds__(kThreads<GROUP
 
   if (warp == 0) {
     // ---------------- producer: one weight slab and two activation halves per super-block ----------------
-    // L2 prefetch of an item's weights: 128 rows x (blocksPerRow x 144) bytes per matrix, four rows per lane.
-    auto prefetch = [&](int item) {
-      const int tile = item % p.tiles, firstBlock = (item / p.tiles) * blocksPerRow;
-      int segment = 0;
-      while (segment + 1 < p.nseg && tile >= p.seg[segment + 1].tile0)
-        ++segment;
-      const size_t rowBytes = size_t(p.k / 256) * 144, row0 = size_t(tile - p.seg[segment].tile0) * kRows;
-      for (int mat = 0; mat < NMAT; ++mat) {
-        const uint8_t* base = (mat ? p.seg[segment].w2 : p.seg[segment].w) + row0 * rowBytes + size_t(firstBlock) * 144;
-        for (int r = lane; r < kRows; r += 32)
-          prefetch_l2(base + r * rowBytes, uint32_t(blocksPerRow) * 144);
-      }
-    };
-    if (int(blockIdx.x) < items)
-      prefetch(blockIdx.x);
     const uint32_t halfBytes = uint32_t(p.actRows) * 256;  // 8 k-steps x [actRows x 16] fp16
     uint32_t it = 0, slabs = 0, halves = 0;  // slabs, halves: copies issued
     bool ok = true, waited = false;
     for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
-      if (item + int(gridDim.x) < items)
-        prefetch(item + gridDim.x);
       const int tile = item % p.tiles, firstBlock = (item / p.tiles) * blocksPerRow;
       int segment = 0;
       while (segment + 1 < p.nseg && tile >= p.seg[segment + 1].tile0)
