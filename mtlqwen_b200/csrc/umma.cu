@@ -9,8 +9,10 @@
 //     activations, from shared memory through a matrix descriptor. The activations were rounded to fp16 beforehand
 //     (umma_prepare_rows_kernel), already laid out as canonical no-swizzle K-major core matrices under the same K
 //     permutation that the nibble extraction produces;
-//   * one 128-column fp32 accumulator per (tile, matrix), double-buffered, so the epilogue of one overlaps the MMAs of
-//     the next.
+//   * one 128-column fp32 accumulator per tile, double-buffered, so the epilogue of one overlaps the MMAs of the next. A gate /
+//     up pair takes both: every super-block of the activations is copied once and multiplied with both matrices (one after the other,
+//     with 96 CTAs on the activations twice, the copies were what the tensor cores waited for: 46.9 us for 12288 x 4096 with 128
+//     rows, 35.0 now), and silu(gate) * up is formed from the two accumulators.
 // Warp roles: 0 = TMA producer, 1 = MMA issuer (owns the TMEM allocation), 4..11 (4..19) = dequant (two or four groups of
 // four, one TMEM lane quadrant each), the last four = epilogue. Every mbarrier wait is bounded; on a timeout the kernel raises an abort
 // flag, records a status code, and every role leaves its loops.
@@ -20,8 +22,9 @@
 // 92.0 -> 84.3; all projections of a layer 88.3 -> 82.1 and 121.7 -> 112.9).
 // The kernel is launched programmatically dependent on the kernel that lays out the activations: set-up and the first
 // weight slab run while that one is still at work, and only the activation copies and the epilogue wait for it.
-// Measured: about 0.8 us per super-block, of which the 16 MMAs are 0.55 at 128 rows (64 cycles each; 11 at 16 rows), bounded by
-// the dequantisation; 96 tiles (n = 12288) occupy 96 of 148 SMs.
+// What bounds it, by its own clocks (18944 x 8192, every SM at work): with 128 rows the copies, 82 KB a super-block of which 64 are
+// activations, at 45 bytes a clock and SM (0.95 us; the 16 MMAs are 0.55); with few rows a dequant group's 1200 clocks a half. 96 tiles
+// (n = 12288) occupy 96 of 148 SMs.
 #include "common.cuh"
 #include "kernels.h"
 
@@ -102,40 +105,33 @@ __device__ __forceinline__ uint64_t smem_descriptor(uint32_t address, uint32_t l
   return uint64_t((address & 0x3FFFFu) >> 4) | (uint64_t(leading >> 4) << 16) | (uint64_t(stride >> 4) << 32) | (uint64_t(1) << 46);
 }
 
-// The epilogue of one (item, matrix) accumulator for the 32 TMEM lanes (= weight rows = output columns) of the calling
+// The epilogue of one item for the 32 TMEM lanes (= weight rows = output columns) of the calling
 // warp: groups of eight activation rows `first`, `first + stride`, ... of the 16. Everything the store loop needs is
 // copied out of the parameter block first: the segment is a run-time index, so the block is reached through a generic
 // address, and the compiler must assume that the stores change it and would read pointer and pitch again after every
 // one of them (measured: 110 ns per store instead of 10).
-template <int NMAT> __device__ __forceinline__ void store_accumulator(const UmmaParams& p, int item, int mat, uint32_t accumulator, int row, int first,
-                                                                      int stride) {
+template <int NMAT> __device__ __forceinline__ void store_accumulator(const UmmaParams& p, int item, uint32_t accumulator, int row, int first, int stride) {
   const int tile = item % p.tiles, slice = item / p.tiles;
   int segment = 0;
   while (segment + 1 < p.nseg && tile >= p.seg[segment + 1].tile0)
     ++segment;
-  float* const y = p.seg[segment].y;
-  const float* const residual = p.seg[segment].res;
   const size_t pitch = size_t(p.seg[segment].ldy), column = size_t(tile - p.seg[segment].tile0) * kRows + row;
   const int liveRows = p.m;
-  float* const partial = NMAT == 1 && p.splits > 1 ? p.partial + size_t(slice) * p.m * pitch : nullptr;
+  // a K slice: the partial sums are added up, with the residual, by umma_reduce_kernel
+  const bool parts = NMAT == 1 && p.splits > 1;
+  float* const y = parts ? p.partial + size_t(slice) * p.m * pitch : p.seg[segment].y;
+  const float* const residual = NMAT == 2 || parts ? nullptr : p.seg[segment].res;
   for (int c = first; c < kActs / 8 && c * 8 < liveRows; c += stride) {
-    float v[8];
+    float v[8], up[8];
     tmem_load8(accumulator + c * 8, v);
+    if (NMAT == 2)  // post == 2 epilogue, quant_linear.metal:224-232
+      tmem_load8(accumulator + kActs + c * 8, up);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int m = c * 8 + i;
       if (m < liveRows) {
         const size_t at = size_t(m) * pitch + column;
-        float value = v[i];
-        if (partial) {  // a K slice: the partial sums are added up, with the residual, by umma_reduce_kernel
-          partial[at] = value;
-          continue;
-        }
-        if (NMAT == 2)  // the gate half parks in y until the up half arrives (post == 2 epilogue, quant_linear.metal:224-232)
-          value = mat == 0 ? value : silu_f(y[at]) * value;
-        else if (residual)
-          value += residual[at];
-        y[at] = value;
+        y[at] = NMAT == 2 ? silu_f(v[i]) * up[i] : residual ? v[i] + residual[at] : v[i];
       }
     }
   }
@@ -151,9 +147,10 @@ template <int NMAT, int GROUPS> __global__ void __launch_bounds__(kThreads<GROUP
   pdl_launch_dependents();
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   // With p.splits > 1 (one matrix) the work items are (tile, K slice) pairs, so that a matrix of few 128-row tiles still
-  // fills the GPU; `blocksPerRow` is then the super-blocks of one slice. One accumulator buffer per (item, matrix).
+  // fills the GPU; `blocksPerRow` is then the super-blocks of one slice.
   const int blocksPerRow = p.k / 256 / p.splits, items = p.tiles * p.splits;
-  const uint32_t units = int(blockIdx.x) < items ? uint32_t((items - 1 - int(blockIdx.x)) / int(gridDim.x) + 1) * NMAT : 0u;  // accumulators of this CTA
+  const uint32_t units = int(blockIdx.x) < items ? uint32_t((items - 1 - int(blockIdx.x)) / int(gridDim.x) + 1) : 0u;  // items of this CTA
+  constexpr uint32_t kDBuffers = 2 / NMAT;  // a pair's accumulators take both
   volatile int* abortFlag = &ctl.abort;
 
   if (tid == 0) {
@@ -195,9 +192,9 @@ template <int NMAT, int GROUPS> __global__ void __launch_bounds__(kThreads<GROUP
         ++segment;
       const int row0 = (tile - p.seg[segment].tile0) * kRows;
       if (elect_one())  // the same lane every time: it keeps the counters
-        for (int mat = 0; mat < NMAT && ok; ++mat)
-          for (int sb = firstBlock; sb < firstBlock + blocksPerRow && ok; ++sb, ++it) {
-            const uint32_t slot = it % kStages, round = it / kStages;
+        for (int sb = firstBlock; sb < firstBlock + blocksPerRow && ok; ++sb, ++it) {
+          for (int mat = 0; mat < NMAT && ok; ++mat) {
+            const uint32_t slab = it * NMAT + mat, slot = slab % kStages, round = slab / kStages;
             if (round > 0)
               ok = mbar_wait_bounded(&ctl.slotFree[slot], (round - 1) & 1, abortFlag);
             if (ok) {
@@ -205,25 +202,26 @@ template <int NMAT, int GROUPS> __global__ void __launch_bounds__(kThreads<GROUP
               tma_load_2d(ring + size_t(slot) * kSlabBytes, &p.map[segment][mat], sb * 18, row0, &ctl.full[slot]);
               ++slabs;
             }
-            if (!waited) {  // the activations are the preceding kernel's output
-              pdl_wait();
-              waited = true;
-            }
-            for (int h = 0; h < 2 && ok; ++h) {  // the two activation halves of this super-block
-              const uint32_t half = 2 * it + h, actSlot = half % kActStages, actRound = half / kActStages;
-              if (actRound > 0)
-                ok = mbar_wait_bounded(&ctl.actFree[actSlot], (actRound - 1) & 1, abortFlag);
-              if (ok) {
-                mbar_arrive_expect_tx(&ctl.actFull[actSlot], halfBytes);
-                bulk_load(actRing + size_t(actSlot) * kActHalfBytes, p.acts + (size_t(sb) * 2 + h) * halfBytes, halfBytes, &ctl.actFull[actSlot]);
-                ++halves;
-              }
-            }
-            if (!ok) {
-              *abortFlag = 1;
-              atomicExch(p.status, kStatusBarrierTimeout);
+          }
+          if (!waited) {  // the activations are the preceding kernel's output
+            pdl_wait();
+            waited = true;
+          }
+          for (int h = 0; h < 2 && ok; ++h) {  // the two activation halves of this super-block
+            const uint32_t half = 2 * it + h, actSlot = half % kActStages, actRound = half / kActStages;
+            if (actRound > 0)
+              ok = mbar_wait_bounded(&ctl.actFree[actSlot], (actRound - 1) & 1, abortFlag);
+            if (ok) {
+              mbar_arrive_expect_tx(&ctl.actFull[actSlot], halfBytes);
+              bulk_load(actRing + size_t(actSlot) * kActHalfBytes, p.acts + (size_t(sb) * 2 + h) * halfBytes, halfBytes, &ctl.actFull[actSlot]);
+              ++halves;
             }
           }
+          if (!ok) {
+            *abortFlag = 1;
+            atomicExch(p.status, kStatusBarrierTimeout);
+          }
+        }
       ok = __all_sync(0xffffffffu, ok);
     }
     // no copy may be in flight when the CTA ends, whoever gave up
@@ -239,34 +237,34 @@ template <int NMAT, int GROUPS> __global__ void __launch_bounds__(kThreads<GROUP
       uint32_t it = 0, unit = 0;
       bool ok = true;
       const uint32_t instruction = instruction_descriptor(p.actRows), stepBytes = uint32_t(p.actRows) * 32;
-      for (int item = blockIdx.x; item < items && ok; item += gridDim.x)
-        for (int mat = 0; mat < NMAT && ok; ++mat, ++unit) {
-          const uint32_t buffer = unit & 1;
-          if (unit >= 2)
-            ok = mbar_wait_bounded(&ctl.dFree[buffer], ((unit >> 1) - 1) & 1, abortFlag);
-          const uint32_t dColumn = tmem + kColD + buffer * 128;
-          for (int j = 0; j < blocksPerRow && ok; ++j, ++it) {
-            for (int h = 0; h < 2 && ok; ++h) {  // eight k-steps per half of a super-block
-              const uint32_t half = 2 * it + h, actSlot = half % kActStages, aBuffer = half % kABuffers;
-              ok = mbar_wait_bounded(&ctl.aReady[aBuffer], (half / kABuffers) & 1, abortFlag) &&
-                   mbar_wait_bounded(&ctl.actFull[actSlot], (half / kActStages) & 1, abortFlag);
-              if (!ok)
-                break;
-              fence_after_sync();
-              const uint32_t actBase = smem_u32(actRing + size_t(actSlot) * kActHalfBytes);
-#pragma unroll
-              for (int step = 0; step < 8; ++step)
-                umma_ts(dColumn, tmem + kColA + aBuffer * 64 + step * 8, smem_descriptor(actBase + step * stepBytes, 128, 256), instruction,
-                        (j | h | step) != 0);
-              umma_commit(&ctl.actFree[actSlot]);
-              umma_commit(&ctl.aFree[aBuffer]);
-            }
+      for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++unit) {
+        const uint32_t buffer = unit % kDBuffers;
+        if (unit >= kDBuffers)
+          ok = mbar_wait_bounded(&ctl.dFree[buffer], (unit / kDBuffers - 1) & 1, abortFlag);
+        for (int j = 0; j < blocksPerRow && ok; ++j, ++it) {
+          for (int turn = 0; turn < 2 * NMAT && ok; ++turn) {  // eight k-steps per half of a super-block, of one matrix and the other
+            const uint32_t mat = turn >> 1, h = turn & 1, act = 2 * it + h, half = 2 * (it * NMAT + mat) + h, actSlot = act % kActStages, aBuffer = half % kABuffers;
+            const uint32_t dColumn = tmem + kColD + (NMAT == 2 ? mat : buffer) * 128;
+            ok = mbar_wait_bounded(&ctl.aReady[aBuffer], (half / kABuffers) & 1, abortFlag) &&
+                 mbar_wait_bounded(&ctl.actFull[actSlot], (act / kActStages) & 1, abortFlag);
             if (!ok)
               break;
-            if (j == blocksPerRow - 1)
-              umma_commit(&ctl.dReady[buffer]);
+            fence_after_sync();
+            const uint32_t actBase = smem_u32(actRing + size_t(actSlot) * kActHalfBytes);
+#pragma unroll
+            for (int step = 0; step < 8; ++step)
+              umma_ts(dColumn, tmem + kColA + aBuffer * 64 + step * 8, smem_descriptor(actBase + step * stepBytes, 128, 256), instruction,
+                      (j | h | step) != 0);
+            if (mat == NMAT - 1)
+              umma_commit(&ctl.actFree[actSlot]);
+            umma_commit(&ctl.aFree[aBuffer]);
           }
+          if (!ok)
+            break;
+          if (j == blocksPerRow - 1)
+            umma_commit(&ctl.dReady[buffer]);
         }
+      }
       if (!ok) {
         *abortFlag = 1;
         atomicExch(p.status, kStatusBarrierTimeout);
@@ -275,73 +273,74 @@ template <int NMAT, int GROUPS> __global__ void __launch_bounds__(kThreads<GROUP
   } else if (warp >= 4 && warp < 4 + 4 * GROUPS) {
     // ---------------- dequant: thread = weight row; a group takes one half of every super-block (two groups) or of every
     // second one (four). A lies in tensor memory as a ring of four halves, so a group fills one while the MMAs of another run.
-    // Four groups keep up with MMAs of up to 128 rows (layer projections of 128 rows 124.6 against 128.6 us), two start and
-    // drain faster, which counts for more with few rows (40 rows: 97.1 against 104.6 us): see launch_tiles.
+    // See umma_launch for which.
     const int group = (warp - 4) >> 2, side = group & 1, quadrant = warp & 3, row = quadrant * 32 + lane;
     constexpr uint32_t k1024 = 0x64006400u;
     uint32_t it = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < items && ok; item += gridDim.x)
-      for (int mat = 0; mat < NMAT && ok; ++mat)
-        for (int j = 0; j < blocksPerRow && ok; ++j, ++it) {
-          if (GROUPS == 4 && (it & 1) != uint32_t(group >> 1))
-            continue;
-          const uint32_t slot = it % kStages, round = it / kStages, half = 2 * it + side, aBuffer = half % kABuffers;
-          ok = mbar_wait_bounded(&ctl.full[slot], round & 1, abortFlag);
-          if (ok && half >= kABuffers)
-            ok = mbar_wait_bounded(&ctl.aFree[aBuffer], (half / kABuffers - 1) & 1, abortFlag);
-          if (!ok)
-            break;
-          fence_after_sync();
-          const uint8_t* block = ring + size_t(slot) * kSlabBytes + row * 144;
-          const uint4 header = *reinterpret_cast<const uint4*>(block);
-          const float2 dm = __half22float2(*reinterpret_cast<const __half2*>(&header.x));
-          // 6-bit scales / mins of this half's four sub-blocks (scale_min_k4, quant_linear.metal:12-20)
-          const uint32_t scales = side == 0 ? header.y & 0x3f3f3f3fu : (header.w & 0x0f0f0f0fu) | ((header.y >> 2) & 0x30303030u);
-          const uint32_t mins = side == 0 ? header.z & 0x3f3f3f3fu : ((header.w >> 4) & 0x0f0f0f0fu) | ((header.z >> 2) & 0x30303030u);
-          const uint32_t aAddress = tmem + (uint32_t(quadrant * 32) << 16) + kColA + aBuffer * 64;
+      for (int j = 0; j < blocksPerRow * NMAT && ok; ++j, ++it) {  // of a pair, the matrices in turn
+        if (GROUPS == 4 && (it & 1) != uint32_t(group >> 1))
+          continue;
+        const uint32_t slot = it % kStages, round = it / kStages, half = 2 * it + side, aBuffer = half % kABuffers;
+        ok = mbar_wait_bounded(&ctl.full[slot], round & 1, abortFlag);
+        if (ok && half >= kABuffers)
+          ok = mbar_wait_bounded(&ctl.aFree[aBuffer], (half / kABuffers - 1) & 1, abortFlag);
+        if (!ok)
+          break;
+        fence_after_sync();
+        const uint8_t* block = ring + size_t(slot) * kSlabBytes + row * 144;
+        const uint4 header = *reinterpret_cast<const uint4*>(block);
+        const uint4* const quants = reinterpret_cast<const uint4*>(block + 16 + 64 * side);
+        uint4 quads[4];  // read ahead where other warps wait for the same pipe (a pair with 128 rows 37.3 -> 35.0 us; with two groups 1 % slower)
+        if (GROUPS == 4)
 #pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            const uint32_t pair = (scales >> (16 * t)) & 0xffffu, minPair = (mins >> (16 * t)) & 0xffffu;
-            const uint8_t* const quants = block + 16 + 64 * side + 32 * t;
-            const uint4 q0 = *reinterpret_cast<const uint4*>(quants), q1 = *reinterpret_cast<const uint4*>(quants + 16);
-            const uint32_t words[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-            // dequantised weight d*sc*q - dmin*m, in fp16: q is made exact first, then one fused multiply-add
-            const uint32_t sL = pack_half2(dm.x * float(pair & 0xffu), dm.x * float(pair & 0xffu));
-            const uint32_t sH = pack_half2(dm.x * float(pair >> 8), dm.x * float(pair >> 8));
-            const uint32_t nL = pack_half2(-dm.y * float(minPair & 0xffu), -dm.y * float(minPair & 0xffu));
-            const uint32_t nH = pack_half2(-dm.y * float(minPair >> 8), -dm.y * float(minPair >> 8));
-            uint32_t v[32];
+          for (int i = 0; i < 4; ++i)
+            quads[i] = quants[i];
+        const float2 dm = __half22float2(*reinterpret_cast<const __half2*>(&header.x));
+        // 6-bit scales / mins of this half's four sub-blocks (scale_min_k4, quant_linear.metal:12-20)
+        const uint32_t scales = side == 0 ? header.y & 0x3f3f3f3fu : (header.w & 0x0f0f0f0fu) | ((header.y >> 2) & 0x30303030u);
+        const uint32_t mins = side == 0 ? header.z & 0x3f3f3f3fu : ((header.w >> 4) & 0x0f0f0f0fu) | ((header.z >> 2) & 0x30303030u);
+        const uint32_t aAddress = tmem + (uint32_t(quadrant * 32) << 16) + kColA + aBuffer * 64;
 #pragma unroll
-            for (int w = 0; w < 8; ++w) {
-              const uint32_t a = words[w];
-              v[2 * w] = hfma2_u32(hsub2_u32((a & 0x000f000fu) | k1024, k1024), sL, nL);
-              v[2 * w + 1] = hfma2_u32(hsub2_u32(((a >> 8) & 0x000f000fu) | k1024, k1024), sL, nL);
-              v[16 + 2 * w] = hfma2_u32(hsub2_u32(((a >> 4) & 0x000f000fu) | k1024, k1024), sH, nH);
-              v[16 + 2 * w + 1] = hfma2_u32(hsub2_u32(((a >> 12) & 0x000f000fu) | k1024, k1024), sH, nH);
-            }
-            tmem_store32(aAddress + 32 * t, v);
+        for (int t = 0; t < 2; ++t) {
+          const uint32_t pair = (scales >> (16 * t)) & 0xffffu, minPair = (mins >> (16 * t)) & 0xffffu;
+          const uint4 q0 = GROUPS == 4 ? quads[2 * t] : quants[2 * t], q1 = GROUPS == 4 ? quads[2 * t + 1] : quants[2 * t + 1];
+          const uint32_t words[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+          // dequantised weight d*sc*q - dmin*m, in fp16: q is made exact first, then one fused multiply-add
+          const uint32_t sL = pack_half2(dm.x * float(pair & 0xffu), dm.x * float(pair & 0xffu));
+          const uint32_t sH = pack_half2(dm.x * float(pair >> 8), dm.x * float(pair >> 8));
+          const uint32_t nL = pack_half2(-dm.y * float(minPair & 0xffu), -dm.y * float(minPair & 0xffu));
+          const uint32_t nH = pack_half2(-dm.y * float(minPair >> 8), -dm.y * float(minPair >> 8));
+          uint32_t v[32];
+#pragma unroll
+          for (int w = 0; w < 8; ++w) {
+            const uint32_t a = words[w];
+            v[2 * w] = hfma2_u32(hsub2_u32((a & 0x000f000fu) | k1024, k1024), sL, nL);
+            v[2 * w + 1] = hfma2_u32(hsub2_u32(((a >> 8) & 0x000f000fu) | k1024, k1024), sL, nL);
+            v[16 + 2 * w] = hfma2_u32(hsub2_u32(((a >> 4) & 0x000f000fu) | k1024, k1024), sH, nH);
+            v[16 + 2 * w + 1] = hfma2_u32(hsub2_u32(((a >> 12) & 0x000f000fu) | k1024, k1024), sH, nH);
           }
-          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-          fence_before_sync();
-          __syncwarp();
-          if (lane == 0) {
-            mbar_arrive(&ctl.aReady[aBuffer]);
-            mbar_arrive(&ctl.slotFree[slot]);
-          }
+          tmem_store32(aAddress + 32 * t, v);
         }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(&ctl.aReady[aBuffer]);
+          mbar_arrive(&ctl.slotFree[slot]);
+        }
+      }
     if (ok && units > 0) {
       // their share of the CTA's last accumulator (see the epilogue warps): groups of eight activation rows 1 + group,
       // 2 + GROUPS + group, ...; the accumulator has no later user, so nobody waits for these reads
-      const uint32_t unit = units - 1, buffer = unit & 1;
+      const uint32_t unit = units - 1, buffer = unit % kDBuffers;
       pdl_wait();
-      ok = mbar_wait_bounded(&ctl.dReady[buffer], (unit >> 1) & 1, abortFlag);
-      if (ok && NMAT == 2)  // the up half reads the gate half that the epilogue warps parked in y: wait until they are through with it
-        ok = mbar_wait_bounded(&ctl.dFree[(unit - 1) & 1], ((unit - 1) >> 1) & 1, abortFlag);
+      ok = mbar_wait_bounded(&ctl.dReady[buffer], (unit / kDBuffers) & 1, abortFlag);
       if (ok) {
         fence_after_sync();
-        const int lastItem = int(blockIdx.x) + int((units - 1) / NMAT) * int(gridDim.x);
-        store_accumulator<NMAT>(p, lastItem, NMAT - 1, tmem + (uint32_t(quadrant * 32) << 16) + kColD + buffer * 128, row, 1 + group, 1 + GROUPS);
+        const int lastItem = int(blockIdx.x) + int(units - 1) * int(gridDim.x);
+        store_accumulator<NMAT>(p, lastItem, tmem + (uint32_t(quadrant * 32) << 16) + kColD + buffer * 128, row, 1 + group, 1 + GROUPS);
       }
     }
     if (!ok && lane == 0) {
@@ -350,26 +349,24 @@ template <int NMAT, int GROUPS> __global__ void __launch_bounds__(kThreads<GROUP
     }
   } else if (warp >= 4 + 4 * GROUPS) {
     // ---------------- epilogue: thread = weight row ----------------
-    pdl_wait();  // residuals, the parked gate half and the partial-sum buffer belong to earlier kernels
+    pdl_wait();  // residuals, results and the partial-sum buffer belong to earlier kernels
     const int quadrant = warp & 3, row = quadrant * 32 + lane;
     const uint32_t laneBase = tmem + (uint32_t(quadrant * 32) << 16) + kColD;
     uint32_t unit = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < items && ok; item += gridDim.x)
-      for (int mat = 0; mat < NMAT && ok; ++mat, ++unit) {
-        const uint32_t buffer = unit & 1;
-        ok = mbar_wait_bounded(&ctl.dReady[buffer], (unit >> 1) & 1, abortFlag);
-        if (!ok)
-          break;
-        fence_after_sync();
-        // the CTA's last accumulator: the dequant warps, idle by then, take most of it
-        const bool last = unit + 1 == units;
-        store_accumulator<NMAT>(p, item, mat, laneBase + buffer * 128, row, 0, last ? 1 + GROUPS : 1);
-        fence_before_sync();
-        __syncwarp();
-        if (lane == 0)
-          mbar_arrive(&ctl.dFree[buffer]);
-      }
+    for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++unit) {
+      const uint32_t buffer = unit % kDBuffers;
+      ok = mbar_wait_bounded(&ctl.dReady[buffer], (unit / kDBuffers) & 1, abortFlag);
+      if (!ok)
+        break;
+      fence_after_sync();
+      // the CTA's last accumulator: the dequant warps, idle by then, take most of it
+      store_accumulator<NMAT>(p, item, laneBase + buffer * 128, row, 0, unit + 1 == units ? 1 + GROUPS : 1);
+      fence_before_sync();
+      __syncwarp();
+      if (lane == 0)
+        mbar_arrive(&ctl.dFree[buffer]);
+    }
     if (!ok && lane == 0) {
       *abortFlag = 1;
       atomicExch(p.status, kStatusBarrierTimeout);
@@ -451,9 +448,13 @@ template <int NMAT, int GROUPS> cudaError_t launch_tiles(const UmmaParams& param
 
 // 9 to 128 activation rows (p.m), rows of x `ldx` floats apart (a multiple of 4).
 cudaError_t umma_launch(bool pair, const UmmaParams& p, const float* x, int ldx, int sms, cudaStream_t stream) {
-  if (p.m > 96)  // layer projections of 64 rows: 106.2 us with two groups, 109.8 with four; of 128 rows 128.6 and 124.6
-    return pair ? launch_tiles<2, 4>(p, x, ldx, sms, stream) : launch_tiles<1, 4>(p, x, ldx, sms, stream);
-  return pair ? launch_tiles<2, 2>(p, x, ldx, sms, stream) : launch_tiles<1, 2>(p, x, ldx, sms, stream);
+  // Two dequant groups take a half of every super-block each, four of every second one. A pair wants four (12288 x 4096 with 9, 40 and
+  // 64 rows 28.8, 30.1 and 32.0 us, with two 32.4, 33.9 and 35.6): its activations come once for two super-blocks, so the dequantisation is what
+  // the MMAs wait for. One matrix with few rows wants two, which start and drain faster (4096 x 12288 with 9 and 64 rows 17.6 and 20.5,
+  // with four 18.7 and 21.1); with 128 rows four keep up with the MMAs (projections of a layer 124.6 us, with two 128.6).
+  if (pair)
+    return launch_tiles<2, 4>(p, x, ldx, sms, stream);
+  return p.m > 96 ? launch_tiles<1, 4>(p, x, ldx, sms, stream) : launch_tiles<1, 2>(p, x, ldx, sms, stream);
 }
 
 }  // namespace infdev
