@@ -239,16 +239,18 @@ __device__ __forceinline__ void q6k_unit(const uint8_t* pA, const uint8_t* pB, i
 #pragma unroll
         for (int sh = 0; sh < 2; ++sh) {
           const int s = sl + 2 * sh, gi = hh * 8 + s * 2 + u;
-          const uint32_t bytesA = ((sh ? loA >> 4 : loA) & 0x0f0f0f0fu) | (((hiA >> (2 * s)) & 0x03030303u) << 4);
-          const uint32_t bytesB = ((sh ? loB >> 4 : loB) & 0x0f0f0f0fu) | (((hiB >> (2 * s)) & 0x03030303u) << 4);
+          const uint32_t bytesA = ((sh ? loA >> 4 : loA) & 0x0f0f0f0fu) | ((s < 3 ? hiA << (4 - 2 * s) : hiA >> 2) & 0x30303030u);
+          const uint32_t bytesB = ((sh ? loB >> 4 : loB) & 0x0f0f0f0fu) | ((s < 3 ? hiB << (4 - 2 * s) : hiB >> 2) & 0x30303030u);
           uint32_t a[1][4];
           byte_fragment(a[0], bytesA, bytesB, k1056);
-          const float sA = dA * float(int(reinterpret_cast<const int8_t*>(pA + 192)[gi])), sB = dB * float(int(reinterpret_cast<const int8_t*>(pB + 192)[gi]));
-          scaled_products<false>(sum, a, b, gi, sA, sB);
+          scaled_products<false>(sum, a, b, gi, float(int(reinterpret_cast<const int8_t*>(pA + 192)[gi])), float(int(reinterpret_cast<const int8_t*>(pB + 192)[gi])));
         }
       }
     }
   }
+#pragma unroll
+  for (int tile = 0; tile < NT; ++tile)
+    sum[tile][0] *= dA, sum[tile][1] *= dA, sum[tile][2] *= dB, sum[tile][3] *= dB;
   add_totals(total, b, sum);
 }
 
