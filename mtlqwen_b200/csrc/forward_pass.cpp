@@ -11,6 +11,9 @@
 #include "gguf_reader.hpp"
 #include "runtime.hpp"
 
+// A device layer that has no norm_supply gets the norm and the projection as two calls.
+#pragma weak infdev_norm_supply
+
 namespace infeng::qwen35 {
 
 // Read-only mapping of a file.
@@ -159,24 +162,43 @@ struct Ops {
   // Decode-sized passes hand the quantised form of each projection's input from the kernel that produces it to the
   // GEMV that consumes it, which saves the GEMV its own quantisation launch.
   void capture(const Tensor& image) {
-    if (rows <= imageRows)
+    if (rows <= imageRows && !selfServed())
       check(infdev_image_capture(ctx, image.as<uint8_t>()));
   }
   void supply(const Tensor& image) {
-    if (rows <= imageRows)
+    if (rows <= imageRows && !selfServed())
       check(infdev_image_supply(ctx, image.as<uint8_t>()));
+  }
+
+  // With one or two rows the Q4_K GEMV quantises and normalises its input itself for less than the launches, or the turns of the
+  // producers, that would do it for it: 64 tokens of one sequence 121.0 ms with norms and images apart, 114.8 with the norms on
+  // the way in, 109.5 with the images too. With eight rows reading them in every CTA costs as much as it saves (157.5, 160.6, 162.6).
+  bool selfServed() const { return rows <= 2; }
+
+  // Announces the RMS norm of `hidden` as the activations of the projections that follow at once, and returns what to pass them.
+  // store: the normalised rows are wanted in scratch.norm in any case.
+  const Tensor& normalised(const Tensor& hidden, const float* norm, std::initializer_list<const Weight*> targets, bool store) {
+    bool fold = infdev_norm_supply && selfServed();
+    for (const Weight* target : targets)
+      fold = fold && target->type == INFDEV_Q4_K;
+    if (fold) {
+      check(infdev_norm_supply(ctx, norm, scratch.norm.as<float>(), store));
+      return hidden;
+    }
+    capture(scratch.normImage);
+    check(infdev_rms_norm(ctx, hidden.as<float>(), norm, rows, hiddenSize, scratch.norm.as<float>()));
+    supply(scratch.normImage);
+    return scratch.norm;
   }
 
   void decoder(uint32_t layer, const Tensor& hidden) {
     prefix = "blk." + std::to_string(layer) + ".";
     const bool fullAttention = layer >= engine.targetLayers || (layer + 1) % fullAttentionInterval == 0;
-    const Tensor& x = scratch.norm;
-    capture(scratch.normImage);
-    check(infdev_rms_norm(ctx, hidden.as<float>(), f32("attn_norm.weight"), rows, hiddenSize, x.as<float>()));
-    supply(scratch.normImage);
+    const float* attentionNorm = f32("attn_norm.weight");
     if (fullAttention) {
       const uint32_t kvLayer = layer < engine.targetLayers ? layer / fullAttentionInterval : engine.kvLayers + layer - engine.targetLayers;
-      linearGroup(x, {{&weight("attn_q.weight"), scratch.mixed}, {&weight("attn_k.weight"), scratch.k}, {&weight("attn_v.weight"), scratch.v}}, rows);
+      Weight &q = weight("attn_q.weight"), &k = weight("attn_k.weight"), &v = weight("attn_v.weight");
+      linearGroup(normalised(hidden, attentionNorm, {&q, &k, &v}, false), {{&q, scratch.mixed}, {&k, scratch.k}, {&v, scratch.v}}, rows);
       check(infdev_attention_prepare(ctx, scratch.mixed.as<float>(), scratch.k.as<float>(), scratch.v.as<float>(), f32("attn_q_norm.weight"),
                                      f32("attn_k_norm.weight"), engine.rope.as<float>(), queries, int(queryCount), rows, engine.kv->blockTable(),
                                      int32_t(engine.kv->tableStride()), int32_t(engine.blockTokens), scratch.attnQ.as<float>(),
@@ -189,7 +211,9 @@ struct Ops {
       supply(scratch.temporaryImage);
       linear(scratch.temporary, weight("attn_output.weight"), rows, hidden, hidden);
     } else {
-      linearGroup(x, {{&weight("attn_qkv.weight"), scratch.mixed}, {&weight("attn_gate.weight"), scratch.gate}}, rows);
+      Weight &qkv = weight("attn_qkv.weight"), &z = weight("attn_gate.weight");
+      linearGroup(normalised(hidden, attentionNorm, {&qkv, &z}, true), {{&qkv, scratch.mixed}, {&z, scratch.gate}}, rows);
+      const Tensor& x = scratch.norm;
       const uint64_t offset = uint64_t(layer - layer / fullAttentionInterval) * INFDEV_GDN_LAYER_STATE_BYTES;
       if (!prefill) {
         // every query of the pass is short: preparation and recurrence in one launch
@@ -213,10 +237,8 @@ struct Ops {
       supply(scratch.temporaryImage);
       linear(scratch.temporary, weight("ssm_out.weight"), rows, hidden, hidden);
     }
-    capture(scratch.normImage);
-    check(infdev_rms_norm(ctx, hidden.as<float>(), f32("post_attention_norm.weight"), rows, hiddenSize, x.as<float>()));
     Weight &gate = weight("ffn_gate.weight"), &up = weight("ffn_up.weight");
-    supply(scratch.normImage);
+    const Tensor& x = normalised(hidden, f32("post_attention_norm.weight"), {&gate, &up}, false);
     capture(scratch.mlpImage);
     check(infdev_gate_up(ctx, int(gate.type), gate.as<void>(), up.as<void>(), gate.n, gate.k, x.as<float>(), rows, scratch.mlpGate.as<float>()));
     supply(scratch.mlpImage);
