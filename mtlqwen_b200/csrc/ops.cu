@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(512) rms_norm_4096_kernel(const float* x, cons
   const float4 a = *reinterpret_cast<const float4*>(src + d), b = *reinterpret_cast<const float4*>(src + d + 4);
   const float4 ga = *reinterpret_cast<const float4*>(w + d), gb = *reinterpret_cast<const float4*>(w + d + 4);
   __shared__ float sums[16];
-  const float sum = warp_sum((a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w) + (b.x * b.x + b.y * b.y + b.z * b.z + b.w * b.w));
+  const float sum = warp_sum(square_sum(a, b));
   if (lane == 0)
     sums[warp] = sum;
   __syncthreads();

@@ -130,14 +130,10 @@ template <int NMAT, int ROWS> __global__ void __launch_bounds__(kThreads, 1) q4k
     const int myBlock = (groups == 2 ? half * kGemvStageBlocks : 0) + unit;
     const bool live = myBlock < chunkBlocks;
     Fragments fragments;
-    float squares;
-    if (live)
+    if (live)  // with a norm every warp: the row is one chunk of 16 super-blocks; one of the CTAs stores what a warp normalises
       fragments = p.image ? load_fragments<ROWS>(p.image + size_t(chunk * kChunkBlocks + myBlock) * kImageBlockBytes, lane)
-                          : quantize_fragments<ROWS>(p.x + size_t(chunk * kChunkBlocks + myBlock) * 256, p.ldx, p.m,
-                                                     p.norm ? p.norm + myBlock * 256 : nullptr, lane, squares);
-    if (p.norm)  // one chunk of 16 super-blocks
-      normalise_fragments<ROWS>(fragments, squares, squaresOfBlock, myBlock, p.m, p.x, p.ldx, p.norm,
-                                myBlock % int(gridDim.x) == int(blockIdx.x) ? p.normalised : nullptr, lane);
+                          : quantize_fragments<ROWS>(p.x + size_t(chunk * kChunkBlocks + myBlock) * 256, p.ldx, p.m, lane,
+                                                     {p.norm, myBlock % int(gridDim.x) == int(blockIdx.x) ? p.normalised : nullptr, squaresOfBlock, myBlock});
     int buffer = 0;
     for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, buffer = buffer == kFinisherWarps - 1 ? 0 : buffer + 1) {
       float total[NMAT][4];

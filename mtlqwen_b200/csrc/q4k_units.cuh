@@ -57,9 +57,17 @@ __device__ __forceinline__ uint32_t level_bits(float v, float inv) { return __fl
 
 // The same from fp32 activations: what image_store_block writes of this super-block and load_fragments reads, bit for bit, without the
 // launch between. A lane owns row g % ROWS and, of it, the eight values of quarter t of every sub-block that its column stands for.
-// With `norm` (the block's 256 weights) it quantises x * norm, which has the same levels as the normalised row, and `squares` becomes
-// the block's sum of squares of x of row g % ROWS, summed in the same order whatever ROWS.
-template <int ROWS> __device__ __forceinline__ Fragments quantize_fragments(const float* x, int ldx, int m, const float* norm, int lane, float& squares) {
+//
+// With norm.weight the activations are the RMS norm of the row, bit for bit as rms_norm_4096_kernel computes it, for 16 warps that hold
+// a row of 4096 between them: a block's squares are summed over the lanes of that kernel's warp, in its order whatever ROWS.
+struct RowNorm {
+  const float* weight;  // the row's 4096 weights; null: x as it is
+  float* normalised;    // [m][4096], where this warp's super-block of the result goes; null: nowhere
+  float* squares;       // shared [super-block][row]
+  int block;            // the warp's super-block
+};
+
+template <int ROWS> __device__ __forceinline__ Fragments quantize_fragments(const float* x, int ldx, int m, int lane, const RowNorm& norm) {
   constexpr int kShare = 8 / ROWS;
   const int g = lane >> 2, t = lane & 3, row = g % ROWS;
   const float* src = x + size_t(row) * ldx + (g / ROWS) * 32 + t * 8;
@@ -71,30 +79,41 @@ template <int ROWS> __device__ __forceinline__ Fragments quantize_fragments(cons
       a = *reinterpret_cast<const float4*>(src + i * kShare * 32), b = *reinterpret_cast<const float4*>(src + i * kShare * 32 + 4);
     v[i][0] = a.x, v[i][1] = a.y, v[i][2] = a.z, v[i][3] = a.w, v[i][4] = b.x, v[i][5] = b.y, v[i][6] = b.z, v[i][7] = b.w;
   }
-  squares = 0.f;
-  if (norm) {
-    float sum[ROWS];
+  if (norm.weight) {
+    constexpr int kBlocks = kGemvNormK / 256;
+    float sum[ROWS];  // of sub-block j, quarter t: lane 4 j + t of the other kernel
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i)
+      sum[i] = square_sum(make_float4(v[i][0], v[i][1], v[i][2], v[i][3]), make_float4(v[i][4], v[i][5], v[i][6], v[i][7]));
+    // j = kShare * i + g / ROWS: the bits of i are the upper ones of j
+#pragma unroll
+    for (int step = ROWS / 2; step; step /= 2)
+#pragma unroll
+      for (int i = 0; i < step; ++i)
+        sum[i] += sum[i + step];
+#pragma unroll
+    for (int lanes = 16; lanes; lanes /= 2)
+      if (lanes < 4 || lanes >= 4 * ROWS)
+        sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], lanes);
+    if (t == 0 && g < ROWS)
+      norm.squares[norm.block * kImageRows + g] = sum[0];
+    named_barrier(1, kBlocks * kWarp);
+    float total = 0.f;
+#pragma unroll
+    for (int b = 0; b < kBlocks; ++b)
+      total += norm.squares[b * kImageRows + row];
+    const float scale = rsqrtf(total / float(kGemvNormK) + 1.0e-6f);
 #pragma unroll
     for (int i = 0; i < ROWS; ++i) {
-      sum[i] = ((v[i][0] * v[i][0] + v[i][1] * v[i][1]) + (v[i][2] * v[i][2] + v[i][3] * v[i][3])) +
-               ((v[i][4] * v[i][4] + v[i][5] * v[i][5]) + (v[i][6] * v[i][6] + v[i][7] * v[i][7]));
-      const float* weight = norm + (kShare * i + g / ROWS) * 32 + t * 8;
-      const float4 a = *reinterpret_cast<const float4*>(weight), b = *reinterpret_cast<const float4*>(weight + 4);
-      v[i][0] *= a.x, v[i][1] *= a.y, v[i][2] *= a.z, v[i][3] *= a.w, v[i][4] *= b.x, v[i][5] *= b.y, v[i][6] *= b.z, v[i][7] *= b.w;
+      const int at = norm.block * 256 + (kShare * i + g / ROWS) * 32 + t * 8;
+      const float4 a = *reinterpret_cast<const float4*>(norm.weight + at), b = *reinterpret_cast<const float4*>(norm.weight + at + 4);
+      v[i][0] = v[i][0] * scale * a.x, v[i][1] = v[i][1] * scale * a.y, v[i][2] = v[i][2] * scale * a.z, v[i][3] = v[i][3] * scale * a.w;
+      v[i][4] = v[i][4] * scale * b.x, v[i][5] = v[i][5] * scale * b.y, v[i][6] = v[i][6] * scale * b.z, v[i][7] = v[i][7] * scale * b.w;
+      if (norm.normalised && row < m) {
+        float4* to = reinterpret_cast<float4*>(norm.normalised + size_t(row) * kGemvNormK + at);
+        to[0] = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]), to[1] = make_float4(v[i][4], v[i][5], v[i][6], v[i][7]);
+      }
     }
-    // a tree over the sub-blocks, those of other lanes first, then the quarters
-#pragma unroll
-    for (int lanes = 4 * ROWS; lanes < 32; lanes *= 2)
-#pragma unroll
-      for (int i = 0; i < ROWS; ++i)
-        sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], lanes);
-#pragma unroll
-    for (int step = 1; step < ROWS; step *= 2)
-#pragma unroll
-      for (int i = 0; i + step < ROWS; i += 2 * step)
-        sum[i] += sum[i + step];
-    squares = sum[0] + __shfl_xor_sync(0xffffffffu, sum[0], 1);
-    squares += __shfl_xor_sync(0xffffffffu, squares, 2);
   }
   float amax = 0.f, finite = 0.f;
 #pragma unroll
@@ -171,40 +190,6 @@ template <int ROWS> __device__ __forceinline__ Fragments quantize_fragments(cons
   f.scales.x = __float_as_uint(__shfl_sync(0xffffffffu, xs, (2 * t % ROWS) * 4));
   f.scales.y = __float_as_uint(__shfl_sync(0xffffffffu, xs, ((2 * t + 1) % ROWS) * 4));
   return f;
-}
-
-// Turns the fragments of x * norm into those of the row's RMS norm, for the 16 consumer warps that hold a row of 4096 between them:
-// squares is what quantize_fragments found, squaresOfBlock their shared [super-block][row]. One warp of the launch stores the
-// normalised super-block where `normalised` is not null.
-template <int ROWS>
-__device__ __forceinline__ void normalise_fragments(Fragments& f, float squares, float* squaresOfBlock, int block, int m, const float* x, int ldx, const float* norm,
-                                                    float* normalised, int lane) {
-  constexpr int kBlocks = kGemvNormK / 256;
-  const int g = lane >> 2, t = lane & 3;
-  if (t == 0 && g < ROWS)
-    squaresOfBlock[block * kImageRows + g] = squares;
-  named_barrier(1, kBlocks * kWarp);
-  float scale[2] = {0.f, 0.f};  // of the rows of columns 2t and 2t + 1
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {
-#pragma unroll
-    for (int b = 0; b < kBlocks; ++b)
-      scale[r] += squaresOfBlock[b * kImageRows + (2 * t + r) % ROWS];
-    scale[r] = rsqrtf(scale[r] / float(kGemvNormK) + 1.0e-6f);
-  }
-  f.scales.x = __float_as_uint(__uint_as_float(f.scales.x) * scale[0]);
-  f.scales.y = __float_as_uint(__uint_as_float(f.scales.y) * scale[1]);
-  if (normalised)
-    for (int row = 0; row < m; ++row) {
-      const float mine = __shfl_sync(0xffffffffu, row & 1 ? scale[1] : scale[0], row % ROWS >> 1);
-      const size_t at = size_t(block) * 256 + lane * 8;
-#pragma unroll
-      for (int e = 0; e < 8; e += 4) {
-        const float4 a = *reinterpret_cast<const float4*>(x + size_t(row) * ldx + at + e), w = *reinterpret_cast<const float4*>(norm + at + e);
-        *reinterpret_cast<float4*>(normalised + size_t(row) * kGemvNormK + at + e) =
-            make_float4(a.x * mine * w.x, a.y * mine * w.y, a.z * mine * w.z, a.w * mine * w.w);
-      }
-    }
 }
 
 // One 16-row x 256-k unit. Lane (g, t) owns weight rows g and g+8 (shared-memory addresses pA, pB) and, in each

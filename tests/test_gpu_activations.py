@@ -52,6 +52,10 @@ def test_norm_on_the_way_in(dev, m, n):
   y = linear(dev, w, n, k, x, norm=(dev.array(gain), normalised, True))
   want = oracle.rms_norm(x, gain)
   assert np.abs(normalised.download() - want).max() <= 1e-6 * np.abs(want).max()  # three roundings and a reciprocal root of a sum
+  apart = dev.empty((m, k))
+  dev.rms_norm(dev.array(x), dev.array(gain), m, k, apart)
+  assert normalised.download().tobytes() == apart.download().tobytes()
+  assert linear(dev, w, n, k, apart.download()).tobytes() == y.tobytes()
   error = np.linalg.norm(y - oracle.linear(weights, D.Q4_K, n, k, want)) / np.linalg.norm(y)
   assert error <= (1e-4 if m <= 8 else 1e-3)  # the levels of an activation block; fp16 operands above eight rows
   # a row does not depend on the others, nor on whether the normalised rows are stored
