@@ -4,7 +4,7 @@
 //                             reference does inside attention_scan (:126-133)
 // attention_scan_kernel    <- attention_scan   (attention.metal:103-183), row by row: queries of one row, and passes whose
 //                             queries have few rows on average
-// attention_group_kernel   <- the same, for the queries of several rows of the other passes
+// attention_tile_kernel   <- the same, for the queries of several rows of the other passes
 // attention_reduce_kernel  <- attention_reduce (attention.metal:185-216)
 //
 // K/V pool of one layer: [physical block][4 kv heads][blockTokens][256] fp16, so the 16 tokens of a tile of
@@ -20,6 +20,7 @@
 #include <mutex>
 #include "act_image.cuh"
 #include "ops.h"
+#include "tcgen05.cuh"
 
 namespace infdev {
 namespace {
@@ -104,9 +105,9 @@ __device__ __forceinline__ void copy_async16(void* dst, const void* src, uint32_
 // chain of load latencies. Both contractions run on the tensor cores as m16n8k16 with fp16 operands split hi + lo where
 // they are not fp16 already: warp 0 scores the tile's 16 tokens for the four query heads of the group, then warp w
 // accumulates the weighted values of dims 64w .. 64w+63 for all four heads.
-// SINGLES: grid (maxSplits + 1, 4 kv heads, queries), for the queries of one row of a pass whose other queries the group kernel
+// SINGLES: grid (maxSplits + 1, 4 kv heads, queries), for the queries of one row of a pass whose other queries the tile kernel
 // takes, beside that kernel: launched after it and early, it reads nothing that kernel writes and does not wait for it. The
-// group kernel lets it start only after its own wait, so what the kernels before both wrote is there; the fence keeps this
+// tile kernel lets it start only after its own wait, so what the kernels before both wrote is there; the fence keeps this
 // CTA's reads behind. One CTA does wait, so that the end of this kernel still means the end of all before it.
 template <bool SINGLES>
 __global__ void __launch_bounds__(128, 6) attention_scan_kernel(const float* q, const __half* cacheK, const __half* cacheV,
@@ -267,31 +268,48 @@ __global__ void __launch_bounds__(128, 6) attention_scan_kernel(const float* q, 
 
 // ---- rows of one query together: prompt chunks and speculative rows --------------------------------------------------
 // The scan above reads K and V once per row: 128 prompt rows behind 2000 tokens pull 1 GB through the L2 (170 us, and
-// 18 us to merge 32 splits of every row). Here up to 16 consecutive rows of a query share every K/V tile: a CTA holds the
-// 16 rows x 4 query heads of one kv head as 64 rows of the two contractions, and walks its piece of the context in tiles
-// of 64 tokens, softmax online. 8 warps = 4 heads x 2 halves: a warp scores 32 tokens of the tile, hands its weights to
-// its partner through shared memory and accumulates 128 of the 256 value dims for all 64. Operands as in the scan: fp16
-// keys and values, query and softmax weights as fp16 hi + lo, fp32 accumulation.
-// 128 rows behind 1920 tokens are 4.2 G multiply-adds with both halves of q and p, 14 us at the 1016 per clock and SM of
-// mma.sync; the kernel takes about 38, because with two warps a scheduler the products, the fragment reads and the exchange
-// between the halves wait for each other (tensor pipe 42 % of the active cycles, 0.29 issued per cycle and scheduler). In an
-// earlier form sixteen warps instead of eight measured 66 instead of 61 us for the whole call, and two groups of four warps
-// with tiles and softmax of their own, nothing exchanged, the same 61.
+// 18 us to merge 32 splits of every row). Here up to 32 consecutive rows of a query share every K/V tile: the 32 rows x 4 query
+// heads of one kv head are the 128 rows of two tcgen05 contractions. A CTA takes its piece of the context in rounds of up to four
+// tiles of 64 tokens:
+//   * loader warps copy the tiles of K, then those of V, with cp.async into a ring of three 32 KB slots, as 16-byte chunks
+//     [8 dims][token], which is the no-swizzle layout of K as a K-major operand and of V as an MN-major one at once;
+//   * scores of the round: q hi and q lo (fp16, 128 KB of shared memory, laid out once per item) x K into 64 columns of tensor
+//     memory a tile;
+//   * worker warps (a thread has one row, and every second tile) take maximum and weights of the whole round, so there is no
+//     rescaling between tiles, and write the weights as fp16 hi and lo over the scores. Their loops are kept short: most of this code
+//     runs once or a few times in a launch, with thirteen warps at work on different parts of it at once, so instruction fetch counts;
+//   * values: the weights in tensor memory x V into 256 columns. Between rounds the workers rescale them.
+// Operands as in the scan: fp16 keys and values, query and softmax weights as fp16 hi + lo, fp32 accumulation. A tile of 64 tokens is
+// 1.6 k cycles of MMAs for the scores (bounded by shared memory: A and B both come from there) and 1 k for the values; mma.sync,
+// with 16 rows x 4 heads, was 8 k for half the rows.
+// Measured, with the merge, and before, with mma.sync: 128 rows behind 1920 tokens 51.0 -> 32.1 us, four times 30 rows behind up to 1970
+// 49.3 -> 32.4, 2048 rows behind 2048 1070 -> 449; 64 rows of 64 tokens 13.7 -> 16.1: a fixed start of laying out q and an end of
+// reading tensor memory, which little work has to pay for.
 //
 // Work items (tile of rows, piece of context, kv head) are dealt to one CTA per SM; which exist only the device knows, so
 // a CTA finds its next item by a scan over the queries. The pieces of a tile follow from its context and from `most`, which
 // the host sets so that the items of the pass fill the SMs about once; a tile of few rows (speculative rows that share a pass
-// with a prompt) is cut as finely as the caller's scratch allows. Queries of one row are no items: the arithmetic of 16 rows
-// for one made them the longest part of a pass (seven decode rows of 4000 tokens beside a prompt of 121 rows 97 us, 47 with
+// with a prompt) is cut as finely as the caller's scratch allows. Queries of one row are no items: the arithmetic of a whole tile
+// for one row made them the longest part of a pass (seven decode rows of 4000 tokens beside a prompt of 121 rows 97 us, 47 with
 // the scan beside this kernel, 63 with all rows in the scan; seven of 32000 tokens 518, 194 and 198).
-constexpr int kGroupRows = 16, kGroupTokens = 64, kGroupThreads = 256, kGroupPitch = kDim + 8, kWeightPitch = kGroupTokens + 8;
+constexpr int kGroupRows = 32, kGroupTokens = 64, kRoundTiles = 4;
+constexpr int kWorkers = 8, kMmaWarp = kWorkers, kLoaders = 4, kTileThreads = (kWorkers + 1 + kLoaders) * kWarp;  // warps
+constexpr int kSlots = 3, kSlotBytes = kGroupTokens * kDim * 2;
+constexpr int kQueryGroup = kGroup * kGroupRows * 16 + 16, kQueryBytes = kDim / 8 * kQueryGroup;  // 16 bytes more, so that the lanes of a row of q write to different banks
+constexpr int kStagePitch = 36;  // floats of a row of 32 staged results
 
-struct GroupShared {
-  __half q[2][kGroup * kGroupRows][kGroupPitch];                         // hi, lo; row 16 * head + r
-  __half k[2][kGroupTokens][kGroupPitch], v[2][kGroupTokens][kGroupPitch];  // two buffers
-  __half p[2][kGroup * kGroupRows][kWeightPitch];                        // hi, lo
+struct TileShared {
+  uint64_t full[kSlots], slotFree[kSlots], queryReady, scoresReady[kRoundTiles], weightsReady[kRoundTiles], valuesReady, valuesFree, drained;
+  uint32_t tmemBase;
+  int abort;
+  int broken[2];  // by item parity: a value was not finite of a token that some rows do not attend to
   float exchange[2][kGroup * kGroupRows];
 };
+constexpr int kTileControlBytes = 2048;
+static_assert(sizeof(TileShared) <= kTileControlBytes, "control block too large");
+constexpr size_t kTileSharedBytes = kTileControlBytes + 2 * kQueryBytes + kSlots * kSlotBytes;
+static_assert(kTileSharedBytes <= 227 * 1024 && kWorkers * 32 * kStagePitch * 4 <= 2 * kQueryBytes, "shared memory");
+constexpr uint32_t kColScores = 0, kColValues = 256;  // tensor memory: four tiles of 64 score columns, 256 value columns
 
 struct RowTile {
   uint32_t start, rows, first, attended, slot;  // first: position of its first row; attended: context of its last row
@@ -317,67 +335,62 @@ __device__ __forceinline__ uint32_t piece_tokens(uint32_t attended, uint32_t row
 __device__ __forceinline__ uint32_t piece_count(uint32_t attended, uint32_t piece) { return (attended + piece - 1) / piece; }
 
 // Work item `item` of the pass, found by one warp together; false when there are fewer. `items`: how many there are, where one
-// round over the queries tells.
+// round tells. A lane has one tile of rows at a time, whichever query it is of: with a lane per query, which counted its tiles one
+// after the other, this took 2.2 us of the 128 rows of one prompt, most of it the divisions of four tiles in a row.
 __device__ __forceinline__ bool find_item(const infdev_query* queries, int queryCount, uint32_t most, uint32_t maxSplits, uint32_t item, RowTile& tile,
                                           uint32_t& split, uint32_t& piece, uint32_t& items) {
   const uint32_t lane = threadIdx.x & 31;
-  for (int base = 0; base < queryCount; base += 32) {
-    uint32_t mine = 0, tiles = 0;
-    infdev_query query = {};
-    if (base + int(lane) < queryCount) {
-      query = queries[base + lane];
-      tiles = tiles_of(query);
-      for (uint32_t t = 0; t < tiles; ++t) {
-        const RowTile each = tile_of(query, t);
-        mine += piece_count(each.attended, piece_tokens(each.attended, each.rows, most, maxSplits));
-      }
-    }
-    uint32_t inclusive = mine;
+  auto running_sum = [&](uint32_t value) {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t other = __shfl_up_sync(0xffffffffu, inclusive, o);
+      const uint32_t other = __shfl_up_sync(0xffffffffu, value, o);
       if (int(lane) >= o)
-        inclusive += other;
+        value += other;
     }
-    const uint32_t total = __shfl_sync(0xffffffffu, inclusive, 31);
-    items = queryCount <= 32 ? total : 0xffffffffu;
-    if (item >= total) {
-      item -= total;
-      continue;
-    }
-    const int owner = __ffs(__ballot_sync(0xffffffffu, inclusive > item)) - 1;
-    uint32_t found[7] = {};
-    if (int(lane) == owner) {
-      uint32_t local = item - (inclusive - mine);
-      for (uint32_t t = 0; t < tiles; ++t) {
-        const RowTile each = tile_of(query, t);
-        const uint32_t tokens = piece_tokens(each.attended, each.rows, most, maxSplits), count = piece_count(each.attended, tokens);
-        if (local < count) {
-          found[0] = each.start, found[1] = each.rows, found[2] = each.first, found[3] = each.attended, found[4] = each.slot, found[5] = local,
-          found[6] = tokens;
-          break;
-        }
-        local -= count;
-      }
-    }
+    return value;
+  };
+  items = 0xffffffffu;
+  for (int base = 0; base < queryCount; base += 32) {
+    infdev_query query = {};
+    if (base + int(lane) < queryCount)
+      query = queries[base + lane];
+    const uint32_t tilesUpTo = running_sum(tiles_of(query)), tiles = __shfl_sync(0xffffffffu, tilesUpTo, 31);
+    for (uint32_t first = 0; first < tiles; first += 32) {
+      // the query of this lane's tile: how many queries end at or before it
+      const uint32_t mine = first + lane;
+      uint32_t owner = 0;
 #pragma unroll
-    for (int i = 0; i < 7; ++i)
-      found[i] = __shfl_sync(0xffffffffu, found[i], owner);
-    tile = {found[0], found[1], found[2], found[3], found[4]};
-    split = found[5], piece = found[6];
-    return true;
+      for (uint32_t step = 16; step > 0; step >>= 1) {
+        if (__shfl_sync(0xffffffffu, tilesUpTo, owner + step - 1) <= mine)
+          owner += step;
+      }
+      infdev_query whose = {};
+      whose.start = __shfl_sync(0xffffffffu, query.start, owner), whose.count = __shfl_sync(0xffffffffu, query.count, owner);
+      whose.position = __shfl_sync(0xffffffffu, query.position, owner), whose.slot = __shfl_sync(0xffffffffu, query.slot, owner);
+      const uint32_t before = __shfl_sync(0xffffffffu, tilesUpTo - tiles_of(query), owner);
+      RowTile each = {};
+      uint32_t tokens = 0, count = 0;
+      if (mine < tiles) {
+        each = tile_of(whose, mine - before);
+        tokens = piece_tokens(each.attended, each.rows, most, maxSplits), count = piece_count(each.attended, tokens);
+      }
+      const uint32_t inclusive = running_sum(count), total = __shfl_sync(0xffffffffu, inclusive, 31);
+      if (queryCount <= 32 && tiles <= 32)
+        items = total;
+      if (item >= total) {
+        item -= total;
+        continue;
+      }
+      const int holder = __ffs(__ballot_sync(0xffffffffu, inclusive > item)) - 1;
+      tile = {__shfl_sync(0xffffffffu, each.start, holder), __shfl_sync(0xffffffffu, each.rows, holder), __shfl_sync(0xffffffffu, each.first, holder),
+              __shfl_sync(0xffffffffu, each.attended, holder), __shfl_sync(0xffffffffu, each.slot, holder)};
+      split = item - __shfl_sync(0xffffffffu, inclusive - count, holder), piece = __shfl_sync(0xffffffffu, tokens, holder);
+      return true;
+    }
   }
   return false;
 }
 
-__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const __half* address) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(address)));
-}
-__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], const __half* address) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(smem_u32(address)));
-}
 // {a, b} as fp16 hi and lo pairs
 __device__ __forceinline__ uint2 split_pair(float a, float b) {
   const uint32_t hi = pack_half2(a, b);
@@ -388,200 +401,364 @@ __device__ __forceinline__ uint2 split_pair(float a, float b) {
 // 0x8000 in each half of `pair` that is an infinity or a NaN.
 __device__ __forceinline__ uint32_t not_finite(uint32_t pair) { return ((pair & 0x7c007c00u) + 0x04000400u) & 0x80008000u; }
 
-__global__ void __launch_bounds__(kGroupThreads, 1)
-    attention_group_kernel(const float* q, const __half* cacheK, const __half* cacheV, const infdev_query* queries, int queryCount, const int32_t* table,
-                           int tableStride, int blockTokens, uint32_t most, uint32_t maxSplits, float* partials) {
+__device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+__global__ void __launch_bounds__(kTileThreads, 1)
+    attention_tile_kernel(const float* q, const __half* cacheK, const __half* cacheV, const infdev_query* queries, int queryCount, const int32_t* table,
+                          int tableStride, int blockTokens, uint32_t most, uint32_t maxSplits, float* partials, int* status) {
   pdl_wait();  // first: the scan of the queries of one row starts beside this kernel and relies on it
   pdl_launch_dependents();
-  extern __shared__ __align__(16) uint8_t groupRaw[];
-  GroupShared& sh = *reinterpret_cast<GroupShared*>(groupRaw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, head = warp & 3, half = warp >> 2, g = lane >> 2, t = lane & 3;
-  const int rowBase = head * kGroupRows;  // this warp's 16 rows of q, p and exchange
+  extern __shared__ __align__(128) uint8_t tileRaw[];
+  TileShared& sh = *reinterpret_cast<TileShared*>(tileRaw);
+  uint8_t* const query = tileRaw + kTileControlBytes;  // [hi, lo][8 dims][row] of 16 bytes, row = 32 * head + r, 8 dims kQueryGroup apart
+  uint8_t* const ring = query + 2 * kQueryBytes;       // [slot][8 dims][token] of 16 bytes
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  volatile int* abortFlag = &sh.abort;
+  if (tid == 0) {
+    for (int s = 0; s < kSlots; ++s) {
+      mbar_init(&sh.full[s], kLoaders * kWarp);
+      mbar_init(&sh.slotFree[s], 1);
+    }
+    mbar_init(&sh.queryReady, kWorkers);
+    for (int j = 0; j < kRoundTiles; ++j) {
+      mbar_init(&sh.scoresReady[j], 1);
+      mbar_init(&sh.weightsReady[j], kWorkers);
+    }
+    mbar_init(&sh.valuesReady, 1);
+    mbar_init(&sh.valuesFree, kWorkers);
+    mbar_init(&sh.drained, 1);
+    sh.abort = sh.broken[0] = sh.broken[1] = 0;
+    mbar_fence_init();
+  }
+  if (warp == kMmaWarp)
+    tmem_alloc(&sh.tmemBase, 512);
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = sh.tmemBase;
+  bool ok = true;
   RowTile tile;
-  uint32_t split, piece, items = 0xffffffffu;
-  for (uint32_t item = blockIdx.x;
-       item / kKvHeads < items && find_item(queries, queryCount, most, maxSplits, item / kKvHeads, tile, split, piece, items); item += gridDim.x) {
-    const uint32_t kvHead = item % kKvHeads, begin = split * piece, end = min(tile.attended, begin + piece);
-    const int32_t* slotTable = table + size_t(tile.slot) * tableStride;
-    auto fetch = [&](uint32_t from, int buffer) {  // a warp copies one token's 512 bytes at a time
-#pragma unroll
-      for (int c = 0; c < kGroupTokens / 8; ++c) {
-        const uint32_t token = c * 8 + warp, at = min(from + token, end - 1);
-        const uint32_t bytes = from + token < end ? 16u : 0u;  // zeros past the end
-        const size_t base = ((size_t(slotTable[at / blockTokens]) * kKvHeads + kvHead) * blockTokens + at % blockTokens) * kDim + lane * 8;
-        copy_async16(&sh.k[buffer][token][lane * 8], cacheK + base, bytes);
-        copy_async16(&sh.v[buffer][token][lane * 8], cacheV + base, bytes);
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    __syncthreads();  // the item before this one is finished with the shared arrays
-    // the 16 rows x 4 heads of q, hi and lo; rows past the tile's are zero. All loads are in flight before the first is used.
-    constexpr int kQuads = kGroup * kGroupRows * (kDim / 4) / kGroupThreads;
-    float4 value[kQuads];
-#pragma unroll
-    for (int i = 0; i < kQuads; ++i) {
-      const int at = i * kGroupThreads + threadIdx.x, row = at / (kDim / 4), d = at % (kDim / 4) * 4, r = row % kGroupRows, h = row / kGroupRows;
-      value[i] = r < int(tile.rows) ? *reinterpret_cast<const float4*>(q + (size_t(tile.start + r) * kQHeads + kvHead * kGroup + h) * kDim + d)
-                                    : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    fetch(begin, 0);
-#pragma unroll
-    for (int i = 0; i < kQuads; ++i) {
-      const int at = i * kGroupThreads + threadIdx.x, row = at / (kDim / 4), d = at % (kDim / 4) * 4;
-      const uint2 a = split_pair(value[i].x, value[i].y), b = split_pair(value[i].z, value[i].w);
-      *reinterpret_cast<uint2*>(&sh.q[0][row][d]) = make_uint2(a.x, b.x);
-      *reinterpret_cast<uint2*>(&sh.q[1][row][d]) = make_uint2(a.y, b.y);
-    }
-    float maximum[2] = {-1.0e30f, -1.0e30f}, norm[2] = {0.f, 0.f}, acc[16][4];  // rows g and g + 8
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-    int buffer = 0;
-    for (uint32_t from = begin; from < end; from += kGroupTokens, buffer ^= 1) {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-      __syncthreads();  // the tile has landed, and everybody is done with the one before
-      if (from + kGroupTokens < end)
-        fetch(from + kGroupTokens, buffer ^ 1);
-      float score[4][4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        score[j][0] = score[j][1] = score[j][2] = score[j][3] = 0.f;
-#pragma unroll
-      for (int step = 0; step < kDim / 16; ++step) {
-        uint32_t hi[4], lo[4];
-        ldmatrix4(hi, &sh.q[0][rowBase + (lane & 15)][16 * step + 8 * (lane >> 4)]);
-        ldmatrix4(lo, &sh.q[1][rowBase + (lane & 15)][16 * step + 8 * (lane >> 4)]);
-#pragma unroll
-        for (int pair = 0; pair < 2; ++pair) {
-          if (from + 32 * half + 16 * pair >= end)  // past the piece: these scores are masked below
+  uint32_t split, piece, items = 0xffffffffu, itemCount = 0, roundCount = 0;
+  auto next_item = [&](uint32_t item) {
+    return item / kKvHeads < items && find_item(queries, queryCount, most, maxSplits, item / kKvHeads, tile, split, piece, items);
+  };
+  auto tiles_in_round = [](uint32_t from, uint32_t end) { return min(uint32_t(kRoundTiles), (end - from + kGroupTokens - 1) / kGroupTokens); };
+  constexpr uint32_t kRoundTokens = kRoundTiles * kGroupTokens;
+
+  if (warp > kMmaWarp) {
+    // ---------------- loaders: the K tiles of a round, then its V tiles ----------------
+    const int loader = warp - kMmaWarp - 1;
+    uint32_t count = 0;    // tiles asked for
+    bool pending = false;  // the last of them has not been handed over yet
+    uint32_t pendingMasked = 0, pendingPast = 0, pendingParity = 0;  // V: its tokens [masked, past) are masked for some rows
+    const uint32_t blockShift = blockTokens & (blockTokens - 1) ? 32u : uint32_t(__ffs(blockTokens) - 1);  // 32: not a power of two
+    const uint32_t chunkOffset = (4 * loader + (lane >> 3)) * (kGroupTokens * 16) + (lane & 7) * 16;
+    auto hand_over = [&] {  // this thread's part of the pending tile has landed
+      uint8_t* slot = ring + (count - 1) % kSlots * kSlotBytes + chunkOffset;
+      if (pendingMasked < pendingPast) {
+        // A value that is not finite, of a token that some rows of the tile do not attend to, times their weights of zero would
+        // reach them: it stands as zero, and the rows that do attend to it get NaN at the end.
+        bool bad = false;
+        for (int c = 0; c < 16; ++c) {
+          const uint32_t token = (c & 7) * 8 + (lane & 7);
+          if (token < pendingMasked || token >= pendingPast)
             continue;
-          uint32_t b[4];
-          ldmatrix4(b, &sh.k[buffer][32 * half + 16 * pair + 8 * (lane >> 4) + (lane & 7)][16 * step + 8 * ((lane >> 3) & 1)]);
-          mma_16816(score[2 * pair], hi, b[0], b[1]);
-          mma_16816(score[2 * pair + 1], hi, b[2], b[3]);
-          mma_16816(score[2 * pair], lo, b[0], b[1]);
-          mma_16816(score[2 * pair + 1], lo, b[2], b[3]);
-        }
-      }
-      // scale, causal mask, row maxima over both halves of the tile
-      float best[2] = {-INFINITY, -INFINITY};
+          uint4* at = reinterpret_cast<uint4*>(slot + (c >> 3) * (16 * kGroupTokens * 16) + (c & 7) * 128);
+          const uint4 v = *at;
+          uint32_t words[4] = {v.x, v.y, v.z, v.w}, found = 0;
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint32_t token = from + 32 * half + 8 * j + 2 * t + (i & 1), limit = min(end, tile.first + g + 8 * (i >> 1) + 1);
-          score[j][i] = token < limit ? score[j][i] * (1.0f / 16.0f) : -INFINITY;
-          best[i >> 1] = fmaxf(best[i >> 1], score[j][i]);
-        }
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        best[r] = fmaxf(best[r], __shfl_xor_sync(0xffffffffu, best[r], 1));
-        best[r] = fmaxf(best[r], __shfl_xor_sync(0xffffffffu, best[r], 2));
-        if (t == 0)
-          sh.exchange[half][rowBase + g + 8 * r] = best[r];
-      }
-      named_barrier(1 + head, 64);
-      float rescale[2];
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const float next = fmaxf(maximum[r], fmaxf(best[r], sh.exchange[half ^ 1][rowBase + g + 8 * r]));
-        rescale[r] = expf(maximum[r] - next);
-        maximum[r] = next;
-        norm[r] *= rescale[r];
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          const float w0 = expf(score[j][2 * r] - maximum[r]), w1 = expf(score[j][2 * r + 1] - maximum[r]);
-          norm[r] += w0 + w1;
-          const uint2 w = split_pair(w0, w1);
-          *reinterpret_cast<uint32_t*>(&sh.p[0][rowBase + g + 8 * r][32 * half + 8 * j + 2 * t]) = w.x;
-          *reinterpret_cast<uint32_t*>(&sh.p[1][rowBase + g + 8 * r][32 * half + 8 * j + 2 * t]) = w.y;
-        }
-      // A value that is not finite, of a token that some rows of the tile do not attend to, times their weights of zero would
-      // reach them: in such a tile it stands as zero, and the rows that do attend to it get NaN afterwards. (128 rows behind 1920
-      // tokens 55.4 -> 56.3 us with the test; a test within the loop of products 58.)
-      const uint32_t masked = max(from, tile.first + 1), past = min(from + kGroupTokens, end);
-      uint32_t broken = 0;
-      for (uint32_t token = masked; token < past; ++token) {
-        const uint2 four = *reinterpret_cast<const uint2*>(&sh.v[buffer][token - from][128 * half + 4 * lane]);
-        broken |= not_finite(four.x) | not_finite(four.y);
-      }
-      broken = __any_sync(0xffffffffu, broken != 0);
-      named_barrier(1 + head, 64);  // both halves of the weights are there
-#pragma unroll
-      for (int j = 0; j < 16; ++j)
-        acc[j][0] *= rescale[0], acc[j][1] *= rescale[0], acc[j][2] *= rescale[1], acc[j][3] *= rescale[1];
-      auto add_values = [&](int step, bool clean) {
-        uint32_t hi[4], lo[4];
-        ldmatrix4(hi, &sh.p[0][rowBase + (lane & 15)][16 * step + 8 * (lane >> 4)]);
-        ldmatrix4(lo, &sh.p[1][rowBase + (lane & 15)][16 * step + 8 * (lane >> 4)]);
-#pragma unroll
-        for (int pair = 0; pair < 8; ++pair) {
-          uint32_t b[4];
-          ldmatrix4_trans(b, &sh.v[buffer][16 * step + (lane & 15)][128 * half + 16 * pair + 8 * (lane >> 4)]);
-          if (clean) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              b[i] &= ~((not_finite(b[i]) >> 15) * 0xffffu);
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t mask = not_finite(words[i]);
+            found |= mask;
+            words[i] &= ~((mask >> 15) * 0xffffu);
           }
-          mma_16816(acc[2 * pair], hi, b[0], b[1]);
-          mma_16816(acc[2 * pair + 1], hi, b[2], b[3]);
-          mma_16816(acc[2 * pair], lo, b[0], b[1]);
-          mma_16816(acc[2 * pair + 1], lo, b[2], b[3]);
+          if (found)
+            *at = make_uint4(words[0], words[1], words[2], words[3]), bad = true;
         }
-      };
-      if (!broken) {
-#pragma unroll
-        for (int step = 0; step < kGroupTokens / 16; ++step) {
-          if (from + 16 * step >= end)  // weights of zero
-            break;
-          add_values(step, false);
-        }
-      } else {
-#pragma unroll 1
-        for (int step = 0; step < kGroupTokens / 16; ++step)
-          add_values(step, true);
-#pragma unroll 1
-        for (uint32_t token = from; token < past; ++token)
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const uint32_t bad = not_finite(*reinterpret_cast<const uint32_t*>(&sh.v[buffer][token - from][128 * half + 8 * j + 2 * t]));
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              if ((bad & (i & 1 ? 0x80000000u : 0x8000u)) && token <= tile.first + g + 8 * (i >> 1))
-                acc[j][i] = NAN;
+        if (bad)
+          *reinterpret_cast<volatile int*>(&sh.broken[pendingParity]) = 1;
+      }
+      fence_async_proxy();
+      mbar_arrive(&sh.full[(count - 1) % kSlots]);
+      pending = false;
+    };
+    for (uint32_t item = blockIdx.x; ok && next_item(item); item += gridDim.x, ++itemCount) {
+      const uint32_t kvHead = item % kKvHeads, begin = split * piece, end = min(tile.attended, begin + piece);
+      const int32_t* slotTable = table + size_t(tile.slot) * tableStride;
+      for (uint32_t from = begin; ok && from < end; from += kRoundTokens) {
+        const uint32_t tiles = tiles_in_round(from, end);
+        for (uint32_t j = 0; ok && j < 2 * tiles; ++j) {
+          const bool values = j >= tiles;
+          const uint32_t first = from + (values ? j - tiles : j) * kGroupTokens, slot = count % kSlots;
+          if (count >= uint32_t(kSlots)) {
+            const uint32_t parity = (count / kSlots - 1) & 1;
+            if (pending && !__all_sync(0xffffffffu, mbar_test_wait(&sh.slotFree[slot], parity))) {  // not while what may free it is held back
+              asm volatile("cp.async.wait_group 0;" ::: "memory");
+              hand_over();
+            }
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&sh.slotFree[slot], parity, abortFlag));
+            if (!ok)
+              break;
           }
+          const __half* cache = (values ? cacheV : cacheK) + (lane >> 3) * 8 + loader * 32;
+          uint8_t* to = ring + slot * kSlotBytes + chunkOffset;
+#pragma unroll 4
+          for (int c = 0; c < 8; ++c) {  // eight tokens x four groups of eight dims, twice
+            const uint32_t token = first + c * 8 + (lane & 7), at = min(token, end - 1);
+            const uint32_t bytes = token < end ? 16u : 0u;  // zeros past the end
+            const uint32_t block = blockShift < 32 ? at >> blockShift : at / blockTokens;
+            const __half* source = cache + ((size_t(slotTable[block]) * kKvHeads + kvHead) * blockTokens + (at - block * blockTokens)) * kDim;
+            copy_async16(to + c * 128, source, bytes);
+            copy_async16(to + 16 * kGroupTokens * 16 + c * 128, source + 128, bytes);
+          }
+          asm volatile("cp.async.commit_group;" ::: "memory");
+          if (pending) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            hand_over();
+          }
+          ++count;
+          pending = true;
+          pendingMasked = values && tile.first + 1 > first ? tile.first + 1 - first : 0u;
+          pendingPast = values ? min(uint32_t(kGroupTokens), end - first) : 0u;
+          pendingParity = itemCount & 1;
+        }
       }
     }
-    // the norm over both halves, then this piece's record of every live row
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      norm[r] += __shfl_xor_sync(0xffffffffu, norm[r], 1);
-      norm[r] += __shfl_xor_sync(0xffffffffu, norm[r], 2);
-      if (t == 0)
-        sh.exchange[half][rowBase + g + 8 * r] = norm[r];
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (pending)
+      hand_over();
+  } else if (warp == kMmaWarp) {
+    // ---------------- MMA issuer ----------------
+    constexpr uint32_t kScores = (1u << 4) | (uint32_t(kGroupTokens >> 3) << 17) | (8u << 24);       // fp16 x fp16 -> fp32, M 128, N 64, both K-major
+    constexpr uint32_t kValues = (1u << 4) | (1u << 16) | (uint32_t(kDim >> 3) << 17) | (8u << 24);  // N 256, B MN-major
+    constexpr uint32_t kQueryStep = 2 * kQueryGroup, kTokenStep = 2 * kGroupTokens * 16;  // 16 dims of q and of K
+    const uint32_t queryBase = smem_u32(query);
+    uint32_t count = 0, weightPhases = 0;
+    for (uint32_t item = blockIdx.x; ok && next_item(item); item += gridDim.x, ++itemCount) {
+      const uint32_t begin = split * piece, end = min(tile.attended, begin + piece);
+      for (uint32_t from = begin; ok && from < end; from += kRoundTokens, ++roundCount) {
+        const uint32_t tiles = tiles_in_round(from, end);
+        if (elect_one()) {
+          if (from == begin)
+            ok = mbar_wait_bounded(&sh.queryReady, itemCount & 1, abortFlag);
+          else  // the round before has read its weights, whose columns the scores take now
+            ok = mbar_wait_bounded(&sh.valuesReady, (roundCount - 1) & 1, abortFlag);
+          for (uint32_t j = 0; ok && j < tiles; ++j) {
+            const uint32_t n = count + j, slot = n % kSlots, base = smem_u32(ring + slot * kSlotBytes);
+            ok = mbar_wait_bounded(&sh.full[slot], (n / kSlots) & 1, abortFlag);
+            if (!ok)
+              break;
+            fence_after_sync();
+#pragma unroll 2
+            for (uint32_t step = 0; step < kDim / 16; ++step) {
+              const uint64_t keys = smem_descriptor(base + step * kTokenStep, kTokenStep / 2, 128);
+              umma_ss(tmem + kColScores + j * 64, smem_descriptor(queryBase + step * kQueryStep, kQueryStep / 2, 128), keys, kScores, step != 0);
+              umma_ss(tmem + kColScores + j * 64, smem_descriptor(queryBase + kQueryBytes + step * kQueryStep, kQueryStep / 2, 128), keys, kScores, 1);
+            }
+            umma_commit(&sh.slotFree[slot]);
+            umma_commit(&sh.scoresReady[j]);
+          }
+          if (ok && from == begin && itemCount > 0)  // the workers have read the values of the item before
+            ok = mbar_wait_bounded(&sh.valuesFree, (itemCount - 1) & 1, abortFlag);
+          for (uint32_t j = 0; ok && j < tiles; ++j) {
+            const uint32_t n = count + tiles + j, slot = n % kSlots, base = smem_u32(ring + slot * kSlotBytes);
+            ok = mbar_wait_bounded(&sh.full[slot], (n / kSlots) & 1, abortFlag) &&
+                 mbar_wait_bounded(&sh.weightsReady[j], (weightPhases >> j) & 1, abortFlag);
+            if (!ok)
+              break;
+            fence_after_sync();
+#pragma unroll 2
+            for (uint32_t step = 0; step < kGroupTokens / 16; ++step) {
+              const uint64_t values = smem_descriptor(base + step * 256, 128, kGroupTokens * 16);
+              umma_ts(tmem + kColValues, tmem + kColScores + j * 64 + step * 16, values, kValues, from != begin || j != 0 || step != 0);
+              umma_ts(tmem + kColValues, tmem + kColScores + j * 64 + step * 16 + 8, values, kValues, 1);
+            }
+            umma_commit(&sh.slotFree[slot]);
+          }
+          if (ok)
+            umma_commit(&sh.valuesReady);
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        count += 2 * tiles;
+        weightPhases ^= (1u << tiles) - 1;
+      }
     }
-    named_barrier(1 + head, 64);
+    if (elect_one()) {  // no product may be under way when the CTA ends, whoever gave up
+      umma_commit(&sh.drained);
+      mbar_wait_bounded(&sh.drained, 0, abortFlag);
+    }
+  } else {
+    // ---------------- workers: rows of q, softmax, results ----------------
+    const int quadrant = warp & 3, side = warp >> 2;  // head; the tiles side, side + 2 and value columns 128 side .. 128 side + 127
+    const int row = quadrant * 32 + lane;
+    const uint32_t laneBase = tmem + (uint32_t(quadrant * 32) << 16);
+    uint32_t scorePhases = 0;
+    // Nobody leaves a loop early: the named barriers have no time limit, so who gave up goes on without waiting for the others.
+    auto wait = [&](uint64_t* bar, uint32_t parity) { ok = __all_sync(0xffffffffu, ok && mbar_wait_bounded(bar, parity, abortFlag)); };
+    for (uint32_t item = blockIdx.x; next_item(item); item += gridDim.x, ++itemCount) {
+      const uint32_t kvHead = item % kKvHeads, begin = split * piece, end = min(tile.attended, begin + piece);
+      named_barrier(5, kWorkers * kWarp);  // the item before is done with the shared memory of q, which its results were staged in
+      if (tid == 0)
+        sh.broken[(itemCount + 1) & 1] = 0;  // of the item before; the next one of that parity has no V tile yet
+      // A warp takes half of a head's 32 rows, eight at a time, a lane eight dims of each: whole rows of 1 KB. Rows past the tile's are zero.
+#pragma unroll 1
+      for (int r0 = (warp & 1) * 16; r0 < (warp & 1) * 16 + 16; r0 += 8) {
+        const int head = warp >> 1;
+        const float* from = q + ((size_t(tile.start) + r0) * kQHeads + kvHead * kGroup + head) * kDim + lane * 8;
+        float4 value[8][2];
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      const uint32_t row = g + 8 * r;
-      if (row >= tile.rows)
-        continue;
-      float* record = partials + ((size_t(tile.start + row) * kQHeads + kvHead * kGroup + head) * maxSplits + split) * kPartialStride;
+        for (int r = 0; r < 8; ++r) {
+          value[r][0] = value[r][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (r0 + r < int(tile.rows)) {
+            const float4* src = reinterpret_cast<const float4*>(from + size_t(r) * kQHeads * kDim);
+            value[r][0] = src[0], value[r][1] = src[1];
+          }
+        }
+        uint8_t* const to = query + lane * kQueryGroup + (head * kGroupRows + r0) * 16;
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        *reinterpret_cast<float2*>(record + 128 * half + 8 * j + 2 * t) = make_float2(acc[j][2 * r], acc[j][2 * r + 1]);
-      if (half == 0 && t == 0)
-        *reinterpret_cast<float2*>(record + kDim) = make_float2(maximum[r], sh.exchange[0][rowBase + row] + sh.exchange[1][rowBase + row]);
+        for (int r = 0; r < 8; ++r) {
+          const float4 a = value[r][0], b = value[r][1];
+          const uint2 s0 = split_pair(a.x, a.y), s1 = split_pair(a.z, a.w), s2 = split_pair(b.x, b.y), s3 = split_pair(b.z, b.w);
+          *reinterpret_cast<uint4*>(to + r * 16) = make_uint4(s0.x, s1.x, s2.x, s3.x);
+          *reinterpret_cast<uint4*>(to + r * 16 + kQueryBytes) = make_uint4(s0.y, s1.y, s2.y, s3.y);
+        }
+      }
+      fence_async_proxy();
+      __syncwarp();
+      if (lane == 0)
+        mbar_arrive(&sh.queryReady);
+      float maximum = -1.0e30f, norm = 0.f;
+      const uint32_t limit = min(end, tile.first + lane + 1);  // this row's scores from here on are masked
+      for (uint32_t from = begin; from < end; from += kRoundTokens, ++roundCount) {
+        const uint32_t tiles = tiles_in_round(from, end);
+        float best = -INFINITY;
+        for (uint32_t j = side; j < tiles; j += 2) {
+          wait(&sh.scoresReady[j], (scorePhases >> j) & 1);
+          fence_after_sync();
+          const uint32_t first = from + j * kGroupTokens, live = limit > first ? limit - first : 0u;
+#pragma unroll 1
+          for (uint32_t c = 0; c < kGroupTokens; c += 16) {
+            uint32_t score[16];
+            tmem_load16(laneBase + kColScores + j * 64 + c, score);
+            tmem_wait_load();
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              best = fmaxf(best, c + i < live ? __uint_as_float(score[i]) * (1.0f / 16.0f) : -INFINITY);
+          }
+        }
+        sh.exchange[side][row] = best;
+        named_barrier(1 + quadrant, 64);
+        const float next = fmaxf(maximum, fmaxf(best, sh.exchange[side ^ 1][row])), rescale = expf(maximum - next);
+        maximum = next, norm *= rescale;
+        if (from != begin) {  // the values so far are of the maximum so far
+          wait(&sh.valuesReady, (roundCount - 1) & 1);
+          fence_after_sync();
+#pragma unroll 1
+          for (int c = 0; c < 8; ++c) {
+            uint32_t v[16];
+            tmem_load16(laneBase + kColValues + side * 128 + c * 16, v);
+            tmem_wait_load();
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              v[i] = __float_as_uint(__uint_as_float(v[i]) * rescale);
+            tmem_store16(laneBase + kColValues + side * 128 + c * 16, v);
+          }
+          tmem_wait_store();
+        }
+        for (uint32_t j = 0; j < tiles; ++j) {
+          if (int(j & 1) == side) {
+            const uint32_t first = from + j * kGroupTokens, live = limit > first ? limit - first : 0u;
+#pragma unroll 1
+            for (uint32_t c = 0; c < kGroupTokens; c += 16) {  // the halves of 16 weights take the columns of their scores
+              uint32_t score[16], halves[16];
+              tmem_load16(laneBase + kColScores + j * 64 + c, score);
+              tmem_wait_load();
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                // the mask before the exponential, which would be branched around otherwise
+                const float s0 = c + 2 * i < live ? __uint_as_float(score[2 * i]) * (1.0f / 16.0f) : -INFINITY;
+                const float s1 = c + 2 * i + 1 < live ? __uint_as_float(score[2 * i + 1]) * (1.0f / 16.0f) : -INFINITY;
+                const float w0 = expf(s0 - maximum), w1 = expf(s1 - maximum);
+                norm += w0 + w1;
+                const uint2 w = split_pair(w0, w1);
+                halves[i] = w.x, halves[8 + i] = w.y;
+              }
+              tmem_store16(laneBase + kColScores + j * 64 + c, halves);
+            }
+            tmem_wait_store();
+          }
+          fence_before_sync();
+          __syncwarp();
+          if (lane == 0)
+            mbar_arrive(&sh.weightsReady[j]);
+        }
+        scorePhases ^= (1u << tiles) - 1;
+        named_barrier(1 + quadrant, 64);  // both sides have read the exchange
+      }
+      // the norm over both sides' tiles, then this piece's record of every live row
+      sh.exchange[side][row] = norm;
+      named_barrier(1 + quadrant, 64);
+      norm = sh.exchange[0][row] + sh.exchange[1][row];
+      wait(&sh.valuesReady, (roundCount - 1) & 1);
+      fence_after_sync();
+      const bool broken = *reinterpret_cast<volatile int*>(&sh.broken[itemCount & 1]) != 0;
+      const size_t headPitch = size_t(maxSplits) * kPartialStride;
+      float* const records = partials + ((size_t(tile.start) * kQHeads + kvHead * kGroup + quadrant) * maxSplits + split) * kPartialStride;
+      float* const stage = reinterpret_cast<float*>(query) + warp * 32 * kStagePitch;
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c) {
+        const int column = side * 128 + c * 32;
+#pragma unroll 1
+        for (int half = 0; half < 32; half += 16) {
+          uint32_t v[16];
+          tmem_load16(laneBase + kColValues + column + half, v);
+          tmem_wait_load();
+          if (broken) {
+            const int32_t* slotTable = table + size_t(tile.slot) * tableStride;
+            for (uint32_t token = max(begin, tile.first + 1); token < limit; ++token) {
+              const __half* source =
+                  cacheV + ((size_t(slotTable[token / blockTokens]) * kKvHeads + kvHead) * blockTokens + token % blockTokens) * kDim + column + half;
+#pragma unroll
+              for (int i = 0; i < 16; ++i)
+                if (not_finite(uint32_t(__half_as_ushort(source[i]))) & 0x8000u)
+                  v[i] = __float_as_uint(NAN);
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 16; i += 4)
+            *reinterpret_cast<uint4*>(stage + lane * kStagePitch + half + i) = make_uint4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+        }
+        __syncwarp();
+#pragma unroll 4
+        for (int step = 0; step < 8; ++step) {  // four rows x 128 bytes a store
+          const int r = step * 4 + (lane >> 3);
+          if (r < int(tile.rows))
+            *reinterpret_cast<float4*>(records + size_t(r) * kQHeads * headPitch + column + (lane & 7) * 4) =
+                *reinterpret_cast<const float4*>(stage + r * kStagePitch + (lane & 7) * 4);
+        }
+        __syncwarp();
+      }
+      if (side == 0 && lane < int(tile.rows))
+        *reinterpret_cast<float2*>(records + size_t(lane) * kQHeads * headPitch + kDim) = make_float2(maximum, norm);
+      fence_before_sync();
+      named_barrier(1 + quadrant, 64);  // both sides have read the exchange
+      if (lane == 0)
+        mbar_arrive(&sh.valuesFree);
     }
   }
+  if (!ok && lane == 0) {
+    *abortFlag = 1;
+    atomicExch(status, kStatusBarrierTimeout);
+  }
+  fence_before_sync();
+  __syncthreads();
+  if (warp == kMmaWarp)
+    tmem_dealloc(tmem, 512);
 }
 
 // grid (rows * 16), 256 threads: merge the splits, normalise, multiply by sigmoid(gate).
 // `image`, when not null, also receives the activation image of the output rows: a head is one 256-value block.
-// GROUPED: the splits of a row whose query has several are those of attention_group_kernel.
+// GROUPED: the splits of a row whose query has several are those of attention_tile_kernel.
 template <bool GROUPED>
 __global__ void __launch_bounds__(256) attention_reduce_kernel(const float* partials, const float* qg, const infdev_query* queries, int queryCount,
                                                                uint32_t most, uint32_t maxSplits, float* out, uint8_t* image) {
@@ -645,35 +822,36 @@ cudaError_t attention_prepare_launch(const float* qg, const float* rawK, const f
 
 cudaError_t attention_launch(const float* q, const float* qg, const void* cacheK, const void* cacheV, const infdev_query* queries,
                              int queryCount, const int32_t* table, int tableStride, int blockTokens, int64_t rows, uint32_t maxSplits, float* partials, float* out,
-                             uint8_t* image, bool rowwise, int sms, cudaStream_t stream, int* launches) {
+                             uint8_t* image, bool rowwise, int sms, int* status, cudaStream_t stream, int* launches) {
   *launches = 0;
   if (rows <= 0)
     return cudaSuccess;
   *launches = 2;
   const uint32_t splits = std::min<uint32_t>(maxSplits, 32);  // the merge keeps one split per lane
-  // The group kernel takes passes whose queries have five rows or more on average, unless no context of the pass can be long
-  // (the table has no room for it): with r rows a query, its longer chain costs 2 us where r x context is below about 4096 (8
-  // rows of 128 tokens 18.7 against 16.7 us for prepare and attention), from there on it is level or faster (8 rows of 2008
-  // tokens 20.8 against 29.1, 16 of 616 22.8 against 23.6, 16 of 2016 22.8 against 39.4, 64 of 128 24.0 against 28.0).
+  // The tile kernel takes passes whose queries have five rows or more on average, unless no context of the pass can be long
+  // (the table has no room for it): with r rows a query, its longer chain costs 2 us and more where r x context is below about 4096;
+  // from there on it is level or faster (64 rows of 64 tokens 16.1 us against 17.8, 64 of 256 18.5 against 22.4, 128 of 128
+  // 18.8 against 29.0, four queries of 20 to 64 rows and as many tokens 19.2 against 29.7; below it 33 rows of 33 tokens 15.7
+  // against 11.7, which only passes of 32 rows a query and more take, whose contexts the host does not know).
   const int64_t capacity = int64_t(tableStride) * blockTokens;
   const bool grouped = rows >= 32 * int64_t(queryCount) || (rows >= 5 * int64_t(queryCount) && rows * capacity >= 4096 * int64_t(queryCount));
-  // The group kernel copies q in pieces of 16 bytes, the scan in pieces of 8.
-  if (grouped && !rowwise && reinterpret_cast<uintptr_t>(q) % 16 == 0) {
+  // The tile kernel copies q and the partial results in pieces of 16 bytes, the scan in pieces of 8 and less.
+  if (grouped && !rowwise && (reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(partials)) % 16 == 0) {
     static PerDeviceOnce configured;
-    if (const cudaError_t e = configure_shared_memory(attention_group_kernel, sizeof(GroupShared), configured))
+    if (const cudaError_t e = configure_shared_memory(attention_tile_kernel, kTileSharedBytes, configured))
       return e;
     const int64_t tiles = std::max<int64_t>((rows + kGroupRows - 1) / kGroupRows, queryCount);
     const uint32_t most = uint32_t(std::clamp<int64_t>(sms / (kKvHeads * tiles), 1, splits));
     const int64_t items = (rows + queryCount) * kKvHeads * splits;  // no more than these
-    launch_kernel<2>(attention_group_kernel, unsigned(std::min<int64_t>(items, sms)), kGroupThreads, sizeof(GroupShared), stream, q,
+    launch_kernel<2>(attention_tile_kernel, unsigned(std::min<int64_t>(items, sms)), kTileThreads, kTileSharedBytes, stream, q,
                   static_cast<const __half*>(cacheK), static_cast<const __half*>(cacheV), queries, queryCount, table, tableStride, blockTokens, most, splits,
-                  partials);
+                  partials, status);
     // Queries of one row stay with the scan, which is faster there: no query rows to share a tile with, and six small CTAs per
-    // SM hide the copies that the group kernel's single CTA waits for. Which queries they are only the device knows; with a
+    // SM hide the copies that the tile kernel's single CTA waits for. Which queries they are only the device knows; with a
     // single query there are none.
     if (queryCount > 1) {
       *launches = 3;
-      // Its CTAs start on the SMs that the group kernel leaves first: shared memory that nobody uses spreads the few of a pass with
+      // Its CTAs start on the SMs that the tile kernel leaves first: shared memory that nobody uses spreads the few of a pass with
       // few queries over all SMs (one row of 32000 tokens beside a prompt: six on an SM 124 us, one 89).
       constexpr size_t kSmShared = 228 * 1024, kScanShared = sizeof(float) * kGroup * kTile + sizeof(__half) * 2 * 2 * kTile * (kDim + 8) + 1024;
       static PerDeviceOnce scanConfigured;

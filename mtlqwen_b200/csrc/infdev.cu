@@ -827,7 +827,7 @@ int infdev_attention(infdev_ctx* ctx, const float* q, const float* qg, const voi
     return fail(ctx, INFDEV_E_ARGUMENT, "attention: blockTokens must be a multiple of 16 and maxSplits in 1..64");
   int launches = 0;
   const cudaError_t e = infdev::attention_launch(q, qg, cacheK, cacheV, queries, queryCount, table, tableStride, blockTokens, rows, maxSplits, partials, out,
-                                                 take_capture(ctx), !ctx->umma, ctx->sms, ctx->stream, &launches);
+                                                 take_capture(ctx), !ctx->umma, ctx->sms, ctx->status, ctx->stream, &launches);
   ctx->launches += launches;
   return check(ctx, e, "attention");
 }

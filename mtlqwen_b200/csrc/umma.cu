@@ -25,8 +25,8 @@
 // What bounds it, by its own clocks (18944 x 8192, every SM at work): with 128 rows the copies, 82 KB a super-block of which 64 are
 // activations, at 45 bytes a clock and SM (0.95 us; the 16 MMAs are 0.55); with few rows a dequant group's 1200 clocks a half. 96 tiles
 // (n = 12288) occupy 96 of 148 SMs.
-#include "common.cuh"
 #include "kernels.h"
+#include "tcgen05.cuh"
 
 namespace infdev {
 namespace {
@@ -56,53 +56,16 @@ constexpr int kControlBytes = 512;
 static_assert(sizeof(Control) <= kControlBytes, "control block too large");
 constexpr size_t kSharedBytes = 1024 + kControlBytes + size_t(kStages) * kSlabBytes + size_t(kActStages) * kActHalfBytes;
 
-__device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t columns) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(columns) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t base, uint32_t columns) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(columns) : "memory");
-}
-__device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// D[128 x N] (+)= A[128 x 16] (TMEM) * B[16 x N] (shared memory descriptor)
-__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint64_t bDesc, uint32_t iDesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(d),
-      "r"(a), "l"(bDesc), "r"(iDesc), "r"(accumulate), "r"(0u)
-      : "memory");
-}
-// 32 lanes x 32 consecutive columns, one 32-bit value per (lane, column)
-__device__ __forceinline__ void tmem_store32(uint32_t address, const uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,"
-      "%28,%29,%30,%31,%32};" ::"r"(address),
-      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]),
-      "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]),
-      "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-      : "memory");
-}
 __device__ __forceinline__ void tmem_load8(uint32_t address, float (&v)[8]) {
   uint32_t r[8];
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "r"(address)
                : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  tmem_wait_load();
 #pragma unroll
   for (int i = 0; i < 8; ++i)
     v[i] = __uint_as_float(r[i]);
-}
-
-// Shared-memory matrix descriptor of a K-major, no-swizzle operand: 8-row x 16-byte core matrices, the two K halves
-// `leading` bytes apart, successive 8-row groups `stride` bytes apart (descriptor version 1 = Blackwell).
-__device__ __forceinline__ uint64_t smem_descriptor(uint32_t address, uint32_t leading, uint32_t stride) {
-  return uint64_t((address & 0x3FFFFu) >> 4) | (uint64_t(leading >> 4) << 16) | (uint64_t(stride >> 4) << 32) | (uint64_t(1) << 46);
 }
 
 // The epilogue of one item for the 32 TMEM lanes (= weight rows = output columns) of the calling
@@ -323,7 +286,7 @@ template <int NMAT, int GROUPS> __global__ void __launch_bounds__(kThreads<GROUP
           }
           tmem_store32(aAddress + 32 * t, v);
         }
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          tmem_wait_store();
         fence_before_sync();
         __syncwarp();
         if (lane == 0) {
