@@ -49,49 +49,77 @@ __device__ __forceinline__ void split_range(uint32_t attended, uint32_t maxSplit
   end = min(attended, begin + per);
 }
 
-// grid (rows * 20), 256 threads: heads 0..15 are queries, 16..19 keys (which also store the value head).
+// One warp per (row, head), eight consecutive dims a lane: heads 0..15 are queries, 16..19 keys (which also store the value head). A CTA
+// of 256 threads per head spent its time on two barriers and a chain of single loads: 128 rows 5.6 us, 3.5 now. ALIGNED: all
+// operands lie on 16-byte boundaries (a caller's views may start at any element).
+template <bool ALIGNED> __device__ __forceinline__ void load_eight(float (&to)[8], const float* from) {
+#pragma unroll
+  for (int i = 0; i < 8; i += 4) {
+    const float4 v = ALIGNED ? *reinterpret_cast<const float4*>(from + i) : make_float4(from[i], from[i + 1], from[i + 2], from[i + 3]);
+    to[i] = v.x, to[i + 1] = v.y, to[i + 2] = v.z, to[i + 3] = v.w;
+  }
+}
+__device__ __forceinline__ uint4 pack_eight(const float (&v)[8]) {
+  return make_uint4(pack_half2(v[0], v[1]), pack_half2(v[2], v[3]), pack_half2(v[4], v[5]), pack_half2(v[6], v[7]));
+}
+template <bool ALIGNED>
 __global__ void __launch_bounds__(256) attention_prepare_kernel(const float* qg, const float* rawK, const float* rawV, const float* qNorm,
                                                                 const float* kNorm, const float* rope, const infdev_query* queries, int queryCount,
-                                                                const int32_t* table, int tableStride, int blockTokens, float* q, __half* cacheK,
+                                                                const int32_t* table, int tableStride, int blockTokens, int heads, float* q, __half* cacheK,
                                                                 __half* cacheV) {
   pdl_launch_dependents();
   pdl_wait();
-  const int row = blockIdx.x / 20, head = blockIdx.x % 20, lane = threadIdx.x;
+  const int item = blockIdx.x * 8 + (threadIdx.x >> 5), row = item / 20, head = item % 20, lane = threadIdx.x & 31;
   const bool query = head < kQHeads;
-  if (query && !qg)  // K/V store only (mtp_store_kv, attention.metal:53-100)
+  if (item >= heads || (query && !qg))  // K/V store only (mtp_store_kv, attention.metal:53-100)
     return;
   const int local = query ? head : head - kQHeads;
-  const float* source = query ? qg + (size_t(row) * kQHeads + local) * kDim * 2 : rawK + (size_t(row) * kKvHeads + local) * kDim;
-  const float* weight = query ? qNorm : kNorm;
-  const float value = source[lane];
-  __shared__ float partial[8], scale;
-  const float sum = warp_sum(value * value);
-  if ((lane & 31) == 0)
-    partial[lane >> 5] = sum;
-  __syncthreads();
-  if (lane == 0) {
-    float total = 0.f;
-    for (int i = 0; i < 8; ++i)
-      total += partial[i];
-    scale = rsqrtf(total / float(kDim) + 1.0e-6f);
-  }
-  __syncthreads();
+  float v[8], weight[8], values[8];
+  load_eight<ALIGNED>(v, (query ? qg + (size_t(row) * kQHeads + local) * kDim * 2 : rawK + (size_t(row) * kKvHeads + local) * kDim) + lane * 8);
+  load_eight<ALIGNED>(weight, (query ? qNorm : kNorm) + lane * 8);
+  if (!query)
+    load_eight<ALIGNED>(values, rawV + (size_t(row) * kKvHeads + local) * kDim + lane * 8);
   const infdev_query& info = query_of_row(queries, queryCount, row);
   const uint32_t position = info.position + row - info.start;
-  float result = value * scale * weight[lane];
-  if (lane < 64) {
-    const int other = lane < 32 ? lane + 32 : lane - 32, pair = lane & 31;
-    const float paired = source[other] * scale * weight[other];
-    const float2 cs = *reinterpret_cast<const float2*>(rope + (size_t(position) * 32 + pair) * 2);
-    result = result * cs.x + (lane < 32 ? -paired : paired) * cs.y;
+  const float sum = warp_sum(((v[0] * v[0] + v[1] * v[1]) + (v[2] * v[2] + v[3] * v[3])) + ((v[4] * v[4] + v[5] * v[5]) + (v[6] * v[6] + v[7] * v[7])));
+  const float scale = rsqrtf(sum / float(kDim) + 1.0e-6f);
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    v[i] = v[i] * scale * weight[i];
+  // dims d and d + 32 of the first 64 turn together: lanes 0..3 and 4..7
+  float other[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    other[i] = __shfl_xor_sync(0xffffffffu, v[i], 4);
+  if (lane < 8) {
+    float angle[2][8];  // cos, sin of pairs 8 (lane % 4) .. + 3, then of the next four
+    const float* entry = rope + (size_t(position) * 32 + (lane & 3) * 8) * 2;
+    load_eight<ALIGNED>(angle[0], entry);
+    load_eight<ALIGNED>(angle[1], entry + 8);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      v[i] = v[i] * angle[i >> 2][2 * (i & 3)] + (lane < 4 ? -other[i] : other[i]) * angle[i >> 2][2 * (i & 3) + 1];
   }
   if (query) {
-    q[(size_t(row) * kQHeads + local) * kDim + lane] = result;
+    float* to = q + (size_t(row) * kQHeads + local) * kDim + lane * 8;
+#pragma unroll
+    for (int i = 0; i < 8; i += 4) {
+      if (ALIGNED)
+        *reinterpret_cast<float4*>(to + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+      else
+        to[i] = v[i], to[i + 1] = v[i + 1], to[i + 2] = v[i + 2], to[i + 3] = v[i + 3];
+    }
+    return;
+  }
+  const size_t block = table[size_t(info.slot) * tableStride + position / blockTokens];
+  const size_t at = ((block * kKvHeads + local) * blockTokens + position % blockTokens) * kDim + lane * 8;
+  if (ALIGNED) {
+    *reinterpret_cast<uint4*>(cacheK + at) = pack_eight(v);
+    *reinterpret_cast<uint4*>(cacheV + at) = pack_eight(values);
   } else {
-    const size_t block = table[size_t(info.slot) * tableStride + position / blockTokens];
-    const size_t at = ((block * kKvHeads + local) * blockTokens + position % blockTokens) * kDim + lane;
-    cacheK[at] = __float2half_rn(result);
-    cacheV[at] = __float2half_rn(rawV[(size_t(row) * kKvHeads + local) * kDim + lane]);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      cacheK[at + i] = __float2half_rn(v[i]), cacheV[at + i] = __float2half_rn(values[i]);
   }
 }
 
@@ -815,8 +843,14 @@ cudaError_t attention_prepare_launch(const float* qg, const float* rawK, const f
                                      void* cacheK, void* cacheV, cudaStream_t stream) {
   if (rows <= 0)
     return cudaSuccess;
-  launch_kernel<2>(attention_prepare_kernel, unsigned(rows * 20), 256, 0, stream, qg, rawK, rawV, qNorm, kNorm, rope, queries, queryCount, table, tableStride, blockTokens, q,
-                                                                     static_cast<__half*>(cacheK), static_cast<__half*>(cacheV));
+  uintptr_t addresses = reinterpret_cast<uintptr_t>(cacheK) | reinterpret_cast<uintptr_t>(cacheV);
+  for (const float* p : {qg, rawK, rawV, qNorm, kNorm, rope, static_cast<const float*>(q)})
+    addresses |= reinterpret_cast<uintptr_t>(p);
+  auto launch = [&](auto kernel) {
+    launch_kernel<2>(kernel, unsigned((rows * 20 + 7) / 8), 256, 0, stream, qg, rawK, rawV, qNorm, kNorm, rope, queries, queryCount, table, tableStride, blockTokens,
+                     int(rows * 20), q, static_cast<__half*>(cacheK), static_cast<__half*>(cacheV));
+  };
+  launch(addresses & 15 ? attention_prepare_kernel<false> : attention_prepare_kernel<true>);
   return cudaGetLastError();
 }
 
