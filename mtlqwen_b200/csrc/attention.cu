@@ -4,7 +4,8 @@
 //                             reference does inside attention_scan (:126-133)
 // attention_scan_kernel    <- attention_scan   (attention.metal:103-183), row by row: queries of one row, and passes whose
 //                             queries have few rows on average
-// attention_tile_kernel   <- the same, for the queries of several rows of the other passes
+// attention_tile_kernel    <- the same, for the queries of several rows of the other passes
+// attention_group_kernel   <- the same, where the contexts of those passes are short
 // attention_reduce_kernel  <- attention_reduce (attention.metal:185-216)
 //
 // K/V pool of one layer: [physical block][4 kv heads][blockTokens][256] fp16, so the 16 tokens of a tile of
@@ -311,8 +312,8 @@ __global__ void __launch_bounds__(128, 6) attention_scan_kernel(const float* q, 
 // 1.6 k cycles of MMAs for the scores (bounded by shared memory: A and B both come from there) and 1 k for the values; mma.sync,
 // with 16 rows x 4 heads, was 8 k for half the rows.
 // Measured, with the merge, and before, with mma.sync: 128 rows behind 1920 tokens 51.0 -> 32.1 us, four times 30 rows behind up to 1970
-// 49.3 -> 32.4, 2048 rows behind 2048 1070 -> 449; 64 rows of 64 tokens 13.7 -> 16.1: a fixed start of laying out q and an end of
-// reading tensor memory, which little work has to pay for.
+// 49.3 -> 32.4, 2048 rows behind 2048 1070 -> 449; 64 rows of 64 tokens 13.0 -> 16.1: a fixed start of laying out q and an end of
+// reading tensor memory, which little work has to pay for, so short contexts stay with attention_group_kernel below.
 //
 // Work items (tile of rows, piece of context, kv head) are dealt to one CTA per SM; which exist only the device knows, so
 // a CTA finds its next item by a scan over the queries. The pieces of a tile follow from its context and from `most`, which
@@ -343,13 +344,13 @@ struct RowTile {
   uint32_t start, rows, first, attended, slot;  // first: position of its first row; attended: context of its last row
 };
 
-__device__ __forceinline__ uint32_t tiles_of(const infdev_query& query) { return query.count > 1 ? (query.count + kGroupRows - 1) / kGroupRows : 0u; }
+template <uint32_t ROWS> __device__ __forceinline__ uint32_t tiles_of(const infdev_query& query) { return query.count > 1 ? (query.count + ROWS - 1) / ROWS : 0u; }
 
-__device__ __forceinline__ RowTile tile_of(const infdev_query& query, uint32_t index) {
+template <uint32_t ROWS> __device__ __forceinline__ RowTile tile_of(const infdev_query& query, uint32_t index) {
   RowTile tile;
-  tile.start = query.start + index * kGroupRows;
-  tile.rows = min(uint32_t(kGroupRows), query.count - index * kGroupRows);
-  tile.first = query.position + index * kGroupRows;
+  tile.start = query.start + index * ROWS;
+  tile.rows = min(ROWS, query.count - index * ROWS);
+  tile.first = query.position + index * ROWS;
   tile.attended = tile.first + tile.rows;
   tile.slot = query.slot;
   return tile;
@@ -365,6 +366,7 @@ __device__ __forceinline__ uint32_t piece_count(uint32_t attended, uint32_t piec
 // Work item `item` of the pass, found by one warp together; false when there are fewer. `items`: how many there are, where one
 // round tells. A lane has one tile of rows at a time, whichever query it is of: with a lane per query, which counted its tiles one
 // after the other, this took 2.2 us of the 128 rows of one prompt, most of it the divisions of four tiles in a row.
+template <uint32_t ROWS>
 __device__ __forceinline__ bool find_item(const infdev_query* queries, int queryCount, uint32_t most, uint32_t maxSplits, uint32_t item, RowTile& tile,
                                           uint32_t& split, uint32_t& piece, uint32_t& items) {
   const uint32_t lane = threadIdx.x & 31;
@@ -382,7 +384,7 @@ __device__ __forceinline__ bool find_item(const infdev_query* queries, int query
     infdev_query query = {};
     if (base + int(lane) < queryCount)
       query = queries[base + lane];
-    const uint32_t tilesUpTo = running_sum(tiles_of(query)), tiles = __shfl_sync(0xffffffffu, tilesUpTo, 31);
+    const uint32_t tilesUpTo = running_sum(tiles_of<ROWS>(query)), tiles = __shfl_sync(0xffffffffu, tilesUpTo, 31);
     for (uint32_t first = 0; first < tiles; first += 32) {
       // the query of this lane's tile: how many queries end at or before it
       const uint32_t mine = first + lane;
@@ -395,11 +397,11 @@ __device__ __forceinline__ bool find_item(const infdev_query* queries, int query
       infdev_query whose = {};
       whose.start = __shfl_sync(0xffffffffu, query.start, owner), whose.count = __shfl_sync(0xffffffffu, query.count, owner);
       whose.position = __shfl_sync(0xffffffffu, query.position, owner), whose.slot = __shfl_sync(0xffffffffu, query.slot, owner);
-      const uint32_t before = __shfl_sync(0xffffffffu, tilesUpTo - tiles_of(query), owner);
+      const uint32_t before = __shfl_sync(0xffffffffu, tilesUpTo - tiles_of<ROWS>(query), owner);
       RowTile each = {};
       uint32_t tokens = 0, count = 0;
       if (mine < tiles) {
-        each = tile_of(whose, mine - before);
+        each = tile_of<ROWS>(whose, mine - before);
         tokens = piece_tokens(each.attended, each.rows, most, maxSplits), count = piece_count(each.attended, tokens);
       }
       const uint32_t inclusive = running_sum(count), total = __shfl_sync(0xffffffffu, inclusive, 31);
@@ -468,7 +470,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
   RowTile tile;
   uint32_t split, piece, items = 0xffffffffu, itemCount = 0, roundCount = 0;
   auto next_item = [&](uint32_t item) {
-    return item / kKvHeads < items && find_item(queries, queryCount, most, maxSplits, item / kKvHeads, tile, split, piece, items);
+    return item / kKvHeads < items && find_item<kGroupRows>(queries, queryCount, most, maxSplits, item / kKvHeads, tile, split, piece, items);
   };
   auto tiles_in_round = [](uint32_t from, uint32_t end) { return min(uint32_t(kRoundTiles), (end - from + kGroupTokens - 1) / kGroupTokens); };
   constexpr uint32_t kRoundTokens = kRoundTiles * kGroupTokens;
@@ -784,10 +786,223 @@ __global__ void __launch_bounds__(kTileThreads, 1)
     tmem_dealloc(tmem, 512);
 }
 
+// The same for passes of short contexts, with mma.sync: 16 rows a tile and a warp, two warps a scheduler. K and V tiles come through
+// a cp.async double buffer; warp = (head, half), a half takes 32 of a tile's 64 tokens for the scores and 128 of the 256 value
+// dims, and the halves exchange maxima, weights and norms. Each tile of tokens is a chain of all of that, 8 k cycles of MMAs in it, which
+// long contexts cannot afford, but there is next to nothing before the first one: 64 rows of 64 tokens 13.0 us with the merge (13.7 before
+// items were found a lane per tile), 16.1 with attention_tile_kernel, and row by row 17.8; attention_launch has the line between the two.
+constexpr int kShortRows = 16, kGroupThreads = 256, kGroupPitch = kDim + 8, kWeightPitch = kGroupTokens + 8;
+
+struct GroupShared {
+  __half q[2][kGroup * kShortRows][kGroupPitch];                         // hi, lo; row 16 * head + r
+  __half k[2][kGroupTokens][kGroupPitch], v[2][kGroupTokens][kGroupPitch];  // two buffers
+  __half p[2][kGroup * kShortRows][kWeightPitch];                        // hi, lo
+  float exchange[2][kGroup * kShortRows];
+};
+
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const __half* address) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(address)));
+}
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], const __half* address) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(smem_u32(address)));
+}
+__global__ void __launch_bounds__(kGroupThreads, 1)
+    attention_group_kernel(const float* q, const __half* cacheK, const __half* cacheV, const infdev_query* queries, int queryCount, const int32_t* table,
+                           int tableStride, int blockTokens, uint32_t most, uint32_t maxSplits, float* partials) {
+  pdl_wait();  // first: the scan of the queries of one row starts beside this kernel and relies on it
+  pdl_launch_dependents();
+  extern __shared__ __align__(16) uint8_t groupRaw[];
+  GroupShared& sh = *reinterpret_cast<GroupShared*>(groupRaw);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, head = warp & 3, half = warp >> 2, g = lane >> 2, t = lane & 3;
+  const int rowBase = head * kShortRows;  // this warp's 16 rows of q, p and exchange
+  RowTile tile;
+  uint32_t split, piece, items = 0xffffffffu;
+  for (uint32_t item = blockIdx.x;
+       item / kKvHeads < items && find_item<kShortRows>(queries, queryCount, most, maxSplits, item / kKvHeads, tile, split, piece, items); item += gridDim.x) {
+    const uint32_t kvHead = item % kKvHeads, begin = split * piece, end = min(tile.attended, begin + piece);
+    const int32_t* slotTable = table + size_t(tile.slot) * tableStride;
+    auto fetch = [&](uint32_t from, int buffer) {  // a warp copies one token's 512 bytes at a time
+#pragma unroll
+      for (int c = 0; c < kGroupTokens / 8; ++c) {
+        const uint32_t token = c * 8 + warp, at = min(from + token, end - 1);
+        const uint32_t bytes = from + token < end ? 16u : 0u;  // zeros past the end
+        const size_t base = ((size_t(slotTable[at / blockTokens]) * kKvHeads + kvHead) * blockTokens + at % blockTokens) * kDim + lane * 8;
+        copy_async16(&sh.k[buffer][token][lane * 8], cacheK + base, bytes);
+        copy_async16(&sh.v[buffer][token][lane * 8], cacheV + base, bytes);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    __syncthreads();  // the item before this one is finished with the shared arrays
+    // the 16 rows x 4 heads of q, hi and lo; rows past the tile's are zero. All loads are in flight before the first is used.
+    constexpr int kQuads = kGroup * kShortRows * (kDim / 4) / kGroupThreads;
+    float4 value[kQuads];
+#pragma unroll
+    for (int i = 0; i < kQuads; ++i) {
+      const int at = i * kGroupThreads + threadIdx.x, row = at / (kDim / 4), d = at % (kDim / 4) * 4, r = row % kShortRows, h = row / kShortRows;
+      value[i] = r < int(tile.rows) ? *reinterpret_cast<const float4*>(q + (size_t(tile.start + r) * kQHeads + kvHead * kGroup + h) * kDim + d)
+                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    fetch(begin, 0);
+#pragma unroll
+    for (int i = 0; i < kQuads; ++i) {
+      const int at = i * kGroupThreads + threadIdx.x, row = at / (kDim / 4), d = at % (kDim / 4) * 4;
+      const uint2 a = split_pair(value[i].x, value[i].y), b = split_pair(value[i].z, value[i].w);
+      *reinterpret_cast<uint2*>(&sh.q[0][row][d]) = make_uint2(a.x, b.x);
+      *reinterpret_cast<uint2*>(&sh.q[1][row][d]) = make_uint2(a.y, b.y);
+    }
+    float maximum[2] = {-1.0e30f, -1.0e30f}, norm[2] = {0.f, 0.f}, acc[16][4];  // rows g and g + 8
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+    int buffer = 0;
+    for (uint32_t from = begin; from < end; from += kGroupTokens, buffer ^= 1) {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();  // the tile has landed, and everybody is done with the one before
+      if (from + kGroupTokens < end)
+        fetch(from + kGroupTokens, buffer ^ 1);
+      float score[4][4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        score[j][0] = score[j][1] = score[j][2] = score[j][3] = 0.f;
+#pragma unroll
+      for (int step = 0; step < kDim / 16; ++step) {
+        uint32_t hi[4], lo[4];
+        ldmatrix4(hi, &sh.q[0][rowBase + (lane & 15)][16 * step + 8 * (lane >> 4)]);
+        ldmatrix4(lo, &sh.q[1][rowBase + (lane & 15)][16 * step + 8 * (lane >> 4)]);
+#pragma unroll
+        for (int pair = 0; pair < 2; ++pair) {
+          if (from + 32 * half + 16 * pair >= end)  // past the piece: these scores are masked below
+            continue;
+          uint32_t b[4];
+          ldmatrix4(b, &sh.k[buffer][32 * half + 16 * pair + 8 * (lane >> 4) + (lane & 7)][16 * step + 8 * ((lane >> 3) & 1)]);
+          mma_16816(score[2 * pair], hi, b[0], b[1]);
+          mma_16816(score[2 * pair + 1], hi, b[2], b[3]);
+          mma_16816(score[2 * pair], lo, b[0], b[1]);
+          mma_16816(score[2 * pair + 1], lo, b[2], b[3]);
+        }
+      }
+      // scale, causal mask, row maxima over both halves of the tile
+      float best[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t token = from + 32 * half + 8 * j + 2 * t + (i & 1), limit = min(end, tile.first + g + 8 * (i >> 1) + 1);
+          score[j][i] = token < limit ? score[j][i] * (1.0f / 16.0f) : -INFINITY;
+          best[i >> 1] = fmaxf(best[i >> 1], score[j][i]);
+        }
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        best[r] = fmaxf(best[r], __shfl_xor_sync(0xffffffffu, best[r], 1));
+        best[r] = fmaxf(best[r], __shfl_xor_sync(0xffffffffu, best[r], 2));
+        if (t == 0)
+          sh.exchange[half][rowBase + g + 8 * r] = best[r];
+      }
+      named_barrier(1 + head, 64);
+      float rescale[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float next = fmaxf(maximum[r], fmaxf(best[r], sh.exchange[half ^ 1][rowBase + g + 8 * r]));
+        rescale[r] = expf(maximum[r] - next);
+        maximum[r] = next;
+        norm[r] *= rescale[r];
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const float w0 = expf(score[j][2 * r] - maximum[r]), w1 = expf(score[j][2 * r + 1] - maximum[r]);
+          norm[r] += w0 + w1;
+          const uint2 w = split_pair(w0, w1);
+          *reinterpret_cast<uint32_t*>(&sh.p[0][rowBase + g + 8 * r][32 * half + 8 * j + 2 * t]) = w.x;
+          *reinterpret_cast<uint32_t*>(&sh.p[1][rowBase + g + 8 * r][32 * half + 8 * j + 2 * t]) = w.y;
+        }
+      // A value that is not finite, of a token that some rows of the tile do not attend to, times their weights of zero would
+      // reach them: in such a tile it stands as zero, and the rows that do attend to it get NaN afterwards. (128 rows behind 1920
+      // tokens 55.4 -> 56.3 us with the test; a test within the loop of products 58.)
+      const uint32_t masked = max(from, tile.first + 1), past = min(from + kGroupTokens, end);
+      uint32_t broken = 0;
+      for (uint32_t token = masked; token < past; ++token) {
+        const uint2 four = *reinterpret_cast<const uint2*>(&sh.v[buffer][token - from][128 * half + 4 * lane]);
+        broken |= not_finite(four.x) | not_finite(four.y);
+      }
+      broken = __any_sync(0xffffffffu, broken != 0);
+      named_barrier(1 + head, 64);  // both halves of the weights are there
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        acc[j][0] *= rescale[0], acc[j][1] *= rescale[0], acc[j][2] *= rescale[1], acc[j][3] *= rescale[1];
+      auto add_values = [&](int step, bool clean) {
+        uint32_t hi[4], lo[4];
+        ldmatrix4(hi, &sh.p[0][rowBase + (lane & 15)][16 * step + 8 * (lane >> 4)]);
+        ldmatrix4(lo, &sh.p[1][rowBase + (lane & 15)][16 * step + 8 * (lane >> 4)]);
+#pragma unroll
+        for (int pair = 0; pair < 8; ++pair) {
+          uint32_t b[4];
+          ldmatrix4_trans(b, &sh.v[buffer][16 * step + (lane & 15)][128 * half + 16 * pair + 8 * (lane >> 4)]);
+          if (clean) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              b[i] &= ~((not_finite(b[i]) >> 15) * 0xffffu);
+          }
+          mma_16816(acc[2 * pair], hi, b[0], b[1]);
+          mma_16816(acc[2 * pair + 1], hi, b[2], b[3]);
+          mma_16816(acc[2 * pair], lo, b[0], b[1]);
+          mma_16816(acc[2 * pair + 1], lo, b[2], b[3]);
+        }
+      };
+      if (!broken) {
+#pragma unroll
+        for (int step = 0; step < kGroupTokens / 16; ++step) {
+          if (from + 16 * step >= end)  // weights of zero
+            break;
+          add_values(step, false);
+        }
+      } else {
+#pragma unroll 1
+        for (int step = 0; step < kGroupTokens / 16; ++step)
+          add_values(step, true);
+#pragma unroll 1
+        for (uint32_t token = from; token < past; ++token)
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const uint32_t bad = not_finite(*reinterpret_cast<const uint32_t*>(&sh.v[buffer][token - from][128 * half + 8 * j + 2 * t]));
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if ((bad & (i & 1 ? 0x80000000u : 0x8000u)) && token <= tile.first + g + 8 * (i >> 1))
+                acc[j][i] = NAN;
+          }
+      }
+    }
+    // the norm over both halves, then this piece's record of every live row
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      norm[r] += __shfl_xor_sync(0xffffffffu, norm[r], 1);
+      norm[r] += __shfl_xor_sync(0xffffffffu, norm[r], 2);
+      if (t == 0)
+        sh.exchange[half][rowBase + g + 8 * r] = norm[r];
+    }
+    named_barrier(1 + head, 64);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const uint32_t row = g + 8 * r;
+      if (row >= tile.rows)
+        continue;
+      float* record = partials + ((size_t(tile.start + row) * kQHeads + kvHead * kGroup + head) * maxSplits + split) * kPartialStride;
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        *reinterpret_cast<float2*>(record + 128 * half + 8 * j + 2 * t) = make_float2(acc[j][2 * r], acc[j][2 * r + 1]);
+      if (half == 0 && t == 0)
+        *reinterpret_cast<float2*>(record + kDim) = make_float2(maximum[r], sh.exchange[0][rowBase + row] + sh.exchange[1][rowBase + row]);
+    }
+  }
+}
+
 // grid (rows * 16), 256 threads: merge the splits, normalise, multiply by sigmoid(gate).
 // `image`, when not null, also receives the activation image of the output rows: a head is one 256-value block.
-// GROUPED: the splits of a row whose query has several are those of attention_tile_kernel.
-template <bool GROUPED>
+// ROWS: the splits of a row whose query has several are those of the kernel with tiles of so many rows; 0: of the scan.
+template <uint32_t ROWS>
 __global__ void __launch_bounds__(256) attention_reduce_kernel(const float* partials, const float* qg, const infdev_query* queries, int queryCount,
                                                                uint32_t most, uint32_t maxSplits, float* out, uint8_t* image) {
   pdl_launch_dependents();
@@ -795,8 +1010,8 @@ __global__ void __launch_bounds__(256) attention_reduce_kernel(const float* part
   const uint32_t headRow = blockIdx.x, row = headRow / kQHeads, dim = threadIdx.x;
   const infdev_query& info = query_of_row(queries, queryCount, row);
   uint32_t count;
-  if (GROUPED && info.count > 1) {
-    const RowTile tile = tile_of(info, (row - info.start) / kGroupRows);
+  if (ROWS > 0 && info.count > 1) {
+    const RowTile tile = tile_of<ROWS>(info, (row - info.start) / max(ROWS, 1u));
     count = piece_count(tile.attended, piece_tokens(tile.attended, tile.rows, most, maxSplits));
   } else {
     uint32_t begin, end;
@@ -862,24 +1077,34 @@ cudaError_t attention_launch(const float* q, const float* qg, const void* cacheK
     return cudaSuccess;
   *launches = 2;
   const uint32_t splits = std::min<uint32_t>(maxSplits, 32);  // the merge keeps one split per lane
-  // The tile kernel takes passes whose queries have five rows or more on average, unless no context of the pass can be long
-  // (the table has no room for it): with r rows a query, its longer chain costs 2 us and more where r x context is below about 4096;
-  // from there on it is level or faster (64 rows of 64 tokens 16.1 us against 17.8, 64 of 256 18.5 against 22.4, 128 of 128
-  // 18.8 against 29.0, four queries of 20 to 64 rows and as many tokens 19.2 against 29.7; below it 33 rows of 33 tokens 15.7
-  // against 11.7, which only passes of 32 rows a query and more take, whose contexts the host does not know).
+  // Tiles take passes whose queries have five rows or more on average, unless no context of the pass can be long (the table has no
+  // room for it): with r rows a query, their longer chain costs 2 us where r x context is below about 4096 (8 rows of 128 tokens
+  // 18.7 against 16.7 us for preparation and attention), from there on it is level or faster (8 rows of 2008 tokens 20.8 against
+  // 29.1, 64 of 64 13.0 against 17.8 for the attention alone, 64 of 256 15.1 against 22.4, 128 of 128 15.8 against 29.0).
   const int64_t capacity = int64_t(tableStride) * blockTokens;
   const bool grouped = rows >= 32 * int64_t(queryCount) || (rows >= 5 * int64_t(queryCount) && rows * capacity >= 4096 * int64_t(queryCount));
-  // The tile kernel copies q and the partial results in pieces of 16 bytes, the scan in pieces of 8 and less.
-  if (grouped && !rowwise && (reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(partials)) % 16 == 0) {
-    static PerDeviceOnce configured;
-    if (const cudaError_t e = configure_shared_memory(attention_tile_kernel, kTileSharedBytes, configured))
+  // The tile kernels copy q in pieces of 16 bytes, that of 32 rows the partial results too, the scan in pieces of 8 and less.
+  if (grouped && !rowwise && reinterpret_cast<uintptr_t>(q) % 16 == 0) {
+    // Where r x context stays below about 24576, the tiles of 16 rows have the shorter chain: 64 rows of 64 tokens 13.0 us against
+    // 16.1 with tiles of 32, 64 of 256 15.1 against 18.5, 128 of 128 15.8 against 18.8, eight queries of 64 rows and tokens 31.3 against
+    // 34.7; 50 rows on average of up to 600 23.3 against 23.2, 30 of up to 2000 49 against 32.
+    // They also take partial results that are not on 16 bytes.
+    const bool shortPass = rows * capacity < 24576 * int64_t(queryCount) || reinterpret_cast<uintptr_t>(partials) % 16 != 0;
+    const int tileRows = shortPass ? kShortRows : kGroupRows;
+    static PerDeviceOnce configured, shortConfigured;
+    if (const cudaError_t e = shortPass ? configure_shared_memory(attention_group_kernel, sizeof(GroupShared), shortConfigured)
+                                        : configure_shared_memory(attention_tile_kernel, kTileSharedBytes, configured))
       return e;
-    const int64_t tiles = std::max<int64_t>((rows + kGroupRows - 1) / kGroupRows, queryCount);
+    const int64_t tiles = std::max<int64_t>((rows + tileRows - 1) / tileRows, queryCount);
     const uint32_t most = uint32_t(std::clamp<int64_t>(sms / (kKvHeads * tiles), 1, splits));
     const int64_t items = (rows + queryCount) * kKvHeads * splits;  // no more than these
-    launch_kernel<2>(attention_tile_kernel, unsigned(std::min<int64_t>(items, sms)), kTileThreads, kTileSharedBytes, stream, q,
-                  static_cast<const __half*>(cacheK), static_cast<const __half*>(cacheV), queries, queryCount, table, tableStride, blockTokens, most, splits,
-                  partials, status);
+    const unsigned grid = unsigned(std::min<int64_t>(items, sms));
+    if (shortPass)
+      launch_kernel<2>(attention_group_kernel, grid, kGroupThreads, sizeof(GroupShared), stream, q, static_cast<const __half*>(cacheK),
+                       static_cast<const __half*>(cacheV), queries, queryCount, table, tableStride, blockTokens, most, splits, partials);
+    else
+      launch_kernel<2>(attention_tile_kernel, grid, kTileThreads, kTileSharedBytes, stream, q, static_cast<const __half*>(cacheK),
+                       static_cast<const __half*>(cacheV), queries, queryCount, table, tableStride, blockTokens, most, splits, partials, status);
     // Queries of one row stay with the scan, which is faster there: no query rows to share a tile with, and six small CTAs per
     // SM hide the copies that the tile kernel's single CTA waits for. Which queries they are only the device knows; with a
     // single query there are none.
@@ -896,13 +1121,13 @@ cudaError_t attention_launch(const float* q, const float* qg, const void* cacheK
       launch_kernel<2>(attention_scan_kernel<true>, dim3(splits + 1, kKvHeads, unsigned(queryCount)), 128, spread, stream, q, static_cast<const __half*>(cacheK),
                        static_cast<const __half*>(cacheV), queries, queryCount, table, tableStride, blockTokens, splits, partials);
     }
-    launch_kernel<2>(attention_reduce_kernel<true>, unsigned(rows * kQHeads), 256, 0, stream, partials, qg, queries, queryCount, most, splits, out, image);
+    launch_kernel<2>(shortPass ? attention_reduce_kernel<kShortRows> : attention_reduce_kernel<kGroupRows>, unsigned(rows * kQHeads), 256, 0, stream, partials, qg, queries, queryCount, most, splits, out, image);
     return cudaGetLastError();
   }
   launch_kernel(attention_scan_kernel<false>, dim3(splits, kKvHeads, unsigned(rows)), 128, 0, stream, q, static_cast<const __half*>(cacheK),
                                                                                        static_cast<const __half*>(cacheV), queries, queryCount, table,
                                                                                        tableStride, blockTokens, splits, partials);
-  launch_kernel(attention_reduce_kernel<false>, unsigned(rows * kQHeads), 256, 0, stream, partials, qg, queries, queryCount, 0u, splits, out, image);
+  launch_kernel(attention_reduce_kernel<0>, unsigned(rows * kQHeads), 256, 0, stream, partials, qg, queries, queryCount, 0u, splits, out, image);
   return cudaGetLastError();
 }
 
@@ -943,7 +1168,7 @@ cudaError_t attention_static_launch(const float* q, const float* qg, const void*
   launch_kernel(attention_scan_kernel<false>, dim3(kStaticSplits, kKvHeads, unsigned(rows)), 128, 0, stream, q, static_cast<const __half*>(cacheK),
                                                                                           static_cast<const __half*>(cacheV), queries, queryCount, table,
                                                                                           tableStride, blockTokens, kStaticSplits, partials);
-  launch_kernel(attention_reduce_kernel<false>, unsigned(rows * kQHeads), 256, 0, stream, partials, qg, queries, queryCount, 0u, uint32_t(kStaticSplits), out, nullptr);
+  launch_kernel(attention_reduce_kernel<0>, unsigned(rows * kQHeads), 256, 0, stream, partials, qg, queries, queryCount, 0u, uint32_t(kStaticSplits), out, nullptr);
   return cudaGetLastError();
 }
 
