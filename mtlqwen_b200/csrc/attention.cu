@@ -314,6 +314,8 @@ __global__ void __launch_bounds__(128, 6) attention_scan_kernel(const float* q, 
 // Measured, with the merge, and before, with mma.sync: 128 rows behind 1920 tokens 51.0 -> 32.1 us, four times 30 rows behind up to 1970
 // 49.3 -> 32.4, 2048 rows behind 2048 1070 -> 449; 64 rows of 64 tokens 13.0 -> 16.1: a fixed start of laying out q and an end of
 // reading tensor memory, which little work has to pay for, so short contexts stay with attention_group_kernel below.
+// Errors against fp64 (rms, of the result's): 128 rows behind 1920 tokens 1.4e-6 and 1.9e-6 before, 300 behind 8700 7.6e-6 and 2.1e-5,
+// 32 behind 29968 2.9e-6 and 4.6e-6: fewer roundings between tiles.
 //
 // Work items (tile of rows, piece of context, kv head) are dealt to one CTA per SM; which exist only the device knows, so
 // a CTA finds its next item by a scan over the queries. The pieces of a tile follow from its context and from `most`, which
