@@ -60,6 +60,28 @@ template <bool ALIGNED> __device__ __forceinline__ void load_eight(float (&to)[8
     to[i] = v.x, to[i + 1] = v.y, to[i + 2] = v.z, to[i + 3] = v.w;
   }
 }
+// Sum of the squares of a head's 256 dims, eight a lane, in the order in which a warp for every 32 dims adds them: partners 16, 8, 4, 2
+// and 1 dims apart, then the eight warps in turn. What a key is stored as, and with it a sequence's tokens, hangs on that order.
+__device__ __forceinline__ float head_square_sum(const float (&v)[8], int lane) {
+  const bool upper = lane & 2, odd = lane & 1;  // bits 4 and 3 of the lane's dims
+  float part[4], half[2];  // each step halves the dims that a lane still sums for
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float own = upper ? v[4 + j] : v[j], other = __shfl_xor_sync(0xffffffffu, upper ? v[j] : v[4 + j], 2);
+    part[j] = __fadd_rn(__fmul_rn(own, own), __fmul_rn(other, other));
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    half[j] = (odd ? part[2 + j] : part[j]) + __shfl_xor_sync(0xffffffffu, odd ? part[j] : part[2 + j], 1);
+  float sum = (upper ? half[1] : half[0]) + __shfl_xor_sync(0xffffffffu, upper ? half[0] : half[1], 2);
+  sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+  sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+  float total = __shfl_sync(0xffffffffu, sum, 0);
+#pragma unroll
+  for (int i = 4; i < 32; i += 4)
+    total += __shfl_sync(0xffffffffu, sum, i);
+  return total;
+}
 __device__ __forceinline__ uint4 pack_eight(const float (&v)[8]) {
   return make_uint4(pack_half2(v[0], v[1]), pack_half2(v[2], v[3]), pack_half2(v[4], v[5]), pack_half2(v[6], v[7]));
 }
@@ -82,8 +104,15 @@ __global__ void __launch_bounds__(256) attention_prepare_kernel(const float* qg,
     load_eight<ALIGNED>(values, rawV + (size_t(row) * kKvHeads + local) * kDim + lane * 8);
   const infdev_query& info = query_of_row(queries, queryCount, row);
   const uint32_t position = info.position + row - info.start;
-  const float sum = warp_sum(((v[0] * v[0] + v[1] * v[1]) + (v[2] * v[2] + v[3] * v[3])) + ((v[4] * v[4] + v[5] * v[5]) + (v[6] * v[6] + v[7] * v[7])));
-  const float scale = rsqrtf(sum / float(kDim) + 1.0e-6f);
+  // what hangs on the position is under way while the squares are added
+  float angle[2][8];  // lanes 0..7: cos, sin of pairs 8 (lane % 4) .. + 3, then of the next four
+  if (lane < 8) {
+    const float* entry = rope + (size_t(position) * 32 + (lane & 3) * 8) * 2;
+    load_eight<ALIGNED>(angle[0], entry);
+    load_eight<ALIGNED>(angle[1], entry + 8);
+  }
+  const size_t block = query ? 0 : table[size_t(info.slot) * tableStride + position / blockTokens];
+  const float scale = rsqrtf(head_square_sum(v, lane) / float(kDim) + 1.0e-6f);
 #pragma unroll
   for (int i = 0; i < 8; ++i)
     v[i] = v[i] * scale * weight[i];
@@ -93,10 +122,6 @@ __global__ void __launch_bounds__(256) attention_prepare_kernel(const float* qg,
   for (int i = 0; i < 8; ++i)
     other[i] = __shfl_xor_sync(0xffffffffu, v[i], 4);
   if (lane < 8) {
-    float angle[2][8];  // cos, sin of pairs 8 (lane % 4) .. + 3, then of the next four
-    const float* entry = rope + (size_t(position) * 32 + (lane & 3) * 8) * 2;
-    load_eight<ALIGNED>(angle[0], entry);
-    load_eight<ALIGNED>(angle[1], entry + 8);
 #pragma unroll
     for (int i = 0; i < 8; ++i)
       v[i] = v[i] * angle[i >> 2][2 * (i & 3)] + (lane < 4 ? -other[i] : other[i]) * angle[i >> 2][2 * (i & 3) + 1];
@@ -112,7 +137,6 @@ __global__ void __launch_bounds__(256) attention_prepare_kernel(const float* qg,
     }
     return;
   }
-  const size_t block = table[size_t(info.slot) * tableStride + position / blockTokens];
   const size_t at = ((block * kKvHeads + local) * blockTokens + position % blockTokens) * kDim + lane * 8;
   if (ALIGNED) {
     *reinterpret_cast<uint4*>(cacheK + at) = pack_eight(v);

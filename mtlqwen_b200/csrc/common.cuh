@@ -224,8 +224,8 @@ __device__ __forceinline__ float warp_max(float v) {
 // The squares of eight values, with the roundings spelled out: a row's RMS norm has the same bits in rms_norm_4096_kernel and where a
 // projection normalises its activations itself, so that a token's result does not depend on how many others share its pass.
 __device__ __forceinline__ float square_sum(const float4& a, const float4& b) {
-  return __fadd_rn(__fmaf_rn(a.w, a.w, __fmaf_rn(a.z, a.z, __fmaf_rn(a.y, a.y, __fmul_rn(a.x, a.x)))),
-                   __fmaf_rn(b.w, b.w, __fmaf_rn(b.z, b.z, __fmaf_rn(b.y, b.y, __fmul_rn(b.x, b.x)))));
+  return __fadd_rn(__fmaf_rn(a.w, a.w, __fmaf_rn(a.z, a.z, __fmaf_rn(a.x, a.x, __fmul_rn(a.y, a.y)))),
+                   __fmaf_rn(b.w, b.w, __fmaf_rn(b.z, b.z, __fmaf_rn(b.x, b.x, __fmul_rn(b.y, b.y)))));
 }
 
 __device__ __forceinline__ float silu_f(float v) { return v / (1.0f + expf(-v)); }
