@@ -127,8 +127,8 @@ int infdev_image_capture(infdev_ctx* ctx, uint8_t* image);
 int infdev_image_supply(infdev_ctx* ctx, const uint8_t* image);
 /* One-shot: the activations of the next infdev_linear, infdev_linear_group or infdev_gate_up call (k = 4096) are the RMS norm of
  * its x with weights w[k], as infdev_rms_norm computes it: one launch less where the kernel can do it on the way in (integer
- * Q4_K, up to 8 rows); elsewhere the call launches the norm itself. normalised: [rows, k] scratch for that; with store the
- * normalised rows are left there in either case. No image may be supplied for the same call. */
+ * Q4_K, up to 8 rows); elsewhere the call launches the norm itself. normalised: [rows, k] scratch for that, x itself or a buffer apart
+ * from it; with store the normalised rows are left there in either case. No image may be supplied for the same call. */
 int infdev_norm_supply(infdev_ctx* ctx, const float* w, float* normalised, int store);
 /* CUDA-graph capture of a pass on the context's stream (no reference counterpart: Metal re-encodes every
  * pass). begin/end bracket the launches; launch replays; the handle is freed with graph_destroy. */
@@ -143,7 +143,9 @@ void infdev_graph_destroy(infdev_ctx* ctx, void* graph);
 int infdev_dequant(infdev_ctx* ctx, int type, const void* blocks, int64_t count, float* out);
 /* y[m,n] = x[m,k] . W[n,k]^T (+ residual[m,n]); replaces Ops::linear (forward.cpp:51-70) over
  * linear_decode_q4_k[_add] (quant_linear.metal:245-327), linear_decode_q6_k[_add] (:436-512) and, for
- * m > 8, linear_prefill (:151-233). x, y, residual fp32 row-major; residual may alias y or be null.
+ * m > 8, linear_prefill (:151-233). x, y, residual fp32 row-major; residual may alias y or be null. y may lie over x (here and in
+ * the two calls below) only where a launch of its own reads all of x first: Q4_K through the integer kernel or, up to 128 rows, the
+ * tcgen05 GEMM.
  * Q5_K, Q8_0 and IQ4_XS matrices (linear_decode_q5_k, linear_decode_q8_0, :329-434, 514-570; the types the real
  * Qwen3.5 files mix in) take the tensor-core kernels where n is a multiple of 16 and rows are multiples of 16 bytes, a
  * plain dequantise-and-multiply kernel otherwise. */

@@ -20,6 +20,7 @@ struct NormRequest {
   const float* weight = nullptr;  // null: none
   float* normalised = nullptr;
   bool store = false;
+  bool apart = false;  // a launch of its own, not on the way into the GEMV
 };
 }  // namespace infdev
 
@@ -79,6 +80,11 @@ struct Bind {  // makes the context's device current for the calling thread
 };
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// Whether two ranges of floats share one.
+bool overlap(const float* a, int64_t countA, const float* b, int64_t countB) {
+  return a && b && reinterpret_cast<uintptr_t>(a) < reinterpret_cast<uintptr_t>(b + countB) && reinterpret_cast<uintptr_t>(b) < reinterpret_cast<uintptr_t>(a + countA);
+}
 
 // The one-shot image requests are consumed by the first call that could honour them, whether or not it does.
 uint8_t* take_capture(infdev_ctx* ctx) {
@@ -462,9 +468,21 @@ int infdev_dequant(infdev_ctx* ctx, int type, const void* blocks, int64_t count,
   return check(ctx, infdev::dequant_launch(type, blocks, count, out, ctx->stream), "dequant");
 }
 
-// `supplied`: image of x to read instead of quantising it (integer kernel only).
+// The norm of a request as a launch of its own: x is then the normalised rows.
+static int launch_norm(infdev_ctx* ctx, infdev::NormRequest& norm, const float*& x, int64_t m, int64_t k) {
+  if (!norm.weight || !norm.apart)
+    return INFDEV_OK;
+  ++ctx->launches;
+  if (int r = check(ctx, infdev::rms_norm_launch(x, norm.weight, nullptr, m, k, norm.normalised, nullptr, ctx->stream), "rms_norm"))
+    return r;
+  x = norm.normalised;
+  norm = {};
+  return INFDEV_OK;
+}
+
+// `supplied`: image of x to read instead of quantising it (integer kernel only). Nothing is launched before the arguments are checked.
 static int linear_run(infdev_ctx* ctx, int type, bool pair, int count, const void* const* w, const void* const* w2, const int64_t* n, int64_t k,
-                      const float* x, int64_t m, float* const* y, const float* const* residual, const uint8_t* supplied, const infdev::NormRequest& norm) {
+                      const float* x, int64_t m, float* const* y, const float* const* residual, const uint8_t* supplied, infdev::NormRequest norm) {
   const infdev::GemvBox box = infdev::gemv_box(type);
   if (!box.blockBytes)
     return fail(ctx, INFDEV_E_ARGUMENT, "linear: unsupported weight type " + std::to_string(type));
@@ -512,6 +530,8 @@ static int linear_run(infdev_ctx* ctx, int type, bool pair, int count, const voi
     u.partial = ctx->ummaPartial;
     u.acts = static_cast<const uint8_t*>(ctx->ummaActs);
     u.status = ctx->status;
+    if (int r = launch_norm(ctx, norm, x, m, k))
+      return r;
     const int64_t slice = 128;  // activation rows per launch
     for (int64_t row = 0; row < m; row += slice) {
       u.m = int(m - row < slice ? m - row : slice);
@@ -553,6 +573,8 @@ static int linear_run(infdev_ctx* ctx, int type, bool pair, int count, const voi
     }
     p.blocks = int(k / 256), p.pitch = int(columns);
     p.image = ctx->wideImage, p.partial = ctx->widePartial, p.status = ctx->status;
+    if (int r = launch_norm(ctx, norm, x, m, k))
+      return r;
     for (int64_t row = 0; row < m;) {
       // groups of 128 rows; a rest of up to 8 rows joins the group before it, halved
       const int64_t left = m - row, take = left <= infdev::kWideMaxRows ? left : left <= infdev::kWideMaxRows + 8 ? (left + 15) / 16 * 8 : infdev::kWideMaxRows;
@@ -591,6 +613,13 @@ static int linear_run(infdev_ctx* ctx, int type, bool pair, int count, const voi
   p.ldx = int(k);
   p.k = int(k);
   p.status = ctx->status;
+  if (int r = launch_norm(ctx, norm, x, m, k))
+    return r;
+  // Where every CTA reads x itself, some still do while others store results: a result that lies over x has its activations
+  // quantised by a launch of their own, which has read them all before the first result is there.
+  bool inPlace = false;
+  for (int i = 0; i < count; ++i)
+    inPlace = inPlace || overlap(x, m * k, y[i], m * n[i]);
   // More than 8 activation rows: 8-row slices re-use the weights out of L2.
   for (int64_t row = 0; row < m; row += 8) {
     p.x = x + row * k;
@@ -604,7 +633,7 @@ static int linear_run(infdev_ctx* ctx, int type, bool pair, int count, const voi
         p.norm = norm.weight, p.normalised = norm.store ? norm.normalised + row * k : nullptr;
       } else if (supplied) {  // 8-row slices of k/256 blocks
         p.image = supplied + size_t(row / 8) * size_t(k / 256) * infdev::kActivationImageBlockBytes;
-      } else if (p.m <= 2 ? p.m * k <= 32768 : k <= 4096 && p.tiles > ctx->sms) {
+      } else if (!inPlace && (p.m <= 2 ? p.m * k <= 32768 : k <= 4096 && p.tiles > ctx->sms)) {
         // Every CTA quantises the activations itself, where reading them all takes no longer than a launch more: 12288 x 4096 with its
         // own image 9.7 (one row) and 11.2 us (eight), without 7.7 and 11.1 (4096 x 4096 4.8 and 7.0, 3.7 and 5.9); 4096 x 12288
         // 9.5 and 11.5, without 8.7 and 13.7, and 4096 x 8192 with three rows 8.7 and 9.6; 1024 x 4096, which is a start and an end
@@ -636,14 +665,15 @@ static int linear_common(infdev_ctx* ctx, int type, bool pair, int count, const 
   infdev::NormRequest norm = take_norm(ctx);
   if (norm.weight && (supplied || k != infdev::kGemvNormK))
     return fail(ctx, INFDEV_E_ARGUMENT, "linear: normalised activations need k = 4096 and no image");
-  if (norm.weight && (m > 8 || type != INFDEV_Q4_K || !ctx->integerDecode)) {  // not on the way into the GEMV
-    if (!aligned16(x))
-      return fail(ctx, INFDEV_E_ARGUMENT, "linear: activations must be 16-byte aligned");
-    if (int r = check(ctx, infdev::rms_norm_launch(x, norm.weight, nullptr, m, k, norm.normalised, nullptr, ctx->stream), "rms_norm"))
-      return r;
-    ++ctx->launches;
-    x = norm.normalised;
-    norm = {};
+  if (norm.weight) {
+    if (norm.normalised != x && overlap(norm.normalised, m * k, x, m * k))
+      return fail(ctx, INFDEV_E_ARGUMENT, "linear: normalised rows may replace the activations, but not lie across them");
+    // On the way into the GEMV some CTAs still read x while others store normalised rows and results.
+    norm.apart = m > 8 || type != INFDEV_Q4_K || !ctx->integerDecode || norm.normalised == x;
+    for (int i = 0; i < count; ++i) {
+      norm.apart = norm.apart || overlap(x, m * k, y[i], m * n[i]) || overlap(norm.normalised, m * k, y[i], m * n[i]);
+      norm.apart = norm.apart || (residual && overlap(norm.normalised, m * k, residual[i], m * n[i]));
+    }
   }
   if (captured && (count != 1 || n[0] % 256))
     return fail(ctx, INFDEV_E_ARGUMENT, "linear: an image of the result needs a single matrix with n a multiple of 256");
@@ -660,6 +690,8 @@ static int linear_common(infdev_ctx* ctx, int type, bool pair, int count, const 
   if (plain) {
     if (m < 0 || k <= 0 || k % 256 || !aligned16(x))
       return fail(ctx, INFDEV_E_ARGUMENT, "linear: k must be a positive multiple of 256 and the activations 16-byte aligned");
+    if (int r = launch_norm(ctx, norm, x, m, k))
+      return r;
     for (int i = 0; i < count; ++i) {
       if (int r = check(ctx, infdev::format_linear_launch(type, pair, w[i], pair ? w2[i] : nullptr, n[i], k, x, m, y[i], residual ? residual[i] : nullptr, ctx->stream),
                         "linear"))

@@ -76,3 +76,58 @@ def test_norm_needs_a_row_of_4096_and_no_image(dev):
   dev.quantize(dev.array(x), 1, 4096, image)
   with pytest.raises(RuntimeError, match="no image"):
     linear(dev, w, 16, 4096, x, image, (gain, scratch))
+
+
+def in_place(dev, w, n, k, x, norm=None, normalised=None, residual=False):
+  """The result over the activations (n = k)."""
+  buffer = dev.array(x)
+  if norm is not None:
+    dev.norm_supply(norm, buffer if normalised is None else normalised, True)
+  dev.linear(D.Q4_K, w, n, k, buffer, x.shape[0], buffer, buffer if residual else None)
+  return buffer.download()
+
+
+# more tiles than SMs, fewer, and several K chunks, which read the activations again behind the first stores
+@pytest.mark.parametrize("m", [1, 2, 3, 8])
+@pytest.mark.parametrize("k", [1024, 4096, 8192])
+def test_result_over_its_activations(dev, m, k):
+  w, x = dev.array(synth.weight(D.Q4_K, k, k, 31)), synth.activations(m, k, 32)
+  assert in_place(dev, w, k, k, x).tobytes() == linear(dev, w, k, k, x).tobytes()
+
+
+@pytest.mark.parametrize("m", [1, 2, 8, 9])
+def test_norm_over_its_activations_and_results(dev, m):
+  k = 4096
+  w, x = dev.array(synth.weight(D.Q4_K, k, k, 33)), synth.activations(m, k, 34)
+  gain, scratch = dev.array((1 + 0.1 * synth.activations(1, k, 35)[0]).astype(np.float32)), dev.empty((m, k))
+  want = linear(dev, w, k, k, x, norm=(gain, scratch, True))
+  assert in_place(dev, w, k, k, x, gain).tobytes() == want.tobytes()  # norm, activations and result in one buffer
+  assert in_place(dev, w, k, k, x, gain, scratch).tobytes() == want.tobytes()  # result over the activations
+  assert in_place(dev, w, k, k, x, gain, scratch, True).tobytes() == (want + x).astype(np.float32).tobytes()
+  y = dev.empty((m, k))
+  dev.norm_supply(gain, y)  # norm where the result goes
+  dev.linear(D.Q4_K, w, k, k, dev.array(x), m, y)
+  assert y.download().tobytes() == want.tobytes()
+  buffer = dev.array(x)
+  dev.norm_supply(gain, buffer, True)  # norm over the activations
+  dev.linear(D.Q4_K, w, k, k, buffer, m, y)
+  assert y.download().tobytes() == want.tobytes() and buffer.download().tobytes() == scratch.download().tobytes()
+
+
+def test_norm_across_its_activations_is_refused(dev):
+  k, m = 4096, 2
+  w, gain = dev.array(synth.weight(D.Q4_K, 16, k, 36)), dev.array(np.ones(k, np.float32))
+  buffer = dev.array(synth.activations(m + 1, k, 37))
+  dev.norm_supply(gain, type("View", (), {"ptr": buffer.ptr + 4 * k}))
+  with pytest.raises(RuntimeError, match="across"):
+    dev.linear(D.Q4_K, w, 16, k, buffer, m, dev.empty((m, 16)))
+
+
+@pytest.mark.parametrize("qtype,n,m", [(D.Q6_K, 24, 1), (D.Q4_K, 24, 9), (D.Q4_K, 24, 1)])
+def test_a_refused_call_leaves_the_normalised_rows_alone(dev, qtype, n, m):
+  k = 4096
+  w, gain, scratch = dev.empty(n * k, np.uint8), dev.array(np.ones(k, np.float32)), dev.array(np.zeros((m, k), np.float32))
+  dev.norm_supply(gain, scratch, True)
+  with pytest.raises(RuntimeError, match="multiple of 16"):
+    dev.linear(qtype, w, n, k, dev.array(synth.activations(m, k, 38)), m, dev.empty((m, n)))
+  assert not scratch.download().any()
