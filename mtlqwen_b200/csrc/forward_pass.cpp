@@ -11,9 +11,6 @@
 #include "gguf_reader.hpp"
 #include "runtime.hpp"
 
-// A device layer that has no norm_supply gets the norm and the projection as two calls.
-#pragma weak infdev_norm_supply
-
 namespace infeng::qwen35 {
 
 // Read-only mapping of a file.
@@ -178,7 +175,7 @@ struct Ops {
   // Announces the RMS norm of `hidden` as the activations of the projections that follow at once, and returns what to pass them.
   // store: the normalised rows are wanted in scratch.norm in any case.
   const Tensor& normalised(const Tensor& hidden, const float* norm, std::initializer_list<const Weight*> targets, bool store) {
-    bool fold = infdev_norm_supply && selfServed();
+    bool fold = selfServed();
     for (const Weight* target : targets)
       fold = fold && target->type == INFDEV_Q4_K;
     if (fold) {

@@ -11,7 +11,7 @@
 //
 // fake_infdev_fail_commits(n) makes the next n infdev_commit calls report a device failure. A commit takes
 // fake_infdev_commit_delay_us (default 10 ms) so that, as on a GPU, a client that reads one token and cancels does so
-// well before the next pass has finished.
+// well before the next pass has finished. fake_infdev_norms_supplied() counts infdev_norm_supply calls.
 #include <atomic>
 #include <chrono>
 #include <thread>
@@ -27,17 +27,31 @@ struct infdev_ctx {
   const int32_t* rowTokens = nullptr;  // set by infdev_gather_tokens
   uint64_t rowHash[128] = {};          // state hash after each packed row of the current target pass
   uint64_t carried[8] = {};            // drafter: hash chain of each speculative query across the drafting steps
+  bool normPending = false;            // an infdev_norm_supply that no projection has taken yet
 };
 
 namespace {
 
-std::atomic<int> failingCommits{0}, commitDelayMicros{10000};
+std::atomic<int> failingCommits{0}, commitDelayMicros{10000}, normsSupplied{0};
 constexpr uint32_t kUnbound = 0xffffffffu;
 
 uint64_t mix(uint64_t hash, int32_t token) {
   hash ^= uint64_t(uint32_t(token)) + 0x9e3779b97f4a7c15ull + (hash << 6) + (hash >> 2);
   hash *= 0x100000001b3ull;
   return hash ^ (hash >> 29);
+}
+
+// A kernel of the pass. A supplied norm belongs to the projection that follows at once: any other kernel in between is a mistake.
+int launch(infdev_ctx* ctx) {
+  if (ctx->normPending)
+    return ctx->error = "a norm was supplied to a call that takes none", INFDEV_E_ARGUMENT;
+  return ++ctx->launches, 0;
+}
+int projection(infdev_ctx* ctx, int64_t k) {
+  if (ctx->normPending && k != 4096)
+    return ctx->error = "a supplied norm needs rows of 4096", INFDEV_E_ARGUMENT;
+  ctx->normPending = false;
+  return launch(ctx);
 }
 
 int32_t pick(uint64_t hash, int64_t vocab) { return int32_t((hash >> 11) % uint64_t(vocab)); }
@@ -70,6 +84,7 @@ extern "C" {
 
 void fake_infdev_fail_commits(int count) { failingCommits = count; }
 void fake_infdev_commit_delay_us(int micros) { commitDelayMicros = micros; }
+int fake_infdev_norms_supplied() { return normsSupplied; }
 
 infdev_ctx* infdev_create(int, char*) { return new infdev_ctx; }
 void infdev_destroy(infdev_ctx* ctx) { delete ctx; }
@@ -103,31 +118,36 @@ void infdev_graph_destroy(infdev_ctx*, void*) {}
 size_t infdev_image_bytes(int64_t rows, int64_t k) { return size_t((rows + 7) / 8) * size_t(k / 256) * 4384; }
 int infdev_image_capture(infdev_ctx*, uint8_t*) { return 0; }
 int infdev_image_supply(infdev_ctx*, const uint8_t*) { return 0; }
+int infdev_norm_supply(infdev_ctx* ctx, const float* w, float* normalised, int) {
+  if (!w || !normalised || ctx->normPending)
+    return ctx->error = "norm_supply", INFDEV_E_ARGUMENT;
+  return ctx->normPending = true, ++normsSupplied, 0;
+}
 int infdev_set_umma(infdev_ctx*, int) { return 0; }
 int infdev_set_settled_records(infdev_ctx*, int) { return 0; }
 size_t infdev_attention_scratch_bytes(int64_t rows, uint32_t maxSplits) { return size_t(rows) * 16 * maxSplits * 260 * sizeof(float); }
 
-int infdev_linear(infdev_ctx* ctx, int, const void*, int64_t, int64_t, const float*, int64_t, float*, const float*) { return ++ctx->launches, 0; }
-int infdev_linear_group(infdev_ctx* ctx, int, int, const void* const*, const int64_t*, int64_t, const float*, int64_t, float* const*) {
-  return ++ctx->launches, 0;
+int infdev_linear(infdev_ctx* ctx, int, const void*, int64_t, int64_t k, const float*, int64_t, float*, const float*) { return projection(ctx, k); }
+int infdev_linear_group(infdev_ctx* ctx, int, int, const void* const*, const int64_t*, int64_t k, const float*, int64_t, float* const*) {
+  return projection(ctx, k);
 }
-int infdev_gate_up(infdev_ctx* ctx, int, const void*, const void*, int64_t, int64_t, const float*, int64_t, float*) { return ++ctx->launches, 0; }
-int infdev_embedding(infdev_ctx* ctx, int, const void*, int64_t, const int32_t*, int64_t, float*) { return ++ctx->launches, 0; }
-int infdev_dequant(infdev_ctx* ctx, int, const void*, int64_t, float*) { return ++ctx->launches, 0; }
-int infdev_rms_norm(infdev_ctx* ctx, const float*, const float*, int64_t, int64_t, float*) { return ++ctx->launches, 0; }
-int infdev_rms_norm_gather(infdev_ctx* ctx, const float*, const float*, const infdev_query*, int, int64_t, float*) { return ++ctx->launches, 0; }
+int infdev_gate_up(infdev_ctx* ctx, int, const void*, const void*, int64_t, int64_t k, const float*, int64_t, float*) { return projection(ctx, k); }
+int infdev_embedding(infdev_ctx* ctx, int, const void*, int64_t, const int32_t*, int64_t, float*) { return launch(ctx); }
+int infdev_dequant(infdev_ctx* ctx, int, const void*, int64_t, float*) { return launch(ctx); }
+int infdev_rms_norm(infdev_ctx* ctx, const float*, const float*, int64_t, int64_t, float*) { return launch(ctx); }
+int infdev_rms_norm_gather(infdev_ctx* ctx, const float*, const float*, const infdev_query*, int, int64_t, float*) { return launch(ctx); }
 int infdev_rope_table(infdev_ctx*, int64_t, float*) { return 0; }
 int infdev_attention_prepare(infdev_ctx* ctx, const float*, const float*, const float*, const float*, const float*, const float*, const infdev_query*,
                              int, int64_t, const int32_t*, int32_t, int32_t, float*, void*, void*) {
-  return ++ctx->launches, 0;
+  return launch(ctx);
 }
 int infdev_attention(infdev_ctx* ctx, const float*, const float*, const void*, const void*, const infdev_query*, int, int64_t, const int32_t*, int32_t,
                      int32_t, uint32_t, float*, float*) {
-  return ++ctx->launches, 0;
+  return launch(ctx);
 }
 int infdev_mtp_fuse(infdev_ctx* ctx, const float*, const float*, const infdev_query*, int, const float*, const float*, int64_t, uint32_t, uint64_t,
                     uint64_t, float*) {
-  return ++ctx->launches, 0;
+  return launch(ctx);
 }
 
 int infdev_gather_tokens(infdev_ctx* ctx, const infdev_query* queries, int queryCount, const int32_t* requestData, uint32_t capacity,
@@ -145,19 +165,19 @@ int infdev_gather_tokens(infdev_ctx* ctx, const infdev_query* queries, int query
     }
   }
   ctx->rowTokens = rowTokens;
-  return ++ctx->launches, 0;
+  return launch(ctx);
 }
 
 // The first GDN layer of a pass (its conv taps sit at offset 0 of a record) advances the toy state.
 int infdev_gdn_prepare(infdev_ctx* ctx, const float*, const float*, const float*, const float*, const float*, const float*, const float*,
                        const infdev_query*, int, int64_t, uint64_t, uint64_t, float*, float*, float*, float*, float*) {
-  return ++ctx->launches, 0;
+  return launch(ctx);
 }
 int infdev_delta_rule(infdev_ctx* ctx, const float*, const float*, const float*, const float*, const float*, const float*, const float*,
                       const infdev_query* queries, int queryCount, uint64_t stateOffset, uint64_t stateBytes, float*) {
   if (stateOffset == INFDEV_CONV_STATE_BYTES)
     update_state(ctx, queries, queryCount, stateBytes);
-  return ++ctx->launches, 0;
+  return launch(ctx);
 }
 int infdev_delta_rule_prefill(infdev_ctx* ctx, const float* q, const float* k, const float* v, const float* g, const float* beta, const float* z,
                               const float* normWeight, const infdev_query* queries, int queryCount, uint64_t stateOffset, uint64_t stateBytes,
@@ -168,7 +188,7 @@ int infdev_gdn_decode(infdev_ctx* ctx, const float*, const float*, const float*,
                       const float*, const infdev_query* queries, int queryCount, uint64_t convStateOffset, uint64_t, uint64_t stateBytes, float*) {
   if (convStateOffset == 0)
     update_state(ctx, queries, queryCount, stateBytes);
-  return ++ctx->launches, 0;
+  return launch(ctx);
 }
 
 int infdev_sample(infdev_ctx* ctx, const float*, int64_t vocab, infdev_query* queries, int, int64_t count, uint32_t mode, int32_t* tokens) {
@@ -191,7 +211,7 @@ int infdev_sample(infdev_ctx* ctx, const float*, int64_t vocab, infdev_query* qu
       tokens[i] = pick(ctx->rowHash[row], vocab);
     }
   }
-  return ++ctx->launches, 0;
+  return launch(ctx);
 }
 
 int infdev_pack_queries(infdev_ctx* ctx, const infdev_query* in, int count, int drafting, uint32_t, const uint64_t* statePrevious,
@@ -219,7 +239,7 @@ int infdev_pack_queries(infdev_ctx* ctx, const infdev_query* in, int count, int 
     rows += query.count;
   }
   meta[0] = rows, meta[1] = logits, meta[2] = flags, meta[3] = packed;
-  return ++ctx->launches, 0;
+  return launch(ctx);
 }
 
 int infdev_verify_drafts(infdev_ctx* ctx, const infdev_query* queries, int count, const int32_t* sampled, const int32_t* proposed,
@@ -239,7 +259,7 @@ int infdev_verify_drafts(infdev_ctx* ctx, const infdev_query* queries, int count
     }
     verdict[3 * i] = accepted, verdict[3 * i + 1] = emitted, verdict[3 * i + 2] = stopped;
   }
-  return ++ctx->launches, 0;
+  return launch(ctx);
 }
 
 int infdev_commit_states(infdev_ctx* ctx, const infdev_query* queries, int count, const uint32_t* verdict, const uint64_t* stateNext,
@@ -248,7 +268,7 @@ int infdev_commit_states(infdev_ctx* ctx, const infdev_query* queries, int count
     if (queries[i].state != kUnbound)
       std::memcpy(reinterpret_cast<void*>(stateNext[queries[i].slot]),
                   reinterpret_cast<const void*>(candidateBase + uint64_t(queries[i].state + verdict[3 * i]) * stateBytes), stateBytes);
-  return ++ctx->launches, 0;
+  return launch(ctx);
 }
 
 }  // extern "C"

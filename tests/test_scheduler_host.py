@@ -367,3 +367,14 @@ def test_requests_arriving_together_compute_a_shared_prefix_once(library, weight
       sequence.close()
   finally:
     model.close()
+
+
+def test_decode_passes_of_one_row_supply_their_norms(library, weights):
+  """One norm before the mixer and one before the MLP of every layer go to the projections that follow; the stand-in refuses any
+  other order."""
+  engine = engine_of(library, weights)
+  sequence, before = engine.sequence(temperature=0.0), library.fake_infdev_norms_supplied()
+  assert len(complete(sequence, [3, 4, 5], 8)) == 8
+  assert library.fake_infdev_norms_supplied() - before >= 7 * 2 * LAYERS  # the passes behind the prompt's
+  sequence.close()
+  engine.close()
