@@ -218,6 +218,10 @@ int infdev_attention(infdev_ctx* ctx, const float* q, const float* qg, const voi
                      int queryCount, int64_t rows, const int32_t* table, int32_t tableStride, int32_t blockTokens, uint32_t maxSplits,
                      float* partials, float* out);
 size_t infdev_attention_scratch_bytes(int64_t rows, uint32_t maxSplits);
+/* One-shot: no row of the next infdev_attention call attends to more than `tokens` tokens (0: unknown, as without this call). The
+ * call picks its kernel by it instead of by the width of the table, which says how long a context may get and not how long one is.
+ * A bound that is too low costs time and no more. */
+int infdev_attention_context(infdev_ctx* ctx, uint32_t tokens);
 /* No counterpart in the reference. The same attention as infdev_attention for callers that cannot allocate device
  * memory at all (a server that handed every free byte to its K/V pool at start-up, or a decode loop that must not
  * make a device-synchronising allocation call): the split-K partials live in an array built into the library

@@ -1096,8 +1096,8 @@ cudaError_t attention_prepare_launch(const float* qg, const float* rawK, const f
 }
 
 cudaError_t attention_launch(const float* q, const float* qg, const void* cacheK, const void* cacheV, const infdev_query* queries,
-                             int queryCount, const int32_t* table, int tableStride, int blockTokens, int64_t rows, uint32_t maxSplits, float* partials, float* out,
-                             uint8_t* image, bool rowwise, int sms, int* status, cudaStream_t stream, int* launches) {
+                             int queryCount, const int32_t* table, int tableStride, int blockTokens, int64_t rows, int64_t longest, uint32_t maxSplits,
+                             float* partials, float* out, uint8_t* image, bool rowwise, int sms, int* status, cudaStream_t stream, int* launches) {
   *launches = 0;
   if (rows <= 0)
     return cudaSuccess;
@@ -1113,9 +1113,11 @@ cudaError_t attention_launch(const float* q, const float* qg, const void* cacheK
   if (grouped && !rowwise && reinterpret_cast<uintptr_t>(q) % 16 == 0) {
     // Where r x context stays below about 24576, the tiles of 16 rows have the shorter chain: 64 rows of 64 tokens 13.0 us against
     // 16.1 with tiles of 32, 64 of 256 15.1 against 18.5, 128 of 128 15.8 against 18.8, eight queries of 64 rows and tokens 31.3 against
-    // 34.7; 50 rows on average of up to 600 23.3 against 23.2, 30 of up to 2000 49 against 32.
+    // 34.7; 50 rows on average of up to 600 23.3 against 23.2, 30 of up to 2000 49 against 32. The longest context of the pass is what
+    // its caller says, or else what a table row holds (a table for 4096 tokens without it: 16 rows of 16 tokens 13.7 us, 11.1 with it).
     // They also take partial results that are not on 16 bytes.
-    const bool shortPass = rows * capacity < 24576 * int64_t(queryCount) || reinterpret_cast<uintptr_t>(partials) % 16 != 0;
+    const int64_t context = longest > 0 ? std::min(longest, capacity) : capacity;
+    const bool shortPass = rows * context < 24576 * int64_t(queryCount) || reinterpret_cast<uintptr_t>(partials) % 16 != 0;
     const int tileRows = shortPass ? kShortRows : kGroupRows;
     static PerDeviceOnce configured, shortConfigured;
     if (const cudaError_t e = shortPass ? configure_shared_memory(attention_group_kernel, sizeof(GroupShared), shortConfigured)

@@ -90,7 +90,7 @@ void loadWeights(Engine& engine, const std::filesystem::path& path, Weights& wei
 // One pass over `rows` packed tokens (Ops, forward.cpp:25-131).
 struct Ops {
   Engine& engine;
-  uint32_t rows = 0, queryCount = 0;
+  uint32_t rows = 0, queryCount = 0, longestContext = 0;
   bool prefill = false;                   // the pass holds a non-speculative query of more than one row
   const infdev_query* queries = nullptr;  // device records of this pass
   Scratch& scratch;
@@ -201,6 +201,7 @@ struct Ops {
                                      int32_t(engine.kv->tableStride()), int32_t(engine.blockTokens), scratch.attnQ.as<float>(),
                                      engine.kv->key(kvLayer).as<void>(), engine.kv->value(kvLayer).as<void>()));
       capture(scratch.temporaryImage);
+      check(infdev_attention_context(ctx, longestContext));
       check(infdev_attention(ctx, scratch.attnQ.as<float>(), scratch.mixed.as<float>(), engine.kv->key(kvLayer).as<void>(),
                              engine.kv->value(kvLayer).as<void>(), queries, int(queryCount), rows, engine.kv->blockTable(),
                              int32_t(engine.kv->tableStride()), int32_t(engine.blockTokens), maxAttentionSplits, scratch.attnPartials.as<float>(),
@@ -416,6 +417,7 @@ PassShape forward(Engine& engine, Batch& batch, bool drafting, bool launch) {
   ops.rows = shape.rows;
   ops.prefill = shape.prefill && !drafting;
   ops.queryCount = shape.queries;
+  ops.longestContext = batch.longestContext;
   ops.queries = deviceQueries;
   Scratch& scratch = engine.workspace;
   const Tensor& hidden = scratch.hidden;

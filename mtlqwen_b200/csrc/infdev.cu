@@ -34,6 +34,7 @@ struct infdev_ctx {
   uint8_t* captureImage = nullptr;     // one-shot: where the next producer call writes the image of its result
   const uint8_t* supplyImage = nullptr;  // one-shot: image the next linear call reads instead of quantising x
   infdev::NormRequest norm;              // one-shot: the next linear call's activations are the RMS norm of its x
+  uint32_t longestContext = 0;           // one-shot: bound on the contexts of the next attention call (0: what a table row holds)
   float* ummaPartial = nullptr;  // K-slice partial results of the tcgen05 prefill GEMM: [4][128][8192] floats, allocated on first use
   uint8_t* wideImage = nullptr;  // activations laid out for the GEMM of the other block types
   float* widePartial = nullptr;  // its K-slice partial results
@@ -403,6 +404,11 @@ int infdev_norm_supply(infdev_ctx* ctx, const float* w, float* normalised, int s
   if (!w || !normalised || !aligned16(w) || !aligned16(normalised))
     return fail(ctx, INFDEV_E_ARGUMENT, "norm_supply: weights and scratch must be given, 16-byte aligned");
   ctx->norm = {w, normalised, store != 0};
+  return INFDEV_OK;
+}
+
+int infdev_attention_context(infdev_ctx* ctx, uint32_t tokens) {
+  ctx->longestContext = tokens;
   return INFDEV_OK;
 }
 
@@ -853,12 +859,14 @@ int infdev_attention(infdev_ctx* ctx, const float* q, const float* qg, const voi
                      int queryCount, int64_t rows, const int32_t* table, int32_t tableStride, int32_t blockTokens, uint32_t maxSplits,
                      float* partials, float* out) {
   Bind bind(ctx);
+  const uint32_t longest = ctx->longestContext;
+  ctx->longestContext = 0;
   if (rows > 0 && queryCount < 1)
     return fail(ctx, INFDEV_E_ARGUMENT, "attention: rows without queries");
   if (blockTokens <= 0 || blockTokens % 16 || maxSplits < 1 || maxSplits > 64)
     return fail(ctx, INFDEV_E_ARGUMENT, "attention: blockTokens must be a multiple of 16 and maxSplits in 1..64");
   int launches = 0;
-  const cudaError_t e = infdev::attention_launch(q, qg, cacheK, cacheV, queries, queryCount, table, tableStride, blockTokens, rows, maxSplits, partials, out,
+  const cudaError_t e = infdev::attention_launch(q, qg, cacheK, cacheV, queries, queryCount, table, tableStride, blockTokens, rows, longest, maxSplits, partials, out,
                                                  take_capture(ctx), !ctx->umma, ctx->sms, ctx->status, ctx->stream, &launches);
   ctx->launches += launches;
   return check(ctx, e, "attention");

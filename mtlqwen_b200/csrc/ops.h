@@ -37,8 +37,8 @@ cudaError_t attention_prepare_launch(const float* qg, const float* rawK, const f
                                      const infdev_query* queries, int queryCount, const int32_t* table, int tableStride, int blockTokens, int64_t rows, float* q,
                                      void* cacheK, void* cacheV, cudaStream_t stream);
 cudaError_t attention_launch(const float* q, const float* qg, const void* cacheK, const void* cacheV, const infdev_query* queries,
-                             int queryCount, const int32_t* table, int tableStride, int blockTokens, int64_t rows, uint32_t maxSplits, float* partials, float* out,
-                             uint8_t* image, bool rowwise, int sms, int* status, cudaStream_t stream, int* launches);
+                             int queryCount, const int32_t* table, int tableStride, int blockTokens, int64_t rows, int64_t longest, uint32_t maxSplits,
+                             float* partials, float* out, uint8_t* image, bool rowwise, int sms, int* status, cudaStream_t stream, int* launches);
 cudaError_t attention_static_launch(const float* q, const float* qg, const void* cacheK, const void* cacheV, const infdev_query* queries,
                                     int queryCount, const int32_t* table, int tableStride, int blockTokens, int64_t rows, int device, float* out,
                                     cudaStream_t stream);

@@ -64,6 +64,7 @@ struct Batch {
   // The same records finished on the host (start, samples, logit, state addresses): target frame, then drafter frame.
   std::array<infdev_query, 2 * maxBatchSequences> finished{};
   uint32_t size = 0, candidateRows = 0;
+  uint32_t longestContext = 0;  // no row of the pass attends to more tokens
 };
 
 struct Engine {
@@ -114,9 +115,11 @@ struct Engine {
   void* passEvents[2] = {nullptr, nullptr};  // CUDA events bracketing each pass on the stream
   // Pure-decode passes (every query one row, nothing speculative) have a fixed launch sequence for a given number of
   // live sequences; from its second occurrence such a pass is captured once into a CUDA graph and then replayed.
-  // The same holds for passes in which every query is a speculative decode of draftWidth + 1 rows (second index 1).
-  void* decodeGraphs[maxBatchSequences + 1][2] = {};
-  uint32_t decodeSeen[maxBatchSequences + 1][2] = {};
+  // The same holds for passes in which every query is a speculative decode of draftWidth + 1 rows (second index 1 + the class of
+  // their longest context: the attention kernel that a graph holds was chosen by it).
+  static constexpr uint32_t contextClasses = 21;  // contexts up to 2^12, 2^13, .., 2^32 tokens
+  void* decodeGraphs[maxBatchSequences + 1][1 + contextClasses] = {};
+  uint32_t decodeSeen[maxBatchSequences + 1][1 + contextClasses] = {};
   bool useGraphs = true;
 
   Engine(const std::filesystem::path& weights, uint32_t maxContext, const std::filesystem::path& draftWeights);

@@ -350,10 +350,21 @@ void Engine::schedule() {
         const auto started = std::chrono::steady_clock::now();
         infdev_event_record(device.ctx, passEvents[0]);
         // Uniform passes have a fixed launch sequence: every query one decode row, or every query a speculative decode.
-        const uint32_t kind = batch.candidateRows ? 1 : 0, rowsEach = kind ? draftWidth + 1 : 1;
-        bool uniform = useGraphs && batch.candidateRows == kind * batch.size * rowsEach;
-        for (uint32_t i = 0; i < batch.size && uniform; ++i)
-          uniform = batch.queries[i].count == rowsEach;
+        const uint32_t rowsEach = batch.candidateRows ? draftWidth + 1 : 1;
+        bool uniform = !batch.candidateRows || batch.candidateRows == batch.size * rowsEach;
+        uint32_t kind = 0;
+        for (uint32_t i = 0; i < batch.size; ++i) {
+          uniform = uniform && batch.queries[i].count == rowsEach;
+          batch.longestContext = std::max(batch.longestContext, batch.queries[i].position + batch.queries[i].count);
+        }
+        // A speculative pass knows the class of its contexts only, with a graph or without, so that its arithmetic is the same.
+        if (uniform && batch.candidateRows) {
+          uint64_t bound = 4096;
+          for (kind = 1; bound < batch.longestContext; bound *= 2)
+            ++kind;
+          batch.longestContext = uint32_t(std::min<uint64_t>(bound, UINT32_MAX));
+        }
+        uniform = uniform && useGraphs;
         void*& graph = decodeGraphs[batch.size][kind];
         auto launchAll = [&] {
           if (batch.candidateRows)

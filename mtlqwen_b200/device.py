@@ -82,6 +82,7 @@ def library():
     "infdev_rope_table": (i32, (vp, i64, f32p)),
     "infdev_attention_prepare": (i32, (vp, f32p, f32p, f32p, f32p, f32p, f32p, vp, i32, i64, vp, i32, i32, f32p, vp, vp)),
     "infdev_attention": (i32, (vp, f32p, f32p, vp, vp, vp, i32, i64, vp, i32, i32, u32, f32p, f32p)),
+    "infdev_attention_context": (i32, (vp, u32)),
     "infdev_attention_scratch_bytes": (ctypes.c_size_t, (i64, u32)),
     "infdev_attention_static": (i32, (vp, f32p, f32p, vp, vp, vp, i32, i64, vp, i32, i32, f32p)),
     "infdev_mtp_fuse": (i32, (vp, f32p, f32p, vp, i32, f32p, f32p, i64, u32, u64, u64, f32p)),
@@ -264,6 +265,10 @@ class Device:
   def attention(self, q, qg, cache_k, cache_v, queries, nq, rows, table, table_stride, block_tokens, max_splits, partials, out):
     self.check(self.lib.infdev_attention(self.ctx, q.ptr, qg.ptr, cache_k.ptr, cache_v.ptr, queries.ptr, nq, rows, table.ptr, table_stride,
                                          block_tokens, max_splits, partials.ptr, out.ptr))
+
+  def attention_context(self, tokens):
+    """No row of the next attention call attends to more than `tokens` tokens."""
+    self.check(self.lib.infdev_attention_context(self.ctx, tokens))
 
   def attention_scratch_bytes(self, rows, max_splits):
     return int(self.lib.infdev_attention_scratch_bytes(rows, max_splits))

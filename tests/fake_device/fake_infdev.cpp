@@ -28,11 +28,13 @@ struct infdev_ctx {
   uint64_t rowHash[128] = {};          // state hash after each packed row of the current target pass
   uint64_t carried[8] = {};            // drafter: hash chain of each speculative query across the drafting steps
   bool normPending = false;            // an infdev_norm_supply that no projection has taken yet
+  uint32_t longestContext = 0;         // an infdev_attention_context that no attention call has taken yet
 };
 
 namespace {
 
 std::atomic<int> failingCommits{0}, commitDelayMicros{10000}, normsSupplied{0};
+std::atomic<uint32_t> sharedContext{0};  // the bound of the latest attention call with queries of several rows
 constexpr uint32_t kUnbound = 0xffffffffu;
 
 uint64_t mix(uint64_t hash, int32_t token) {
@@ -85,6 +87,7 @@ extern "C" {
 void fake_infdev_fail_commits(int count) { failingCommits = count; }
 void fake_infdev_commit_delay_us(int micros) { commitDelayMicros = micros; }
 int fake_infdev_norms_supplied() { return normsSupplied; }
+uint32_t fake_infdev_shared_context() { return sharedContext; }
 
 infdev_ctx* infdev_create(int, char*) { return new infdev_ctx; }
 void infdev_destroy(infdev_ctx* ctx) { delete ctx; }
@@ -125,6 +128,7 @@ int infdev_norm_supply(infdev_ctx* ctx, const float* w, float* normalised, int) 
 }
 int infdev_set_umma(infdev_ctx*, int) { return 0; }
 int infdev_set_settled_records(infdev_ctx*, int) { return 0; }
+int infdev_attention_context(infdev_ctx* ctx, uint32_t tokens) { return ctx->longestContext = tokens, 0; }
 size_t infdev_attention_scratch_bytes(int64_t rows, uint32_t maxSplits) { return size_t(rows) * 16 * maxSplits * 260 * sizeof(float); }
 
 int infdev_linear(infdev_ctx* ctx, int, const void*, int64_t, int64_t k, const float*, int64_t, float*, const float*) { return projection(ctx, k); }
@@ -141,8 +145,14 @@ int infdev_attention_prepare(infdev_ctx* ctx, const float*, const float*, const 
                              int, int64_t, const int32_t*, int32_t, int32_t, float*, void*, void*) {
   return launch(ctx);
 }
-int infdev_attention(infdev_ctx* ctx, const float*, const float*, const void*, const void*, const infdev_query*, int, int64_t, const int32_t*, int32_t,
-                     int32_t, uint32_t, float*, float*) {
+int infdev_attention(infdev_ctx* ctx, const float*, const float*, const void*, const void*, const infdev_query* queries, int queryCount, int64_t rows,
+                     const int32_t*, int32_t, int32_t, uint32_t, float*, float*) {
+  for (int i = 0; i < queryCount; ++i)
+    if (queries[i].position + queries[i].count > ctx->longestContext)
+      return ctx->error = "a context is longer than was said", INFDEV_E_ARGUMENT;
+  if (rows > queryCount)
+    sharedContext = ctx->longestContext;
+  ctx->longestContext = 0;
   return launch(ctx);
 }
 int infdev_mtp_fuse(infdev_ctx* ctx, const float*, const float*, const infdev_query*, int, const float*, const float*, int64_t, uint32_t, uint64_t,

@@ -2,6 +2,7 @@
 import numpy as np
 import pytest
 
+from mtlqwen_b200 import device as D
 from test_gpu_attention import run_attention
 
 pytestmark = pytest.mark.gpu
@@ -20,3 +21,47 @@ pytestmark = pytest.mark.gpu
 def test_tiles_rounds_and_items(dev, contexts, counts, block_tokens, max_splits):
   rng = np.random.default_rng(sum(contexts) + 7 * len(counts) + max_splits)
   assert run_attention(dev, rng, contexts, counts, block_tokens, max_splits) < 1e-5
+
+
+class Pass:
+  """Queries of `counts` rows at the end of `contexts` tokens, with a table of `stride` blocks a slot."""
+
+  def __init__(self, dev, seed, contexts, counts, block_tokens=16, stride=None):
+    rng = np.random.default_rng(seed)
+    blocks = [-(-c // block_tokens) for c in contexts]
+    self.dev, self.contexts, self.counts, self.block_tokens, self.stride = dev, contexts, counts, block_tokens, stride or max(blocks)
+    order = rng.permutation(sum(blocks)).astype(np.int32)
+    self.table, at = np.zeros((len(contexts), self.stride), np.int32), 0
+    for i, n in enumerate(blocks):
+      self.table[i, :n] = order[at:at + n]
+      at += n
+    self.rows = sum(counts)
+    self.keys, self.values = (rng.standard_normal((sum(blocks), 4, block_tokens, 256)).astype(np.float16) for _ in range(2))
+    self.q, self.qg = (rng.standard_normal((self.rows, 16, width)).astype(np.float32) for width in (256, 512))
+    self.starts = np.concatenate([[0], np.cumsum(counts)])[:-1]
+    queries = []
+    for i, (context, count) in enumerate(zip(contexts, counts)):
+      info = D.Query()
+      info.start, info.count, info.position, info.slot, info.state = int(self.starts[i]), count, context - count, i, D.UNBOUND
+      queries.append(info)
+    self.held = [dev.array(self.q), dev.array(self.qg), dev.array(self.keys.view(np.uint16)), dev.queries(queries), dev.array(self.table)]
+
+  def run(self, values=None, context=0, max_splits=32, offset=0):
+    """offset: floats by which the partial results miss a 16-byte boundary."""
+    dev, (q, qg, keys, queries, table) = self.dev, self.held
+    out, partials = dev.empty((self.rows, 16, 256)), dev.empty(dev.attention_scratch_bytes(self.rows, max_splits) // 4 + 4)
+    if context:
+      dev.attention_context(context)
+    dev.attention(q, qg, keys, dev.array((self.values if values is None else values).view(np.uint16)), queries, len(self.counts), self.rows, table, self.stride,
+                  self.block_tokens, max_splits, type("View", (), {"ptr": partials.ptr + 4 * offset}), out)
+    dev.commit()
+    return out.download()
+
+
+@pytest.mark.parametrize("contexts,counts", [([64], [64]), ([33, 64, 80], [33, 64, 30]), ([700] * 8, [6] * 8), ([700, 40], [20, 40])])
+def test_the_longest_context_counts_and_not_the_width_of_the_table(dev, contexts, counts):
+  narrow = Pass(dev, 81, contexts, counts).run()
+  wide = Pass(dev, 81, contexts, counts, stride=512)
+  assert wide.run(context=max(contexts)).tobytes() == narrow.tobytes()
+  other = wide.run()  # the bound is gone after one call: tiles of 32 rows
+  assert other.tobytes() != narrow.tobytes() and np.abs(other - narrow).max() < 1e-5 * np.abs(narrow).max()

@@ -369,6 +369,22 @@ def test_requests_arriving_together_compute_a_shared_prefix_once(library, weight
     model.close()
 
 
+def test_attention_hears_how_long_the_contexts_are(library, weights):
+  """Not how long max_context would let them get; a speculative pass says the power of two that its graph was captured for. (The
+  stand-in refuses a pass with a longer context than was said.)"""
+  library.fake_infdev_shared_context.restype = ctypes.c_uint32
+  engine = engine_of(library, weights, drafter=True)
+  sequence = engine.sequence(temperature=0.0)
+  one(sequence, tokens_of(20, 64))
+  assert library.fake_infdev_shared_context() == 64
+  sequence.close()
+  sequence = engine.sequence(temperature=0.0, speculative=True)
+  assert len(complete(sequence, tokens_of(21, 30), 8)) == 8
+  assert library.fake_infdev_shared_context() == 4096
+  sequence.close()
+  engine.close()
+
+
 def test_decode_passes_of_one_row_supply_their_norms(library, weights):
   """One norm before the mixer and one before the MLP of every layer go to the projections that follow; the stand-in refuses any
   other order."""
