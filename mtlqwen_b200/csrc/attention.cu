@@ -410,24 +410,30 @@ __device__ __forceinline__ bool find_item(const infdev_query* queries, int query
     infdev_query query = {};
     if (base + int(lane) < queryCount)
       query = queries[base + lane];
-    const uint32_t tilesUpTo = running_sum(tiles_of<ROWS>(query)), tiles = __shfl_sync(0xffffffffu, tilesUpTo, 31);
+    const uint32_t own = tiles_of<ROWS>(query);
+    const bool single = !__any_sync(0xffffffffu, own > 1);  // a lane's tile is its query's then, and there is nothing to look for
+    const uint32_t tilesUpTo = single ? 0u : running_sum(own), tiles = single ? 32u : __shfl_sync(0xffffffffu, tilesUpTo, 31);
     for (uint32_t first = 0; first < tiles; first += 32) {
-      // the query of this lane's tile: how many queries end at or before it
-      const uint32_t mine = first + lane;
-      uint32_t owner = 0;
+      infdev_query whose = query;
+      uint32_t index = 0;
+      bool live = own > 0;
+      if (!single) {  // the query of this lane's tile: how many queries end at or before it
+        const uint32_t mine = first + lane;
+        uint32_t owner = 0;
 #pragma unroll
-      for (uint32_t step = 16; step > 0; step >>= 1) {
-        if (__shfl_sync(0xffffffffu, tilesUpTo, owner + step - 1) <= mine)
-          owner += step;
+        for (uint32_t step = 16; step > 0; step >>= 1) {
+          if (__shfl_sync(0xffffffffu, tilesUpTo, owner + step - 1) <= mine)
+            owner += step;
+        }
+        whose.start = __shfl_sync(0xffffffffu, query.start, owner), whose.count = __shfl_sync(0xffffffffu, query.count, owner);
+        whose.position = __shfl_sync(0xffffffffu, query.position, owner), whose.slot = __shfl_sync(0xffffffffu, query.slot, owner);
+        index = mine - __shfl_sync(0xffffffffu, tilesUpTo - own, owner);
+        live = mine < tiles;
       }
-      infdev_query whose = {};
-      whose.start = __shfl_sync(0xffffffffu, query.start, owner), whose.count = __shfl_sync(0xffffffffu, query.count, owner);
-      whose.position = __shfl_sync(0xffffffffu, query.position, owner), whose.slot = __shfl_sync(0xffffffffu, query.slot, owner);
-      const uint32_t before = __shfl_sync(0xffffffffu, tilesUpTo - tiles_of<ROWS>(query), owner);
       RowTile each = {};
       uint32_t tokens = 0, count = 0;
-      if (mine < tiles) {
-        each = tile_of<ROWS>(whose, mine - before);
+      if (live) {
+        each = tile_of<ROWS>(whose, index);
         tokens = piece_tokens(each.attended, each.rows, most, maxSplits), count = piece_count(each.attended, tokens);
       }
       const uint32_t inclusive = running_sum(count), total = __shfl_sync(0xffffffffu, inclusive, 31);
