@@ -1117,19 +1117,26 @@ cudaError_t attention_launch(const float* q, const float* qg, const void* cacheK
   const bool grouped = rows >= 32 * int64_t(queryCount) || (rows >= 5 * int64_t(queryCount) && rows * capacity >= 4096 * int64_t(queryCount));
   // The tile kernels copy q in pieces of 16 bytes, that of 32 rows the partial results too, the scan in pieces of 8 and less.
   if (grouped && !rowwise && reinterpret_cast<uintptr_t>(q) % 16 == 0) {
-    // Where r x context stays below about 24576, the tiles of 16 rows have the shorter chain: 64 rows of 64 tokens 13.0 us against
-    // 16.1 with tiles of 32, 64 of 256 15.1 against 18.5, 128 of 128 15.8 against 18.8, eight queries of 64 rows and tokens 31.3 against
-    // 34.7; 50 rows on average of up to 600 23.3 against 23.2, 30 of up to 2000 49 against 32. The longest context of the pass is what
-    // its caller says, or else what a table row holds (a table for 4096 tokens without it: 16 rows of 16 tokens 13.7 us, 11.1 with it).
+    // The tiles of 16 rows have the shorter chain, those of 32 the higher rate: the line is drawn by the work of the whole pass, its rows times
+    // its longest context, which is what its caller says or else what a table row holds. us with tiles of 16 / 32, by queries x rows at
+    // tokens: 1x64 at 64 13.0 / 16.5, 8x5 at 100 12.4 / 15.5, 1x128 at 256 17.4 / 20.6, 4x32 at 256 18.5 / 21.6, 1x128 at 512 22.3 / 22.6,
+    // 4x32 at 512 23.3 / 23.5; at the line 1x128 at 768 26.7 / 25.4, 1x96 at 1024 26.7 / 22.6, 4x16 at 1536 26.2 / 25.5, 8x12 at 1024 33.6 / 33.1;
+    // above 1x128 at 2048 49.1 / 32.2, 8x32 at 1024 56.5 / 43.0. One query of few rows gains later: 1x8 at 8192 28.1 / 30.9, at 12288 37.2 / 40.2, at
+    // 16384 46.0 / 46.6, at 24000 63.7 / 61.4. Several queries of 17 to 31 rows on average gain earlier, because their tiles of 16 are reckoned
+    // too few (below): 2x24 at 1536 32.9 / 22.6, 4x24 at 768 36.9 / 24.7.
     // They also take partial results that are not on 16 bytes.
     const int64_t context = longest > 0 ? std::min(longest, capacity) : capacity;
-    const bool shortPass = rows * context < 24576 * int64_t(queryCount) || reinterpret_cast<uintptr_t>(partials) % 16 != 0;
+    const int64_t line = rows < 10 ? 131072 : queryCount > 1 && rows > 16 * int64_t(queryCount) && rows < 32 * int64_t(queryCount) ? 73728 : 98304;
+    const bool shortPass = rows * context < line || reinterpret_cast<uintptr_t>(partials) % 16 != 0;
     const int tileRows = shortPass ? kShortRows : kGroupRows;
     static PerDeviceOnce configured, shortConfigured;
     if (const cudaError_t e = shortPass ? configure_shared_memory(attention_group_kernel, sizeof(GroupShared), shortConfigured)
                                         : configure_shared_memory(attention_tile_kernel, kTileSharedBytes, configured))
       return e;
-    const int64_t tiles = std::max<int64_t>((rows + tileRows - 1) / tileRows, queryCount);
+    // How many rows each query has only the device knows. Queries of 33 to 63 rows on average are taken to have two tiles of 32 each: too few
+    // reckoned with is a second turn of items for some CTAs (4x48 at 1024 tokens with six tiles 51.6 us, with eight 37).
+    const int64_t perQuery = !shortPass && rows > 32 * int64_t(queryCount) && rows < 64 * int64_t(queryCount) ? 2 : 1;
+    const int64_t tiles = std::max<int64_t>((rows + tileRows - 1) / tileRows, perQuery * queryCount);
     const uint32_t most = uint32_t(std::clamp<int64_t>(sms / (kKvHeads * tiles), 1, splits));
     const int64_t items = (rows + queryCount) * kKvHeads * splits;  // no more than these
     const unsigned grid = unsigned(std::min<int64_t>(items, sms));

@@ -65,3 +65,13 @@ def test_the_longest_context_counts_and_not_the_width_of_the_table(dev, contexts
   assert wide.run(context=max(contexts)).tobytes() == narrow.tobytes()
   other = wide.run()  # the bound is gone after one call: tiles of 32 rows
   assert other.tobytes() != narrow.tobytes() and np.abs(other - narrow).max() < 1e-5 * np.abs(narrow).max()
+
+
+# The work of a pass (rows x the tokens a table row holds) below the line between the two kinds of tiles and on it: whole passes, passes of few rows, several
+# queries of 17 to 31 rows; queries of 33 to 63 rows, which are reckoned as two tiles each, and one beside a decode row.
+@pytest.mark.parametrize("contexts,counts,block_tokens", [
+  ([752], [128], 16), ([768], [128], 16), ([14560], [9], 16), ([14576], [9], 16), ([1520, 900], [24, 24], 16), ([1536, 900], [24, 24], 16),
+  ([320, 640, 1700], [33, 95, 40], 16), ([1000] * 4, [48] * 4, 16), ([1400, 1500, 1700], [40, 33, 62], 16), ([2000, 1500], [63, 1], 128)])
+def test_either_side_of_the_line_between_the_tiles(dev, contexts, counts, block_tokens):
+  rng = np.random.default_rng(sum(contexts) + len(counts))
+  assert run_attention(dev, rng, contexts, counts, block_tokens) < 1e-5
