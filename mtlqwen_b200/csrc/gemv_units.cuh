@@ -230,7 +230,7 @@ __device__ __forceinline__ void q6k_unit(const uint8_t* pA, const uint8_t* pB, i
   constexpr uint32_t k1056 = 0x64206420u;
 #pragma unroll(NT > 2 ? 1 : 2)
   for (int hh = 0; hh < 2; ++hh) {
-#pragma unroll(NT > 4 ? 1 : 2)
+#pragma unroll(NT > 3 ? 1 : 2)
     for (int u = 0; u < 2; ++u) {
       const uint32_t hiA = lds_u32_unaligned(pA + 128 + 32 * hh + 16 * u + 4 * t), hiB = lds_u32_unaligned(pB + 128 + 32 * hh + 16 * u + 4 * t);
 #pragma unroll
