@@ -394,10 +394,16 @@ template <class Q, int NMAT, int XSPLIT> __global__ void __launch_bounds__(kThre
           } else {
             q6k_unit(pA, pB, lane, rows, sum);
           }
-          const int mat = NMAT == 2 && int(mine - it) >= groups;
+          // a branch: chosen by a run-time index the sums would live in local memory
+          if (NMAT == 2 && int(mine - it) >= groups) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            (NMAT == 2 && mat ? total[NMAT - 1] : total[0])[0][i] += sum[0][i];
+            for (int i = 0; i < 4; ++i)
+              total[NMAT - 1][0][i] += sum[0][i];
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              total[0][0][i] += sum[0][i];
+          }
         }
         __syncwarp();
         if (lane == 0)

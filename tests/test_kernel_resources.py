@@ -27,6 +27,14 @@ def reports(tmp_path_factory):
     return dict(zip(("gemv.cu", "gemv_wide.cu"), pool.map(lambda name: compiled(name, directory), ("gemv.cu", "gemv_wide.cu"))))
 
 
+def test_gemv_keeps_no_array_in_local_memory(reports):
+  """A frame beyond the spills (rounded to eight bytes) is an array that is chosen from at run time."""
+  kernels = reports["gemv.cu"]
+  assert len(kernels) >= 12
+  for kernel, (stack, spills) in kernels.items():
+    assert stack <= (spills + 7) // 8 * 8, kernel
+
+
 def test_q6k_of_few_rows_is_decoded_without_spills(reports):
   kernels = {tiles: spills for (qtype, tiles), (_, spills) in reports["gemv_wide.cu"].items() if qtype == "Q6K"}
   assert sorted(kernels) == [(2, ), (3, ), (4, ), (5, )] and not any(kernels.values()), kernels
