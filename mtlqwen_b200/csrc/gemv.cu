@@ -36,13 +36,9 @@
 namespace infdev {
 namespace {
 
-constexpr int kConsumerWarps = 16;  // two halves of 8; consecutive ring stages alternate between the halves
 constexpr int kStageBlocks = kGemvStageBlocks;  // super-blocks per ring stage: one per warp of a half
 constexpr int kStageWarps = kStageBlocks;
-constexpr int kFinisherWarps = 2;
-constexpr int kProducerWarp = kConsumerWarps + kFinisherWarps;
-constexpr int kThreads = (kProducerWarp + 1) * kWarp;  // 608: 104 registers a thread
-constexpr int kChunkBlocks = 16;   // super-blocks of K per pass over the tiles (4096 values): two slabs, one per half
+
 constexpr int kTileRows = kGemvTileRows;
 
 // How a block type lies in a ring stage: kBoxes tiled copies of 16 rows x kStageBlocks / kBoxes super-blocks (a box is at
@@ -73,19 +69,28 @@ template <class Q> constexpr int row_pitch() { return box_blocks<Q>() * Q::kBloc
 template <class Q> constexpr int box_bytes() { return kTileRows * row_pitch<Q>(); }
 template <class Q> constexpr int stage_bytes() { return Q::kBoxes * box_bytes<Q>(); }
 
-constexpr int kLowBytes = kConsumerWarps * 16 * 32 * 8;  // low halves of the activations: [warp][fragment][lane]
-template <int NMAT, int XSPLIT> constexpr size_t fixed_bytes() {
-  return kRingControlBytes + (XSPLIT == 2 ? kLowBytes : 0) + size_t(kFinisherWarps) * NMAT * kConsumerWarps * 128 * 4;
-}
-// As many ring stages as fit beside that in the 227 KB a CTA may use; even, so that a slot always belongs to the same half of the
-// consumers (a half that ran ahead in a slot of the other one could find the parity of the phase before last).
-template <class Q, int NMAT, int XSPLIT> constexpr int stage_count() {
-  const int stages = int((size_t(227) * 1024 - fixed_bytes<NMAT, XSPLIT>()) / stage_bytes<Q>());
-  return (stages > kMaxStages ? kMaxStages : stages) / 2 * 2;
-}
-template <class Q, int NMAT, int XSPLIT> constexpr size_t smem_bytes() {
-  return fixed_bytes<NMAT, XSPLIT>() + size_t(stage_count<Q, NMAT, XSPLIT>()) * stage_bytes<Q>();
-}
+// Roles and shared memory of a CTA. HALVES: groups of eight consumer warps; with two, consecutive ring stages alternate between them.
+template <class Q, int NMAT, int XSPLIT, int HALVES> struct Layout {
+  static constexpr int kConsumers = kStageWarps * HALVES;
+  static constexpr int kChunkBlocks = kStageBlocks * HALVES;  // super-blocks of K per pass over the tiles: a slab per half
+  static constexpr int kLowBytes = XSPLIT == 2 ? kConsumers * 16 * 32 * 8 : 0;  // low halves of the activations: [warp][fragment][lane]
+  static constexpr size_t fixed_bytes(int finishers) { return kRingControlBytes + kLowBytes + size_t(finishers) * NMAT * kConsumers * 128 * 4; }
+  // As many ring stages as fit beside that in the 227 KB a CTA may use; with two halves an even number, so that a slot always belongs to
+  // the same one (a half that ran ahead in a slot of the other one could find the parity of the phase before last).
+  static constexpr int stages(int finishers) {
+    const int fit = int((size_t(227) * 1024 - fixed_bytes(finishers)) / stage_bytes<Q>());
+    return (fit > kMaxStages ? kMaxStages : fit) / HALVES * HALVES;
+  }
+  // A second finisher's buffer may not cost a half its second stage, without which it computes and copies in turn: a pair of Q8_0
+  // (12288 x 4096, eight rows) 36.8 us with two finishers and two stages, 25.8 with one and four; IQ4_XS and Q5_K, which have four and six
+  // with two finishers, 32.6 and 27.1 against 33.4 and 27.5.
+  static constexpr int kFinishers = stages(2) < 2 * HALVES ? 1 : 2;
+  static constexpr int kStages = stages(kFinishers);
+  static constexpr size_t kBytes = fixed_bytes(kFinishers) + size_t(kStages) * stage_bytes<Q>();
+  static constexpr int kProducer = kConsumers + kFinishers;  // warps: consumers, finishers, producer
+  static constexpr int kThreads = (kProducer + 1) * kWarp;
+  static_assert(kStages >= 2 && kStages >= HALVES, "a slot for each half");
+};
 
 // ---- Q4_K: one 16-row x 256-k unit -------------------------------------------------------------
 // Lane (g = lane/4, t = lane%4) owns weight rows g and g+8 and, in each, the 16-byte quant chunks t and
@@ -269,13 +274,14 @@ __device__ __forceinline__ void q4k_unit(uint32_t pA, uint32_t pB, int t, const 
   total[3] += xs.y * (dB.x * ((acc[0][3] + acc[1][3]) + (acc[2][3] + acc[3][3])) - dB.y * accm[3]);
 }
 
-template <class Q, int NMAT, int XSPLIT> __global__ void __launch_bounds__(kThreads, 1) gemv_kernel(const __grid_constant__ GemvParams p) {
-  constexpr int kStages = stage_count<Q, NMAT, XSPLIT>();
-  static_assert(kStages >= 2, "a slot for each half");
+template <class Q, int NMAT, int XSPLIT, int HALVES>
+__global__ void __launch_bounds__(Layout<Q, NMAT, XSPLIT, HALVES>::kThreads, 1) gemv_kernel(const __grid_constant__ GemvParams p) {
+  using L = Layout<Q, NMAT, XSPLIT, HALVES>;
+  constexpr int kConsumerWarps = L::kConsumers, kFinisherWarps = L::kFinishers, kProducerWarp = L::kProducer, kChunkBlocks = L::kChunkBlocks, kStages = L::kStages;
   extern __shared__ __align__(128) uint8_t smemRaw[];
   RingControl& ctl = *reinterpret_cast<RingControl*>(smemRaw);
   uint2* low = reinterpret_cast<uint2*>(smemRaw + kRingControlBytes);
-  float* partial = reinterpret_cast<float*>(smemRaw + kRingControlBytes + (XSPLIT == 2 ? kLowBytes : 0));
+  float* partial = reinterpret_cast<float*>(smemRaw + kRingControlBytes + L::kLowBytes);
   uint8_t* ring = reinterpret_cast<uint8_t*>(partial + kFinisherWarps * NMAT * kConsumerWarps * 128);
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -367,10 +373,10 @@ template <class Q, int NMAT, int XSPLIT> __global__ void __launch_bounds__(kThre
 #pragma unroll
       for (int mat = 0; mat < NMAT; ++mat)
         clear(total[mat]);
-      // `mine` is the next stage of this half (they are the stages congruent to `half` modulo 2), `slot` and `phase`
+      // `mine` is the next stage of this half (they are the stages congruent to `half` modulo HALVES), `slot` and `phase`
       // its place in the ring.
       const int perTile = NMAT * groups;
-      for (; mine < it + perTile; mine += 2, slot += 2) {
+      for (; mine < it + perTile; mine += HALVES, slot += HALVES) {
         if (slot >= kStages) {
           slot -= kStages;
           phase ^= 1;
@@ -426,15 +432,16 @@ template <class Q, int NMAT, int XSPLIT> __global__ void __launch_bounds__(kThre
   }
 }
 
-template <class Q, int NMAT, int XSPLIT> cudaError_t launch(const GemvParams& p, int sms, cudaStream_t stream) {
+template <class Q, int NMAT, int XSPLIT, int HALVES> cudaError_t launch_halves(const GemvParams& p, int sms, cudaStream_t stream) {
+  using L = Layout<Q, NMAT, XSPLIT, HALVES>;
   static PerDeviceOnce configured;
-  constexpr size_t bytes = smem_bytes<Q, NMAT, XSPLIT>();
-  if (cudaError_t e = configure_shared_memory(gemv_kernel<Q, NMAT, XSPLIT>, bytes, configured))
+  if (cudaError_t e = configure_shared_memory(gemv_kernel<Q, NMAT, XSPLIT, HALVES>, L::kBytes, configured))
     return e;
   const int grid = p.tiles < sms ? p.tiles : sms;
-  launch_kernel<1>(gemv_kernel<Q, NMAT, XSPLIT>, grid, kThreads, bytes, stream, p);
+  launch_kernel<1>(gemv_kernel<Q, NMAT, XSPLIT, HALVES>, grid, L::kThreads, L::kBytes, stream, p);
   return cudaGetLastError();
 }
+template <class Q, int NMAT, int XSPLIT> cudaError_t launch(const GemvParams& p, int sms, cudaStream_t stream) { return launch_halves<Q, NMAT, XSPLIT, 2>(p, sms, stream); }
 
 }  // namespace
 
