@@ -41,7 +41,7 @@ template <int NMAT> constexpr int stage_count() {
 }
 template <int NMAT> constexpr size_t smem_bytes() { return fixed_bytes<NMAT>() + size_t(stage_count<NMAT>()) * kQ4StageBytes; }
 
-template <int NMAT, int ROWS, bool IMAGE> __global__ void __launch_bounds__(kThreads, 1) q4k_decode_kernel(const __grid_constant__ GemvParams p) {
+template <int NMAT, int ROWS> __global__ void __launch_bounds__(kThreads, 1) q4k_decode_kernel(const __grid_constant__ GemvParams p) {
   constexpr int kStages = stage_count<NMAT>();
   extern __shared__ __align__(128) uint8_t smemRaw[];
   RingControl& ctl = *reinterpret_cast<RingControl*>(smemRaw);
@@ -131,9 +131,9 @@ template <int NMAT, int ROWS, bool IMAGE> __global__ void __launch_bounds__(kThr
     const bool live = myBlock < chunkBlocks;
     Fragments fragments;
     if (live)  // with a norm every warp: the row is one chunk of 16 super-blocks; one of the CTAs stores what a warp normalises
-      fragments = IMAGE ? load_fragments<ROWS>(p.image + size_t(chunk * kChunkBlocks + myBlock) * kImageBlockBytes, lane)
-                        : quantize_fragments<ROWS>(p.x + size_t(chunk * kChunkBlocks + myBlock) * 256, p.ldx, p.m, lane,
-                                                   {p.norm, myBlock % int(gridDim.x) == int(blockIdx.x) ? p.normalised : nullptr, squaresOfBlock, myBlock});
+      fragments = p.image ? load_fragments<ROWS>(p.image + size_t(chunk * kChunkBlocks + myBlock) * kImageBlockBytes, lane)
+                          : quantize_fragments<ROWS>(p.x + size_t(chunk * kChunkBlocks + myBlock) * 256, p.ldx, p.m, lane,
+                                                     {p.norm, myBlock % int(gridDim.x) == int(blockIdx.x) ? p.normalised : nullptr, squaresOfBlock, myBlock});
     int buffer = 0;
     for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, buffer = buffer == kFinisherWarps - 1 ? 0 : buffer + 1) {
       float total[NMAT][4];
@@ -204,17 +204,14 @@ __global__ void __launch_bounds__(256) activation_image_kernel(const float* x, i
   image_store_block(out, row, lane, v);
 }
 
-template <int NMAT, int ROWS, bool IMAGE> cudaError_t launch_source(const GemvParams& p, int sms, cudaStream_t stream) {
+template <int NMAT, int ROWS> cudaError_t launch(const GemvParams& p, int sms, cudaStream_t stream) {
   static PerDeviceOnce configured;
   constexpr size_t bytes = smem_bytes<NMAT>();
-  if (cudaError_t e = configure_shared_memory(q4k_decode_kernel<NMAT, ROWS, IMAGE>, bytes, configured))
+  if (cudaError_t e = configure_shared_memory(q4k_decode_kernel<NMAT, ROWS>, bytes, configured))
     return e;
   const int grid = p.tiles < sms ? p.tiles : sms;
-  launch_kernel<1>(q4k_decode_kernel<NMAT, ROWS, IMAGE>, grid, kThreads, bytes, stream, p);
+  launch_kernel<1>(q4k_decode_kernel<NMAT, ROWS>, grid, kThreads, bytes, stream, p);
   return cudaGetLastError();
-}
-template <int NMAT, int ROWS> cudaError_t launch(const GemvParams& p, int sms, cudaStream_t stream) {
-  return p.image ? launch_source<NMAT, ROWS, true>(p, sms, stream) : launch_source<NMAT, ROWS, false>(p, sms, stream);
 }
 
 // One or two rows pay for their own columns only: 12288 x 4096 with its image launch 12.5 -> 11.0 us at one row, 11.5 at two;
