@@ -117,7 +117,7 @@ struct Engine {
   // live sequences; from its second occurrence such a pass is captured once into a CUDA graph and then replayed.
   // The same holds for passes in which every query is a speculative decode of draftWidth + 1 rows (second index 1 + the class of
   // their longest context: the attention kernel that a graph holds was chosen by it).
-  static constexpr uint32_t contextClasses = 21;  // contexts up to 2^12, 2^13, .., 2^32 tokens
+  static constexpr uint32_t contextClasses = 23;  // contexts up to 2^10, 2^11, .., 2^32 tokens
   void* decodeGraphs[maxBatchSequences + 1][1 + contextClasses] = {};
   uint32_t decodeSeen[maxBatchSequences + 1][1 + contextClasses] = {};
   bool useGraphs = true;

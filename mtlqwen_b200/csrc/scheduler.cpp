@@ -359,7 +359,7 @@ void Engine::schedule() {
         }
         // A speculative pass knows the class of its contexts only, with a graph or without, so that its arithmetic is the same.
         if (uniform && batch.candidateRows) {
-          uint64_t bound = 4096;
+          uint64_t bound = 1024;  // up to there every pass of this kind takes the same kernels
           for (kind = 1; bound < batch.longestContext; bound *= 2)
             ++kind;
           batch.longestContext = uint32_t(std::min<uint64_t>(bound, UINT32_MAX));

@@ -380,7 +380,11 @@ def test_attention_hears_how_long_the_contexts_are(library, weights):
   sequence.close()
   sequence = engine.sequence(temperature=0.0, speculative=True)
   assert len(complete(sequence, tokens_of(21, 30), 8)) == 8
-  assert library.fake_infdev_shared_context() == 4096
+  assert library.fake_infdev_shared_context() == 1024
+  sequence.close()
+  sequence = engine.sequence(temperature=0.0, speculative=True)
+  assert len(complete(sequence, tokens_of(22, 1030), 8)) == 8
+  assert library.fake_infdev_shared_context() == 2048
   sequence.close()
   engine.close()
 
