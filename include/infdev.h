@@ -213,7 +213,8 @@ int infdev_attention_prepare(infdev_ctx* ctx, const float* qg, const float* k, c
                              int32_t tableStride, int32_t blockTokens, float* q, void* cacheK, void* cacheV);
 /* With qg == NULL only the K/V store runs: mtp_store_kv (attention.metal:53-100, drafter_store_kv<256>). */
 /* attention_scan + attention_reduce (attention.metal:103-216): causal GQA over the cache, times
- * sigmoid(gate). partials: scratch of infdev_attention_scratch_bytes(rows, maxSplits) bytes. */
+ * sigmoid(gate). partials: scratch of infdev_attention_scratch_bytes(rows, maxSplits) bytes. q and partials lie on 8-byte boundaries, the cache on
+ * 16-byte ones (anything else is refused); the rows of a prompt are served faster where q and partials lie on 16. */
 int infdev_attention(infdev_ctx* ctx, const float* q, const float* qg, const void* cacheK, const void* cacheV, const infdev_query* queries,
                      int queryCount, int64_t rows, const int32_t* table, int32_t tableStride, int32_t blockTokens, uint32_t maxSplits,
                      float* partials, float* out);

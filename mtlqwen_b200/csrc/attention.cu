@@ -1124,7 +1124,7 @@ cudaError_t attention_launch(const float* q, const float* qg, const void* cacheK
     // above 1x128 at 2048 49.1 / 32.2, 8x32 at 1024 56.5 / 43.0. One query of few rows gains later: 1x8 at 8192 28.1 / 30.9, at 12288 37.2 / 40.2, at
     // 16384 46.0 / 46.6, at 24000 63.7 / 61.4. Several queries of 17 to 31 rows on average gain earlier, because their tiles of 16 are reckoned
     // too few (below): 2x24 at 1536 32.9 / 22.6, 4x24 at 768 36.9 / 24.7.
-    // They also take partial results that are not on 16 bytes.
+    // They also take partial results that are on 8 bytes only.
     const int64_t context = longest > 0 ? std::min(longest, capacity) : capacity;
     const int64_t line = rows < 10 ? 131072 : queryCount > 1 && rows > 16 * int64_t(queryCount) && rows < 32 * int64_t(queryCount) ? 73728 : 98304;
     const bool shortPass = rows * context < line || reinterpret_cast<uintptr_t>(partials) % 16 != 0;

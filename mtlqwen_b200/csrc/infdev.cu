@@ -82,6 +82,11 @@ struct Bind {  // makes the context's device current for the calling thread
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+// The scan and the merge read q and partial results in pairs of floats, every kernel copies the cache in pieces of 16 bytes.
+bool attention_aligned(const float* q, const float* partials, const void* cacheK, const void* cacheV) {
+  return (reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(partials)) % 8 == 0 && aligned16(cacheK) && aligned16(cacheV);
+}
+
 // Whether two ranges of floats share one.
 bool overlap(const float* a, int64_t countA, const float* b, int64_t countB) {
   return a && b && reinterpret_cast<uintptr_t>(a) < reinterpret_cast<uintptr_t>(b + countB) && reinterpret_cast<uintptr_t>(b) < reinterpret_cast<uintptr_t>(a + countA);
@@ -865,6 +870,8 @@ int infdev_attention(infdev_ctx* ctx, const float* q, const float* qg, const voi
     return fail(ctx, INFDEV_E_ARGUMENT, "attention: rows without queries");
   if (blockTokens <= 0 || blockTokens % 16 || maxSplits < 1 || maxSplits > 64)
     return fail(ctx, INFDEV_E_ARGUMENT, "attention: blockTokens must be a multiple of 16 and maxSplits in 1..64");
+  if (!attention_aligned(q, partials, cacheK, cacheV))
+    return fail(ctx, INFDEV_E_ARGUMENT, "attention: q and partials must lie on 8-byte boundaries, the cache on 16-byte boundaries");
   int launches = 0;
   const cudaError_t e = infdev::attention_launch(q, qg, cacheK, cacheV, queries, queryCount, table, tableStride, blockTokens, rows, longest, maxSplits, partials, out,
                                                  take_capture(ctx), !ctx->umma, ctx->sms, ctx->status, ctx->stream, &launches);
@@ -890,6 +897,8 @@ int infdev_attention_static(infdev_ctx* ctx, const float* q, const float* qg, co
     return fail(ctx, INFDEV_E_ARGUMENT, "attention: rows without queries");
   if (blockTokens <= 0 || blockTokens % 16)
     return fail(ctx, INFDEV_E_ARGUMENT, "attention_static: blockTokens must be a positive multiple of 16");
+  if (!attention_aligned(q, nullptr, cacheK, cacheV))
+    return fail(ctx, INFDEV_E_ARGUMENT, "attention_static: q must lie on an 8-byte boundary, the cache on 16-byte boundaries");
   if (rows > infdev::attention_static_max_rows())
     return fail(ctx, INFDEV_E_ARGUMENT, "attention_static: at most " + std::to_string(infdev::attention_static_max_rows()) +
                                             " packed rows fit the built-in scratch; use infdev_attention with a caller-provided buffer");

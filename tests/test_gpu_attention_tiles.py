@@ -75,3 +75,23 @@ def test_the_longest_context_counts_and_not_the_width_of_the_table(dev, contexts
 def test_either_side_of_the_line_between_the_tiles(dev, contexts, counts, block_tokens):
   rng = np.random.default_rng(sum(contexts) + len(counts))
   assert run_attention(dev, rng, contexts, counts, block_tokens) < 1e-5
+
+
+@pytest.mark.parametrize("operand,offset", [("q", 1), ("partials", 1), ("partials", 3), ("keys", 2), ("values", 4)])
+def test_operands_that_the_copies_cannot_take_are_refused(dev, operand, offset):
+  """Floats by which q and the partial results miss a multiple of 8 bytes, halves by which the cache misses one of 16."""
+  work = Pass(dev, 93, [40], [1])
+  q, qg, keys, queries, table = work.held
+  values, out = dev.array(work.values.view(np.uint16)), dev.empty((1, 16, 256))
+  partials = dev.empty(dev.attention_scratch_bytes(1, 32) // 4 + 4)
+  operands = {"q": q.ptr, "keys": keys.ptr, "values": values.ptr, "partials": partials.ptr}
+  operands[operand] += offset * (2 if operand in ("keys", "values") else 4)
+  view = {name: type("View", (), {"ptr": ptr}) for name, ptr in operands.items()}
+  before = dev.lib.infdev_launch_count(dev.ctx)
+  with pytest.raises(RuntimeError, match="boundaries"):
+    dev.attention(view["q"], qg, view["keys"], view["values"], queries, 1, 1, table, work.stride, work.block_tokens, 32, view["partials"], out)
+  if operand != "partials":
+    with pytest.raises(RuntimeError, match="boundaries"):
+      dev.check(dev.lib.infdev_attention_static(dev.ctx, operands["q"], qg.ptr, operands["keys"], operands["values"], queries.ptr, 1, 1, table.ptr, work.stride,
+                                                work.block_tokens, out.ptr))
+  assert dev.lib.infdev_launch_count(dev.ctx) == before
