@@ -95,3 +95,74 @@ def test_operands_that_the_copies_cannot_take_are_refused(dev, operand, offset):
       dev.check(dev.lib.infdev_attention_static(dev.ctx, operands["q"], qg.ptr, operands["keys"], operands["values"], queries.ptr, 1, 1, table.ptr, work.stride,
                                                 work.block_tokens, out.ptr))
   assert dev.lib.infdev_launch_count(dev.ctx) == before
+
+
+def broken_rows(work, clean, got, query, token, dims):
+  """The rows of `query` from `token` on, in the heads of kv head 1, and nothing else, are not finite."""
+  first = int(work.starts[query]) + max(0, token - (work.contexts[query] - work.counts[query]))
+  hit = np.zeros_like(clean, bool)
+  for dim in dims:
+    hit[first:int(work.starts[query]) + work.counts[query], 4:8, dim] = True
+  assert not np.isfinite(got[hit]).any()
+  assert got[~hit].tobytes() == clean[~hit].tobytes()
+
+
+def break_value(work, values, query, token, dims, value):
+  values[work.table[query, token // work.block_tokens], 1, token % work.block_tokens, dims] = value
+
+
+# Contexts that the table is cut to, so that the first ones are served in tiles of 16 rows; the others in tiles of 32: several rounds of 256 tokens in one
+# piece, with the value in the first, at the ends and in the last; pieces of several rounds.
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("context,rows,token,max_splits", [
+  (40, 40, 39, 32), (40, 40, 17, 32), (200, 64, 150, 32), (90, 48, 60, 32), (90, 48, 3, 32),
+  (1200, 1100, 100, 1), (1200, 1100, 355, 1), (1200, 1100, 356, 1), (1200, 1100, 1199, 1), (1300, 64, 1260, 1), (1300, 64, 700, 1), (1300, 400, 1100, 2)])
+def test_rows_before_a_value_that_is_not_finite_do_not_notice(dev, context, rows, token, max_splits, value):
+  work, dims = Pass(dev, token, [context], [rows]), [7, 200]
+  clean, values = work.run(max_splits=max_splits), work.values.copy()
+  break_value(work, values, 0, token, dims, value)
+  broken_rows(work, clean, work.run(values, max_splits=max_splits), 0, token, dims)
+
+
+# 40 tiles of 32 rows in one piece each are 160 items: some CTAs take two, one after the other. The value is in an item of the first
+# turn, of the second, or in a tile that several items later has nothing of it.
+@pytest.mark.parametrize("query", [0, 17, 18, 19])
+def test_a_broken_value_stays_with_its_item(dev, query):
+  contexts, counts = [600 + 8 * i for i in range(20)], [64] * 20
+  work, dims = Pass(dev, 90, contexts, counts), [0, 255]
+  clean, values, token = work.run(max_splits=1), work.values.copy(), contexts[query] - 20
+  break_value(work, values, query, token, dims, np.nan)
+  broken_rows(work, clean, work.run(values, max_splits=1), query, token, dims)
+
+
+@pytest.mark.parametrize("contexts,counts", [([300], [128]), ([2000, 50], [100, 28])])
+def test_partial_results_eight_bytes_off(dev, contexts, counts):
+  work = Pass(dev, 91, contexts, counts)
+  want = work.run()
+  assert np.abs(work.run(offset=2) - want).max() < 1e-5 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("which", ["qg", "k", "v", "q_norm", "rope", "q", "cache"])
+def test_preparation_at_any_element(dev, which):
+  """An operand that misses a 16-byte boundary is read or written element by element, to the same bits."""
+  rows, block_tokens, rng = 37, 16, np.random.default_rng(92)
+  qg, k, v, q_norm, k_norm = (rng.standard_normal(shape).astype(np.float32) for shape in ((rows, 16, 512), (rows, 4, 256), (rows, 4, 256), 256, 256))
+  rope, blocks = dev.rope_table(rows + 5), -(-(rows + 5) // block_tokens)
+  table = dev.array(rng.permutation(blocks).astype(np.int32))
+  info = D.Query()
+  info.start, info.count, info.position, info.slot, info.state = 0, rows, 5, 0, D.UNBOUND
+
+  def run(moved):
+    def place(array, name):
+      array = np.ascontiguousarray(array)
+      shift = int(name == moved)
+      buffer = dev.array(np.concatenate([np.zeros(shift, array.dtype), array.reshape(-1), np.zeros(8, array.dtype)]))
+      return buffer, type("View", (), {"ptr": buffer.ptr + shift * array.itemsize}), lambda: buffer.download()[shift:shift + array.size].tobytes()
+
+    inputs = [place(a, name) for a, name in ((qg, "qg"), (k, "k"), (v, "v"), (q_norm, "q_norm"), (k_norm, "k_norm"), (rope.download(), "rope"))]
+    outputs = [place(np.zeros((rows, 16, 256), np.float32), "q")] + [place(np.zeros((blocks, 4, block_tokens, 256), np.uint16), "cache") for _ in range(2)]
+    dev.attention_prepare(*(view for _, view, _ in inputs), dev.queries([info]), 1, rows, table, blocks, block_tokens, *(view for _, view, _ in outputs))
+    dev.commit()
+    return [download() for _, _, download in outputs]
+
+  assert run(which) == run(None)
