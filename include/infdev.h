@@ -91,8 +91,9 @@ float infdev_event_elapsed_ms(infdev_ctx* ctx, void* start, void* stop);
  * than 8 rows decode a weight once for up to 40 rows (1) or go through the GEMV in slices (0). Environment: INFENG_UMMA. With 0,
  * infdev_attention also treats every row on its own. Otherwise, in a pass of 32 rows a query or more on average (of five, where
  * rows a query times the tokens that a table row can hold reach 4096), up to 16 rows of a query of several share the reading
- * of K and V, and the rounding of such a row's sums depends on its query's other rows and on how much else is in the pass; a
- * query of one row keeps the arithmetic that it has alone. */
+ * of K and V, or up to 32 where the rows of the pass times its longest context (infdev_attention_context, or else the tokens that a
+ * table row can hold) are many and q and partials lie on 16-byte boundaries. The rounding of such a row's sums depends on its
+ * query's other rows, on how much else is in the pass and on that bound; a query of one row keeps the arithmetic that it has alone. */
 int infdev_set_umma(infdev_ctx* ctx, int enabled);
 /* Activation split of the fp16 tensor-core GEMV: 2 = hi+lo fp16 (fp32-accurate, default), 1 = hi only. */
 int infdev_set_xsplit(infdev_ctx* ctx, int xsplit);
@@ -110,9 +111,10 @@ int infdev_set_integer_decode(infdev_ctx* ctx, int enabled);
 /* ---- activation images (no reference counterpart) ----
  * The integer Q4_K decode kernel reads its activations as an "image": per (row, 256-value block) 16-bit integers
  * split into a high and a low byte plane in tensor-core fragment order, the block's scale and its sub-block sums;
- * rows come in 8-row slices of k/256 blocks (4384 bytes per block and slice). A linear call builds the image from
- * its fp32 activations with one extra small launch; a pass avoids that launch by letting the kernel that produces
- * the activations write their image as well, and handing it to the linear call that follows. */
+ * rows come in 8-row slices of k/256 blocks (4384 bytes per block and slice). A linear call of one or two rows, or of
+ * up to eight with many results and k up to 4096, quantises its fp32 activations on the way into the kernel, with the
+ * same bits; any other builds the image with one extra small launch. A pass avoids that launch by letting the kernel that
+ * produces the activations write their image as well, and handing it to the linear call that follows. */
 size_t infdev_image_bytes(int64_t rows, int64_t k);
 /* image = quantised x[rows,k] (k a multiple of 256). */
 int infdev_quantize(infdev_ctx* ctx, const float* x, int64_t rows, int64_t k, uint8_t* image);

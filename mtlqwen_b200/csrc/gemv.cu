@@ -6,7 +6,8 @@
 // mlp_gate_up of Q4_K, Q5_K and IQ4_XS (fused_kernels.metal:11-200). The reference re-reads the weights once per
 // activation row (grid.y = rows); here up to 8 rows share one pass over the weights.
 //
-// Design (one persistent CTA per SM: 16 consumer warps, 2 finisher warps and 1 producer warp):
+// Design (one persistent CTA per SM: 16 consumer warps, or 8 where K is one slab, 2 finisher warps (1 where a pair's ring would be too
+// short) and 1 producer warp):
 //  * The weight matrix is a contiguous byte stream (row n = K/256 super-blocks). The producer warp moves
 //    16-row x 8-super-block slabs into a shared-memory ring with one tiled TMA copy each (a tensor map over
 //    the packed rows as 8-byte elements) that completes on an mbarrier; nothing else touches HBM for the weights.
@@ -21,10 +22,11 @@
 //    output head 248320 x 4096 Q6_K, eight rows 232 -> 211 us, 12288 x 4096 Q5_K 17.7 -> 16.0, Q8_0 16.7 -> 14.4, IQ4_XS 19.9 -> 18.2,
 //    4096 x 12288 (three chunks) Q6_K 24.8 -> 21.2, Q8_0 23.7 -> 19.9. Eight warps that held all their activations in registers,
 //    216 of them by setmaxnreg, measured 250 on the head: two warps a scheduler leave it idle while one waits for a product.
+//    (Sixteen leave a thread 96 registers: Q5_K spills five of them, which 12288 x 4096 does not show.)
 //  * Q4_K: A holds the exact integers sc*q (<= 945, exact in fp16); the super-block scale d is applied to
 //    the fp32 accumulator after each super-block, and the -dmin*m term is one more MMA against the
-//    per-sub-block activation sums. Q6_K: A holds q-32 exactly and the per-16 scale d*sc is applied to
-//    the accumulator after each MMA (one MMA = one scale group).
+//    per-sub-block activation sums. Q6_K: A holds q-32 exactly, the per-16 scale sc is applied to the
+//    accumulator after each MMA (one MMA = one scale group) and d once per super-block.
 //  * Activations are split x = hi + lo into two fp16 fragments (XSPLIT = 2) so the result keeps fp32
 //    accuracy; XSPLIT = 1 drops lo (relative error ~3e-4, still inside the 1e-3 contract).
 //  * Every mbarrier wait is bounded; on a timeout the kernel raises an abort flag, records a status code

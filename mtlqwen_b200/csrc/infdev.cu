@@ -644,7 +644,7 @@ static int linear_run(infdev_ctx* ctx, int type, bool pair, int count, const voi
         p.norm = norm.weight, p.normalised = norm.store ? norm.normalised + row * k : nullptr;
       } else if (supplied) {  // 8-row slices of k/256 blocks
         p.image = supplied + size_t(row / 8) * size_t(k / 256) * infdev::kActivationImageBlockBytes;
-      } else if (!inPlace && (p.m <= 2 ? p.m * k <= 24576 || p.tiles > ctx->sms : k <= 4096 && p.tiles > ctx->sms)) {
+      } else if (!inPlace && ((p.m <= 2 && p.m * k <= 24576) || (p.tiles > ctx->sms && (p.m <= 2 || k <= 4096)))) {
         // Every CTA quantises the activations itself, where reading them all takes no longer than a launch more: 12288 x 4096 with its
         // own image 9.7 (one row) and 11.2 us (eight), without 7.7 and 11.1 (4096 x 4096 4.8 and 7.0, 3.7 and 5.9); 4096 x 12288
         // 9.5 and 11.5, without 8.7 and 13.7, and 4096 x 8192 with three rows 8.7 and 9.6; 1024 x 4096, which is a start and an end
