@@ -54,7 +54,8 @@ struct UmmaParams {
   int splits;
   float* partial;
   int m, k;
-  int actRows;           // MMA N: m rounded up to a multiple of 16 (set by umma_launch)
+  int actRows;           // MMA N: m rounded up to a multiple of 16 (this and the next two set by umma_launch)
+  int stages, actStages; // ring slots: slabs of 128 rows x one super-block, activations of half a super-block
   const uint8_t* acts;   // prepared activations: k/256 blocks of actRows x 512 bytes
   int* status;
 };

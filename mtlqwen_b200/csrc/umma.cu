@@ -9,22 +9,26 @@
 //     activations, from shared memory through a matrix descriptor. The activations were rounded to fp16 beforehand
 //     (umma_prepare_rows_kernel), already laid out as canonical no-swizzle K-major core matrices under the same K
 //     permutation that the nibble extraction produces;
-//   * one 128-column fp32 accumulator per tile, double-buffered, so the epilogue of one overlaps the MMAs of the next. A gate /
-//     up pair takes both: every super-block of the activations is copied once and multiplied with both matrices (one after the other,
-//     with 96 CTAs on the activations twice, the copies were what the tensor cores waited for: 47.5 us for 12288 x 4096 with 128
-//     rows, 35.0 now), and silu(gate) * up is formed from the two accumulators.
-// Warp roles: 0 = TMA producer, 1 = MMA issuer (owns the TMEM allocation), 4..11 (4..19) = dequant (two or four groups of
-// four, one TMEM lane quadrant each), the last four = epilogue. Every mbarrier wait is bounded; on a timeout the kernel raises an abort
-// flag, records a status code, and every role leaves its loops.
-// The fp16 activations of a super-block are 64 KB, so weight slabs and activations travel through separate rings, the
-// activations in two halves of eight k-steps each: 4 slab stages + 4 half stages. Bulk prefetches of whole tiles into the L2, which
-// the producer once began with, got in the way of the copies (18944 x 16384 with 9 rows 71.9 -> 64.6 us without them, with 128 rows
-// 92.0 -> 84.3; all projections of a layer 88.3 -> 82.1 and 121.7 -> 112.9).
+//   * two fp32 accumulators of 128 columns: the halves of every super-block, added up at the end, or a gate / up pair, whose matrices
+//     share every copy of the activations and whose silu(gate) * up is formed from the two.
+// Warp roles: 0 = weight slabs, 1 = activations (one thread each issues the copies), 2 and 3 = MMA issuers (warp 2 owns the TMEM
+// allocation), 4..19 = four dequant groups of four warps (one TMEM lane quadrant each), which also store the results. Every mbarrier wait is
+// bounded; on a timeout the kernel raises an abort flag, records a status code, and every role leaves its loops.
+// Weight slabs (a super-block of 128 rows, 18 KB) and activations (half a super-block, 4 to 32 KB by the rows of the launch) travel through
+// rings of their own. The operand A has four places in tensor memory, half a super-block each, one per dequant group; the accumulators are two, one
+// per issuer. An issuer spends 430 to 700 clocks on the waits, eight MMAs and two commits of a half, whatever N; one issuer of both
+// halves was what set the pace of a pair (12288 x 4096, 128 rows 35.3 us, 29.1 with two; 9 rows 28.8 and 23.3).
+// Bulk prefetches of whole tiles into the L2 got in the way of the copies (18944 x 16384 with 9 rows 71.9 -> 64.6 us without them).
 // The kernel is launched programmatically dependent on the kernel that lays out the activations: set-up and the first
-// weight slab run while that one is still at work, and only the activation copies and the epilogue wait for it.
-// What bounds it, by its own clocks (18944 x 8192, every SM at work): with 128 rows the copies, 82 KB a super-block of which 64 are
-// activations, at 45 bytes a clock and SM (0.95 us; the 16 MMAs are 0.55); with few rows a dequant group's 1200 clocks a half. 96 tiles
-// (n = 12288) occupy 96 of 148 SMs.
+// weight slabs run while that one is still at work, and only the activation copies and the epilogue wait for it.
+// What bounds it, by its own clocks: a super-block of 128 rows takes a CTA 1000 to 1050 clocks with few rows (the dequant groups: 1200
+// warp instructions a scheduler for two, half the slots taken) and 1150 to 1220 with 128 (of which the MMAs are 1024). What is left is not in the loop: 4 to 5 us
+// from the end of the kernel before to the first MMA, through the layout kernel and two launches, and 1.5 us (a pair with 128 rows 3.3 us: silu)
+// of stores. 96 tiles (n = 12288) occupy 96 of 148 SMs. All projections of a layer, before the two issuers, the cheaper dequantisation and the
+// rings by row count, and now: 9 rows 78.1 -> 64.0 us, 40 rows 82.9 -> 68.5, 128 rows 101.0 -> 83.2.
+// Tried and left out: fp32 activations converted by four warps of the kernel itself instead of the layout kernel (12288 x 4096, 9 rows 16.0 us
+// against 14.1, 40 rows 20.5 against 14.9: copies of twice the bytes, and a proxy fence between every conversion and its MMAs); K slices as
+// clusters that add up over distributed shared memory instead of umma_reduce_kernel (4096 x 4096, 9 rows 8.8 against 8.6 us, 40 rows 10.1 against 9.5).
 #include "kernels.h"
 #include "tcgen05.cuh"
 
@@ -34,310 +38,308 @@ namespace {
 constexpr int kRows = kUmmaTileRows;      // weight rows per tile = TMEM lanes
 constexpr int kActs = 128;                // most activation rows per launch; the MMA N is the live rows rounded up to 16
 constexpr int kSlabBytes = kRows * 144;   // 18,432
-template <int GROUPS> constexpr int kThreads = (8 + 4 * GROUPS) * kWarp;  // GROUPS: dequant groups of four warps, 2 or 4
-// An even number of slab slots: a slot then always belongs to the same dequant groups (four groups take the super-blocks in
-// pairs by turns). Otherwise a group could find the parity of the phase before last in a slot whose slab for another group
-// had not landed yet, and read it ahead of its own copy.
-constexpr int kStages = 4, kActStages = 4;
-static_assert(kStages % 2 == 0, "a slot serves the same dequant groups throughout");
-constexpr int kActHalfBytes = 8 * kActs * 16 * 2;  // ring stage: 8 k-steps x [128 x 16] fp16; a launch of N rows uses N x 256 of it
+constexpr int kGroups = 4;                // dequant groups of four warps
+constexpr int kWeightWarp = 0, kActWarp = 1, kIssueWarp = 2, kFirstDequantWarp = 4;  // two issuers: warps 2 and 3
+constexpr int kThreads = (kFirstDequantWarp + 4 * kGroups) * kWarp;
+constexpr int kMaxStages = 10, kMaxActStages = 8;
 // kind::f16 instruction descriptor: fp32 accumulate, fp16 A and B, both K-major, M = 128
 __device__ __forceinline__ uint32_t instruction_descriptor(int n) { return (1u << 4) | (uint32_t(n >> 3) << 17) | (uint32_t(kRows >> 4) << 24); }
 constexpr int kTmemCols = 512;
-constexpr uint32_t kColA = 0, kColD = 256;  // A: ring of 4 x 64 columns, half a super-block each; D: 2 x 128 columns
-constexpr uint32_t kABuffers = 4;
+constexpr uint32_t kColA = 0, kColD = 256;  // A: 64 columns (half a super-block) per dequant group; D: 128 columns per issuer
 
 struct Control {
-  uint64_t full[8], slotFree[8], actFull[8], actFree[8], aReady[kABuffers], aFree[kABuffers], dReady[2], dFree[2];
+  uint64_t full[kMaxStages], slotFree[kMaxStages], actFull[kMaxActStages], actFree[kMaxActStages], aReady[kGroups], aFree[kGroups], dReady, dFree;
   uint32_t tmemBase;
   int abort;
 };
 constexpr int kControlBytes = 512;
 static_assert(sizeof(Control) <= kControlBytes, "control block too large");
-constexpr size_t kSharedBytes = 1024 + kControlBytes + size_t(kStages) * kSlabBytes + size_t(kActStages) * kActHalfBytes;
+// 222 KB, and registers for 768 threads, leave an SM room for a block of the small kernels before and after, which start early: with all of the
+// shared memory (a block without any takes 1 KB) they waited for SMs that have no CTA of this kernel (4096 x 4096, 24 rows 10.2 -> 8.9 us).
+constexpr int kBoundThreads = 768;
+constexpr size_t kSharedBytes = 222 * 1024, kRingBytes = kSharedBytes - 1024 - kControlBytes;
 
-__device__ __forceinline__ void tmem_load8(uint32_t address, float (&v)[8]) {
-  uint32_t r[8];
+__device__ __forceinline__ void tmem_load8(uint32_t address, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "r"(address)
                : "memory");
-  tmem_wait_load();
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-    v[i] = __uint_as_float(r[i]);
 }
 
-// The epilogue of one item for the 32 TMEM lanes (= weight rows = output columns) of the calling
-// warp: groups of eight activation rows `first`, `first + stride`, ... of the 16. Everything the store loop needs is
-// copied out of the parameter block first: the segment is a run-time index, so the block is reached through a generic
-// address, and the compiler must assume that the stores change it and would read pointer and pitch again after every
-// one of them (measured: 110 ns per store instead of 10).
-template <int NMAT> __device__ __forceinline__ void store_accumulator(const UmmaParams& p, int item, uint32_t accumulator, int row, int first, int stride) {
-  const int tile = item % p.tiles, slice = item / p.tiles;
+__device__ __forceinline__ int find_segment(const UmmaParams& p, int tile) {
   int segment = 0;
   while (segment + 1 < p.nseg && tile >= p.seg[segment + 1].tile0)
     ++segment;
-  const size_t pitch = size_t(p.seg[segment].ldy), column = size_t(tile - p.seg[segment].tile0) * kRows + row;
-  const int liveRows = p.m;
-  // a K slice: the partial sums are added up, with the residual, by umma_reduce_kernel
-  const bool parts = NMAT == 1 && p.splits > 1;
-  float* const y = parts ? p.partial + size_t(slice) * p.m * pitch : p.seg[segment].y;
-  const float* const residual = NMAT == 2 || parts ? nullptr : p.seg[segment].res;
-  for (int c = first; c < kActs / 8 && c * 8 < liveRows; c += stride) {
-    float v[8], up[8];
-    tmem_load8(accumulator + c * 8, v);
-    if (NMAT == 2)  // post == 2 epilogue, quant_linear.metal:224-232
-      tmem_load8(accumulator + kActs + c * 8, up);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int m = c * 8 + i;
-      if (m < liveRows) {
-        const size_t at = size_t(m) * pitch + column;
-        y[at] = NMAT == 2 ? silu_f(v[i]) * up[i] : residual ? v[i] + residual[at] : v[i];
-      }
-    }
-  }
+  return segment;
 }
 
-template <int NMAT, int GROUPS> __global__ void __launch_bounds__(kThreads<GROUPS>, 1) umma_linear_kernel(const __grid_constant__ UmmaParams p) {
+// Where the 32 TMEM lanes (= weight rows = output columns) of the calling warp go. Everything the store loop needs is copied out of the
+// parameter block: the segment is a run-time index, so the block is reached through a generic address, and the compiler must assume that
+// the stores change it and would read pointer and pitch again after every one of them (measured: 110 ns per store instead of 10).
+struct Destination {
+  float* y;
+  const float* residual;
+  size_t pitch;
+};
+template <bool PAIR> __device__ __forceinline__ Destination destination(const UmmaParams& p, int item, int row) {
+  const int tile = item % p.tiles, slice = item / p.tiles, segment = find_segment(p, tile);
+  Destination d;
+  d.pitch = size_t(p.seg[segment].ldy);
+  const size_t column = size_t(tile - p.seg[segment].tile0) * kRows + row;
+  // a K slice: the partial sums are added up, with the residual, by umma_reduce_kernel
+  const bool parts = !PAIR && p.splits > 1;
+  d.y = (parts ? p.partial + size_t(slice) * p.m * d.pitch : p.seg[segment].y) + column;
+  d.residual = PAIR || parts || !p.seg[segment].res ? nullptr : p.seg[segment].res + column;
+  return d;
+}
+// Eight activation rows of an item from `first` on.
+template <bool PAIR> __device__ __forceinline__ void store_rows(const Destination& d, int m, uint32_t accumulator, int first, const float (&residual)[8]) {
+  uint32_t v[8], w[8];
+  tmem_load8(accumulator + first, v);
+  tmem_load8(accumulator + kActs + first, w);
+  float* y = d.y + size_t(first) * d.pitch;
+  tmem_wait_load();
+#pragma unroll
+  for (int i = 0; i < 8; ++i, y += d.pitch) {
+    const float a = __uint_as_float(v[i]), b = __uint_as_float(w[i]);  // of a pair gate and up (post == 2 epilogue, quant_linear.metal:224-232)
+    if (first + i < m)
+      *y = PAIR ? silu_f(a) * b : a + b + residual[i];
+  }
+}
+template <bool PAIR> __device__ __forceinline__ void load_residual(const Destination& d, int m, int first, float (&residual)[8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    residual[i] = !PAIR && d.residual && first + i < m ? d.residual[size_t(first + i) * d.pitch] : 0.f;
+}
+
+template <bool PAIR> __global__ void __launch_bounds__(kBoundThreads, 1) umma_linear_kernel(const __grid_constant__ UmmaParams p) {
+  constexpr int kMats = PAIR ? 2 : 1;
   extern __shared__ uint8_t smemRaw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
   Control& ctl = *reinterpret_cast<Control*>(smem);
   uint8_t* ring = smem + kControlBytes;
-  uint8_t* actRing = ring + size_t(kStages) * kSlabBytes;  // halves of a super-block's activations
+  uint8_t* actRing = ring + size_t(p.stages) * kSlabBytes;
 
   pdl_launch_dependents();
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   // With p.splits > 1 (one matrix) the work items are (tile, K slice) pairs, so that a matrix of few 128-row tiles still
   // fills the GPU; `blocksPerRow` is then the super-blocks of one slice.
   const int blocksPerRow = p.k / 256 / p.splits, items = p.tiles * p.splits;
-  const uint32_t units = int(blockIdx.x) < items ? uint32_t((items - 1 - int(blockIdx.x)) / int(gridDim.x) + 1) : 0u;  // items of this CTA
-  constexpr uint32_t kDBuffers = 2 / NMAT;  // a pair's accumulators take both
+  const uint32_t stages = uint32_t(p.stages), actStages = uint32_t(p.actStages);
+  const uint32_t actBytes = uint32_t(p.actRows) * 256;  // half a super-block: 8 k-steps x [actRows x 16] fp16
   volatile int* abortFlag = &ctl.abort;
+  auto give_up = [&] {
+    *abortFlag = 1;
+    atomicExch(p.status, kStatusBarrierTimeout);
+  };
 
   if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (uint32_t s = 0; s < stages; ++s) {
       mbar_init(&ctl.full[s], 1);
       mbar_init(&ctl.slotFree[s], 8);  // the warps of the two groups that share a super-block
     }
-    for (int s = 0; s < kActStages; ++s) {
+    for (uint32_t s = 0; s < actStages; ++s) {
       mbar_init(&ctl.actFull[s], 1);
-      mbar_init(&ctl.actFree[s], 1);
+      mbar_init(&ctl.actFree[s], kMats);  // the issuers that read it
     }
-    for (uint32_t b = 0; b < kABuffers; ++b) {
-      mbar_init(&ctl.aReady[b], 4);  // the warps of one dequant group
-      mbar_init(&ctl.aFree[b], 1);
+    for (int g = 0; g < kGroups; ++g) {
+      mbar_init(&ctl.aReady[g], 4);  // the warps of the group
+      mbar_init(&ctl.aFree[g], 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&ctl.dReady[b], 1);
-      mbar_init(&ctl.dFree[b], 4);
-    }
+    mbar_init(&ctl.dReady, 2);
+    mbar_init(&ctl.dFree, 4 * kGroups);
     ctl.abort = 0;
     mbar_fence_init();
   }
-  if (warp == 1)
+  if (warp == kIssueWarp)
     tmem_alloc(&ctl.tmemBase, kTmemCols);
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem = ctl.tmemBase;
 
-  if (warp == 0) {
-    // ---------------- producer: one weight slab and two activation halves per super-block ----------------
-    const uint32_t halfBytes = uint32_t(p.actRows) * 256;  // 8 k-steps x [actRows x 16] fp16
-    uint32_t it = 0, slabs = 0, halves = 0;  // slabs, halves: copies issued
-    bool ok = true, waited = false;
-    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
-      const int tile = item % p.tiles, firstBlock = (item / p.tiles) * blocksPerRow;
-      int segment = 0;
-      while (segment + 1 < p.nseg && tile >= p.seg[segment + 1].tile0)
-        ++segment;
-      const int row0 = (tile - p.seg[segment].tile0) * kRows;
-      if (elect_one())  // the same lane every time: it keeps the counters
-        for (int sb = firstBlock; sb < firstBlock + blocksPerRow && ok; ++sb, ++it) {
-          for (int mat = 0; mat < NMAT && ok; ++mat) {
-            const uint32_t slab = it * NMAT + mat, slot = slab % kStages, round = slab / kStages;
-            if (round > 0)
-              ok = mbar_wait_bounded(&ctl.slotFree[slot], (round - 1) & 1, abortFlag);
+  if (warp == kWeightWarp) {
+    // ---------------- weight slabs: do not depend on the kernels before this one ----------------
+    if (elect_one()) {
+      uint32_t slot = 0, lap = 0, slabs = 0;
+      bool ok = true;
+      for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+        const int tile = item % p.tiles, firstBlock = (item / p.tiles) * blocksPerRow;
+        const int segment = find_segment(p, tile);
+        const int row0 = (tile - p.seg[segment].tile0) * kRows;
+        for (int sb = firstBlock; sb < firstBlock + blocksPerRow && ok; ++sb)
+          for (int mat = 0; mat < kMats && ok; ++mat) {
+            if (lap > 0)
+              ok = mbar_wait_bounded(&ctl.slotFree[slot], (lap - 1) & 1, abortFlag);
             if (ok) {
               mbar_arrive_expect_tx(&ctl.full[slot], kSlabBytes);
               tma_load_2d(ring + size_t(slot) * kSlabBytes, &p.map[segment][mat], sb * 18, row0, &ctl.full[slot]);
               ++slabs;
+              if (++slot == stages)
+                slot = 0, ++lap;
             }
           }
-          if (!waited) {  // the activations are the preceding kernel's output
-            pdl_wait();
-            waited = true;
-          }
-          for (int h = 0; h < 2 && ok; ++h) {  // the two activation halves of this super-block
-            const uint32_t half = 2 * it + h, actSlot = half % kActStages, actRound = half / kActStages;
-            if (actRound > 0)
-              ok = mbar_wait_bounded(&ctl.actFree[actSlot], (actRound - 1) & 1, abortFlag);
-            if (ok) {
-              mbar_arrive_expect_tx(&ctl.actFull[actSlot], halfBytes);
-              bulk_load(actRing + size_t(actSlot) * kActHalfBytes, p.acts + (size_t(sb) * 2 + h) * halfBytes, halfBytes, &ctl.actFull[actSlot]);
-              ++halves;
-            }
-          }
-          if (!ok) {
-            *abortFlag = 1;
-            atomicExch(p.status, kStatusBarrierTimeout);
+      }
+      if (!ok)
+        give_up();
+      // no copy may be in flight when the CTA ends, whoever gave up
+      for (uint32_t i = slabs > stages ? slabs - stages : 0; i < slabs; ++i)
+        mbar_wait_bounded(&ctl.full[i % stages], (i / stages) & 1, abortFlag);
+    }
+  } else if (warp == kActWarp) {
+    // ---------------- activations, by halves of a super-block: the preceding kernel's output ----------------
+    pdl_wait();
+    if (elect_one()) {
+      uint32_t slot = 0, lap = 0, copies = 0;
+      bool ok = true;
+      for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+        const int firstHalf = (item / p.tiles) * blocksPerRow * 2;
+        for (int half = firstHalf; half < firstHalf + blocksPerRow * 2 && ok; ++half) {
+          if (lap > 0)
+            ok = mbar_wait_bounded(&ctl.actFree[slot], (lap - 1) & 1, abortFlag);
+          if (ok) {
+            mbar_arrive_expect_tx(&ctl.actFull[slot], actBytes);
+            bulk_load(actRing + size_t(slot) * actBytes, p.acts + size_t(half) * actBytes, actBytes, &ctl.actFull[slot]);
+            ++copies;
+            if (++slot == actStages)
+              slot = 0, ++lap;
           }
         }
-      ok = __all_sync(0xffffffffu, ok);
+      }
+      if (!ok)
+        give_up();
+      for (uint32_t i = copies > actStages ? copies - actStages : 0; i < copies; ++i)
+        mbar_wait_bounded(&ctl.actFull[i % actStages], (i / actStages) & 1, abortFlag);
     }
-    // no copy may be in flight when the CTA ends, whoever gave up
+  } else if (warp < kFirstDequantWarp) {
+    // ---------------- MMA issuers: of a pair one matrix each, otherwise one half of every super-block ----------------
     if (elect_one()) {
-      for (uint32_t i = slabs > uint32_t(kStages) ? slabs - kStages : 0; i < slabs; ++i)
-        mbar_wait_bounded(&ctl.full[i % kStages], (i / kStages) & 1, abortFlag);
-      for (uint32_t i = halves > uint32_t(kActStages) ? halves - kActStages : 0; i < halves; ++i)
-        mbar_wait_bounded(&ctl.actFull[i % kActStages], (i / kActStages) & 1, abortFlag);
-    }
-  } else if (warp == 1) {
-    // ---------------- MMA issuer (one lane) ----------------
-    if (elect_one()) {
-      uint32_t it = 0, unit = 0;
+      const uint32_t issuer = uint32_t(warp - kIssueWarp);
+      uint32_t slot = PAIR ? 0 : issuer, parity = 0, count = 0, unit = 0;  // count: super-blocks
       bool ok = true;
       const uint32_t instruction = instruction_descriptor(p.actRows), stepBytes = uint32_t(p.actRows) * 32;
+      const uint32_t dColumn = tmem + kColD + issuer * kActs;
       for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++unit) {
-        const uint32_t buffer = unit % kDBuffers;
-        if (unit >= kDBuffers)
-          ok = mbar_wait_bounded(&ctl.dFree[buffer], (unit / kDBuffers - 1) & 1, abortFlag);
-        for (int j = 0; j < blocksPerRow && ok; ++j, ++it) {
-          for (int turn = 0; turn < 2 * NMAT && ok; ++turn) {  // eight k-steps per half of a super-block, of one matrix and the other
-            const uint32_t mat = turn >> 1, h = turn & 1, act = 2 * it + h, half = 2 * (it * NMAT + mat) + h, actSlot = act % kActStages, aBuffer = half % kABuffers;
-            const uint32_t dColumn = tmem + kColD + (NMAT == 2 ? mat : buffer) * 128;
-            ok = mbar_wait_bounded(&ctl.aReady[aBuffer], (half / kABuffers) & 1, abortFlag) &&
-                 mbar_wait_bounded(&ctl.actFull[actSlot], (act / kActStages) & 1, abortFlag);
+        if (unit > 0)
+          ok = mbar_wait_bounded(&ctl.dFree, (unit - 1) & 1, abortFlag);
+        for (int j = 0; j < blocksPerRow && ok; ++j, ++count) {
+#pragma unroll
+          for (int turn = 0; turn < kMats; ++turn) {
+            // the dequant group that fills this operand, and how often it has
+            const uint32_t half = PAIR ? uint32_t(turn) : issuer, group = PAIR ? 2 * issuer + half : 2 * (count & 1) + half, fill = PAIR ? count : count >> 1;
+            ok = ok && mbar_wait_bounded(&ctl.actFull[slot], parity, abortFlag) && mbar_wait_bounded(&ctl.aReady[group], fill & 1, abortFlag);
             if (!ok)
               break;
+            const uint64_t act = smem_descriptor(smem_u32(actRing + size_t(slot) * actBytes), 128, 256);
             fence_after_sync();
-            const uint32_t actBase = smem_u32(actRing + size_t(actSlot) * kActHalfBytes);
 #pragma unroll
-            for (int step = 0; step < 8; ++step)
-              umma_ts(dColumn, tmem + kColA + aBuffer * 64 + step * 8, smem_descriptor(actBase + step * stepBytes, 128, 256), instruction,
-                      (j | h | step) != 0);
-            if (mat == NMAT - 1)
-              umma_commit(&ctl.actFree[actSlot]);
-            umma_commit(&ctl.aFree[aBuffer]);
+            for (uint32_t step = 0; step < 8; ++step)
+              umma_ts(dColumn, tmem + kColA + group * 64 + step * 8, act + (step * stepBytes >> 4), instruction, uint32_t(j | turn) | step);
+            umma_commit(&ctl.aFree[group]);
+            umma_commit(&ctl.actFree[slot]);
+            if ((slot += PAIR ? 1 : 2) >= actStages)
+              slot -= actStages, parity ^= 1;
           }
-          if (!ok)
-            break;
-          if (j == blocksPerRow - 1)
-            umma_commit(&ctl.dReady[buffer]);
         }
+        if (ok)
+          umma_commit(&ctl.dReady);
       }
-      if (!ok) {
-        *abortFlag = 1;
-        atomicExch(p.status, kStatusBarrierTimeout);
-      }
+      if (!ok)
+        give_up();
     }
-  } else if (warp >= 4 && warp < 4 + 4 * GROUPS) {
-    // ---------------- dequant: thread = weight row; a group takes one half of every super-block (two groups) or of every
-    // second one (four). A lies in tensor memory as a ring of four halves, so a group fills one while the MMAs of another run.
-    // See umma_launch for which.
-    const int group = (warp - 4) >> 2, side = group & 1, quadrant = warp & 3, row = quadrant * 32 + lane;
-    constexpr uint32_t k1024 = 0x64006400u;
-    uint32_t it = 0;
+  } else {
+    // ---------------- dequant: thread = weight row; a group takes one half of every second slab and has a place of its own in tensor
+    // memory for it, so that a group fills its operand while the MMAs of the others run ----------------
+    const uint32_t group = uint32_t(warp - kFirstDequantWarp) >> 2, side = group & 1;
+    const int quadrant = warp & 3, row = quadrant * 32 + lane;
+    const uint32_t laneBase = tmem + (uint32_t(quadrant * 32) << 16), aAddress = laneBase + kColA + group * 64;
+    constexpr uint32_t k1024 = 0x64006400u, kSixteenth = 0x2c002c00u, kMinus64 = 0xd400d400u;
+    uint32_t slot = group >> 1, parity = 0, fills = 0, unit = 0, slab = group >> 1;  // slab: the next of this group, counted over all items
     bool ok = true;
-    for (int item = blockIdx.x; item < items && ok; item += gridDim.x)
-      for (int j = 0; j < blocksPerRow * NMAT && ok; ++j, ++it) {  // of a pair, the matrices in turn
-        if (GROUPS == 4 && (it & 1) != uint32_t(group >> 1))
-          continue;
-        const uint32_t slot = it % kStages, round = it / kStages, half = 2 * it + side, aBuffer = half % kABuffers;
-        ok = mbar_wait_bounded(&ctl.full[slot], round & 1, abortFlag);
-        if (ok && half >= kABuffers)
-          ok = mbar_wait_bounded(&ctl.aFree[aBuffer], (half / kABuffers - 1) & 1, abortFlag);
+    for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++unit) {
+      const uint32_t end = (unit + 1) * uint32_t(blocksPerRow * kMats);
+      for (; slab < end && ok; slab += 2, ++fills) {
+        ok = mbar_wait_bounded(&ctl.full[slot], parity, abortFlag);
         if (!ok)
           break;
-        fence_after_sync();
         const uint8_t* block = ring + size_t(slot) * kSlabBytes + row * 144;
         const uint4 header = *reinterpret_cast<const uint4*>(block);
-        const uint4* const quants = reinterpret_cast<const uint4*>(block + 16 + 64 * side);
-        uint4 quads[4];  // read ahead where other warps wait for the same pipe (a pair with 128 rows 37.3 -> 35.0 us; with two groups 1 % slower)
-        if (GROUPS == 4)
+        uint4 quads[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            quads[i] = quants[i];
-        const float2 dm = __half22float2(*reinterpret_cast<const __half2*>(&header.x));
+        for (int i = 0; i < 4; ++i)
+          quads[i] = *reinterpret_cast<const uint4*>(block + 16 + 64 * side + 16 * i);
         // 6-bit scales / mins of this half's four sub-blocks (scale_min_k4, quant_linear.metal:12-20)
         const uint32_t scales = side == 0 ? header.y & 0x3f3f3f3fu : (header.w & 0x0f0f0f0fu) | ((header.y >> 2) & 0x30303030u);
         const uint32_t mins = side == 0 ? header.z & 0x3f3f3f3fu : ((header.w >> 4) & 0x0f0f0f0fu) | ((header.z >> 2) & 0x30303030u);
-        const uint32_t aAddress = tmem + (uint32_t(quadrant * 32) << 16) + kColA + aBuffer * 64;
+        const __half2 dm = *reinterpret_cast<const __half2*>(&header.x), d = __low2half2(dm), dmin = __hneg2(__high2half2(dm));
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
-          const uint32_t pair = (scales >> (16 * t)) & 0xffffu, minPair = (mins >> (16 * t)) & 0xffffu;
-          const uint4 q0 = GROUPS == 4 ? quads[2 * t] : quants[2 * t], q1 = GROUPS == 4 ? quads[2 * t + 1] : quants[2 * t + 1];
+          // dequantised weight d*sc*q - dmin*m, in fp16: q, sc and m are made exact first (of the nibbles that lie as 16 q by a multiply-add,
+          // which saves two shifts of three), then the products d*sc and dmin*m are rounded once, as is the multiply-add of q.
+          const uint32_t scalePair = hsub2_u32(__byte_perm(scales, 0x64u, t == 0 ? 0x4140 : 0x4342), k1024);
+          const uint32_t minPair = hsub2_u32(__byte_perm(mins, 0x64u, t == 0 ? 0x4140 : 0x4342), k1024);
+          const __half2 s = __hmul2(d, *reinterpret_cast<const __half2*>(&scalePair)), n = __hmul2(dmin, *reinterpret_cast<const __half2*>(&minPair));
+          const __half2 sLow = __low2half2(s), sHigh = __high2half2(s), nLow = __low2half2(n), nHigh = __high2half2(n);
+          const uint32_t sL = *reinterpret_cast<const uint32_t*>(&sLow), sH = *reinterpret_cast<const uint32_t*>(&sHigh);
+          const uint32_t nL = *reinterpret_cast<const uint32_t*>(&nLow), nH = *reinterpret_cast<const uint32_t*>(&nHigh);
+          const uint4 q0 = quads[2 * t], q1 = quads[2 * t + 1];
           const uint32_t words[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-          // dequantised weight d*sc*q - dmin*m, in fp16: q is made exact first, then one fused multiply-add
-          const uint32_t sL = pack_half2(dm.x * float(pair & 0xffu), dm.x * float(pair & 0xffu));
-          const uint32_t sH = pack_half2(dm.x * float(pair >> 8), dm.x * float(pair >> 8));
-          const uint32_t nL = pack_half2(-dm.y * float(minPair & 0xffu), -dm.y * float(minPair & 0xffu));
-          const uint32_t nH = pack_half2(-dm.y * float(minPair >> 8), -dm.y * float(minPair >> 8));
           uint32_t v[32];
 #pragma unroll
           for (int w = 0; w < 8; ++w) {
-            const uint32_t a = words[w];
+            const uint32_t a = words[w], b = a >> 8;
             v[2 * w] = hfma2_u32(hsub2_u32((a & 0x000f000fu) | k1024, k1024), sL, nL);
-            v[2 * w + 1] = hfma2_u32(hsub2_u32(((a >> 8) & 0x000f000fu) | k1024, k1024), sL, nL);
-            v[16 + 2 * w] = hfma2_u32(hsub2_u32(((a >> 4) & 0x000f000fu) | k1024, k1024), sH, nH);
-            v[16 + 2 * w + 1] = hfma2_u32(hsub2_u32(((a >> 12) & 0x000f000fu) | k1024, k1024), sH, nH);
+            v[2 * w + 1] = hfma2_u32(hsub2_u32((b & 0x000f000fu) | k1024, k1024), sL, nL);
+            v[16 + 2 * w] = hfma2_u32(hfma2_u32((a & 0x00f000f0u) | k1024, kSixteenth, kMinus64), sH, nH);
+            v[16 + 2 * w + 1] = hfma2_u32(hfma2_u32((b & 0x00f000f0u) | k1024, kSixteenth, kMinus64), sH, nH);
+          }
+          if (t == 0) {  // the slab is in registers by now; the MMAs of this group's operand before may run until here
+            __syncwarp();
+            if (lane == 0)
+              mbar_arrive(&ctl.slotFree[slot]);
+            if (fills > 0)
+              ok = mbar_wait_bounded(&ctl.aFree[group], (fills - 1) & 1, abortFlag);
+            fence_after_sync();
           }
           tmem_store32(aAddress + 32 * t, v);
         }
-          tmem_wait_store();
+        tmem_wait_store();
         fence_before_sync();
         __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(&ctl.aReady[aBuffer]);
-          mbar_arrive(&ctl.slotFree[slot]);
-        }
+        if (lane == 0)
+          mbar_arrive(&ctl.aReady[group]);
+        if ((slot += 2) >= stages)
+          slot -= stages, parity ^= 1;
       }
-    if (ok && units > 0) {
-      // their share of the CTA's last accumulator (see the epilogue warps): groups of eight activation rows 1 + group,
-      // 2 + GROUPS + group, ...; the accumulator has no later user, so nobody waits for these reads
-      const uint32_t unit = units - 1, buffer = unit % kDBuffers;
-      pdl_wait();
-      ok = mbar_wait_bounded(&ctl.dReady[buffer], (unit / kDBuffers) & 1, abortFlag);
-      if (ok) {
-        fence_after_sync();
-        const int lastItem = int(blockIdx.x) + int(units - 1) * int(gridDim.x);
-        store_accumulator<NMAT>(p, lastItem, tmem + (uint32_t(quadrant * 32) << 16) + kColD + buffer * 128, row, 1 + group, 1 + GROUPS);
-      }
-    }
-    if (!ok && lane == 0) {
-      *abortFlag = 1;
-      atomicExch(p.status, kStatusBarrierTimeout);
-    }
-  } else if (warp >= 4 + 4 * GROUPS) {
-    // ---------------- epilogue: thread = weight row ----------------
-    pdl_wait();  // residuals, results and the partial-sum buffer belong to earlier kernels
-    const int quadrant = warp & 3, row = quadrant * 32 + lane;
-    const uint32_t laneBase = tmem + (uint32_t(quadrant * 32) << 16) + kColD;
-    uint32_t unit = 0;
-    bool ok = true;
-    for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++unit) {
-      const uint32_t buffer = unit % kDBuffers;
-      ok = mbar_wait_bounded(&ctl.dReady[buffer], (unit / kDBuffers) & 1, abortFlag);
+      // ---- epilogue: thread = weight row ----
+      pdl_wait();  // residuals, results and the partial-sum buffer belong to earlier kernels
+      const Destination to = destination<PAIR>(p, item, row);
+      const int m = p.m;
+      float residual[8];
+      load_residual<PAIR>(to, m, int(group) * 8, residual);
+      ok = ok && mbar_wait_bounded(&ctl.dReady, unit & 1, abortFlag);
       if (!ok)
         break;
       fence_after_sync();
-      // the CTA's last accumulator: the dequant warps, idle by then, take most of it
-      store_accumulator<NMAT>(p, item, laneBase + buffer * 128, row, 0, unit + 1 == units ? 1 + GROUPS : 1);
+      for (int first = int(group) * 8; first < m; first += kGroups * 8) {
+        float next[8];
+        load_residual<PAIR>(to, m, first + kGroups * 8, next);
+        store_rows<PAIR>(to, m, laneBase + kColD, first, residual);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          residual[i] = next[i];
+      }
       fence_before_sync();
       __syncwarp();
       if (lane == 0)
-        mbar_arrive(&ctl.dFree[buffer]);
+        mbar_arrive(&ctl.dFree);
     }
-    if (!ok && lane == 0) {
-      *abortFlag = 1;
-      atomicExch(p.status, kStatusBarrierTimeout);
-    }
+    if (!ok && lane == 0)
+      give_up();
   }
   fence_before_sync();
   __syncthreads();
-  if (warp == 1)
+  if (warp == kIssueWarp)
     tmem_dealloc(tmem, kTmemCols);
 }
 
@@ -388,18 +390,26 @@ __global__ void __launch_bounds__(256) umma_reduce_kernel(const float* partial, 
   *reinterpret_cast<float4*>(y + at) = sum;
 }
 
-template <int NMAT, int GROUPS> cudaError_t launch_tiles(const UmmaParams& params, const float* x, int ldx, int sms, cudaStream_t stream) {
+template <bool PAIR> cudaError_t launch_tiles(const UmmaParams& params, const float* x, int ldx, int sms, cudaStream_t stream) {
   static PerDeviceOnce configured;
-  if (const cudaError_t e = configure_shared_memory(umma_linear_kernel<NMAT, GROUPS>, kSharedBytes, configured))
+  if (const cudaError_t e = configure_shared_memory(umma_linear_kernel<PAIR>, kSharedBytes, configured))
     return e;
   // The MMA is as wide as the launch has rows, in steps of 16: a speculative pass of 40 rows moves 24 KB of activations
   // per super-block instead of 64 KB and spends a third of the tensor time.
   UmmaParams p = params;
   p.actRows = (p.m + 15) / 16 * 16;
+  const int actBytes = p.actRows * 256;
+  p.actStages = int((kRingBytes - 4 * kSlabBytes) / actBytes) / 2 * 2;
+  p.actStages = p.actStages > kMaxActStages ? kMaxActStages : p.actStages;
+  // An even number of slab slots: a slot then always belongs to the same dequant groups (they take the slabs in pairs by turns). Otherwise
+  // a group could find the parity of the phase before last in a slot whose slab for another group had not landed yet, and read it
+  // ahead of its own copy.
+  p.stages = int((kRingBytes - size_t(p.actStages) * actBytes) / kSlabBytes) / 2 * 2;
+  p.stages = p.stages > kMaxStages ? kMaxStages : p.stages;
   launch_kernel<1>(umma_prepare_rows_kernel, dim3(p.k / 256, p.actRows / 8), 256, 0, stream, x, ldx, p.m, p.actRows,
                 reinterpret_cast<__half*>(const_cast<uint8_t*>(p.acts)));
   const int items = p.tiles * p.splits, grid = items < sms ? items : sms;
-  launch_kernel<1>(umma_linear_kernel<NMAT, GROUPS>, grid, kThreads<GROUPS>, kSharedBytes, stream, p);
+  launch_kernel<1>(umma_linear_kernel<PAIR>, grid, kThreads, kSharedBytes, stream, p);
   if (p.splits > 1) {
     const size_t count = size_t(p.m) * p.seg[0].ldy;
     launch_kernel<1>(umma_reduce_kernel, unsigned((count / 4 + 255) / 256), 256, 0, stream, p.partial, p.splits, count, p.seg[0].res, p.seg[0].y);
@@ -411,13 +421,7 @@ template <int NMAT, int GROUPS> cudaError_t launch_tiles(const UmmaParams& param
 
 // 9 to 128 activation rows (p.m), rows of x `ldx` floats apart (a multiple of 4).
 cudaError_t umma_launch(bool pair, const UmmaParams& p, const float* x, int ldx, int sms, cudaStream_t stream) {
-  // Two dequant groups take a half of every super-block each, four of every second one. A pair wants four (12288 x 4096 with 9, 40 and
-  // 64 rows 28.8, 30.1 and 32.0 us, with two 32.4, 33.9 and 35.6): its activations come once for two super-blocks, so the dequantisation is what
-  // the MMAs wait for. One matrix with few rows wants two, which start and drain faster (4096 x 12288 with 9 and 64 rows 17.6 and 20.5,
-  // with four 18.7 and 21.1); with 128 rows four keep up with the MMAs (projections of a layer 124.6 us, with two 128.6).
-  if (pair)
-    return launch_tiles<2, 4>(p, x, ldx, sms, stream);
-  return p.m > 96 ? launch_tiles<1, 4>(p, x, ldx, sms, stream) : launch_tiles<1, 2>(p, x, ldx, sms, stream);
+  return pair ? launch_tiles<true>(p, x, ldx, sms, stream) : launch_tiles<false>(p, x, ldx, sms, stream);
 }
 
 }  // namespace infdev
