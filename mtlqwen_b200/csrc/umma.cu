@@ -21,14 +21,16 @@
 // Bulk prefetches of whole tiles into the L2 got in the way of the copies (18944 x 16384 with 9 rows 71.9 -> 64.6 us without them).
 // The kernel is launched programmatically dependent on the kernel that lays out the activations: set-up and the first
 // weight slabs run while that one is still at work, and only the activation copies and the epilogue wait for it.
-// What bounds it, by its own clocks: a super-block of 128 rows takes a CTA 1000 to 1050 clocks with few rows (the dequant groups: 1200
-// warp instructions a scheduler for two, half the slots taken) and 1150 to 1220 with 128 (of which the MMAs are 1024). What is left is not in the loop: 4 to 5 us
+// What bounds it, by its own clocks: a super-block of 128 rows takes a CTA about 850 clocks with few rows (the dequant groups, 500 warp
+// instructions a scheduler) and 1250 with 128 (of which the MMAs are 1024). What is left is not in the loop: 4 to 5 us
 // from the end of the kernel before to the first MMA, through the layout kernel and two launches, and 1.5 us (a pair with 128 rows 3.3 us: silu)
 // of stores. 96 tiles (n = 12288) occupy 96 of 148 SMs. All projections of a layer, before the two issuers, the cheaper dequantisation and the
-// rings by row count, and now: 9 rows 78.1 -> 64.0 us, 40 rows 82.9 -> 68.5, 128 rows 101.0 -> 83.2.
+// rings by row count, and now: 9 rows 78.1 -> 56.6 us, 40 rows 82.6 -> 59.7, 128 rows 100.8 -> 80.3.
 // Tried and left out: fp32 activations converted by four warps of the kernel itself instead of the layout kernel (12288 x 4096, 9 rows 16.0 us
 // against 14.1, 40 rows 20.5 against 14.9: copies of twice the bytes, and a proxy fence between every conversion and its MMAs); K slices as
-// clusters that add up over distributed shared memory instead of umma_reduce_kernel (4096 x 4096, 9 rows 8.8 against 8.6 us, 40 rows 10.1 against 9.5).
+// clusters that add up over distributed shared memory instead of umma_reduce_kernel (4096 x 4096, 9 rows 8.8 against 8.6 us, 40 rows 10.1 against 9.5);
+// equal parts of all tiles' super-blocks for all SMs, the last CTA of a shared tile adding up what the others left in global memory
+// (12288 x 4096, 9 rows 18.7 against 14.3, 128 rows 32.6 against 18.4: every CTA then ends two tiles, not one).
 #include "kernels.h"
 #include "tcgen05.cuh"
 
@@ -110,6 +112,42 @@ template <bool PAIR> __device__ __forceinline__ void load_residual(const Destina
 #pragma unroll
   for (int i = 0; i < 8; ++i)
     residual[i] = !PAIR && d.residual && first + i < m ? d.residual[size_t(first + i) * d.pitch] : 0.f;
+}
+
+// Whether one of two scales is not below 2^-6 (or not a number).
+__device__ __forceinline__ bool reaches_64th(const __half2& scales) {
+  return (((*reinterpret_cast<const uint32_t*>(&scales) & 0x7fff7fffu) + 0x5c005c00u) & 0x80008000u) != 0;
+}
+
+// 64 weights scale * q + low of two sub-blocks, in the order of the operand's columns: the low nibbles of eight words belong to the first, the
+// high ones to the second. SMALL: scales below 2^-6. The nibbles in bits 2..5 or 6..9 of a 16-bit group are fp16 numbers as they are, q x 2^-22
+// and q x 2^-18, and one multiply-add with the scale times 2^22 or 2^18, which is exact, gives the bits that the general form has: there q is
+// brought to an exponent of its own and made exact first (13 instructions for eight weights; 10 here, of which five on the
+// half-rate ALU pipe: projections of a layer with 9, 40 and 128 rows 64.1 -> 56.6, 67.2 -> 59.7 and 83.3 -> 80.3 us).
+template <bool SMALL> __device__ __forceinline__ void dequantise(const uint4& q0, const uint4& q1, const __half2& scale, const __half2& low, uint32_t (&v)[32]) {
+  constexpr uint32_t k1024 = 0x64006400u, kSixteenth = 0x2c002c00u, kMinus64 = 0xd400d400u, k2048 = 0x68006800u, k512 = 0x60006000u;
+  const __half2 scaleLow = __low2half2(scale), scaleHigh = __high2half2(scale), lowLow = __low2half2(low), lowHigh = __high2half2(low);
+  uint32_t sL = *reinterpret_cast<const uint32_t*>(&scaleLow), sH = *reinterpret_cast<const uint32_t*>(&scaleHigh);
+  const uint32_t nL = *reinterpret_cast<const uint32_t*>(&lowLow), nH = *reinterpret_cast<const uint32_t*>(&lowHigh);
+  if (SMALL)
+    sL = hmul2_u32(hmul2_u32(sL, k2048), k2048), sH = hmul2_u32(hmul2_u32(sH, k512), k512);
+  const uint32_t words[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    if (SMALL) {
+      const uint32_t a = words[w] << 2, b = words[w] >> 6;
+      v[2 * w] = hfma2_u32(a & 0x003c003cu, sL, nL);
+      v[2 * w + 1] = hfma2_u32(b & 0x003c003cu, sL, nL);
+      v[16 + 2 * w] = hfma2_u32(a & 0x03c003c0u, sH, nH);
+      v[16 + 2 * w + 1] = hfma2_u32(b & 0x03c003c0u, sH, nH);
+    } else {
+      const uint32_t a = words[w], b = a >> 8;
+      v[2 * w] = hfma2_u32(hsub2_u32((a & 0x000f000fu) | k1024, k1024), sL, nL);
+      v[2 * w + 1] = hfma2_u32(hsub2_u32((b & 0x000f000fu) | k1024, k1024), sL, nL);
+      v[16 + 2 * w] = hfma2_u32(hfma2_u32((a & 0x00f000f0u) | k1024, kSixteenth, kMinus64), sH, nH);
+      v[16 + 2 * w + 1] = hfma2_u32(hfma2_u32((b & 0x00f000f0u) | k1024, kSixteenth, kMinus64), sH, nH);
+    }
+  }
 }
 
 template <bool PAIR> __global__ void __launch_bounds__(kBoundThreads, 1) umma_linear_kernel(const __grid_constant__ UmmaParams p) {
@@ -253,7 +291,7 @@ template <bool PAIR> __global__ void __launch_bounds__(kBoundThreads, 1) umma_li
     const uint32_t group = uint32_t(warp - kFirstDequantWarp) >> 2, side = group & 1;
     const int quadrant = warp & 3, row = quadrant * 32 + lane;
     const uint32_t laneBase = tmem + (uint32_t(quadrant * 32) << 16), aAddress = laneBase + kColA + group * 64;
-    constexpr uint32_t k1024 = 0x64006400u, kSixteenth = 0x2c002c00u, kMinus64 = 0xd400d400u;
+    constexpr uint32_t k1024 = 0x64006400u;
     uint32_t slot = group >> 1, parity = 0, fills = 0, unit = 0, slab = group >> 1;  // slab: the next of this group, counted over all items
     bool ok = true;
     for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++unit) {
@@ -272,36 +310,41 @@ template <bool PAIR> __global__ void __launch_bounds__(kBoundThreads, 1) umma_li
         const uint32_t scales = side == 0 ? header.y & 0x3f3f3f3fu : (header.w & 0x0f0f0f0fu) | ((header.y >> 2) & 0x30303030u);
         const uint32_t mins = side == 0 ? header.z & 0x3f3f3f3fu : ((header.w >> 4) & 0x0f0f0f0fu) | ((header.z >> 2) & 0x30303030u);
         const __half2 dm = *reinterpret_cast<const __half2*>(&header.x), d = __low2half2(dm), dmin = __hneg2(__high2half2(dm));
+        // dequantised weight d*sc*q - dmin*m, in fp16: sc and m are made exact first, then the products d*sc and dmin*m are rounded once
+        __half2 scale[2], low[2];  // of sub-blocks 2t and 2t + 1
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
-          // dequantised weight d*sc*q - dmin*m, in fp16: q, sc and m are made exact first (of the nibbles that lie as 16 q by a multiply-add,
-          // which saves two shifts of three), then the products d*sc and dmin*m are rounded once, as is the multiply-add of q.
           const uint32_t scalePair = hsub2_u32(__byte_perm(scales, 0x64u, t == 0 ? 0x4140 : 0x4342), k1024);
           const uint32_t minPair = hsub2_u32(__byte_perm(mins, 0x64u, t == 0 ? 0x4140 : 0x4342), k1024);
-          const __half2 s = __hmul2(d, *reinterpret_cast<const __half2*>(&scalePair)), n = __hmul2(dmin, *reinterpret_cast<const __half2*>(&minPair));
-          const __half2 sLow = __low2half2(s), sHigh = __high2half2(s), nLow = __low2half2(n), nHigh = __high2half2(n);
-          const uint32_t sL = *reinterpret_cast<const uint32_t*>(&sLow), sH = *reinterpret_cast<const uint32_t*>(&sHigh);
-          const uint32_t nL = *reinterpret_cast<const uint32_t*>(&nLow), nH = *reinterpret_cast<const uint32_t*>(&nHigh);
-          const uint4 q0 = quads[2 * t], q1 = quads[2 * t + 1];
-          const uint32_t words[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-          uint32_t v[32];
+          scale[t] = __hmul2(d, *reinterpret_cast<const __half2*>(&scalePair)), low[t] = __hmul2(dmin, *reinterpret_cast<const __half2*>(&minPair));
+        }
+        // the slab is in registers by now; the MMAs that read this group's operand before may run until the first store
+        auto before_store = [&](int t) {
+          if (t > 0)
+            return;
+          __syncwarp();
+          if (lane == 0)
+            mbar_arrive(&ctl.slotFree[slot]);
+          if (fills > 0)
+            ok = mbar_wait_bounded(&ctl.aFree[group], (fills - 1) & 1, abortFlag);
+          fence_after_sync();
+        };
+        if (__any_sync(0xffffffffu, reaches_64th(scale[0]) || reaches_64th(scale[1]))) {
 #pragma unroll
-          for (int w = 0; w < 8; ++w) {
-            const uint32_t a = words[w], b = a >> 8;
-            v[2 * w] = hfma2_u32(hsub2_u32((a & 0x000f000fu) | k1024, k1024), sL, nL);
-            v[2 * w + 1] = hfma2_u32(hsub2_u32((b & 0x000f000fu) | k1024, k1024), sL, nL);
-            v[16 + 2 * w] = hfma2_u32(hfma2_u32((a & 0x00f000f0u) | k1024, kSixteenth, kMinus64), sH, nH);
-            v[16 + 2 * w + 1] = hfma2_u32(hfma2_u32((b & 0x00f000f0u) | k1024, kSixteenth, kMinus64), sH, nH);
+          for (int t = 0; t < 2; ++t) {
+            uint32_t v[32];
+            dequantise<false>(quads[2 * t], quads[2 * t + 1], scale[t], low[t], v);
+            before_store(t);
+            tmem_store32(aAddress + 32 * t, v);
           }
-          if (t == 0) {  // the slab is in registers by now; the MMAs of this group's operand before may run until here
-            __syncwarp();
-            if (lane == 0)
-              mbar_arrive(&ctl.slotFree[slot]);
-            if (fills > 0)
-              ok = mbar_wait_bounded(&ctl.aFree[group], (fills - 1) & 1, abortFlag);
-            fence_after_sync();
+        } else {
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            uint32_t v[32];
+            dequantise<true>(quads[2 * t], quads[2 * t + 1], scale[t], low[t], v);
+            before_store(t);
+            tmem_store32(aAddress + 32 * t, v);
           }
-          tmem_store32(aAddress + 32 * t, v);
         }
         tmem_wait_store();
         fence_before_sync();
