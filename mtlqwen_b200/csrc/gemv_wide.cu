@@ -36,6 +36,7 @@ namespace {
 constexpr int kConsumerWarps = 8;
 constexpr int kThreads = (kConsumerWarps + 2) * kWarp;  // + weight producer, + activation producer
 constexpr int kTileRows = kGemvTileRows;
+constexpr int kMaxSlices = 8;  // of K
 constexpr int kMaxDepth = 4;  // ring slots of a consumer warp
 constexpr int kMaxTiles = 5;  // a group's tiles of eight rows: the MMAs of four take longer than the decode, more tiles spill registers
 constexpr int kSharedBytes = 227 * 1024, kControlBytes = 1024;
@@ -341,8 +342,10 @@ template <class Q, int NT> __global__ void __launch_bounds__(kThreads, 1) wide_k
 }
 
 // Adds up the slices, four values per thread, and finishes: y = sum (+ residual), or silu(gate) * up for a pair. The columns of
-// all matrices lie side by side in a row of the partial results.
-__global__ void __launch_bounds__(256) wide_reduce_kernel(const __grid_constant__ WideParams p) {
+// all matrices lie side by side in a row of the partial results. AT_ONCE: a thread asks for all slices before it adds (projections of a layer of
+// mixed types with 9 and 16 rows 103.1 -> 99.6 and 104.4 -> 101.3 us); with many rows it is the number of resident blocks that counts, which takes
+// few registers (128 rows 491 us, at once 498).
+template <bool AT_ONCE> __global__ void __launch_bounds__(256) wide_reduce_kernel(const __grid_constant__ WideParams p) {
   pdl_launch_dependents();
   pdl_wait();
   const int width = p.pair ? p.pitch / 2 : p.pitch;
@@ -352,10 +355,21 @@ __global__ void __launch_bounds__(256) wide_reduce_kernel(const __grid_constant_
   const int row = int(at / width), column = int(at % width), slices = p.slices;
   auto total = [&](int from) {
     const float* partial = p.partial + size_t(row) * p.pitch + from;
+    auto add = [](float4& sum, const float4& v) { sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w; };
     float4 sum = *reinterpret_cast<const float4*>(partial);
-    for (int s = 1; s < slices; ++s) {
-      const float4 v = *reinterpret_cast<const float4*>(partial + s * count);
-      sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
+    if (AT_ONCE) {
+      float4 v[kMaxSlices];
+#pragma unroll
+      for (int s = 1; s < kMaxSlices; ++s)
+        if (s < slices)
+          v[s] = *reinterpret_cast<const float4*>(partial + s * count);
+#pragma unroll
+      for (int s = 1; s < kMaxSlices; ++s)
+        if (s < slices)
+          add(sum, v[s]);
+    } else {
+      for (int s = 1; s < slices; ++s)
+        add(sum, *reinterpret_cast<const float4*>(partial + s * count));
     }
     return sum;
   };
@@ -381,7 +395,7 @@ __global__ void __launch_bounds__(256) wide_reduce_kernel(const __grid_constant_
 int slices(const WideParams& p, int tilesPerGroup, int sms) {
   int best = 1;
   double least = 0;
-  for (int s = 1; s <= 8 && s <= p.blocks; ++s) {
+  for (int s = 1; s <= kMaxSlices && s <= p.blocks; ++s) {
     const int ctas = sms / (p.groups * s);
     if (ctas < 1 || ((s > 1 || p.pair) && size_t(s) * p.m * p.pitch > kWidePartialFloats))
       break;
@@ -423,7 +437,7 @@ template <class Q> cudaError_t launch(const WideParams& params, const float* x, 
   }
   *launches = 2;
   if (e == cudaSuccess && (p.pair || p.slices > 1)) {
-    launch_kernel<1>(wide_reduce_kernel, unsigned((size_t(p.m) * p.pitch / (p.pair ? 8 : 4) + 255) / 256), 256, 0, stream, p);
+    launch_kernel<1>(p.m <= 64 ? wide_reduce_kernel<true> : wide_reduce_kernel<false>, unsigned((size_t(p.m) * p.pitch / (p.pair ? 8 : 4) + 255) / 256), 256, 0, stream, p);
     *launches = 3;
     e = cudaGetLastError();
   }

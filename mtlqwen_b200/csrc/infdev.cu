@@ -530,13 +530,13 @@ static int linear_run(infdev_ctx* ctx, int type, bool pair, int count, const voi
     // A matrix of few 128-row tiles (n = 4096: 32 of them) would leave most SMs idle during prefill: cut K into slices.
     u.splits = 1;
     if (!pair && count == 1 && m > 8 && n[0] <= 8192 && n[0] % 4 == 0)
-      for (int s = 4; s > 1; --s)
+      for (int s = infdev::kUmmaMaxSplits; s > 1; --s)
         if ((k / 256) % s == 0 && tiles * s <= ctx->sms) {
           u.splits = s;
           break;
         }
     if (u.splits > 1 && !ctx->ummaPartial)
-      if (int r = check(ctx, cudaMalloc(reinterpret_cast<void**>(&ctx->ummaPartial), size_t(4) * 128 * 8192 * sizeof(float)), "prefill partial buffer"))
+      if (int r = check(ctx, cudaMalloc(reinterpret_cast<void**>(&ctx->ummaPartial), size_t(infdev::kUmmaMaxSplits) * 128 * 8192 * sizeof(float)), "prefill partial buffer"))
         return r;
     u.partial = ctx->ummaPartial;
     u.acts = static_cast<const uint8_t*>(ctx->ummaActs);

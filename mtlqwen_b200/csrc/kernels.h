@@ -43,7 +43,7 @@ constexpr int kImageCounters = 4096;  // arrival counters a context owns for blo
 constexpr int kActivationImageBlockBytes = 4384;  // act_image.cuh: image bytes per 256 activations x 8 rows
 
 // ---- tcgen05 path (umma.cu) ----
-constexpr int kUmmaTileRows = 128, kUmmaMaxActBytesPerBlock = 16 * 128 * 16 * 2;  // 64 KB of fp16 activations per super-block
+constexpr int kUmmaTileRows = 128, kUmmaMaxSplits = 4, kUmmaMaxActBytesPerBlock = 16 * 128 * 16 * 2;  // 64 KB of fp16 activations per super-block
 
 struct UmmaParams {
   alignas(64) CUtensorMap map[4][2];  // box = one super-block (18 x 8 bytes) x 128 rows

@@ -414,21 +414,36 @@ __global__ void __launch_bounds__(256) umma_prepare_rows_kernel(const float* x, 
   }
 }
 
-// y = partial[0] + partial[1] + ... (+ residual), four values per thread.
-__global__ void __launch_bounds__(256) umma_reduce_kernel(const float* partial, int splits, size_t count, const float* residual, float* y) {
+// y = partial[0] + partial[1] + ... (+ residual), four values per thread. AT_ONCE: a thread asks for all of them before it adds, one trip to
+// the L2 instead of one for each slice (4096 x 4096 with 9 and 40 rows 8.2 -> 7.7 and 9.0 -> 8.3 us). With more than 64 rows the blocks are so many that
+// what counts is how many of them fit beside the GEMM's CTAs and are there when it ends, which takes few registers (128 rows 11.5 us, at once 12.6).
+template <bool AT_ONCE> __global__ void __launch_bounds__(256) umma_reduce_kernel(const float* partial, int splits, size_t count, const float* residual, float* y) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t at = (size_t(blockIdx.x) * 256 + threadIdx.x) * 4;
   if (at >= count)
     return;
+  auto add = [](float4& sum, const float4& v) { sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w; };
   float4 sum = *reinterpret_cast<const float4*>(partial + at);
-  for (int s = 1; s < splits; ++s) {
-    const float4 v = *reinterpret_cast<const float4*>(partial + s * count + at);
-    sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
-  }
-  if (residual) {
-    const float4 v = *reinterpret_cast<const float4*>(residual + at);
-    sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
+  if (AT_ONCE) {
+    float4 slice[kUmmaMaxSplits], more = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int s = 1; s < kUmmaMaxSplits; ++s)
+      if (s < splits)
+        slice[s] = *reinterpret_cast<const float4*>(partial + s * count + at);
+    if (residual)
+      more = *reinterpret_cast<const float4*>(residual + at);
+#pragma unroll
+    for (int s = 1; s < kUmmaMaxSplits; ++s)
+      if (s < splits)
+        add(sum, slice[s]);
+    if (residual)
+      add(sum, more);
+  } else {
+    for (int s = 1; s < splits; ++s)
+      add(sum, *reinterpret_cast<const float4*>(partial + s * count + at));
+    if (residual)
+      add(sum, *reinterpret_cast<const float4*>(residual + at));
   }
   *reinterpret_cast<float4*>(y + at) = sum;
 }
@@ -455,7 +470,8 @@ template <bool PAIR> cudaError_t launch_tiles(const UmmaParams& params, const fl
   launch_kernel<1>(umma_linear_kernel<PAIR>, grid, kThreads, kSharedBytes, stream, p);
   if (p.splits > 1) {
     const size_t count = size_t(p.m) * p.seg[0].ldy;
-    launch_kernel<1>(umma_reduce_kernel, unsigned((count / 4 + 255) / 256), 256, 0, stream, p.partial, p.splits, count, p.seg[0].res, p.seg[0].y);
+    launch_kernel<1>(p.m <= 64 ? umma_reduce_kernel<true> : umma_reduce_kernel<false>, unsigned((count / 4 + 255) / 256), 256, 0, stream, p.partial, p.splits, count,
+                     p.seg[0].res, p.seg[0].y);
   }
   return cudaGetLastError();
 }
