@@ -42,10 +42,12 @@ __device__ __forceinline__ const infdev_query& query_of_row(const infdev_query* 
 //    the rows with the last three inputs of its channels in registers: every input is loaded once (a thread per output
 //    element loaded each four times and searched the query table for each: together with the gates 339 us for 2411 rows,
 //    where reading and writing everything once takes 30). State layout: conv taps fp32 [8192][4] at record + stateOffset.
-// CONV_ROWS rows per thread and GATE_HEADS heads per CTA: 8 and 8 where the rows alone fill the GPU, 1 and 1 for short prompt
-// pieces, which have too few CTAs otherwise and wait for one thread's chain of rows (the sums are the same either way).
+// CONV_ROWS rows per thread and GATE_HEADS heads per CTA (the sums are the same whatever they are): the rows of short prompt pieces are spread
+// thinly, so that no thread has a long chain of them; with more rows an SM, which holds two CTAs, would take them in several turns.
+// 1 and 1, 2 and 2, 4 and 4, 8 and 8: 24 rows 6.2 / 6.2 / 7.2 / 10.6 us, 32 rows 7.7 / 6.2 / 6.2 / 9.8, 40 rows 8.7 / 6.3 / 7.3 / 9.8, 64 rows 11.2 / 8.2 /
+// 7.4 / 9.8, 128 rows 17.5 / 11.8 / 9.8 / 10.8, 192 rows 24.1 / 15.2 / 12.9 / 13.0, 256 rows 30.3 / 19.4 / 15.6 / 14.2, 512 rows 55 / 34 / 26.8 / 24.1.
 // ALIGNED: mixed, convWeight, q, k and v lie on 16-byte boundaries; without, they are read and written value by value.
-constexpr int kGateRows = 8, kFewPrepareRows = 64;
+constexpr int kGateRows = 8, kPrepareRows1 = 24, kPrepareRows2 = 48, kPrepareRows4 = 192;  // most rows of each spread
 constexpr int kConvChannels = 4 * 256;  // per CTA
 
 template <bool ALIGNED> __device__ __forceinline__ float4 load_four(const float* p) {
@@ -925,15 +927,18 @@ cudaError_t gdn_prepare_launch(const float* x, const float* mixed, const float* 
     launch_kernel<2>(kernel, unsigned(gateBlocks + convBlocks), 256, 0, stream, x, wBeta, wAlpha, A, dt, mixed, convWeight, queries, int(rows), gateBlocks,
                      stateOffset, stateBytes, q, k, v, beta, g);
   };
-  // With the delta rule after it: 2 rows 17.2 against 22.2 us, 16 rows 19.7 against 25.3, 64 rows level, 96 rows 47.1 against 45.3.
   // A caller's views may start at any float.
   uintptr_t addresses = 0;
   for (const float* p : {mixed, convWeight, static_cast<const float*>(q), static_cast<const float*>(k), static_cast<const float*>(v)})
     addresses |= reinterpret_cast<uintptr_t>(p);
   if (addresses & 15)
     launch(gdn_prepare_kernel<1, 1, false>, 1, 1);
-  else if (rows <= kFewPrepareRows)
+  else if (rows <= kPrepareRows1)
     launch(gdn_prepare_kernel<1, 1, true>, 1, 1);
+  else if (rows <= kPrepareRows2)
+    launch(gdn_prepare_kernel<2, 2, true>, 2, 2);
+  else if (rows <= kPrepareRows4)
+    launch(gdn_prepare_kernel<4, 4, true>, 4, 4);
   else
     launch(gdn_prepare_kernel<8, 8, true>, 8, 8);
   return cudaGetLastError();
