@@ -10,6 +10,7 @@
 // written once (or once per token for speculative queries, whose every row must stay selectable). The
 // reference makes two passes over the state in device memory per token (delta_rule.metal:320-333, 351-360).
 #include <cuda_bf16.h>
+#include <algorithm>
 #include "act_image.cuh"
 #include "kernels.h"
 #include "ops.h"
@@ -184,6 +185,44 @@ __global__ void __launch_bounds__(256, 2) gdn_prepare_kernel(const float* x, con
   }
 }
 
+// The queries that the chunked kernel takes.
+__device__ __forceinline__ bool chunked(const infdev_query& info, uint32_t chunkedFrom) { return chunkedFrom && info.state == kUnbound && info.count >= chunkedFrom; }
+// How many they are among up to 32; more count as 32. Every lane of a warp calls.
+__device__ __forceinline__ uint32_t chunked_queries(const infdev_query* queries, uint32_t count, uint32_t chunkedFrom) {
+  const uint32_t lane = threadIdx.x & 31;
+  return count > 32 ? 32 : __popc(__ballot_sync(0xffffffffu, lane < count && chunked(queries[lane], chunkedFrom)));
+}
+
+// gated_rms_norm_128 of one head of a query's rows, in place: eight warps, eight rows each at a time.
+__device__ __forceinline__ void gated_norm_rows(float* out, const float* z, const float* normWeight, uint32_t start, uint32_t count, int head) {
+  constexpr uint32_t kRows = 8;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr size_t kPitch = size_t(kValueHeads) * kHeadDim;
+  float weight[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    weight[c] = normWeight[lane + 32 * c];
+  for (uint32_t first = warp * kRows; first < count; first += 8 * kRows) {
+    float o[kRows][4], gate[kRows][4];
+    const size_t at = size_t(start + first) * kPitch + size_t(head) * kHeadDim + lane;
+#pragma unroll
+    for (uint32_t r = 0; r < kRows; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        o[r][c] = first + r < count ? out[at + r * kPitch + 32 * c] : 0.f;
+        gate[r][c] = first + r < count ? z[at + r * kPitch + 32 * c] : 0.f;
+      }
+#pragma unroll
+    for (uint32_t r = 0; r < kRows; ++r) {
+      const float scale = rsqrtf(warp_sum(o[r][0] * o[r][0] + o[r][1] * o[r][1] + o[r][2] * o[r][2] + o[r][3] * o[r][3]) / float(kHeadDim) + 1.0e-6f);
+      if (first + r < count)
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          out[at + r * kPitch + 32 * c] = o[r][c] * scale * weight[c] * silu_f(gate[r][c]);
+    }
+  }
+}
+
 // grid (32 value heads, queries), 256 threads. Thread (part = tid/32, lane) owns S[k][4*lane .. 4*lane+3]
 // for k = part + 8*i, i < 16.
 // `image`, when not null, also receives the activation image of `out`. A 256-value block holds two heads, which two
@@ -253,8 +292,11 @@ __global__ void __launch_bounds__(256, 2) delta_rule_kernel(const float* q, cons
   const infdev_query info = queries[blockIdx.y];
   const int head = blockIdx.x, keyHead = head % kKeyHeads, tid = threadIdx.x, part = tid >> 5, lane = tid & 31;
   const bool speculative = info.state != kUnbound;
-  if (chunkedFrom && !speculative && info.count >= chunkedFrom)  // delta_rule_chunked_kernel takes this query
+  if (!FUSED && chunked(info, chunkedFrom)) {  // delta_rule_chunked_kernel had this query, all but its norm
+    if (z)
+      gated_norm_rows(out, z, normWeight, info.start, info.count, head);
     return;
+  }
   __shared__ float qraw[kHeadDim], kraw[kHeadDim], vraw[kHeadDim], red[12], dots[8];
   __shared__ float4 partialPred[8][32], partialQ[8][32];
   const int channels[3] = {keyHead * kHeadDim + (tid & 127), 2048 + keyHead * kHeadDim + (tid & 127), 4096 + head * kHeadDim + (tid & 127)};
@@ -442,15 +484,18 @@ __global__ void __launch_bounds__(256, 2) delta_rule_kernel(const float* q, cons
 //   delta  = A^-1 rhs,   rhs_t = beta_t * (v_t - G_t * S^T k_t)
 //   o_t    = G_t * S^T q_t + sum_{i<=t} R[t][i] (q_t . k_i) delta_i
 //   S      = G_15 * S + sum_i (G_15 / G_i) k_i delta_i^T
-// grid (32 value heads, queries), 8 + 4 warps; serves the non-speculative queries of at least `chunkedFrom` tokens. A last
+// grid (32 value heads, queries and the second halves of some), 12 warps; serves the non-speculative queries of at least `chunkedFrom` tokens, all
+// but the norm of their outputs, which is delta_rule_kernel's launch (gated_norm_rows): here it stood in the chain, 2000 of 8200 clocks a chunk. A last
 // chunk of fewer than 16 tokens is padded with tokens of beta = 0, k = q = v = 0 and decay 1, which change nothing.
 //
 // A query is a chain of chunks per head, so what counts is the time of one chunk. Everything that does not depend on S - the
 // normalised keys and queries, the gates, A^-1 and the weights of the second sum - is prepared by four warps of their own,
 // a chunk or two ahead, in two shared-memory buffers. The eight others hold S^T in registers, 16 value columns each: a warp
-// needs nothing from its neighbours until the norm of the output, because a value column's recurrence is its own. All
+// needs nothing from its neighbours, because a value column's recurrence is its own. All
 // products run on the tensor cores; a warp's accumulators (value column x key dim, or x token) are at the same time, as they
 // lie in its registers, the A operand of the next product.
+// Where no more than two queries are chunked (64 CTAs of 148 SMs), a head's columns go to two CTAs: four computing warps then have the tensor
+// cores of an SM to themselves, and the four that are left over prepare every second chunk.
 //
 // Precision. Keys, queries, S and the update of S are split into fp16 hi + lo after scaling by a power of two (fixed for keys
 // and queries, whose norm is at most 1; by the largest value of each value column for the others), and the three products that
@@ -463,12 +508,14 @@ __global__ void __launch_bounds__(256, 2) delta_rule_kernel(const float* q, cons
 // token by token 1.1e-7 and 0.7e-7. One scale for the 16 columns of a warp, fp16 parts throughout and sums carried in the
 // accumulators gave 4.1e-7 and 5.4e-7, and lost value columns far below their neighbours; they took 278 us for eight queries
 // of 59 to 493 rows, this form 311 us.
-// A chunk takes about 4.7 us (one query of 512 rows: 32 chunks, 173 us with the preparation); its 168 MMAs per warp are 1.4 us
-// of them at the measured 8.06 cycles per MMA and scheduler (tensor pipe 32 % of the active cycles over eight queries, 0.44
-// issued per cycle and scheduler), the rest is the chain of products that wait for each other. The
-// fp32 form, FMAs with eight partial sums per product through shared memory, took 12 us.
+// By its own clocks a chunk takes 5000 with half of the columns (KS and QS 1900, A^-1 rhs 550, the second sum 500, the update 1000, the rest
+// stores, scales and barriers) and 6900 with all (2800, 700, 700, 1400), where the preparing warps are as slow as that; 8200 when the norm was part of
+// the chain and one preparing warp had gates, decays and the inverse. Eight queries of 59 to 493 rows 200 -> 187 us, one of 493 rows 143 -> 110,
+// of 128 rows 42.1 -> 33.9, of 64 rows 24.8 -> 20.6. Tried and left out: the outputs by warps of their own that are handed S through shared
+// memory (200 -> 244 us), two of the preparing warps a stage behind the two others (187 -> 222), 16 warps of 128 registers (237).
 constexpr int kChunk = 16, kComputeWarps = 8, kPrepareWarps = 4;
 constexpr int kChunkThreads = (kComputeWarps + kPrepareWarps) * kWarp;
+constexpr int kSplitWarps = kComputeWarps / 2;  // computing warps of a CTA that has half of a head's value columns
 constexpr float kKeyUnit = 256.f;  // fixed scale of the normalised keys and queries
 using TokenMatrix = __nv_bfloat16[3][kChunk][kChunk + 8];  // lower triangular, [part][token][token]
 struct ChunkBuffer {
@@ -478,14 +525,13 @@ struct ChunkBuffer {
 };
 struct ChunkShared {
   ChunkBuffer buffer[2];
-  // of the chunk being prepared, two sets in turn: warp 1 reads one while warp 0 may already write the next chunk's, and a set
+  // of the chunk being prepared, two sets in turn: warp 1 reads one while warp 3 may already write the next chunk's, and a set
   // comes up again only behind the barrier that frees its buffer
   double cumulative[2][kChunk];
   float gateBeta[2][kChunk];
-  float system[kChunk][kChunk + 1];
-  float squares[2][kComputeWarps][kChunk];
+  float system[2][kChunk][kChunk + 1], ratio[2][kChunk][kChunk + 1];  // of each preparing group: the triangular system; R
 };
-// named barriers: 1, 2 buffer filled; 3, 4 buffer free; 5 the preparing warps; 6 the computing warps
+// named barriers: 1, 2 buffer filled; 3, 4 buffer free; 5, 6 a preparing group
 __device__ __forceinline__ void chunk_ldmatrix(uint32_t (&r)[4], const void* address) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(address)) : "memory");
 }
@@ -613,13 +659,15 @@ __device__ __forceinline__ void store_three(TokenMatrix& to, int t, int i, float
   }
 }
 
-// The four preparing warps: chunk after chunk into the two buffers.
+// The four preparing warps: chunk after chunk into the two buffers. All normalise four tokens each; then warps 0 and 1 have the products
+// k . k and q . k while 2 and 3 form the decays between the tokens, and warp 3 cumulates the gates of the next chunk while warp 0 inverts.
 __device__ __forceinline__ void chunk_prepare(ChunkShared& sh, const infdev_query& info, const float* q, const float* k, const float* g, const float* beta,
-                                              int head) {
-  const int warp = (threadIdx.x >> 5) - kComputeWarps, lane = threadIdx.x & 31, keyHead = head % kKeyHeads;
+                                              int head, int group, int groups, int threads) {
+  const int warp = (threadIdx.x >> 5) % kPrepareWarps, lane = threadIdx.x & 31, keyHead = head % kKeyHeads;
   const int tokenOfB = (lane & 7) + 8 * (lane >> 4), dimOfB = 8 * ((lane >> 3) & 1);  // ldmatrix rows of a B operand stored [n][k]
   float4 nextQ[4], nextK[4];
   float nextG = 0.f, nextBeta = 0.f;
+  double cumulative = 0.0;  // warp 3: of the next chunk's tokens
   auto load = [&](uint32_t first) {  // warp w: tokens 4w .. 4w + 3
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -630,18 +678,34 @@ __device__ __forceinline__ void chunk_prepare(ChunkShared& sh, const infdev_quer
         nextQ[j] = *reinterpret_cast<const float4*>(q + at), nextK[j] = *reinterpret_cast<const float4*>(k + at);
       }
     }
-    if (warp == 0) {
+    if (warp == 3) {
       const bool live = lane < kChunk && first + lane < info.count;
       nextG = live ? g[size_t(info.start + first + lane) * kValueHeads + head] : 0.f;
       nextBeta = live ? beta[size_t(info.start + first + lane) * kValueHeads + head] : 0.f;
     }
   };
-  load(0);
-  uint32_t step = 0;
-  for (uint32_t first = 0; first < info.count; first += kChunk, ++step) {
+  auto cumulate = [&] {  // lanes 16 .. 31: the sum over all 16 tokens
+    cumulative = double(nextG);
+#pragma unroll
+    for (int step = 1; step < kChunk; step *= 2) {
+      const double other = __shfl_up_sync(0xffffffffu, cumulative, step);
+      if (lane >= step)
+        cumulative += other;
+    }
+    const double all = __shfl_sync(0xffffffffu, cumulative, kChunk - 1);
+    cumulative = lane < kChunk ? cumulative : all;
+  };
+  load(group * kChunk);
+  if (warp == 3)
+    cumulate();
+  uint32_t step = group;
+  for (uint32_t first = group * kChunk; first < info.count; first += groups * kChunk, step += groups) {
     ChunkBuffer& out = sh.buffer[step & 1];
     if (step >= 2)
-      named_barrier(3 + (step & 1), kChunkThreads);
+      named_barrier(3 + (step & 1), threads);
+    const float gateBeta = nextBeta;
+    if (warp == 3 && lane < kChunk)
+      sh.cumulative[step & 1][lane] = cumulative, sh.gateBeta[step & 1][lane] = gateBeta;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float4 a = nextQ[j], b = nextK[j];
@@ -653,23 +717,10 @@ __device__ __forceinline__ void chunk_prepare(ChunkShared& sh, const infdev_quer
       split_pair(b.x * kn, b.y * kn, hi.x, lo.x), split_pair(b.z * kn, b.w * kn, hi.y, lo.y);
       *reinterpret_cast<uint2*>(&out.k[0][4 * warp + j][4 * lane]) = hi, *reinterpret_cast<uint2*>(&out.k[1][4 * warp + j][4 * lane]) = lo;
     }
-    if (warp == 0) {
-      double running = 0.0, mine = 0.0;
-#pragma unroll
-      for (int t = 0; t < kChunk; ++t) {
-        running += double(__shfl_sync(0xffffffffu, nextG, t));
-        mine = lane == t ? running : mine;
-      }
-      if (lane < kChunk) {
-        sh.cumulative[step & 1][lane] = mine, sh.gateBeta[step & 1][lane] = nextBeta;
-        out.decay[lane] = exp_of(mine), out.tail[lane] = exp_of(running - mine), out.beta[lane] = nextBeta;
-      }
-    }
-    load(first + kChunk);  // past the end: zeros
-    named_barrier(5, kPrepareWarps * kWarp);
+    load(first + groups * kChunk);  // past the end: zeros
+    named_barrier(5 + group, kPrepareWarps * kWarp);
+    float dot[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
     if (warp < 2) {
-      // warp 0: k . k and the inverse of the triangular system; warp 1: q . k
-      float dot[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
       const auto& left = warp == 0 ? out.k : out.q;
 #pragma unroll
       for (int s = 0; s < kHeadDim / 16; ++s) {
@@ -684,14 +735,24 @@ __device__ __forceinline__ void chunk_prepare(ChunkShared& sh, const infdev_quer
         for (int e = 0; e < 4; ++e)
           dot[0][e] += part[0][e], dot[1][e] += part[1][e];
       }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int t = 8 * (warp - 2) + 2 * j + (lane >> 4), i = lane & 15;
+        sh.ratio[group][t][i] = i <= t ? exp_of(sh.cumulative[step & 1][t] - sh.cumulative[step & 1][i]) : 0.f;
+      }
+    }
+    named_barrier(5 + group, kPrepareWarps * kWarp);
+    if (warp < 2) {
+      // warp 0: the triangular system and its inverse; warp 1: the weights of the second sum
 #pragma unroll
       for (int n = 0; n < 2; ++n)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int t = (lane >> 2) + 8 * (e >> 1), i = 8 * n + 2 * (lane & 3) + (e & 1);
-          const float value = dot[n][e] * (1.0f / (kKeyUnit * kKeyUnit)) * exp_of(sh.cumulative[step & 1][t] - sh.cumulative[step & 1][i]);
+          const float value = dot[n][e] * (1.0f / (kKeyUnit * kKeyUnit)) * sh.ratio[group][t][i];
           if (warp == 0) {
-            sh.system[t][i] = i < t ? value * sh.gateBeta[step & 1][t] : 0.f;
+            sh.system[group][t][i] = i < t ? value * sh.gateBeta[step & 1][t] : 0.f;
           } else {
             store_three(out.mix, t, i, i <= t ? value : 0.f);
           }
@@ -708,25 +769,30 @@ __device__ __forceinline__ void chunk_prepare(ChunkShared& sh, const infdev_quer
         for (int i = 0; i < kChunk; ++i)
 #pragma unroll
           for (int t = i + 1; t < kChunk; ++t)
-            x[t] = fmaf(-sh.system[t][i], x[i], x[t]);
+            x[t] = fmaf(-sh.system[group][t][i], x[i], x[t]);
         if (lane < kChunk)
 #pragma unroll
           for (int t = 0; t < kChunk; ++t) {
             store_three(out.solve, t, column, x[t]);
           }
       }
+    } else if (warp == 3) {
+      const double all = __shfl_sync(0xffffffffu, cumulative, kChunk);
+      if (lane < kChunk)
+        out.decay[lane] = exp_of(cumulative), out.tail[lane] = exp_of(all - cumulative), out.beta[lane] = gateBeta;
+      cumulate();
     }
-    named_barrier_arrive(1 + (step & 1), kChunkThreads);
+    named_barrier_arrive(1 + (step & 1), threads);
   }
 }
 
-// Which query the CTAs of row `rank` of the grid take: the one with the rank-th largest count, so that the longest chains start
-// first and the short ones fill the SMs that are left over (eight queries of 59 to 493 rows, 256 CTAs on 148 SMs, with a
+// Which query the CTAs of row `rank` of the grid take: of those that this kernel takes the one with the rank-th largest count, so that the longest
+// chains start first and the short ones fill the SMs that are left over (eight queries of 59 to 493 rows, 256 CTAs on 148 SMs, with a
 // chunk of 4.2 us: 323 us in the order of the pass, 281 us sorted). Every lane of a warp calls; beyond 32 queries the order of the pass stays.
-__device__ __forceinline__ uint32_t query_by_length(const infdev_query* queries, uint32_t count, uint32_t rank) {
+__device__ __forceinline__ uint32_t query_by_length(const infdev_query* queries, uint32_t count, uint32_t chunkedFrom, uint32_t rank) {
   if (count > 32)
     return rank;
-  const uint32_t lane = threadIdx.x & 31, mine = lane < count ? queries[lane].count : 0u;
+  const uint32_t lane = threadIdx.x & 31, mine = lane < count && chunked(queries[lane], chunkedFrom) ? queries[lane].count : 0u;
   uint32_t before = 0;
   for (uint32_t j = 0; j < count; ++j) {
     const uint32_t other = __shfl_sync(0xffffffffu, mine, j);
@@ -736,25 +802,31 @@ __device__ __forceinline__ uint32_t query_by_length(const infdev_query* queries,
 }
 
 __global__ void __launch_bounds__(kChunkThreads, 1)
-    delta_rule_chunked_kernel(const float* q, const float* k, const float* v, const float* g, const float* beta, const float* z, const float* normWeight,
-                              const infdev_query* queries, uint64_t stateOffset, float* out, uint32_t chunkedFrom) {
+    delta_rule_chunked_kernel(const float* q, const float* k, const float* v, const float* g, const float* beta, const infdev_query* queries, uint64_t stateOffset,
+                              float* out, uint32_t chunkedFrom, uint32_t queryCount, uint32_t sms) {
   pdl_launch_dependents();
   pdl_wait();
-  const infdev_query info = queries[query_by_length(queries, gridDim.y, blockIdx.y)];
-  if (info.state != kUnbound || info.count < chunkedFrom)  // delta_rule_kernel takes this query
+  const uint32_t part = blockIdx.y >= queryCount ? 1 : 0;
+  const infdev_query info = queries[query_by_length(queries, queryCount, chunkedFrom, blockIdx.y - part * queryCount)];
+  if (!chunked(info, chunkedFrom))  // delta_rule_kernel takes this query
     return;
   extern __shared__ __align__(16) uint8_t chunkRaw[];
   ChunkShared& sh = *reinterpret_cast<ChunkShared*>(chunkRaw);
   const int head = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // two CTAs have half of a head's columns each
+  const bool split = 2 * kValueHeads * chunked_queries(queries, queryCount, chunkedFrom) <= sms;
+  if (!split && part)
+    return;
+  const int threads = split ? (kSplitWarps + kPrepareWarps) * kWarp : kChunkThreads;  // at the barriers of a buffer
   // The computing warps hold more than a third of the registers each: 2 x 192 + 120 = 3 x 168 a thread, of the 168 that the launch
   // bounds give all three groups of four warps.
-  if (warp >= kComputeWarps) {
+  if (warp >= (split ? kSplitWarps : kComputeWarps)) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 120;");
-    chunk_prepare(sh, info, q, k, g, beta, head);
+    chunk_prepare(sh, info, q, k, g, beta, head, split ? warp / kPrepareWarps - 1 : 0, split ? 2 : 1, threads);
     return;
   }
   asm volatile("setmaxnreg.inc.sync.aligned.u32 192;");
-  const int row = lane >> 2, t2 = 2 * (lane & 3), column = 16 * warp + row;  // value columns `column` and `column` + 8
+  const int row = lane >> 2, t2 = 2 * (lane & 3), column = 16 * (warp + int(part) * kSplitWarps) + row;  // value columns `column` and `column` + 8
   const int tokenOfB = (lane & 7) + 8 * (lane >> 4), dimOfB = 8 * ((lane >> 3) & 1);
   float S[kHeadDim / 8][4];  // S^T: tile j holds key dims 8j + t2, + 1 of the two value columns
   const size_t state = size_t(head) * kHeadDim * kHeadDim + column;
@@ -763,11 +835,8 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
 #pragma unroll
     for (int e = 0; e < 4; ++e)
       S[j][e] = info.previous ? reinterpret_cast<const float*>(info.previous + stateOffset)[state + (8 * j + t2 + (e & 1)) * kHeadDim + 8 * (e >> 1)] : 0.f;
-  float weight[2] = {0.f, 0.f};
-  if (z)
-    weight[0] = normWeight[column], weight[1] = normWeight[column + 8];
   // element (n, e) of a token tile: token 8n + t2 + e % 2, value column + 8 (e / 2)
-  float value[2][4], gate[2][4];
+  float value[2][4];
   auto load = [&](float (&into)[2][4], const float* from, uint32_t first) {
 #pragma unroll
     for (int n = 0; n < 2; ++n)
@@ -781,8 +850,6 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
   uint32_t step = 0;
   for (uint32_t first = 0; first < info.count; first += kChunk, ++step) {
     const ChunkBuffer& in = sh.buffer[step & 1];
-    if (z)
-      load(gate, z, first);
     float largest[2] = {0.f, 0.f};
 #pragma unroll
     for (int j = 0; j < kHeadDim / 8; ++j)
@@ -790,7 +857,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
       for (int e = 0; e < 4; ++e)
         largest[e >> 1] = fmaxf(largest[e >> 1], fabsf(S[j][e]));
     const float2 unit = column_unit(largest[0]), unit8 = column_unit(largest[1]);
-    named_barrier(1 + (step & 1), kChunkThreads);
+    named_barrier(1 + (step & 1), threads);
     // S^T k and S^T q of the 16 tokens
     float ks[2][4], qs[2][4];
 #pragma unroll
@@ -862,49 +929,15 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
         for (int e = 0; e < 4; ++e)
           S[2 * s + n][e] = fmaf(added[n][e], updateUnit[e >> 1], S[2 * s + n][e] * stateDecay);
     }
-    named_barrier_arrive(3 + (step & 1), kChunkThreads);  // the buffer may be refilled
-    // o, its gated norm over the head's 128 columns (gated_rms_norm_128), and the store
-    float o[2][4], squares[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        o[n][e] = decay[n][e & 1] * (qs[n][e] * productUnit[e >> 1]) + mixed[n][e];
-        squares[n][e & 1] = fmaf(o[n][e], o[n][e], squares[n][e & 1]);
-      }
-    if (z) {
-#pragma unroll
-      for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          float sum = squares[n][e];
-#pragma unroll
-          for (int m = 4; m < 32; m <<= 1)
-            sum += __shfl_xor_sync(0xffffffffu, sum, m);
-          if (row == 0)
-            sh.squares[step & 1][warp][8 * n + t2 + e] = sum;
-        }
-      named_barrier(6, kComputeWarps * kWarp);  // two sets of sums in turn: nobody is two chunks behind
-#pragma unroll
-      for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          float sum = 0.f;
-#pragma unroll
-          for (int w = 0; w < kComputeWarps; ++w)
-            sum += sh.squares[step & 1][w][8 * n + t2 + e];
-          const float norm = rsqrtf(sum / float(kHeadDim) + 1.0e-6f);
-          o[n][e] = o[n][e] * norm * weight[0] * silu_f(gate[n][e]);
-          o[n][e + 2] = o[n][e + 2] * norm * weight[1] * silu_f(gate[n][e + 2]);
-        }
-    }
+    named_barrier_arrive(3 + (step & 1), threads);  // the buffer may be refilled
 #pragma unroll
     for (int n = 0; n < 2; ++n)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const uint32_t token = first + 8 * n + t2 + (e & 1);
         if (token < info.count)
-          out[(size_t(info.start + token) * kValueHeads + head) * kHeadDim + column + 8 * (e >> 1)] = o[n][e];
+          out[(size_t(info.start + token) * kValueHeads + head) * kHeadDim + column + 8 * (e >> 1)] =
+              decay[n][e & 1] * (qs[n][e] * productUnit[e >> 1]) + mixed[n][e];
       }
   }
 #pragma unroll
@@ -946,15 +979,16 @@ cudaError_t gdn_prepare_launch(const float* x, const float* mixed, const float* 
 
 cudaError_t delta_rule_launch(const float* q, const float* k, const float* v, const float* g, const float* beta, const float* z,
                               const float* normWeight, const infdev_query* queries, int queryCount, uint64_t stateOffset, uint64_t stateBytes,
-                              float* out, uint8_t* image, int* counters, uint32_t chunkedFrom, cudaStream_t stream) {
+                              float* out, uint8_t* image, int* counters, uint32_t chunkedFrom, int sms, cudaStream_t stream) {
   if (queryCount <= 0)
     return cudaSuccess;
   if (chunkedFrom) {
     static PerDeviceOnce configured;
     if (cudaError_t e = configure_shared_memory(delta_rule_chunked_kernel, sizeof(ChunkShared), configured))
       return e;
-    launch_kernel<2>(delta_rule_chunked_kernel, dim3(kValueHeads, unsigned(queryCount)), kChunkThreads, sizeof(ChunkShared), stream, q, k, v, g, beta, z, normWeight,
-                  queries, stateOffset, out, chunkedFrom);
+    const int halves = std::min(queryCount, sms / (2 * kValueHeads));  // as many queries as may be split
+    launch_kernel<2>(delta_rule_chunked_kernel, dim3(kValueHeads, unsigned(queryCount + halves)), kChunkThreads, sizeof(ChunkShared), stream, q, k, v, g, beta, queries,
+                  stateOffset, out, chunkedFrom, uint32_t(queryCount), uint32_t(sms));
   }
   // Not launched early: its CTAs would be placed around those of the kernels before it, two on an SM, and the token-by-token chain
   // of short queries runs slower for it (12 rows: 37.5 against 31.0 us; passes that the chunked kernel takes lose 1 us).

@@ -28,7 +28,7 @@ cudaError_t gdn_prepare_launch(const float* x, const float* mixed, const float* 
                                float* q, float* k, float* v, float* beta, float* g, cudaStream_t stream);
 cudaError_t delta_rule_launch(const float* q, const float* k, const float* v, const float* g, const float* beta, const float* z,
                               const float* normWeight, const infdev_query* queries, int queryCount, uint64_t stateOffset, uint64_t stateBytes,
-                              float* out, uint8_t* image, int* counters, uint32_t chunkedFrom, cudaStream_t stream);
+                              float* out, uint8_t* image, int* counters, uint32_t chunkedFrom, int sms, cudaStream_t stream);
 cudaError_t gdn_decode_launch(const float* x, const float* mixed, const float* wBeta, const float* wAlpha, const float* A, const float* dt,
                               const float* convWeight, const float* z, const float* normWeight, const infdev_query* queries, int queryCount,
                               uint64_t convStateOffset, uint64_t stateOffset, uint64_t stateBytes, float* out, uint8_t* image, int* counters,
