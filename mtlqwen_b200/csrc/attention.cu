@@ -335,8 +335,9 @@ __global__ void __launch_bounds__(128, 6) attention_scan_kernel(const float* q, 
 // Operands as in the scan: fp16 keys and values, query and softmax weights as fp16 hi + lo, fp32 accumulation. A tile of 64 tokens is
 // 1.6 k cycles of MMAs for the scores (bounded by shared memory: A and B both come from there) and 1 k for the values; mma.sync,
 // with 16 rows x 4 heads, was 8 k for half the rows.
-// Measured, with the merge, and before, with mma.sync: 128 rows behind 1920 tokens 51.0 -> 32.1 us, four times 30 rows behind up to 1970
-// 49.3 -> 32.4, 2048 rows behind 2048 1070 -> 449; 64 rows of 64 tokens 13.0 -> 16.1: a fixed start of laying out q and an end of
+// Measured, with the merge, and before, with mma.sync: 128 rows behind 1920 tokens 51.0 -> 32.1 us (31.0 with weights by powers of two), four times
+// 30 rows behind up to 1970 49.3 -> 32.4 (31.4), 2048 rows behind 2048 1070 -> 457 (420); by its own clocks the first of these spends 5000 of
+// 38000 on its start, 6500 on q, 10000 on scores, which wait for their copies, 4300 on weights, 4000 on the last values and 5300 on the store of its results; 64 rows of 64 tokens 13.0 -> 16.1: a fixed start of laying out q and an end of
 // reading tensor memory, which little work has to pay for, so short contexts stay with attention_group_kernel below.
 // Errors against fp64 (rms, of the result's): 128 rows behind 1920 tokens 1.4e-6 and 1.9e-6 before, 300 behind 8700 7.6e-6 and 2.1e-5,
 // 32 behind 29968 2.9e-6 and 4.6e-6: fewer roundings between tiles.
@@ -464,6 +465,20 @@ __device__ __forceinline__ uint2 split_pair(float a, float b) {
 __device__ __forceinline__ uint32_t not_finite(uint32_t pair) { return ((pair & 0x7c007c00u) + 0x04000400u) & 0x80008000u; }
 
 __device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// Scores of tokens first .. first + 15 of a tile that a row with `live` of its tokens does not attend to.
+__device__ __forceinline__ void mask_scores(uint32_t (&score)[16], uint32_t first, uint32_t live) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    score[i] = first + i < live ? score[i] : __float_as_uint(-INFINITY);
+}
+// e^((score - largest) / 16) as a power of two: a third of expf's instructions, which the workers' 128 x 256 weights a round are bound by. The rounding of
+// the exponent makes a weight w wrong by up to |ln w| x 2^-24 of itself, most where it counts least.
+__device__ __forceinline__ float softmax_weight(float score, float largest) {
+  float weight;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(weight) : "f"((score - largest) * (1.4426950408889634f / 16.0f)));
+  return weight;
+}
 
 __global__ void __launch_bounds__(kTileThreads, 1)
     attention_tile_kernel(const float* q, const __half* cacheK, const __half* cacheV, const infdev_query* queries, int queryCount, const int32_t* table,
@@ -698,16 +713,20 @@ __global__ void __launch_bounds__(kTileThreads, 1)
           wait(&sh.scoresReady[j], (scorePhases >> j) & 1);
           fence_after_sync();
           const uint32_t first = from + j * kGroupTokens, live = limit > first ? limit - first : 0u;
+          const bool whole = __all_sync(0xffffffffu, live >= kGroupTokens);
 #pragma unroll 1
           for (uint32_t c = 0; c < kGroupTokens; c += 16) {
             uint32_t score[16];
             tmem_load16(laneBase + kColScores + j * 64 + c, score);
             tmem_wait_load();
+            if (!whole)
+              mask_scores(score, c, live);
 #pragma unroll
             for (int i = 0; i < 16; ++i)
-              best = fmaxf(best, c + i < live ? __uint_as_float(score[i]) * (1.0f / 16.0f) : -INFINITY);
+              best = fmaxf(best, __uint_as_float(score[i]));
           }
         }
+        best *= 1.0f / 16.0f;
         sh.exchange[side][row] = best;
         named_barrier(1 + quadrant, 64);
         const float next = fmaxf(maximum, fmaxf(best, sh.exchange[side ^ 1][row])), rescale = expf(maximum - next);
@@ -730,17 +749,17 @@ __global__ void __launch_bounds__(kTileThreads, 1)
         for (uint32_t j = 0; j < tiles; ++j) {
           if (int(j & 1) == side) {
             const uint32_t first = from + j * kGroupTokens, live = limit > first ? limit - first : 0u;
+            const bool whole = __all_sync(0xffffffffu, live >= kGroupTokens);
 #pragma unroll 1
             for (uint32_t c = 0; c < kGroupTokens; c += 16) {  // the halves of 16 weights take the columns of their scores
               uint32_t score[16], halves[16];
               tmem_load16(laneBase + kColScores + j * 64 + c, score);
               tmem_wait_load();
+              if (!whole)
+                mask_scores(score, c, live);
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
-                // the mask before the exponential, which would be branched around otherwise
-                const float s0 = c + 2 * i < live ? __uint_as_float(score[2 * i]) * (1.0f / 16.0f) : -INFINITY;
-                const float s1 = c + 2 * i + 1 < live ? __uint_as_float(score[2 * i + 1]) * (1.0f / 16.0f) : -INFINITY;
-                const float w0 = expf(s0 - maximum), w1 = expf(s1 - maximum);
+                const float w0 = softmax_weight(__uint_as_float(score[2 * i]), 16.f * maximum), w1 = softmax_weight(__uint_as_float(score[2 * i + 1]), 16.f * maximum);
                 norm += w0 + w1;
                 const uint2 w = split_pair(w0, w1);
                 halves[i] = w.x, halves[8 + i] = w.y;
