@@ -220,10 +220,12 @@ template <int NT, class B> __device__ __forceinline__ void iq4_unit(const uint8_
 // Block layout (quant_linear.metal:69-85): ql[128] | qh[64] | int8 sc[16] | fp16 d. Element r = 128*hh + 32*s
 // + l has its low nibble in ql[64*hh + 32*(s&1) + l] (high half of the byte when s >= 2), its top two bits
 // in qh[32*hh + l] >> 2s, and scale sc[r/16]. MMA gi covers elements [16gi, 16gi+16); lane t supplies
-// elements 16gi + 4t + {0,1,2,3}. Blocks are only 2-byte aligned, so words are fetched as two halves.
-template <int NT, class B>
+// elements 16gi + 4t + {0,1,2,3}. Blocks are only 2-byte aligned, so words are fetched as two halves; WORDS: as they are, of a block that is
+// known to lie at a multiple of four bytes.
+template <bool WORDS, int NT, class B>
 __device__ __forceinline__ void q6k_unit(const uint8_t* pA, const uint8_t* pB, int lane, const B& b, float (&total)[NT][4]) {
   const int t = lane & 3;
+  auto load = [](const uint8_t* p) { return WORDS ? lds_u32(p) : lds_u32_unaligned(p); };
   float sum[NT][4];
   clear(sum);
   const float dA = load_half_bits(pA + 208), dB = load_half_bits(pB + 208);
@@ -232,10 +234,10 @@ __device__ __forceinline__ void q6k_unit(const uint8_t* pA, const uint8_t* pB, i
   for (int hh = 0; hh < 2; ++hh) {
 #pragma unroll(NT > 3 ? 1 : 2)
     for (int u = 0; u < 2; ++u) {
-      const uint32_t hiA = lds_u32_unaligned(pA + 128 + 32 * hh + 16 * u + 4 * t), hiB = lds_u32_unaligned(pB + 128 + 32 * hh + 16 * u + 4 * t);
+      const uint32_t hiA = load(pA + 128 + 32 * hh + 16 * u + 4 * t), hiB = load(pB + 128 + 32 * hh + 16 * u + 4 * t);
 #pragma unroll
       for (int sl = 0; sl < 2; ++sl) {
-        const uint32_t loA = lds_u32_unaligned(pA + 64 * hh + 32 * sl + 16 * u + 4 * t), loB = lds_u32_unaligned(pB + 64 * hh + 32 * sl + 16 * u + 4 * t);
+        const uint32_t loA = load(pA + 64 * hh + 32 * sl + 16 * u + 4 * t), loB = load(pB + 64 * hh + 32 * sl + 16 * u + 4 * t);
 #pragma unroll
         for (int sh = 0; sh < 2; ++sh) {
           const int s = sl + 2 * sh, gi = hh * 8 + s * 2 + u;

@@ -307,7 +307,7 @@ template <class Q, int NT> __global__ void __launch_bounds__(kThreads, 1) wide_k
           } else if constexpr (std::is_same_v<Q, IQ4>) {
             iq4_unit(pA, pB, lane, rows, total);
           } else {
-            q6k_unit(pA, pB, lane, rows, total);
+            q6k_unit<false>(pA, pB, lane, rows, total);
           }
           __syncwarp();
           if (lane == 0)
