@@ -34,6 +34,25 @@ __device__ __forceinline__ const infdev_query& query_of_row(const infdev_query* 
   return *queries;
 }
 
+// warp_sum of COUNT sums, in its order, but a lane goes on with one half of them and leaves the other to its partner: 62 exchanges instead of 320 for
+// 64 sums (preparation of 2411 rows 106.7 -> 101.2 us). Lane l is left with the sums from l x COUNT / 32 on: two of 64, otherwise one.
+template <int COUNT, int PARTNER, int SIZE> __device__ __forceinline__ void share_sums(float (&sum)[SIZE], int lane) {
+  if constexpr (PARTNER > 0) {
+    constexpr int kLeft = COUNT > 1 ? COUNT / 2 : 1;
+    const bool upper = lane & PARTNER;
+#pragma unroll
+    for (int o = 0; o < kLeft; ++o) {
+      if constexpr (COUNT > 1) {
+        const float other = __shfl_xor_sync(0xffffffffu, upper ? sum[o] : sum[o + kLeft], PARTNER);
+        sum[o] = (upper ? sum[o + kLeft] : sum[o]) + other;
+      } else {
+        sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], PARTNER);
+      }
+    }
+    share_sums<kLeft, PARTNER / 2>(sum, lane);
+  }
+}
+
 // gdn_prepare_kernel: both preparation steps of a GDN layer in one launch of 256-thread CTAs.
 //  * CTAs [0, gateBlocks): beta / g of eight rows and GATE_HEADS of the 32 value heads. Warps 0..3 share the 4096-long dot
 //    products with wBeta (a quarter each), warps 4..7 those with wAlpha; a warp keeps a tile of rows x heads of partial
@@ -45,10 +64,13 @@ __device__ __forceinline__ const infdev_query& query_of_row(const infdev_query* 
 //    where reading and writing everything once takes 30). State layout: conv taps fp32 [8192][4] at record + stateOffset.
 // CONV_ROWS rows per thread and GATE_HEADS heads per CTA (the sums are the same whatever they are): the rows of short prompt pieces are spread
 // thinly, so that no thread has a long chain of them; with more rows an SM, which holds two CTAs, would take them in several turns.
-// 1 and 1, 2 and 2, 4 and 4, 8 and 8: 24 rows 6.2 / 6.2 / 7.2 / 10.6 us, 32 rows 7.7 / 6.2 / 6.2 / 9.8, 40 rows 8.7 / 6.3 / 7.3 / 9.8, 64 rows 11.2 / 8.2 /
-// 7.4 / 9.8, 128 rows 17.5 / 11.8 / 9.8 / 10.8, 192 rows 24.1 / 15.2 / 12.9 / 13.0, 256 rows 30.3 / 19.4 / 15.6 / 14.2, 512 rows 55 / 34 / 26.8 / 24.1.
+// 1 and 1, 2 and 2, 4 and 4, 8 and 8: 24 rows 5.7 / 5.8 / 6.7 / 9.8 us, 32 rows 7.6 / 5.7 / 5.7 / 8.7, 48 rows 8.8 / 5.7 / 6.2 / 8.8, 64 rows 10.3 / 7.7 /
+// 6.7 / 8.8, 128 rows 15.9 / 10.9 / 8.8 / 9.8, 160 rows 18.5 / 12.4 / 10.3 / 10.8, 192 rows 21.6 / 13.9 / 11.4 / 10.8, 512 rows 50 / 31 / 23.2 / 21.1.
+// What bounds the last is instructions: the parts of 2411 rows, each alone, issue 2.8 a cycle in 46 and 39 us, 45 for a value of the convolution
+// (its division and exponential are most of them). The gates' operands through shared memory by cp.async 103.9 us, the convolution as a launch of
+// more and smaller blocks 102.1, gates and convolution side by side on an SM 121, as below 93.5.
 // ALIGNED: mixed, convWeight, q, k and v lie on 16-byte boundaries; without, they are read and written value by value.
-constexpr int kGateRows = 8, kPrepareRows1 = 24, kPrepareRows2 = 48, kPrepareRows4 = 192;  // most rows of each spread
+constexpr int kGateRows = 8, kPrepareRows1 = 24, kPrepareRows2 = 48, kPrepareRows4 = 176;  // most rows of each spread
 constexpr int kConvChannels = 4 * 256;  // per CTA
 
 template <bool ALIGNED> __device__ __forceinline__ float4 load_four(const float* p) {
@@ -70,12 +92,11 @@ __global__ void __launch_bounds__(256, 2) gdn_prepare_kernel(const float* x, con
     const int warp = tid >> 5, lane = tid & 31, which = warp >> 2, quarter = warp & 3;
     const float* weights = (which ? wAlpha : wBeta) + size_t(head0) * 4096 + quarter * 1024 + lane * 4;
     const float* src = x + size_t(row0) * 4096 + quarter * 1024 + lane * 4;
-    float sum[kGateRows][GATE_HEADS];
+    constexpr int kSums = kGateRows * GATE_HEADS;
+    float sum[kSums];
 #pragma unroll
-    for (int r = 0; r < kGateRows; ++r)
-#pragma unroll
-      for (int h = 0; h < GATE_HEADS; ++h)
-        sum[r][h] = 0.f;
+    for (int o = 0; o < kSums; ++o)
+      sum[o] = 0.f;
 #pragma unroll 2
     for (int i = 0; i < 8; ++i) {
       float4 a[kGateRows];
@@ -87,25 +108,21 @@ __global__ void __launch_bounds__(256, 2) gdn_prepare_kernel(const float* x, con
         const float4 b = *reinterpret_cast<const float4*>(weights + size_t(h) * 4096 + i * 128);
 #pragma unroll
         for (int r = 0; r < kGateRows; ++r)
-          sum[r][h] += dot4(a[r], b);
+          sum[r * GATE_HEADS + h] += dot4(a[r], b);
       }
     }
-    __shared__ float parts[kGateRows][GATE_HEADS][8];
+    share_sums<kSums, 16>(sum, lane);
+    __shared__ float parts[kSums][8];
 #pragma unroll
-    for (int r = 0; r < kGateRows; ++r)
-#pragma unroll
-      for (int h = 0; h < GATE_HEADS; ++h) {
-        const float total = warp_sum(sum[r][h]);
-        if (lane == 0)
-          parts[r][h][warp] = total;
-      }
+    for (int o = 0; o < (kSums + 31) / 32; ++o)
+      parts[lane * kSums / 32 + o][warp] = sum[o];  // fewer than 32: several lanes have the same one
     __syncthreads();
-    if (tid < 2 * kGateRows * GATE_HEADS) {
-      const int r = (tid / GATE_HEADS) % kGateRows, h = tid % GATE_HEADS, head = head0 + h;
+    if (tid < 2 * kSums) {
+      const int r = (tid / GATE_HEADS) % kGateRows, head = head0 + tid % GATE_HEADS;
       if (r < live) {
-        const float* p = parts[r][h] + (tid < kGateRows * GATE_HEADS ? 0 : 4);
+        const float* p = parts[tid % kSums] + (tid < kSums ? 0 : 4);
         const float dot = (p[0] + p[1]) + (p[2] + p[3]);
-        if (tid < kGateRows * GATE_HEADS)
+        if (tid < kSums)
           beta[(row0 + r) * kValueHeads + head] = 1.0f / (1.0f + expf(-dot));
         else
           g[(row0 + r) * kValueHeads + head] = A[head] * logf(1.0f + expf(dot + dt[head]));
@@ -120,6 +137,11 @@ __global__ void __launch_bounds__(256, 2) gdn_prepare_kernel(const float* x, con
   for (int i = 0; i < CONV_ROWS; ++i)
     if (row0 + i < last)
       input[i] = load_four<ALIGNED>(mixed + size_t(row0 + i) * kChannels + c);
+  // The three inputs before this one, oldest first: asked for before it is known whether they are of the same query (101.2 -> 98.4 us).
+  float4 window[3];
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+    window[r] = row0 - 3 + r >= 0 ? load_four<ALIGNED>(mixed + size_t(row0 - 3 + r) * kChannels + c) : make_float4(0.f, 0.f, 0.f, 0.f);
   float4 weight[4];  // of the thread's four channels, oldest tap first
 #pragma unroll
   for (int j = 0; j < 4; ++j)
@@ -127,18 +149,20 @@ __global__ void __launch_bounds__(256, 2) gdn_prepare_kernel(const float* x, con
   float* const out = c < 2048 ? q + c : c < 4096 ? k + (c - 2048) : v + (c - 4096);
   const size_t pitch = c < 4096 ? 2048 : 4096;
   const infdev_query* info = &query_of_row(queries, uint32_t(row0));
-  float4 window[3];  // the three inputs before this one, oldest first
-  bool enter = true;
+  // Kept: the stores below would have them read again for every row (98.4 -> 93.5 us).
+  int start = int(info->start), end = start + int(info->count);
+  bool enter = row0 - 3 < start, speculative = info->state != kUnbound;
 #pragma unroll
   for (int i = 0; i < CONV_ROWS; ++i) {
     const int row = row0 + i;
     if (row >= last)
       break;
-    if (row >= int(info->start + info->count)) {
+    if (row >= end) {
       info = &query_of_row(info, uint32_t(row));
+      start = int(info->start), end = start + int(info->count), speculative = info->state != kUnbound;
       enter = true;
     }
-    const int p = row - int(info->start);
+    const int p = row - start;
     if (enter) {
       // the window at position p of this query: earlier rows of the query, before them the taps of the state record
       const float* prev = reinterpret_cast<const float*>(info->previous + stateOffset) + size_t(c) * 4;
@@ -151,7 +175,7 @@ __global__ void __launch_bounds__(256, 2) gdn_prepare_kernel(const float* x, con
       for (int r = 0; r < 3; ++r) {
         const int position = p - 3 + r;  // tap position + 4 of the record (1 .. 3) when negative
         if (position >= 0)
-          window[r] = load_four<ALIGNED>(mixed + size_t(info->start + position) * kChannels + c);
+          window[r] = load_four<ALIGNED>(mixed + size_t(start + position) * kChannels + c);
         else if (position == -3)
           window[r] = make_float4(taps[0].y, taps[1].y, taps[2].y, taps[3].y);
         else if (position == -2)
@@ -173,8 +197,7 @@ __global__ void __launch_bounds__(256, 2) gdn_prepare_kernel(const float* x, con
       *reinterpret_cast<float4*>(to) = result;
     else
       to[0] = result.x, to[1] = result.y, to[2] = result.z, to[3] = result.w;
-    const bool speculative = info->state != kUnbound;
-    if (speculative || p + 1 == int(info->count)) {
+    if (speculative || row + 1 == end) {
       float4* state = reinterpret_cast<float4*>(info->next + stateOffset + (speculative ? uint64_t(p) * stateBytes : 0)) + c;
       state[0] = make_float4(window[0].x, window[1].x, window[2].x, now.x);
       state[1] = make_float4(window[0].y, window[1].y, window[2].y, now.y);

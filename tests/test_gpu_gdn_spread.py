@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 
 # both sides of every line, with queries that begin and end inside the rows of a thread
-@pytest.mark.parametrize("lengths", [[24], [3, 22], [47, 1], [5, 2, 42], [1, 190, 1], [100, 3, 90]])
+@pytest.mark.parametrize("lengths", [[24], [3, 22], [47, 1], [5, 2, 42], [1, 190, 1], [100, 3, 90], [9, 1, 2, 200, 3, 5]])
 def test_every_spread_has_the_same_bits(dev, lengths):
   rng = np.random.default_rng(41)
   rows, nq = sum(lengths), len(lengths)
