@@ -216,7 +216,7 @@ __device__ __forceinline__ uint32_t chunked_queries(const infdev_query* queries,
   return count > 32 ? 32 : __popc(__ballot_sync(0xffffffffu, lane < count && chunked(queries[lane], chunkedFrom)));
 }
 
-// gated_rms_norm_128 of one head of a query's rows, in place: eight warps, eight rows each at a time.
+// gated_rms_norm_128 of one head of a query's rows, in place: eight warps, eight rows each at a time, in turn with the CTAs of the grid's third dimension.
 __device__ __forceinline__ void gated_norm_rows(float* out, const float* z, const float* normWeight, uint32_t start, uint32_t count, int head) {
   constexpr uint32_t kRows = 8;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -225,7 +225,7 @@ __device__ __forceinline__ void gated_norm_rows(float* out, const float* z, cons
 #pragma unroll
   for (int c = 0; c < 4; ++c)
     weight[c] = normWeight[lane + 32 * c];
-  for (uint32_t first = warp * kRows; first < count; first += 8 * kRows) {
+  for (uint32_t first = (blockIdx.z * 8 + warp) * kRows; first < count; first += gridDim.z * 8 * kRows) {
     float o[kRows][4], gate[kRows][4];
     const size_t at = size_t(start + first) * kPitch + size_t(head) * kHeadDim + lane;
 #pragma unroll
@@ -320,6 +320,8 @@ __global__ void __launch_bounds__(256, 2) delta_rule_kernel(const float* q, cons
       gated_norm_rows(out, z, normWeight, info.start, info.count, head);
     return;
   }
+  if (!FUSED && blockIdx.z > 0)
+    return;
   __shared__ float qraw[kHeadDim], kraw[kHeadDim], vraw[kHeadDim], red[12], dots[8];
   __shared__ float4 partialPred[8][32], partialQ[8][32];
   const int channels[3] = {keyHead * kHeadDim + (tid & 127), 2048 + keyHead * kHeadDim + (tid & 127), 4096 + head * kHeadDim + (tid & 127)};
@@ -534,7 +536,7 @@ __global__ void __launch_bounds__(256, 2) delta_rule_kernel(const float* q, cons
 // By its own clocks a chunk takes 5000 with half of the columns (KS and QS 1900, A^-1 rhs 550, the second sum 500, the update 1000, the rest
 // stores, scales and barriers) and 6900 with all (2800, 700, 700, 1400), where the preparing warps are as slow as that; 8200 when the norm was part of
 // the chain and one preparing warp had gates, decays and the inverse. Eight queries of 59 to 493 rows 200 -> 187 us, one of 493 rows 143 -> 110,
-// of 128 rows 42.1 -> 33.9, of 64 rows 24.8 -> 20.6. Tried and left out: the outputs by warps of their own that are handed S through shared
+// of 128 rows 42.1 -> 33.9, of 64 rows 24.8 -> 20.6, all with norms of one CTA a head (see delta_rule_launch). Tried and left out: the outputs by warps of their own that are handed S through shared
 // memory (200 -> 244 us), two of the preparing warps a stage behind the two others (187 -> 222), 16 warps of 128 registers (237).
 constexpr int kChunk = 16, kComputeWarps = 8, kPrepareWarps = 4;
 constexpr int kChunkThreads = (kComputeWarps + kPrepareWarps) * kWarp;
@@ -1013,9 +1015,13 @@ cudaError_t delta_rule_launch(const float* q, const float* k, const float* v, co
     launch_kernel<2>(delta_rule_chunked_kernel, dim3(kValueHeads, unsigned(queryCount + halves)), kChunkThreads, sizeof(ChunkShared), stream, q, k, v, g, beta, queries,
                   stateOffset, out, chunkedFrom, uint32_t(queryCount), uint32_t(sms));
   }
+  // The norms of long queries are spread over several CTAs a head, which else were a chain of loads and stores after the last chunk: one query of 493
+  // rows 111 -> 96.5 us, six of 17 to 700 rows 202 -> 179, eight of 59 to 493 rows 187 -> 179. Few enough of them that those without rows do not
+  // tell (eight queries of 128 rows 81.0, with four CTAs a head 81.7, with eight 83.4).
+  const int spread = chunkedFrom ? std::clamp(6 * sms / (kValueHeads * queryCount), 1, 8) : 1;
   // Not launched early: its CTAs would be placed around those of the kernels before it, two on an SM, and the token-by-token chain
   // of short queries runs slower for it (12 rows: 37.5 against 31.0 us; passes that the chunked kernel takes lose 1 us).
-  launch_kernel(delta_rule_kernel<false>, dim3(kValueHeads, unsigned(queryCount)), 256, 0, stream, q, k, v, g, beta, z, normWeight, queries, stateOffset,
+  launch_kernel(delta_rule_kernel<false>, dim3(kValueHeads, unsigned(queryCount), unsigned(spread)), 256, 0, stream, q, k, v, g, beta, z, normWeight, queries, stateOffset,
                 stateBytes, out, image, counters, chunkedFrom, GdnInputs{});
   return cudaGetLastError();
 }

@@ -72,3 +72,13 @@ def test_outputs_over_the_gates(mixed):
     (apart, state), (over, other) = mixed.run([i])[0], mixed.run([i], in_place=True)[0]
     # token by token instead of in chunks: a few 1e-7 each (2-norms against fp64)
     assert np.linalg.norm(apart - over) <= 2e-6 * np.linalg.norm(apart) and np.linalg.norm(state - other) <= 2e-6 * np.linalg.norm(state)
+
+
+def test_the_norm_on_one_cta_or_on_eight_has_the_same_bits(dev):
+  """28 queries leave a head of each one CTA for its norms; a query alone has eight of 64 rows at a time, the longest here one row more than they
+  take at once."""
+  lengths = [513, 64, 65, 1] + [16] * 24
+  everything = Pass(dev, lengths, seed=52)
+  together = everything.run(range(len(lengths)))
+  for i in range(5):
+    assert same(everything.run([i])[0], together[i]), lengths[i]
