@@ -245,20 +245,40 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
 
   if (info.topK == 0) {
     // plain temperature sampling over the vocabulary, top-p ignored (native_ops.metal:172-188). The row is summed in
-    // double precision in contiguous chunks, 128 of them per CTA and one at a time per warp; the first CTA finds the chunk
-    // in which the cumulative sum passes the target and walks that one in vocabulary order.
+    // double precision in contiguous chunks, 128 of them per CTA and two at a time per warp; the first CTA finds the chunk
+    // in which the cumulative sum passes the target and walks that one in vocabulary order. What bounds it is latency, so everything is
+    // asked for eight values at a time: one and eight rows of 248320 logits 33.4 -> 17.0 and 37.5 -> 20.5 us, in the order of addition as before.
     maximum = fmaxf(fmaxf(sh.maxima[lane], sh.maxima[lane + 32]), fmaxf(sh.maxima[lane + 64], sh.maxima[lane + 96]));
     maximum = warp_max(maximum) / temperature;
     const int chunks = int(ctas) * kChunks, chunk = (vocab + chunks - 1) / chunks;
-    for (int c = int(part) * kChunks + warp; c < int(part + 1) * kChunks; c += kClusterWarps) {
-      double sum = 0.0;
-      for (int j = c * chunk + lane; j < min(vocab, (c + 1) * chunk); j += 32)
-        sum += double(expf(row[j] / temperature - maximum));
+    for (int c = int(part) * kChunks + warp; c < int(part + 1) * kChunks; c += 2 * kClusterWarps) {
+      double sum[2] = {0.0, 0.0};  // of two chunks at a time
+      int from[2], end[2];
 #pragma unroll
-      for (int o = 16; o; o >>= 1)
-        sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      if (lane == 0)
-        first.chunkSum[c] = sum;
+      for (int s = 0; s < 2; ++s)
+        from[s] = (c + s * kClusterWarps) * chunk, end[s] = min(vocab, from[s] + chunk);
+      for (int at = lane; at < chunk; at += 8 * kWarp) {
+        float value[2][8];
+#pragma unroll
+        for (int s = 0; s < 2; ++s)
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            value[s][e] = from[s] + at + kWarp * e < end[s] ? row[from[s] + at + kWarp * e] : 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+#pragma unroll
+          for (int s = 0; s < 2; ++s)
+            if (from[s] + at + kWarp * e < end[s])
+              sum[s] += double(expf(value[s][e] / temperature - maximum));
+      }
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1)
+          sum[s] += __shfl_xor_sync(0xffffffffu, sum[s], o);
+        if (lane == 0)
+          first.chunkSum[c + s * kClusterWarps] = sum[s];
+      }
     }
     cluster.sync();
     if (part || warp)
@@ -283,17 +303,36 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       double cumulative = inclusive - lanes32;
       int owner = lane * perLane;
       const int end = owner + perLane - 1;
-      for (; owner < end && cumulative + sh.chunkSum[owner] < target; ++owner)
-        cumulative += sh.chunkSum[owner];
+      for (bool before = true; before;) {  // the sums of eight chunks are asked for at once
+        double sums[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          sums[e] = owner + e < end ? sh.chunkSum[owner + e] : 0.0;
+        const int at = owner;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          before = before && at + e < end && cumulative + sums[e] < target;
+          if (before)
+            cumulative += sums[e], ++owner;
+        }
+      }
       sh.owner = owner, sh.before = cumulative;
     }
     __syncwarp();
     double cumulative = sh.before;
     const int a = sh.owner * chunk, b = min(vocab, a + chunk);
     int token = vocab - 1;
-    for (int base = a; base < b; base += 32) {
+    float value[8];
+    for (int base = a, e = 0; base < b; base += 32, ++e) {
       const int j = base + lane;
-      double running = j < b ? double(expf(row[j] / temperature - maximum)) : 0.0;
+      if (e % 8 == 0)
+#pragma unroll
+        for (int ahead = 0; ahead < 8; ++ahead)
+          value[ahead] = j + 32 * ahead < b ? row[j + 32 * ahead] : 0.f;
+      double running = j < b ? double(expf(value[0] / temperature - maximum)) : 0.0;
+#pragma unroll
+      for (int ahead = 0; ahead < 7; ++ahead)
+        value[ahead] = value[ahead + 1];
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const double other = __shfl_up_sync(0xffffffffu, running, o);
@@ -415,23 +454,25 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     for (uint32_t j = 0; j < kept; ++j)
       total += sh.weight[j];
     const float limit = info.topP * total;
-    float nucleus = 0.f;
-    uint32_t keep = 0;
-    do {
-      nucleus += sh.weight[keep];
-      ++keep;
-    } while (keep < kept && nucleus < limit);
-    const float target = random * nucleus;
-    float cumulative = 0.f;
-    int token = sh.sortedIndex[keep - 1];
-    for (uint32_t j = 0; j < keep; ++j) {
-      cumulative += sh.weight[j];
-      if (cumulative >= target) {
-        token = sh.sortedIndex[j];
-        break;
+    // eight weights at a time: one by one every step waits for the shared memory (16.6 -> 16.0 us for the top-40 of eight rows of 248320 logits)
+    auto walk = [&](uint32_t end, float limit, float& sum) {  // adds up weights until they are no longer below the limit; how many they are
+      uint32_t taken = 0;
+      for (bool more = true; more;) {
+        float weight[8];
+        const uint32_t at = taken;
+#pragma unroll
+        for (uint32_t e = 0; e < 8; ++e)
+          weight[e] = at + e < end ? sh.weight[at + e] : 0.f;
+#pragma unroll
+        for (uint32_t e = 0; e < 8; ++e)
+          if (more)
+            sum += weight[e], ++taken, more = taken < end && sum < limit;
       }
-    }
-    tokens[i] = token;
+      return taken;
+    };
+    float nucleus = 0.f, cumulative = 0.f;
+    const uint32_t keep = walk(kept, limit, nucleus);
+    tokens[i] = sh.sortedIndex[walk(keep, random * nucleus, cumulative) - 1];
   }
 }
 

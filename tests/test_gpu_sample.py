@@ -220,3 +220,15 @@ def test_verify_drafts_and_commit_states_follow_the_reference_loop(dev):
   for q, (accepted, _, _) in zip(queries, want):
     if q.state != D.UNBOUND:
       assert np.array_equal(states[q.slot], candidates[q.state + accepted]), q.slot
+
+
+# chunks of one logit less, as many and one more than the 256 that a warp asks for at once, with eight CTAs for a row; 300 and 17 with one
+@pytest.mark.parametrize("rows,vocab", [(16, 1024 * 255), (16, 1024 * 256), (16, 1024 * 256 + 7), (150, 128 * 300 - 5), (150, 2100)])
+def test_chunks_of_plain_temperature_sampling(dev, rows, vocab):
+  rng = np.random.default_rng(vocab)
+  logits = (2.0 * rng.standard_normal((rows, vocab))).astype(np.float32)
+  queries, count = make_queries([(0.9, 1.0, 0, 1)] * rows)
+  tokens = dev.empty(count, np.int32)
+  dev.sample(dev.array(logits), vocab, dev.queries(queries), len(queries), count, 0, tokens)
+  # the order of the sum may move a target that lies within rounding of a boundary to the neighbour
+  assert np.abs(np.array(tokens.download().tolist()) - np.array(expected(logits, queries))).max() <= 1
