@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(256, 2) delta_rule_kernel(const float* q, cons
   const int head = blockIdx.x, keyHead = head % kKeyHeads, tid = threadIdx.x, part = tid >> 5, lane = tid & 31;
   const bool speculative = info.state != kUnbound;
   if (!FUSED && chunked(info, chunkedFrom)) {  // delta_rule_chunked_kernel had this query, all but its norm
-    if (z)
+    if (z && z != out)
       gated_norm_rows(out, z, normWeight, info.start, info.count, head);
     return;
   }
@@ -555,6 +555,7 @@ struct ChunkShared {
   double cumulative[2][kChunk];
   float gateBeta[2][kChunk];
   float system[2][kChunk][kChunk + 1], ratio[2][kChunk][kChunk + 1];  // of each preparing group: the triangular system; R
+  float squares[2][kComputeWarps][kChunk];                            // of the outputs, where they are normalised here
 };
 // named barriers: 1, 2 buffer filled; 3, 4 buffer free; 5, 6 a preparing group
 __device__ __forceinline__ void chunk_ldmatrix(uint32_t (&r)[4], const void* address) {
@@ -826,9 +827,12 @@ __device__ __forceinline__ uint32_t query_by_length(const infdev_query* queries,
   return uint32_t(__ffs(__ballot_sync(0xffffffffu, lane < count && before == rank)) - 1);
 }
 
+// NORM: the outputs go over the gates z, which would be gone before the norm's launch reads them, so they are normalised in the chain. Eight queries of
+// 59 to 493 rows 242 us, 179 without (with the norm's launch).
+template <bool NORM>
 __global__ void __launch_bounds__(kChunkThreads, 1)
-    delta_rule_chunked_kernel(const float* q, const float* k, const float* v, const float* g, const float* beta, const infdev_query* queries, uint64_t stateOffset,
-                              float* out, uint32_t chunkedFrom, uint32_t queryCount, uint32_t sms) {
+    delta_rule_chunked_kernel(const float* q, const float* k, const float* v, const float* g, const float* beta, const float* normWeight,
+                              const infdev_query* queries, uint64_t stateOffset, float* out, uint32_t chunkedFrom, uint32_t queryCount, uint32_t sms) {
   pdl_launch_dependents();
   pdl_wait();
   const uint32_t part = blockIdx.y >= queryCount ? 1 : 0;
@@ -839,7 +843,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
   ChunkShared& sh = *reinterpret_cast<ChunkShared*>(chunkRaw);
   const int head = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // two CTAs have half of a head's columns each
-  const bool split = 2 * kValueHeads * chunked_queries(queries, queryCount, chunkedFrom) <= sms;
+  const bool split = !NORM && 2 * kValueHeads * chunked_queries(queries, queryCount, chunkedFrom) <= sms;
   if (!split && part)
     return;
   const int threads = split ? (kSplitWarps + kPrepareWarps) * kWarp : kChunkThreads;  // at the barriers of a buffer
@@ -872,9 +876,14 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
       }
   };
   load(value, v, 0);
+  [[maybe_unused]] float gate[2][4], weight[2];
+  if constexpr (NORM)
+    weight[0] = normWeight[column], weight[1] = normWeight[column + 8];
   uint32_t step = 0;
   for (uint32_t first = 0; first < info.count; first += kChunk, ++step) {
     const ChunkBuffer& in = sh.buffer[step & 1];
+    if constexpr (NORM)
+      load(gate, out, first);
     float largest[2] = {0.f, 0.f};
 #pragma unroll
     for (int j = 0; j < kHeadDim / 8; ++j)
@@ -955,14 +964,45 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
           S[2 * s + n][e] = fmaf(added[n][e], updateUnit[e >> 1], S[2 * s + n][e] * stateDecay);
     }
     named_barrier_arrive(3 + (step & 1), threads);  // the buffer may be refilled
+    auto output = [&](int n, int e) { return decay[n][e & 1] * (qs[n][e] * productUnit[e >> 1]) + mixed[n][e]; };
+    if constexpr (NORM) {  // gated_rms_norm_128 over the columns of all computing warps
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          mixed[n][e] = output(n, e);
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          float sum = fmaf(mixed[n][e], mixed[n][e], mixed[n][e + 2] * mixed[n][e + 2]);
+#pragma unroll
+          for (int m = 4; m < 32; m <<= 1)
+            sum += __shfl_xor_sync(0xffffffffu, sum, m);
+          if (row == 0)
+            sh.squares[step & 1][warp][8 * n + t2 + e] = sum;
+        }
+      named_barrier(7, kComputeWarps * kWarp);  // two sets of sums in turn: nobody is two chunks behind
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          float sum = 0.f;
+#pragma unroll
+          for (int w = 0; w < kComputeWarps; ++w)
+            sum += sh.squares[step & 1][w][8 * n + t2 + e];
+          const float scale = rsqrtf(sum / float(kHeadDim) + 1.0e-6f);
+          mixed[n][e] = mixed[n][e] * scale * weight[0] * silu_f(gate[n][e]);
+          mixed[n][e + 2] = mixed[n][e + 2] * scale * weight[1] * silu_f(gate[n][e + 2]);
+        }
+    }
 #pragma unroll
     for (int n = 0; n < 2; ++n)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const uint32_t token = first + 8 * n + t2 + (e & 1);
         if (token < info.count)
-          out[(size_t(info.start + token) * kValueHeads + head) * kHeadDim + column + 8 * (e >> 1)] =
-              decay[n][e & 1] * (qs[n][e] * productUnit[e >> 1]) + mixed[n][e];
+          out[(size_t(info.start + token) * kValueHeads + head) * kHeadDim + column + 8 * (e >> 1)] = NORM ? mixed[n][e] : output(n, e);
       }
   }
 #pragma unroll
@@ -1008,12 +1048,14 @@ cudaError_t delta_rule_launch(const float* q, const float* k, const float* v, co
   if (queryCount <= 0)
     return cudaSuccess;
   if (chunkedFrom) {
-    static PerDeviceOnce configured;
-    if (cudaError_t e = configure_shared_memory(delta_rule_chunked_kernel, sizeof(ChunkShared), configured))
+    static PerDeviceOnce configured[2];
+    const bool norm = z == out;
+    const auto kernel = norm ? delta_rule_chunked_kernel<true> : delta_rule_chunked_kernel<false>;
+    if (cudaError_t e = configure_shared_memory(kernel, sizeof(ChunkShared), configured[norm]))
       return e;
-    const int halves = std::min(queryCount, sms / (2 * kValueHeads));  // as many queries as may be split
-    launch_kernel<2>(delta_rule_chunked_kernel, dim3(kValueHeads, unsigned(queryCount + halves)), kChunkThreads, sizeof(ChunkShared), stream, q, k, v, g, beta, queries,
-                  stateOffset, out, chunkedFrom, uint32_t(queryCount), uint32_t(sms));
+    const int halves = norm ? 0 : std::min(queryCount, sms / (2 * kValueHeads));  // as many queries as may be split
+    launch_kernel<2>(kernel, dim3(kValueHeads, unsigned(queryCount + halves)), kChunkThreads, sizeof(ChunkShared), stream, q, k, v, g, beta, normWeight, queries,
+                     stateOffset, out, chunkedFrom, uint32_t(queryCount), uint32_t(sms));
   }
   // The norms of long queries are spread over several CTAs a head, which else were a chain of loads and stores after the last chunk: one query of 493
   // rows 111 -> 96.5 us, six of 17 to 700 rows 202 -> 179, eight of 59 to 493 rows 187 -> 179. Few enough of them that those without rows do not

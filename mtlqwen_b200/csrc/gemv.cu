@@ -402,8 +402,8 @@ __global__ void __launch_bounds__(Layout<Q, NMAT, XSPLIT, HALVES>::kThreads, 1) 
           } else if constexpr (std::is_same_v<Q, IQ4>) {
             iq4_unit(pA, pB, lane, rows, sum);
           } else {
-            // every second super-block of a row lies at a multiple of four bytes: 48 of 634 instructions less (output head 203.5 -> 199.4 us, all rows of
-            // four values at a time by selects 225)
+            // Every second super-block of a row lies at a multiple of four bytes and is read by whole words: 48 of 634 instructions less (output head
+            // 203.5 -> 199.4 us). The others by words that are put together from two: 225 us.
             if (unit & 1)
               q6k_unit<false>(pA, pB, lane, rows, sum);
             else

@@ -810,8 +810,6 @@ static int delta_rule_common(infdev_ctx* ctx, const float* q, const float* k, co
     take_capture(ctx);
     return fail(ctx, INFDEV_E_ARGUMENT, "delta_rule_prefill: writes no image of its result; use infdev_delta_rule for decode-sized passes");
   }
-  if (z == out)  // the chunked form leaves its outputs there before the norm reads the gates
-    chunkedFrom = 0;
   ctx->launches += chunkedFrom ? 2 : 1;
   return check(ctx,
                infdev::delta_rule_launch(q, k, v, g, beta, z, normWeight, queries, queryCount, stateOffset, stateBytes, out, take_capture(ctx), ctx->imageCounters,
