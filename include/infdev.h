@@ -128,8 +128,8 @@ int infdev_image_capture(infdev_ctx* ctx, uint8_t* image);
  * reads images; other kernels ignore the request and read x. */
 int infdev_image_supply(infdev_ctx* ctx, const uint8_t* image);
 /* One-shot: the activations of the next infdev_linear, infdev_linear_group or infdev_gate_up call (k = 4096) are the RMS norm of
- * its x with weights w[k], as infdev_rms_norm computes it: one launch less where the kernel can do it on the way in (integer
- * Q4_K, up to 8 rows); elsewhere the call launches the norm itself. normalised: [rows, k] scratch for that, x itself or a buffer apart
+ * its x with weights w[k], as infdev_rms_norm computes it: one launch less where the kernel can do it on the way in (Q4_K: the integer
+ * kernel with up to 8 rows, the tensor-core GEMM with more); elsewhere the call launches the norm itself. normalised: [rows, k] scratch for that, x itself or a buffer apart
  * from it; with store the normalised rows are left there in either case. No image may be supplied for the same call. */
 int infdev_norm_supply(infdev_ctx* ctx, const float* w, float* normalised, int store);
 /* CUDA-graph capture of a pass on the context's stream (no reference counterpart: Metal re-encodes every

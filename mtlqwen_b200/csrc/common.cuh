@@ -228,6 +228,22 @@ __device__ __forceinline__ float square_sum(const float4& a, const float4& b) {
                    __fmaf_rn(b.w, b.w, __fmaf_rn(b.z, b.z, __fmaf_rn(b.x, b.x, __fmul_rn(b.y, b.y)))));
 }
 
+// The RMS norm of a row of 4096 by 512 threads, each with eight consecutive values a, b and their weights.
+__device__ __forceinline__ void normalise_4096(const float4& a, const float4& b, const float4& ga, const float4& gb, float (&v)[8]) {
+  __shared__ float sums[16];
+  const float sum = warp_sum(square_sum(a, b));
+  if (threadIdx.x % kWarp == 0)
+    sums[threadIdx.x / kWarp] = sum;
+  __syncthreads();
+  float total = 0.f;
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    total += sums[i];
+  const float scale = rsqrtf(total / 4096.0f + 1.0e-6f);
+  v[0] = a.x * scale * ga.x, v[1] = a.y * scale * ga.y, v[2] = a.z * scale * ga.z, v[3] = a.w * scale * ga.w;
+  v[4] = b.x * scale * gb.x, v[5] = b.y * scale * gb.y, v[6] = b.z * scale * gb.z, v[7] = b.w * scale * gb.w;
+}
+
 __device__ __forceinline__ float silu_f(float v) { return v / (1.0f + expf(-v)); }
 __device__ __forceinline__ float sigmoid_f(float v) { return 1.0f / (1.0f + expf(-v)); }
 

@@ -175,7 +175,7 @@ struct Ops {
   // Announces the RMS norm of `hidden` as the activations of the projections that follow at once, and returns what to pass them.
   // store: the normalised rows are wanted in scratch.norm in any case.
   const Tensor& normalised(const Tensor& hidden, const float* norm, std::initializer_list<const Weight*> targets, bool store) {
-    bool fold = selfServed();
+    bool fold = selfServed() || rows > imageRows;  // with many rows the tensor-core GEMM normalises where it lays out its activations
     for (const Weight* target : targets)
       fold = fold && target->type == INFDEV_Q4_K;
     if (fold) {

@@ -541,16 +541,25 @@ static int linear_run(infdev_ctx* ctx, int type, bool pair, int count, const voi
     u.partial = ctx->ummaPartial;
     u.acts = static_cast<const uint8_t*>(ctx->ummaActs);
     u.status = ctx->status;
-    if (int r = launch_norm(ctx, norm, x, m, k))
-      return r;
     const int64_t slice = 128;  // activation rows per launch
+    // The layout of the activations is that of their norm, which is stored where somebody may read it. Results of one slice over the activations
+    // of the next want a norm of all rows before.
+    bool stored = norm.store || norm.normalised == x, over = false;
+    for (int i = 0; i < count; ++i) {
+      stored = stored || (residual && overlap(norm.normalised, m * k, residual[i], m * n[i]));
+      over = over || overlap(x, m * k, y[i], m * n[i]);
+    }
+    if (over && m > slice)
+      if (int r = launch_norm(ctx, norm, x, m, k))
+        return r;
     for (int64_t row = 0; row < m; row += slice) {
       u.m = int(m - row < slice ? m - row : slice);
       for (int i = 0; i < count; ++i) {
         u.seg[i].y = y[i] + row * n[i];
         u.seg[i].res = residual && residual[i] ? residual[i] + row * n[i] : nullptr;
       }
-      if (int r = check(ctx, infdev::umma_launch(pair, u, x + row * k, int(k), ctx->sms, ctx->stream), "umma launch"))
+      if (int r = check(ctx, infdev::umma_launch(pair, u, x + row * k, int(k), norm.weight, norm.weight && stored ? norm.normalised + row * k : nullptr, ctx->sms, ctx->stream),
+                        "umma launch"))
         return r;
       ctx->launches += u.splits > 1 ? 3 : 2;
     }

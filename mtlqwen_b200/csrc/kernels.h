@@ -60,7 +60,7 @@ struct UmmaParams {
   int* status;
 };
 
-cudaError_t umma_launch(bool pair, const UmmaParams& p, const float* x, int ldx, int sms, cudaStream_t stream);
+cudaError_t umma_launch(bool pair, const UmmaParams& p, const float* x, int ldx, const float* norm, float* normalised, int sms, cudaStream_t stream);
 
 // What a tiled copy of the fp16 GEMV moves per row of a matrix of this type: `blocks` super-blocks of `blockBytes` (for
 // Q8_0: eight blocks) and `padBytes` more. blockBytes 0: not a type of that kernel.

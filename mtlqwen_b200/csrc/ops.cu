@@ -161,18 +161,8 @@ __global__ void __launch_bounds__(512) rms_norm_4096_kernel(const float* x, cons
   }
   const float4 a = *reinterpret_cast<const float4*>(src + d), b = *reinterpret_cast<const float4*>(src + d + 4);
   const float4 ga = *reinterpret_cast<const float4*>(w + d), gb = *reinterpret_cast<const float4*>(w + d + 4);
-  __shared__ float sums[16];
-  const float sum = warp_sum(square_sum(a, b));
-  if (lane == 0)
-    sums[warp] = sum;
-  __syncthreads();
-  float total = 0.f;
-#pragma unroll
-  for (int i = 0; i < 16; ++i)
-    total += sums[i];
-  const float scale = rsqrtf(total / float(kDim) + 1.0e-6f);
-  const float v[8] = {a.x * scale * ga.x, a.y * scale * ga.y, a.z * scale * ga.z, a.w * scale * ga.w,
-                      b.x * scale * gb.x, b.y * scale * gb.y, b.z * scale * gb.z, b.w * scale * gb.w};
+  float v[8];
+  normalise_4096(a, b, ga, gb, v);
   if (y) {
     *reinterpret_cast<float4*>(y + size_t(row) * kDim + d) = make_float4(v[0], v[1], v[2], v[3]);
     *reinterpret_cast<float4*>(y + size_t(row) * kDim + d + 4) = make_float4(v[4], v[5], v[6], v[7]);
