@@ -335,10 +335,13 @@ __global__ void __launch_bounds__(128, 6) attention_scan_kernel(const float* q, 
 // Operands as in the scan: fp16 keys and values, query and softmax weights as fp16 hi + lo, fp32 accumulation. A tile of 64 tokens is
 // 1.6 k cycles of MMAs for the scores (bounded by shared memory: A and B both come from there) and 1 k for the values; mma.sync,
 // with 16 rows x 4 heads, was 8 k for half the rows.
-// Measured, with the merge, and before, with mma.sync: 128 rows behind 1920 tokens 51.0 -> 32.1 us (31.0 with weights by powers of two), four times
-// 30 rows behind up to 1970 49.3 -> 32.4 (31.4), 2048 rows behind 2048 1070 -> 457 (420); by its own clocks the first of these spends 5000 of
-// 38000 on its start, 6500 on q, 10000 on scores, which wait for their copies, 4300 on weights, 4000 on the last values and 5300 on the store of its results; 64 rows of 64 tokens 13.0 -> 16.1: a fixed start of laying out q and an end of
+// Measured, with the merge, and before, with mma.sync: 128 rows behind 1920 tokens 51.0 -> 32.0 us, four times 30 rows behind up to 1970 49.3 -> 33.5 (33.8
+// with every tile masked), 2048 rows behind 2048 1070 -> 443 (455 with every tile masked); by its own clocks the first of these spent, with weights by
+// ex2.approx, 5000 of 38000 on its start, 6500 on q, 10000 on scores, which wait for their copies, 4300 on weights, 4000 on the last values and 5300 on the
+// store of its results; 64 rows of 64 tokens 13.0 -> 16.1: a fixed start of laying out q and an end of
 // reading tensor memory, which little work has to pay for, so short contexts stay with attention_group_kernel below.
+// Left out: weights as ex2.approx.ftz of a product rounded once, 31.3, 32.7 and 419 us, but weights between 1/4 and 1/2 then are off by 8.1e-8 rms and
+// -3.7e-8 on average instead of 7.3e-8 and 1.1e-8.
 // Errors against fp64 (rms, of the result's): 128 rows behind 1920 tokens 1.4e-6 and 1.9e-6 before, 300 behind 8700 7.6e-6 and 2.1e-5,
 // 32 behind 29968 2.9e-6 and 4.6e-6: fewer roundings between tiles.
 //
@@ -471,13 +474,6 @@ __device__ __forceinline__ void mask_scores(uint32_t (&score)[16], uint32_t firs
 #pragma unroll
   for (int i = 0; i < 16; ++i)
     score[i] = first + i < live ? score[i] : __float_as_uint(-INFINITY);
-}
-// e^((score - largest) / 16) as a power of two: a third of expf's instructions, which the workers' 128 x 256 weights a round are bound by. The rounding of
-// the exponent makes a weight w wrong by up to |ln w| x 2^-24 of itself, most where it counts least.
-__device__ __forceinline__ float softmax_weight(float score, float largest) {
-  float weight;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(weight) : "f"((score - largest) * (1.4426950408889634f / 16.0f)));
-  return weight;
 }
 
 __global__ void __launch_bounds__(kTileThreads, 1)
@@ -759,7 +755,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
                 mask_scores(score, c, live);
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
-                const float w0 = softmax_weight(__uint_as_float(score[2 * i]), 16.f * maximum), w1 = softmax_weight(__uint_as_float(score[2 * i + 1]), 16.f * maximum);
+                const float w0 = expf(__uint_as_float(score[2 * i]) * (1.0f / 16.0f) - maximum), w1 = expf(__uint_as_float(score[2 * i + 1]) * (1.0f / 16.0f) - maximum);
                 norm += w0 + w1;
                 const uint2 w = split_pair(w0, w1);
                 halves[i] = w.x, halves[8 + i] = w.y;
