@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(Layout<Q, NMAT, XSPLIT, HALVES>::kThreads, 1) 
             iq4_unit(pA, pB, lane, rows, sum);
           } else {
             // Every second super-block of a row lies at a multiple of four bytes and is read by whole words: 48 of 634 instructions less (output head
-            // 203.5 -> 199.4 us). The others by words that are put together from two: 225 us.
+            // 203.5 -> 192.7 us). The others by words that are put together from two: 225 us.
             if (unit & 1)
               q6k_unit<false>(pA, pB, lane, rows, sum);
             else
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(Layout<Q, NMAT, XSPLIT, HALVES>::kThreads, 1) 
           mbar_arrive(&ctl.empty[slot]);
       }
       it += perTile;
-      // Hand the partial sums of the K split to the buffer's finisher and go on with the next tile.
+      // Hand the partial sums of the K split to the buffer's finisher, which adds them in the order of the super-blocks, and go on with the next tile.
       const uint32_t parity = (bufferState >> buffer) & 1u;
       if (((bufferState >> (4 + buffer)) & 1u) && !mbar_wait_bounded(&ctl.partialFree[buffer], parity ^ 1u, abortFlag))
         give_up();
@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(Layout<Q, NMAT, XSPLIT, HALVES>::kThreads, 1) 
       float* sums = partial + size_t(buffer) * NMAT * kConsumerWarps * 128;
 #pragma unroll
       for (int mat = 0; mat < NMAT; ++mat)
-        reinterpret_cast<float4*>(sums + (mat * kConsumerWarps + warp) * 128)[lane] = make_float4(total[mat][0][0], total[mat][0][1], total[mat][0][2], total[mat][0][3]);
+        reinterpret_cast<float4*>(sums + (mat * kConsumerWarps + half * kStageWarps + unit) * 128)[lane] = make_float4(total[mat][0][0], total[mat][0][1], total[mat][0][2], total[mat][0][3]);
       __syncwarp();
       if (lane == 0)
         mbar_arrive(&ctl.partialReady[buffer]);
