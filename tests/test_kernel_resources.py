@@ -38,3 +38,12 @@ def test_gemv_keeps_no_array_in_local_memory(reports):
 def test_q6k_of_few_rows_is_decoded_without_spills(reports):
   kernels = {tiles: spills for (qtype, tiles), (_, spills) in reports["gemv_wide.cu"].items() if qtype == "Q6K"}
   assert sorted(kernels) == [(2, ), (3, ), (4, ), (5, )] and not any(kernels.values()), kernels
+
+
+def test_the_norm_of_long_queries_leaves_short_ones_their_registers(tmp_path):
+  """The launch of the token-by-token delta rule also normalises the outputs of the chunked one: without that it spills 52 bytes, with the norm inlined 68."""
+  nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+  report = subprocess.run([nvcc, *build.ARCH, *build.FLAGS, "-Xptxas=-v", "-I", str(build.PACKAGE.parent / "include"), "-x", "cu", "-cubin", str(build.CSRC / "gdn.cu"),
+                           "-o", str(tmp_path / "gdn.out")], capture_output=True, text=True, check=True).stderr
+  spills = re.findall(r"Function properties for \S*delta_rule_kernelILb0E\S*\s+\d+ bytes stack frame, (\d+) bytes spill stores", report)
+  assert len(spills) == 1 and int(spills[0]) <= 52
