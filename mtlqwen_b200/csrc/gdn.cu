@@ -218,7 +218,10 @@ __device__ __forceinline__ uint32_t chunked_queries(const infdev_query* queries,
 
 // gated_rms_norm_128 of one head of a query's rows, in place: eight warps, eight rows each at a time, in turn with the CTAs of the grid's third dimension.
 // Not inlined: delta_rule_kernel<false>, whose launch this is, would keep fewer registers for its own queries (68 bytes of spills instead of 24; 12 rows
-// 24.7 us instead of 23.8, 215 instead of 211.6 for 128).
+// 24.7 us instead of 23.9, 215 instead of 211.6 for 128).
+// The squares are added in the order in which the chunked kernel with the norm in its chain has them, columns c and c + 8 first, then the eight pairs of
+// 16 columns by halves, then the eight 16s one after the other, so the bits do not depend on which of the two norms a call takes. Rows are halved between
+// lanes as in share_sums: 41 exchanges for eight rows, where warp_sum takes 40 in its own order.
 __device__ __noinline__ void gated_norm_rows(float* out, const float* z, const float* normWeight, uint32_t start, uint32_t count, int head) {
   constexpr uint32_t kRows = 8;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -237,9 +240,42 @@ __device__ __noinline__ void gated_norm_rows(float* out, const float* z, const f
         o[r][c] = first + r < count ? out[at + r * kPitch + 32 * c] : 0.f;
         gate[r][c] = first + r < count ? z[at + r * kPitch + 32 * c] : 0.f;
       }
+    // lanes with bit 3 go on with columns 64 .. 127 and leave the others to their partners, eight columns off
+    const bool high = lane & 8;
+    float pairs[kRows][2];
+#pragma unroll
+    for (uint32_t r = 0; r < kRows; ++r)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float other = __shfl_xor_sync(0xffffffffu, high ? o[r][e] : o[r][e + 2], 8), own = high ? o[r][e + 2] : o[r][e];
+        const float low8 = high ? other : own, high8 = high ? own : other;
+        pairs[r][e] = __fmaf_rn(high8, high8, __fmul_rn(low8, low8));
+      }
+#pragma unroll
+    for (uint32_t partner = 1; partner < 8; partner *= 2) {
+      const uint32_t left = kRows / 2 / partner;
+      const bool upper = lane & partner;
+#pragma unroll
+      for (uint32_t r = 0; r < left; ++r)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float other = __shfl_xor_sync(0xffffffffu, upper ? pairs[r][e] : pairs[r + left][e], partner);
+          pairs[r][e] = (upper ? pairs[r + left][e] : pairs[r][e]) + other;
+        }
+    }
+    // 16 columns each: 32 c + 16 (bit 4) of the row that bits 0, 1 and 2 name, c = e or, with bit 3, e + 2
+    float even[2], odd[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float other = __shfl_xor_sync(0xffffffffu, pairs[0][e], 16);
+      even[e] = lane & 16 ? other : pairs[0][e], odd[e] = lane & 16 ? pairs[0][e] : other;
+    }
+    const float below = __shfl_xor_sync(0xffffffffu, ((even[0] + odd[0]) + even[1]) + odd[1], 8);
+    const float total = (((below + even[0]) + odd[0]) + even[1]) + odd[1];  // of lanes with bit 3
+    const float scales = rsqrtf(total / float(kHeadDim) + 1.0e-6f);
 #pragma unroll
     for (uint32_t r = 0; r < kRows; ++r) {
-      const float scale = rsqrtf(warp_sum(o[r][0] * o[r][0] + o[r][1] * o[r][1] + o[r][2] * o[r][2] + o[r][3] * o[r][3]) / float(kHeadDim) + 1.0e-6f);
+      const float scale = __shfl_sync(0xffffffffu, scales, 8 | (r >> 2 & 1) | (r >> 1 & 1) << 1 | (r & 1) << 2);
       if (first + r < count)
 #pragma unroll
         for (int c = 0; c < 4; ++c)
@@ -977,7 +1013,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
       for (int n = 0; n < 2; ++n)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          float sum = fmaf(mixed[n][e], mixed[n][e], mixed[n][e + 2] * mixed[n][e + 2]);
+          float sum = __fmaf_rn(mixed[n][e + 2], mixed[n][e + 2], __fmul_rn(mixed[n][e], mixed[n][e]));
 #pragma unroll
           for (int m = 4; m < 32; m <<= 1)
             sum += __shfl_xor_sync(0xffffffffu, sum, m);

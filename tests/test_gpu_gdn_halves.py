@@ -74,6 +74,13 @@ def test_outputs_over_the_gates(mixed):
     assert np.linalg.norm(apart - over) <= 7 * 2.0 ** -24 * np.linalg.norm(apart) and state.tobytes() == other.tobytes()
 
 
+@pytest.mark.parametrize("chosen", [[0], [1], [6], [0, 1], [0, 1, 2], [3, 0, 4, 5, 7]])  # whole and short last chunks, one CTA a head and two, short queries beside
+def test_outputs_over_the_gates_have_the_same_bits(mixed, chosen):
+  """The norm in the chain and the one behind it add the squares in one order."""
+  for i, apart, over in zip(chosen, mixed.run(chosen), mixed.run(chosen, in_place=True)):
+    assert same(apart, over), i
+
+
 def test_the_norm_on_one_cta_or_on_eight_has_the_same_bits(dev):
   """28 queries leave a head of each one CTA for its norms; a query alone has eight of 64 rows at a time, the longest here one row more than they
   take at once."""
