@@ -547,7 +547,7 @@ __global__ void __launch_bounds__(256, 2) delta_rule_kernel(const float* q, cons
 //   delta  = A^-1 rhs,   rhs_t = beta_t * (v_t - G_t * S^T k_t)
 //   o_t    = G_t * S^T q_t + sum_{i<=t} R[t][i] (q_t . k_i) delta_i
 //   S      = G_15 * S + sum_i (G_15 / G_i) k_i delta_i^T
-// grid (32 value heads, queries and the second halves of some), 12 warps; serves the non-speculative queries of at least `chunkedFrom` tokens, all
+// grid (32 value heads, queries, or more where so few are split), 12 warps; serves the non-speculative queries of at least `chunkedFrom` tokens, all
 // but the norm of their outputs, which is delta_rule_kernel's launch (gated_norm_rows): here it stood in the chain, 2000 of 8200 clocks a chunk. A last
 // chunk of fewer than 16 tokens is padded with tokens of beta = 0, k = q = v = 0 and decay 1, which change nothing.
 //
@@ -873,17 +873,18 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
                               const infdev_query* queries, uint64_t stateOffset, float* out, uint32_t chunkedFrom, uint32_t queryCount, uint32_t sms) {
   pdl_launch_dependents();
   pdl_wait();
-  const uint32_t part = blockIdx.y >= queryCount ? 1 : 0;
-  const infdev_query info = queries[query_by_length(queries, queryCount, chunkedFrom, blockIdx.y - part * queryCount)];
+  // Two CTAs have half of a head's columns each: rows of the grid from the number of chunked queries on, which else have nothing to do, take the second halves.
+  const uint32_t taken = chunked_queries(queries, queryCount, chunkedFrom);
+  const bool split = !NORM && 2 * kValueHeads * taken <= sms;
+  const uint32_t part = split && blockIdx.y >= taken ? 1 : 0, rank = blockIdx.y - part * taken;
+  if (rank >= (split ? taken : queryCount))
+    return;
+  const infdev_query info = queries[query_by_length(queries, queryCount, chunkedFrom, rank)];
   if (!chunked(info, chunkedFrom))  // delta_rule_kernel takes this query
     return;
   extern __shared__ __align__(16) uint8_t chunkRaw[];
   ChunkShared& sh = *reinterpret_cast<ChunkShared*>(chunkRaw);
   const int head = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // two CTAs have half of a head's columns each
-  const bool split = !NORM && 2 * kValueHeads * chunked_queries(queries, queryCount, chunkedFrom) <= sms;
-  if (!split && part)
-    return;
   const int threads = split ? (kSplitWarps + kPrepareWarps) * kWarp : kChunkThreads;  // at the barriers of a buffer
   // The computing warps hold more than a third of the registers each: 2 x 192 + 120 = 3 x 168 a thread, of the 168 that the launch
   // bounds give all three groups of four warps.
@@ -1091,14 +1092,16 @@ cudaError_t delta_rule_launch(const float* q, const float* k, const float* v, co
     const auto kernel = norm ? delta_rule_chunked_kernel<true> : delta_rule_chunked_kernel<false>;
     if (cudaError_t e = configure_shared_memory(kernel, sizeof(ChunkShared), configured[norm]))
       return e;
-    const int halves = norm ? 0 : std::min(queryCount, sms / (2 * kValueHeads));  // as many queries as may be split
-    launch_kernel<2>(kernel, dim3(kValueHeads, unsigned(queryCount + halves)), kChunkThreads, sizeof(ChunkShared), stream, q, k, v, g, beta, normWeight, queries,
+    // rows for the halves of as many queries as may be split. Rows of their own beside those of all queries made three turns of CTAs out of two where
+    // eight queries are all short (5 rows each 18.6 -> 19.6 us), and a grid too large out of 65535 queries.
+    const int rows = norm ? queryCount : std::max(queryCount, 2 * std::min(queryCount, sms / (2 * kValueHeads)));
+    launch_kernel<2>(kernel, dim3(kValueHeads, unsigned(rows)), kChunkThreads, sizeof(ChunkShared), stream, q, k, v, g, beta, normWeight, queries,
                      stateOffset, out, chunkedFrom, uint32_t(queryCount), uint32_t(sms));
   }
   // The norms of long queries are spread over several CTAs a head, which else were a chain of loads and stores after the last chunk: one query of 493
   // rows 111 -> 96.5 us, six of 17 to 700 rows 202 -> 179, eight of 59 to 493 rows 187 -> 179. Few enough of them that those without rows do not
   // tell (eight queries of 128 rows 81.0, with four CTAs a head 81.7, with eight 83.4).
-  const int spread = chunkedFrom ? std::clamp(6 * sms / (kValueHeads * queryCount), 1, 8) : 1;
+  const int spread = chunkedFrom && z && z != out ? std::clamp(6 * sms / (kValueHeads * queryCount), 1, 8) : 1;
   // Not launched early: its CTAs would be placed around those of the kernels before it, two on an SM, and the token-by-token chain
   // of short queries runs slower for it (12 rows: 37.5 against 31.0 us; passes that the chunked kernel takes lose 1 us).
   launch_kernel(delta_rule_kernel<false>, dim3(kValueHeads, unsigned(queryCount), unsigned(spread)), 256, 0, stream, q, k, v, g, beta, z, normWeight, queries, stateOffset,

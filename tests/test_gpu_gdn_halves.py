@@ -89,3 +89,20 @@ def test_the_norm_on_one_cta_or_on_eight_has_the_same_bits(dev):
   together = everything.run(range(len(lengths)))
   for i in range(5):
     assert same(everything.run([i])[0], together[i]), lengths[i]
+
+
+def test_as_many_queries_as_a_grid_has_rows(dev):
+  """65535 queries, all of them the same row and record, beside each of which nothing more fits into the grid."""
+  rng, count = np.random.default_rng(53), 65535
+  draw = lambda *shape: dev.array(rng.standard_normal(shape).astype(np.float32))
+  q, k, v, z, g, beta, norm, previous, next_ = draw(1, 16, 128), draw(1, 16, 128), draw(1, 32, 128), draw(1, 32, 128), dev.array(np.full((1, 32), -0.1, np.float32)), \
+    dev.array(np.full((1, 32), 0.5, np.float32)), draw(128), draw(1, STATE), dev.empty((1, STATE))
+  query = D.Query()
+  query.previous, query.next, query.start, query.count, query.position, query.slot, query.state = previous.ptr, next_.ptr, 0, 1, 77, 0, D.UNBOUND
+  results = []
+  for queries in ([query], [query] * count):
+    out = dev.empty((1, 32, 128))
+    dev.delta_rule(q, k, v, g, beta, z, norm, dev.queries(queries), len(queries), 0, STATE * 4, out, prefill=True)
+    dev.commit()
+    results.append((out.download().tobytes(), next_.download().tobytes()))
+  assert results[0] == results[1]
