@@ -542,14 +542,15 @@ static int linear_run(infdev_ctx* ctx, int type, bool pair, int count, const voi
     u.acts = static_cast<const uint8_t*>(ctx->ummaActs);
     u.status = ctx->status;
     const int64_t slice = 128;  // activation rows per launch
-    // The layout of the activations is that of their norm, which is stored where somebody may read it. Results of one slice over the activations
-    // of the next want a norm of all rows before.
-    bool stored = norm.store || norm.normalised == x, over = false;
+    // The layout of the activations is that of their norm, which is stored where somebody may read it. A norm of all rows before is wanted by results of
+    // one slice over what the norm of the next reads, its activations and weights, and by a residual of one slice in the normalised rows of the next.
+    bool stored = norm.store || norm.normalised == x, before = false;
     for (int i = 0; i < count; ++i) {
-      stored = stored || (residual && overlap(norm.normalised, m * k, residual[i], m * n[i]));
-      over = over || overlap(x, m * k, y[i], m * n[i]);
+      const bool added = residual && overlap(norm.normalised, m * k, residual[i], m * n[i]);
+      stored = stored || added;
+      before = before || added || overlap(x, m * k, y[i], m * n[i]) || overlap(norm.weight, k, y[i], m * n[i]);
     }
-    if (over && m > slice)
+    if (before && m > slice)
       if (int r = launch_norm(ctx, norm, x, m, k))
         return r;
     for (int64_t row = 0; row < m; row += slice) {
