@@ -292,12 +292,14 @@ template <bool PAIR> __global__ void __launch_bounds__(kBoundThreads, 1) umma_li
     const int quadrant = warp & 3, row = quadrant * 32 + lane;
     const uint32_t laneBase = tmem + (uint32_t(quadrant * 32) << 16), aAddress = laneBase + kColA + group * 64;
     constexpr uint32_t k1024 = 0x64006400u;
+    // of the whole warp, which reads and writes tensor memory together: a lane whose limit runs out takes the others with it
+    auto wait = [&](uint64_t* bar, uint32_t parity) { return bool(__all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abortFlag))); };
     uint32_t slot = group >> 1, parity = 0, fills = 0, unit = 0, slab = group >> 1;  // slab: the next of this group, counted over all items
     bool ok = true;
     for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++unit) {
       const uint32_t end = (unit + 1) * uint32_t(blocksPerRow * kMats);
       for (; slab < end && ok; slab += 2, ++fills) {
-        ok = mbar_wait_bounded(&ctl.full[slot], parity, abortFlag);
+        ok = wait(&ctl.full[slot], parity);
         if (!ok)
           break;
         const uint8_t* block = ring + size_t(slot) * kSlabBytes + row * 144;
@@ -319,33 +321,35 @@ template <bool PAIR> __global__ void __launch_bounds__(kBoundThreads, 1) umma_li
           scale[t] = __hmul2(d, *reinterpret_cast<const __half2*>(&scalePair)), low[t] = __hmul2(dmin, *reinterpret_cast<const __half2*>(&minPair));
         }
         // the slab is in registers by now; the MMAs that read this group's operand before may run until the first store
-        auto before_store = [&](int t) {
-          if (t > 0)
-            return;
-          __syncwarp();
-          if (lane == 0)
-            mbar_arrive(&ctl.slotFree[slot]);
-          if (fills > 0)
-            ok = mbar_wait_bounded(&ctl.aFree[group], (fills - 1) & 1, abortFlag);
-          fence_after_sync();
+        auto store = [&](int t, const uint32_t (&v)[32]) {
+          if (t == 0) {
+            __syncwarp();
+            if (lane == 0)
+              mbar_arrive(&ctl.slotFree[slot]);
+            if (fills > 0)
+              ok = wait(&ctl.aFree[group], (fills - 1) & 1);
+            fence_after_sync();
+          }
+          if (ok)
+            tmem_store32(aAddress + 32 * t, v);
         };
         if (__any_sync(0xffffffffu, reaches_64th(scale[0]) || reaches_64th(scale[1]))) {
 #pragma unroll
           for (int t = 0; t < 2; ++t) {
             uint32_t v[32];
             dequantise<false>(quads[2 * t], quads[2 * t + 1], scale[t], low[t], v);
-            before_store(t);
-            tmem_store32(aAddress + 32 * t, v);
+            store(t, v);
           }
         } else {
 #pragma unroll
           for (int t = 0; t < 2; ++t) {
             uint32_t v[32];
             dequantise<true>(quads[2 * t], quads[2 * t + 1], scale[t], low[t], v);
-            before_store(t);
-            tmem_store32(aAddress + 32 * t, v);
+            store(t, v);
           }
         }
+        if (!ok)
+          break;
         tmem_wait_store();
         fence_before_sync();
         __syncwarp();
@@ -360,7 +364,7 @@ template <bool PAIR> __global__ void __launch_bounds__(kBoundThreads, 1) umma_li
       const int m = p.m;
       float residual[8];
       load_residual<PAIR>(to, m, int(group) * 8, residual);
-      ok = ok && mbar_wait_bounded(&ctl.dReady, unit & 1, abortFlag);
+      ok = ok && wait(&ctl.dReady, unit & 1);
       if (!ok)
         break;
       fence_after_sync();
