@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(Layout<Q, NMAT, XSPLIT, HALVES>::kThreads, 1) 
   // ---- consumers ----
   // The super-block of a warp in its half's slabs: of Q6_K each scheduler has as many of one parity as of the other.
   const int g = lane >> 2, t = lane & 3, half = warp / kStageWarps, unit = std::is_same_v<Q, Q6K> ? (warp % kStageWarps) ^ (warp >> 2 & 1) : warp % kStageWarps;
-  static_assert(stage_bytes<Q>() % 4 == 0 && row_pitch<Q>() % 4 == 0 && (Q::kBlockBytes % 4 == 0 || Q::kBlockBytes * 2 % 4 == 0), "which blocks lie at words");
+  static_assert(row_pitch<Q>() % 4 == 0 && Q::kBlockBytes * 2 % 4 == 0 && box_blocks<Q>() % 2 == 0, "blocks of even number lie at words");
   const uint8_t* const blocks = ring + (unit / box_blocks<Q>()) * box_bytes<Q>() + (unit % box_blocks<Q>()) * Q::kBlockBytes + g * row_pitch<Q>();
   uint32_t it = 0, mine = half, slot = half, phase = 0;
   uint32_t bufferState = 0;  // bit b: parity of the next use of partial-sum buffer b; bit 4 + b: it has been used before

@@ -62,6 +62,7 @@ constexpr int kCandidates = 2048;   // collected logits that fit
 constexpr int kMostTied = 256;      // more at the threshold than these stay out of the collection (ranking all of 1003 took 40 us)
 constexpr int kMostWanted = 64;
 constexpr int kChunks = 128;        // plain temperature sampling sums the row in this many contiguous pieces per CTA
+static_assert(kChunks % (2 * kClusterWarps) == 0, "a warp takes two pieces at a time, all of them of its own CTA");
 
 struct SampleShared {
   float maxima[kParts];  // of the parts; of the warps for the argmax
