@@ -230,5 +230,14 @@ def test_chunks_of_plain_temperature_sampling(dev, rows, vocab):
   queries, count = make_queries([(0.9, 1.0, 0, 1)] * rows)
   tokens = dev.empty(count, np.int32)
   dev.sample(dev.array(logits), vocab, dev.queries(queries), len(queries), count, 0, tokens)
-  # the order of the sum may move a target that lies within rounding of a boundary to the neighbour
-  assert np.abs(np.array(tokens.download().tolist()) - np.array(expected(logits, queries))).max() <= 1
+  got, sure = tokens.download().tolist(), 0
+  for row, (token, q) in enumerate(zip(got, queries)):
+    # the weights' exponents as the kernel rounds them, everything else in 64 bits: weights off by 2^-23 each move the sums by less than 1e-7 of the whole
+    exponent = logits[row] / np.float32(q.temperature) - logits[row].max() / np.float32(q.temperature)
+    sums = np.cumsum(np.exp(exponent.astype(np.float64)))
+    target = float(oracle.uniform(q.seed, q.position + q.count - q.samples + 1)) * sums[-1]
+    want = int(np.searchsorted(sums, target))
+    clear = np.abs(sums[max(want - 1, 0):want + 1] - target).min() > 1e-7 * sums[-1]  # no boundary within rounding of the target
+    sure += clear
+    assert token == want if clear else abs(token - want) <= 1, row
+  assert sure >= 3 * rows // 4
