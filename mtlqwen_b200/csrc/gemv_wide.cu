@@ -342,9 +342,9 @@ template <class Q, int NT> __global__ void __launch_bounds__(kThreads, 1) wide_k
 }
 
 // Adds up the slices, four values per thread, and finishes: y = sum (+ residual), or silu(gate) * up for a pair. The columns of
-// all matrices lie side by side in a row of the partial results. AT_ONCE: a thread asks for all slices before it adds (projections of a layer of
-// mixed types with 9 and 16 rows 103.1 -> 99.6 and 104.4 -> 101.3 us); with many rows it is the number of resident blocks that counts, which takes
-// few registers (128 rows 491 us, at once 498).
+// all matrices lie side by side in a row of the partial results. AT_ONCE: a thread asks for all slices before it adds; with many rows it is the
+// number of resident blocks that counts, which takes few registers. Projections of a layer of mixed types with 9, 16, 32, 48, 64, 80, 96 and 128 rows,
+// one after the other / at once: 102.5 / 102.6, 104.5 / 101.0, 150.5 / 148.2, 218.8 / 223.0, 267.3 / 262.9, 315.6 / 315.7, 366.2 / 368.5 and 491.8 / 498.4 us.
 template <bool AT_ONCE> __global__ void __launch_bounds__(256) wide_reduce_kernel(const __grid_constant__ WideParams p) {
   pdl_launch_dependents();
   pdl_wait();

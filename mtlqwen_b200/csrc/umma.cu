@@ -3,7 +3,7 @@
 // Replaces linear_prefill / linear_prefill_small (quant_linear.metal:151-233, epilogues 0 / 1 / 2) for weight matrices
 // whose row count is a multiple of 128 and whose K is a multiple of 2048, for 9 to 128 activation rows per launch:
 //   * one thread owns one weight row of a 128-row tile: it reads the row's 144-byte super-block from a TMA-filled slab,
-//     dequantises it to fp16 (d*sc*q - dmin*m, q made exact first, then one fused multiply-add per two weights) and
+//     dequantises it to fp16 (d*sc*q - dmin*m, d*sc and dmin*m rounded once, one fused multiply-add per two weights) and
 //     writes it to tensor memory with tcgen05.st;
 //   * tcgen05.mma (kind::f16, M = 128 weight rows, N = 128 activation rows, K = 16) takes A from TMEM and B, the
 //     activations, from shared memory through a matrix descriptor. The activations were rounded to fp16 beforehand
@@ -25,7 +25,7 @@
 // instructions a scheduler) and 1250 with 128 (of which the MMAs are 1024). What is left is not in the loop: 4 to 5 us
 // from the end of the kernel before to the first MMA, through the layout kernel and two launches, and 1.5 us (a pair with 128 rows 3.3 us: silu)
 // of stores. 96 tiles (n = 12288) occupy 96 of 148 SMs. All projections of a layer, before the two issuers, the cheaper dequantisation and the
-// rings by row count, and now: 9 rows 78.1 -> 56.6 us, 40 rows 82.6 -> 59.7, 128 rows 100.8 -> 80.3.
+// rings by row count, and now, back to back in a graph: 9 rows 78.0 -> 55.1 us, 40 rows 82.6 -> 59.0, 128 rows 100.8 -> 79.7.
 // Tried and left out: fp32 activations converted by four warps of the kernel itself instead of the layout kernel (12288 x 4096, 9 rows 16.0 us
 // against 14.1, 40 rows 20.5 against 14.9: copies of twice the bytes, and a proxy fence between every conversion and its MMAs); K slices as
 // clusters that add up over distributed shared memory instead of umma_reduce_kernel (4096 x 4096, 9 rows 8.8 against 8.6 us, 40 rows 10.1 against 9.5);
@@ -441,8 +441,9 @@ __global__ void __launch_bounds__(512) umma_norm_rows_kernel(const float* x, con
 }
 
 // y = partial[0] + partial[1] + ... (+ residual), four values per thread. AT_ONCE: a thread asks for all of them before it adds, one trip to
-// the L2 instead of one for each slice (4096 x 4096 with 9 and 40 rows 8.2 -> 7.7 and 9.0 -> 8.3 us). With more than 64 rows the blocks are so many that
-// what counts is how many of them fit beside the GEMM's CTAs and are there when it ends, which takes few registers (128 rows 11.5 us, at once 12.6).
+// the L2 instead of one for each slice. With more than 64 rows the blocks are so many that what counts is how many of them fit beside the GEMM's
+// CTAs and are there when it ends, which takes few registers. One after the other / at once, 4096 x 4096 with 9, 32, 48, 64, 80, 96 and 128 rows 8.1 / 7.7,
+// 8.6 / 8.0, 9.3 / 8.4, 9.3 / 9.0, 10.2 / 10.5, 10.0 / 11.3 and 11.5 / 12.7 us; 4096 x 12288 with 48, 64 and 80 rows 14.5 / 14.9, 15.4 / 15.2, 15.8 / 15.9.
 template <bool AT_ONCE> __global__ void __launch_bounds__(256) umma_reduce_kernel(const float* partial, int splits, size_t count, const float* residual, float* y) {
   pdl_launch_dependents();
   pdl_wait();
