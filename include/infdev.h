@@ -183,7 +183,8 @@ int infdev_gdn_prepare(infdev_ctx* ctx, const float* x, const float* mixed, cons
                        const float* ssmDt, const float* convWeight, const infdev_query* queries, int queryCount, int64_t rows,
                        uint64_t stateOffset, uint64_t stateBytes, float* q, float* k, float* v, float* beta, float* g);
 /* delta_rule_decode / delta_rule_prefill (delta_rule.metal:73-363) for every query length, followed by
- * gated_rms_norm_128 (fused_kernels.metal:234-254) when z is non-null (z [rows,4096], normWeight [128]).
+ * gated_rms_norm_128 (fused_kernels.metal:234-254) when z is non-null (z [rows,4096], normWeight [128]); out may be z, with the same
+ * bits, or lie apart from it.
  * stateOffset here addresses the layer's recurrent state S fp32 [32][128][128] inside a record. */
 int infdev_delta_rule(infdev_ctx* ctx, const float* q, const float* k, const float* v, const float* g, const float* beta, const float* z,
                       const float* normWeight, const infdev_query* queries, int queryCount, uint64_t stateOffset, uint64_t stateBytes, float* out);

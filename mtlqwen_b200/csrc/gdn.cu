@@ -570,12 +570,13 @@ __global__ void __launch_bounds__(256, 2) delta_rule_kernel(const float* q, cons
 // as a model has them, 512 tokens: outputs 1.8e-7, state 1.4e-7 (2-norms); the fp32 chunk form before it 2.1e-7 and 4.7e-7,
 // token by token 1.1e-7 and 0.7e-7. One scale for the 16 columns of a warp, fp16 parts throughout and sums carried in the
 // accumulators gave 4.1e-7 and 5.4e-7, and lost value columns far below their neighbours; they took 278 us for eight queries
-// of 59 to 493 rows, this form 311 us.
+// of 59 to 493 rows when this form, with its preparation, took 311 us.
 // By its own clocks a chunk takes 5000 with half of the columns (KS and QS 1900, A^-1 rhs 550, the second sum 500, the update 1000, the rest
 // stores, scales and barriers) and 6900 with all (2800, 700, 700, 1400), where the preparing warps are as slow as that; 8200 when the norm was part of
-// the chain and one preparing warp had gates, decays and the inverse. Eight queries of 59 to 493 rows 200 -> 187 us, one of 493 rows 143 -> 110,
-// of 128 rows 42.1 -> 33.9, of 64 rows 24.8 -> 20.6, all with norms of one CTA a head (see delta_rule_launch). Tried and left out: the outputs by warps of their own that are handed S through shared
-// memory (200 -> 244 us), two of the preparing warps a stage behind the two others (187 -> 222), 16 warps of 128 registers (237).
+// the chain and one preparing warp had gates, decays and the inverse. With the norms, before and now: eight queries of 59 to 493 rows 199.9 -> 176.9 us,
+// of 128 rows 88.8 -> 80.4, one of 493 rows 143.4 -> 88.3, of 128 rows 42.1 -> 30.8, of 64 rows 24.7 -> 20.6. Tried and left out: the outputs by
+// warps of their own that are handed S through shared memory (eight queries 200 -> 244 us), two of the preparing warps a stage behind the two others
+// (187 -> 222, without spread norms), 16 warps of 128 registers (237).
 constexpr int kChunk = 16, kComputeWarps = 8, kPrepareWarps = 4;
 constexpr int kChunkThreads = (kComputeWarps + kPrepareWarps) * kWarp;
 constexpr int kSplitWarps = kComputeWarps / 2;  // computing warps of a CTA that has half of a head's value columns
@@ -851,8 +852,8 @@ __device__ __forceinline__ void chunk_prepare(ChunkShared& sh, const infdev_quer
 }
 
 // Which query the CTAs of row `rank` of the grid take: of those that this kernel takes the one with the rank-th largest count, so that the longest
-// chains start first and the short ones fill the SMs that are left over (eight queries of 59 to 493 rows, 256 CTAs on 148 SMs, with a
-// chunk of 4.2 us: 323 us in the order of the pass, 281 us sorted). Every lane of a warp calls; beyond 32 queries the order of the pass stays.
+// chains start first and the short ones fill the SMs that are left over (eight queries of 59 to 493 rows, 256 CTAs on 148 SMs, with an
+// earlier form of the chunk and its preparation: 323 us in the order of the pass, 281 us sorted). Every lane of a warp calls; beyond 32 queries the order of the pass stays.
 __device__ __forceinline__ uint32_t query_by_length(const infdev_query* queries, uint32_t count, uint32_t chunkedFrom, uint32_t rank) {
   if (count > 32)
     return rank;
@@ -865,8 +866,8 @@ __device__ __forceinline__ uint32_t query_by_length(const infdev_query* queries,
   return uint32_t(__ffs(__ballot_sync(0xffffffffu, lane < count && before == rank)) - 1);
 }
 
-// NORM: the outputs go over the gates z, which would be gone before the norm's launch reads them, so they are normalised in the chain. Eight queries of
-// 59 to 493 rows 242 us, 179 without (with the norm's launch).
+// NORM: the outputs go over the gates z, which would be gone before the norm's launch reads them, so they are normalised in the chain, by one CTA a head.
+// Over the gates / apart: eight queries of 59 to 493 rows 195.6 / 176.9 us, one of 493 rows 140.1 / 88.3.
 template <bool NORM>
 __global__ void __launch_bounds__(kChunkThreads, 1)
     delta_rule_chunked_kernel(const float* q, const float* k, const float* v, const float* g, const float* beta, const float* normWeight,
@@ -1099,7 +1100,7 @@ cudaError_t delta_rule_launch(const float* q, const float* k, const float* v, co
                      stateOffset, out, chunkedFrom, uint32_t(queryCount), uint32_t(sms));
   }
   // The norms of long queries are spread over several CTAs a head, which else were a chain of loads and stores after the last chunk: one query of 493
-  // rows 111 -> 96.5 us, six of 17 to 700 rows 202 -> 179, eight of 59 to 493 rows 187 -> 179. Few enough of them that those without rows do not
+  // rows 111 -> 96.5 us, six of 17 to 700 rows 202 -> 179, eight of 59 to 493 rows 187 -> 179, as they were measured then. Few enough of them that those without rows do not
   // tell (eight queries of 128 rows 81.0, with four CTAs a head 81.7, with eight 83.4).
   const int spread = chunkedFrom && z && z != out ? std::clamp(6 * sms / (kValueHeads * queryCount), 1, 8) : 1;
   // Not launched early: its CTAs would be placed around those of the kernels before it, two on an SM, and the token-by-token chain
